@@ -639,6 +639,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
     // Q tile barriers are indexed [buffer][tile]
     __shared__ __align__(8) uint64_t bar_qfull[2][2], bar_qrot[2][2], bar_qfree[2][2];
     __shared__ __align__(8) uint64_t bar_s[P2_NSBUF], bar_p[P2_NSBUF];      // per score buffer
+    __shared__ __align__(8) uint64_t bar_first[2];                          // per tile: the scores of its first step in a unit
     __shared__ __align__(8) uint64_t bar_o[2], bar_rs[2], bar_rp[2];        // per tile: O complete; scores again / redone
     __shared__ __align__(8) uint64_t bar_kvfull[P2_NSTAGE], bar_empty[P2_NSTAGE];   // K and V of a stage arrive on one barrier
     __shared__ uint32_t s_tmem_base;
@@ -665,6 +666,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
                 mbar_init(smem_u32(&bar_qfree[i][u]), 1);
             }
             mbar_init(smem_u32(&bar_o[i]), 1);
+            mbar_init(smem_u32(&bar_first[i]), 1);
             mbar_init(smem_u32(&bar_rs[i]), 1);
             mbar_init(smem_u32(&bar_rp[i]), P2_WPT);
             s_redo[i] = 0;
@@ -814,6 +816,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
                             tc::mma_ss_lohi(tmem + bq * 128, qd + kk * 2, kd + kk * 2, DESC_HI, IDESC_QK, kk > 0);
                     }
                     tc::commit(aBarS + bq * 8);
+                    if (g_j == 0) tc::commit(smem_u32(&bar_first[g_u]));
                     BN_LOG_MMA(20 | g_u << 8 | g_j << 16);
                     uint32_t e = g_u | stage << 4 | (quse & 1u) << 6;
                     if (g_j > 0) e |= 2u;
@@ -990,7 +993,12 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
                 const uint32_t tS = tmem + lane_base + sb * 128 + hf * 64;   // 64 fp32 scores; P goes over the first 32
                 BN_LOG(1 | u << 8 | j << 16);
                 const float k_max2 = __ldg(kmax2 + j);
-                ok = mbar_wait(smem_u32(&bar_s[sb]), (s / P2_NSBUF) & 1, &s_abort);
+                // A parity wait tells only neighbouring phases of a barrier apart, and a tile that some units do not have
+                // (an odd number of query tiles) has let any number of phases of bar_s pass before its first step.  So
+                // that step waits for a barrier of the tile's own, one phase per unit; from then on the tile's previous
+                // step is at most three steps back, and the phase before is known to be over.
+                ok = j == 0 ? mbar_wait(smem_u32(&bar_first[u]), units_done & 1, &s_abort)
+                            : mbar_wait(smem_u32(&bar_s[sb]), (s / P2_NSBUF) & 1, &s_abort);
                 if (!ok) break;
                 tc::fence_after_sync();
                 BN_LOG(2 | u << 8 | j << 16);

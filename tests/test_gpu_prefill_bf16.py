@@ -78,6 +78,19 @@ def test_prefill_group_sizes(lib, Hq, Hkv, S):
         assert np.abs(lse[b].T - ref_lse).max() <= 2e-2
 
 
+@pytest.mark.parametrize("B,S,causal", [(9, 300, True), (3, 1391, True), (7, 641, True), (9, 300, False)])
+def test_prefill_odd_number_of_query_tiles(lib, B, S, causal):
+    """More units of two query tiles than multiprocessors, the first ones with one tile only: the second tile's warps begin
+    many steps into the launch.  Against the oracle, and both kernels against each other on every element."""
+    Hq, Hkv, D = 32, 4, 64
+    q, k, v = make_inputs(B, S, Hq, Hkv, D, 17 * S + B)
+    got, _ = run(q, k, v, 0, causal)
+    other, _ = run(q, k, v, 0, causal, single=True)
+    assert np.abs(got - other).max() <= GATE
+    ref, _ = oracle(q, k, v, 0, causal, B - 1)
+    assert np.abs(got[B - 1].reshape(S, Hq * D) - ref).max() <= GATE
+
+
 def test_prefill_growing_scores_take_the_rescale_path(lib):
     """Keys whose scores grow along the sequence force the running reference to move by more than 2^8
     several times (the rescale-and-redo path of the single-pass softmax)."""
