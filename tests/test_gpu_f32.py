@@ -60,6 +60,30 @@ def test_mm_matches_reference_order(T, cref, M, K, N):
     assert np.array_equal(got, ref), nerr(got, ref)   # same FMA chain -> same bits
 
 
+@pytest.mark.parametrize("M,K,N", [(8, 4, 32), (9, 20, 33), (17, 52, 1000), (33, 68, 4736), (65, 16, 9473), (1151, 24, 2052), (1, 1, 8)])
+@pytest.mark.parametrize("layout", ["nn", "nt", "nn_odd", "nt_odd", "a_t"])
+def test_mm_tiles_and_copies(T, cref, M, K, N, layout):
+    """Every tile size and every way the operands are copied (along K, along N, element by element where a stride or an
+    address is odd, a transposed A), with ragged edges: the bits of the chain."""
+    rng = np.random.default_rng(M + K + N)
+    a, b = rng.standard_normal((M, K), dtype=np.float32), rng.standard_normal((K, N), dtype=np.float32)
+
+    def on_gpu(x, odd):
+        t = T.TensorF(x.shape[0], x.shape[1] + (3 if odd else 0))
+        t.copy_from_numpy(np.pad(x, ((0, 0), (0, 3))) if odd else x)
+        return T.TensorF(x.shape[0], x.shape[1], _base=t.base, _stride_h=t.stride_h)
+    odd = layout.endswith("odd")
+    ta = on_gpu(a.T, False).T if layout == "a_t" else on_gpu(a, odd)
+    tb = on_gpu(b.T, odd).T if layout.startswith("nt") else on_gpu(b, odd)
+    got = (ta @ tb).to_numpy()
+    import ctypes as C
+    ref = np.empty((M, N), dtype=np.float32)
+    fp = C.POINTER(C.c_float)
+    cref.cpu().ref_mm_f32(a.ctypes.data_as(fp), C.c_long(K), C.c_long(1), b.ctypes.data_as(fp), C.c_long(N),
+                          C.c_long(1), ref.ctypes.data_as(fp), C.c_int(M), C.c_int(K), C.c_int(N))
+    assert np.array_equal(got, ref)
+
+
 def test_mm_transposed_and_sliced_views(T):
     rng = np.random.default_rng(2)
     a = rng.standard_normal((40, 96), dtype=np.float32)
