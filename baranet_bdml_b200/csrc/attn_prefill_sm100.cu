@@ -632,6 +632,9 @@ __device__ __forceinline__ bool mma_scores_again(uint32_t tS, uint32_t qd, uint3
 }
 
 // 18 warps = 5 on one scheduler: 16384 / (5 * 32) leaves 96 registers per thread
+// ODD_TILES: the sequences have an odd number of query tiles, so that some units lack their second one.  A form of its own
+// because the extra barrier costs 2 % (238 -> 243 us at 8 x 2048 tokens) where it is not needed.
+template <bool ODD_TILES>
 __global__ void __launch_bounds__(P2_THREADS, 1)
 prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                const __grid_constant__ CUtensorMap tmap_v, const PrefillParams p, const int n_units) {
@@ -816,7 +819,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
                             tc::mma_ss_lohi(tmem + bq * 128, qd + kk * 2, kd + kk * 2, DESC_HI, IDESC_QK, kk > 0);
                     }
                     tc::commit(aBarS + bq * 8);
-                    if (g_j == 0) tc::commit(smem_u32(&bar_first[g_u]));
+                    if (ODD_TILES && g_j == 0) tc::commit(smem_u32(&bar_first[g_u]));
                     BN_LOG_MMA(20 | g_u << 8 | g_j << 16);
                     uint32_t e = g_u | stage << 4 | (quse & 1u) << 6;
                     if (g_j > 0) e |= 2u;
@@ -986,19 +989,19 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
             const int warp_first_last = p.causal ? min(p.S - 1, gi - lane + p.position_offset) : p.S - 1;
             const int warp_last_last = p.causal ? min(p.S - 1, gi - lane + 31 + p.position_offset) : p.S - 1;
 
-            for (int j = 0; j < nt; ++j) {
+            // A parity wait tells only neighbouring phases of a barrier apart, and a tile that some units do not have (an odd
+            // number of query tiles) has let any number of phases of bar_s pass before its first step.  So a unit's first
+            // scores are announced on a barrier of the tile's own, one phase per unit; from then on the tile's previous step
+            // is at most three steps back, and the phase before is known to be over.
+            if (ODD_TILES) ok = mbar_wait(smem_u32(&bar_first[u]), units_done & 1, &s_abort);
+            for (int j = 0; ok && j < nt; ++j) {
                 // this step's place in the CTA's sequence, hence its score buffer
                 const uint32_t s = (uint32_t)(sbase + (j < n_both ? 2 * j + u : n_both + j));
                 const uint32_t sb = s % P2_NSBUF;
                 const uint32_t tS = tmem + lane_base + sb * 128 + hf * 64;   // 64 fp32 scores; P goes over the first 32
                 BN_LOG(1 | u << 8 | j << 16);
                 const float k_max2 = __ldg(kmax2 + j);
-                // A parity wait tells only neighbouring phases of a barrier apart, and a tile that some units do not have
-                // (an odd number of query tiles) has let any number of phases of bar_s pass before its first step.  So
-                // that step waits for a barrier of the tile's own, one phase per unit; from then on the tile's previous
-                // step is at most three steps back, and the phase before is known to be over.
-                ok = j == 0 ? mbar_wait(smem_u32(&bar_first[u]), units_done & 1, &s_abort)
-                            : mbar_wait(smem_u32(&bar_s[sb]), (s / P2_NSBUF) & 1, &s_abort);
+                ok = mbar_wait(smem_u32(&bar_s[sb]), (s / P2_NSBUF) & 1, &s_abort);
                 if (!ok) break;
                 tc::fence_after_sync();
                 BN_LOG(2 | u << 8 | j << 16);
@@ -1311,7 +1314,9 @@ extern "C" int bn_attn_prefill_bf16(const void* q, const void* k, const void* v,
     int dev = 0;
     cudaGetDevice(&dev);
     if (configured_dev != dev) {
-        cudaError_t e = cudaFuncSetAttribute(prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, P2_SMEM_BYTES);
+        cudaError_t e = cudaFuncSetAttribute(prefill_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, P2_SMEM_BYTES);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(prefill_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, P2_SMEM_BYTES);
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(prefill_kernel_v1, cudaFuncAttributeMaxDynamicSharedMemorySize, PF_SMEM_BYTES);
         if (e != cudaSuccess) return fail(BN_ERR_CUDA, "cudaFuncSetAttribute(prefill): %s", cudaGetErrorString(e));
@@ -1328,7 +1333,8 @@ extern "C" int bn_attn_prefill_bf16(const void* q, const void* k, const void* v,
         int sms = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         const unsigned grid = (unsigned)(n_units < sms ? n_units : sms);
-        prefill_kernel<<<grid, P2_THREADS, P2_SMEM_BYTES, st>>>(tmap_q, tmap_k, tmap_v, p, (int)n_units);
+        if (n_qtiles % 2) prefill_kernel<true><<<grid, P2_THREADS, P2_SMEM_BYTES, st>>>(tmap_q, tmap_k, tmap_v, p, (int)n_units);
+        else prefill_kernel<false><<<grid, P2_THREADS, P2_SMEM_BYTES, st>>>(tmap_q, tmap_k, tmap_v, p, (int)n_units);
     }
     return launch_status("bn_attn_prefill_bf16");
 }
