@@ -35,13 +35,19 @@ __global__ void rope_f32_kernel(const float* __restrict__ x, int64_t x_rs, int64
 }
 
 // ---------------------------------------------------------------------------
-// Fused attention core, fp32, two passes over the keys
+// Fused attention core, fp32
 // ---------------------------------------------------------------------------
-constexpr int AF_BM = 16;    // query rows per CTA
-constexpr int AF_BN = 64;    // keys per tile
-constexpr int AF_BK = 32;    // dot-product columns staged per step
-constexpr int AF_MAXHALF = 32;   // head_dim <= 64
-constexpr int AF_MAXOUT = 16;    // distinct output columns per problem <= 256
+// A score is ONE chain of FMAs over the width of its softmax's problem (collapsed heads: all of Hq * D columns, 2048 links of
+// 4 cycles = 4 us), an output one chain over the keys: the kernel is bound by those chains and by reading their operands from
+// shared memory, so it spreads (row, key) pairs as widely as it can.  A CTA owns RPT x GR query rows of one problem; thread =
+// (key of a 128-key tile, group of RPT rows).  The tile's rotated keys stay in shared memory for all the query heads that
+// share them; queries are rotated in pieces of up to 256 columns.  Scores are kept (up to the shared memory that is left)
+// and exponentiated once the row's maximum and sum are known, p = expf(s - m) / l; where they do not fit, they are
+// computed twice, a tile at a time.
+// 128 rows, 32 / 4 heads of 64, collapsed: 72 us; with 16 rows a CTA (8 CTAs) and all scores computed twice 699 us.
+constexpr int AF_KEYS = 128, AF_QCOLS = 256;
+constexpr int AF_MAXD = 64, AF_MAXOUT = 256;    // head_dim; distinct output columns of a problem
+constexpr size_t AF_SMEM = 200 * 1024;
 
 struct AttnF32Params {
     const float *q, *k, *v;
@@ -50,160 +56,221 @@ struct AttnF32Params {
     int S, Hq, Hkv, D;
     float scale, theta;
     int position_offset, causal, heads_mode, apply_rope;
+    int heads_per_piece, k_ld, p_ld, stored;
 };
 
-// Column c of the (virtual) repeated K/V matrix -> column of the stored one.
-__device__ __forceinline__ int kv_col(int c, int D, int n_rep) { return (c / D / n_rep) * D + c % D; }
+// PC: output columns of a problem, rounded up to 64 or 256.  D4: head_dim is a multiple of 4.
+template <int RPT, int GR, int PC, bool D4>
+__global__ void __launch_bounds__(AF_KEYS * GR) attn_f32_kernel(const AttnF32Params p) {
+    constexpr int THREADS = AF_KEYS * GR, BM = RPT * GR;
+    constexpr int CPT = PC > THREADS ? PC / THREADS : 1, NG = PC > THREADS ? 1 : THREADS / PC, ROWS = (BM + NG - 1) / NG;
+    extern __shared__ __align__(16) float af_smem[];
+    __shared__ float inv_freq[AF_MAXD / 2];
+    __shared__ float row_m[BM], row_l[BM];
+    float* Ks = af_smem;                                       // [key][k_ld]
+    float* Qs = Ks + AF_KEYS * p.k_ld;                         // [row][heads_per_piece * D]
+    float2* k_turn = reinterpret_cast<float2*>(Qs + BM * p.heads_per_piece * p.D);   // [key][D / 2] cos, sin
+    float2* q_turn = k_turn + AF_KEYS * (p.D / 2);                                   // [row][D / 2]
+    float* Ps = reinterpret_cast<float*>(q_turn + BM * (p.D / 2));                   // [row][p_ld]
 
-__global__ void __launch_bounds__(256) attn_f32_kernel(AttnF32Params p) {
-    __shared__ float Qs[AF_BM][AF_BK];
-    __shared__ float Ks[AF_BN][AF_BK + 1];
-    __shared__ float Ps[AF_BM][AF_BN];
-    __shared__ float cq[AF_BM][AF_MAXHALF], sq[AF_BM][AF_MAXHALF];
-    __shared__ float ck[AF_BN][AF_MAXHALF], sk[AF_BN][AF_MAXHALF];
-    __shared__ float inv_freq[AF_MAXHALF];
-
-    const int tid = threadIdx.x;
-    const int r = tid / 16, cg = tid % 16;
-    const int row0 = blockIdx.x * AF_BM;
-    const int D = p.D, half = D / 2, n_rep = p.Hq / p.Hkv;
-    // problem = the set of columns one softmax spans
-    const int prob = blockIdx.y;
+    const int tid = threadIdx.x, key = tid % AF_KEYS, group = tid / AF_KEYS, warp = tid / 32, lane = tid % 32;
+    const int D = p.D, half = D / 2, n_rep = p.Hq / p.Hkv, prob = blockIdx.y;
+    const int row0 = (gridDim.x - 1 - blockIdx.x) * BM;        // the rows with most keys first
     const bool collapsed = p.heads_mode == BN_HEADS_COLLAPSED;
-    const int qc0 = collapsed ? 0 : prob * D;              // first q column of the dot product
-    const int Wd = collapsed ? p.Hq * D : D;               // dot-product width
-    const int vc0 = collapsed ? 0 : (prob / n_rep) * D;    // first stored V column of the output
-    const int Wo = collapsed ? p.Hkv * D : D;              // distinct output columns
+    const int heads = collapsed ? p.Hq : 1, kv_heads = collapsed ? p.Hkv : 1;
+    const int head0 = collapsed ? 0 : prob, kv0 = collapsed ? 0 : prob / n_rep, Wo = kv_heads * D;
+    const int last = p.causal ? min(p.S - 1, row0 + BM - 1 + p.position_offset) : p.S - 1;
+    const int n_keys = last + 1, n_tiles = (n_keys + AF_KEYS - 1) / AF_KEYS;
+    const int q_ld = p.heads_per_piece * D, pieces = (heads + p.heads_per_piece - 1) / p.heads_per_piece;
 
     if (tid < half) inv_freq[tid] = rope_inv_freq(tid, D, p.theta);
+    if (tid < BM) { row_m[tid] = -INFINITY; row_l[tid] = 0.f; }
     __syncthreads();
-    if (p.apply_rope) {
-        for (int e = tid; e < AF_BM * half; e += 256) {
-            int rr = e / half, i = e % half;
-            float angle = (row0 + rr + p.position_offset) * inv_freq[i];
-            cq[rr][i] = cosf(angle);
-            sq[rr][i] = sinf(angle);
+
+    // cos and sin of rows g0 .. g0 + n - 1's positions
+    auto turn = [&](int g0, int n, float2* cs) {
+        if (!p.apply_rope) return;
+        for (int e = tid; e < n * half; e += THREADS) {
+            const float angle = (g0 + e / half + p.position_offset) * inv_freq[e % half];
+            float cos_angle, sin_angle;
+            sincosf(angle, &sin_angle, &cos_angle);
+            cs[e] = make_float2(cos_angle, sin_angle);
         }
-    }
-    const int grow = row0 + r;
-    // last valid key for this CTA's rows / for this thread's row
-    int block_last = p.causal ? min(p.S - 1, row0 + AF_BM - 1 + p.position_offset) : p.S - 1;
-    int row_last = p.causal ? min(p.S - 1, grow + p.position_offset) : p.S - 1;
-    if (grow >= p.S) row_last = -1;
-    const int n_tiles = block_last >= 0 ? block_last / AF_BN + 1 : 0;
-
-    float m_run = -INFINITY, l_run = 0.0f;
-    float acc[AF_MAXOUT];
-#pragma unroll
-    for (int j = 0; j < AF_MAXOUT; ++j) acc[j] = 0.0f;
-
-    for (int pass = 0; pass < 2; ++pass) {
-        for (int jt = 0; jt < n_tiles; ++jt) {
-            const int j0 = jt * AF_BN;
-            __syncthreads();  // previous tile's Ps / ck readers are done
+    };
+    // rows [g0, g0 + n) of `heads_n` heads from `head_at` on, rotated, to dst[row][head * D ..]
+    auto stage = [&](const float* x, int64_t rs, int64_t cs, int g0, int n, int head_at, int heads_n, const float2* turned, float* dst, int ld) {
+        const int pairs = heads_n * half;
+#pragma unroll 8
+        for (int e = tid; e < n * pairs; e += THREADS) {
+            const int r = e / pairs, c = e - r * pairs, i = c % half, g = g0 + r;
+            float x0 = 0.f, x1 = 0.f;
+            if (g < p.S) {
+                const float* src = x + g * rs + (head_at * D + 2 * c) * cs;
+                x0 = __ldg(src);
+                x1 = __ldg(src + cs);
+            }
+            float y0 = x0, y1 = x1;
             if (p.apply_rope) {
-                for (int e = tid; e < AF_BN * half; e += 256) {
-                    int jj = e / half, i = e % half;
-                    float angle = (j0 + jj + p.position_offset) * inv_freq[i];
-                    ck[jj][i] = cosf(angle);
-                    sk[jj][i] = sinf(angle);
-                }
+                const float cos_angle = turned[r * half + i].x, sin_angle = turned[r * half + i].y;
+                y0 = x0 * cos_angle - x1 * sin_angle;
+                y1 = x0 * sin_angle + x1 * cos_angle;
             }
-            float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-            for (int c0 = 0; c0 < Wd; c0 += AF_BK) {
-                __syncthreads();
-                // stage rotated Q (16 x 32) and rotated K (64 x 32), pair-wise
-                for (int e = tid; e < (AF_BM + AF_BN) * (AF_BK / 2); e += 256) {
-                    int pr = e % (AF_BK / 2), rr = e / (AF_BK / 2);
-                    int c = c0 + 2 * pr;             // even column inside the dot product
-                    bool isq = rr < AF_BM;
-                    int lr = isq ? rr : rr - AF_BM;
-                    int g = isq ? row0 + lr : j0 + lr;
-                    float x0 = 0.0f, x1 = 0.0f;
-                    if (g < p.S && c < Wd) {
-                        if (isq) {
-                            x0 = p.q[g * p.q_rs + (qc0 + c) * p.q_cs];
-                            x1 = p.q[g * p.q_rs + (qc0 + c + 1) * p.q_cs];
-                        } else {
-                            int kc = kv_col(qc0 + c, D, n_rep);
-                            x0 = p.k[g * p.k_rs + kc * p.k_cs];
-                            x1 = p.k[g * p.k_rs + (kc + 1) * p.k_cs];
+            *reinterpret_cast<float2*>(dst + r * ld + 2 * c) = make_float2(y0, y1);
+        }
+    };
+    turn(row0, BM, q_turn);
+    auto row_last = [&](int r) {
+        const int g = row0 + r;
+        return g >= p.S ? -1 : p.causal ? min(p.S - 1, g + p.position_offset) : p.S - 1;
+    };
+    // the tile's scaled scores to dst[row][key], -inf where masked
+    auto scores = [&](int tile, float* dst) {
+        const int j0 = tile * AF_KEYS;
+        __syncthreads();                                       // the keys before, and what lies in dst, have been read
+        turn(j0, AF_KEYS, k_turn);
+        __syncthreads();
+        stage(p.k, p.k_rs, p.k_cs, j0, AF_KEYS, kv0, kv_heads, k_turn, Ks, p.k_ld);
+        float acc[RPT];
+#pragma unroll
+        for (int r = 0; r < RPT; ++r) acc[r] = 0.f;
+        for (int piece = 0; piece < pieces; ++piece) {
+            const int h0 = piece * p.heads_per_piece, nh = min(p.heads_per_piece, heads - h0);
+            if (piece > 0) __syncthreads();                    // the queries before have been read
+            if (pieces > 1 || tile == 0) stage(p.q, p.q_rs, p.q_cs, row0, BM, head0 + h0, nh, q_turn, Qs, q_ld);
+            __syncthreads();
+            for (int h = 0; h < nh; ++h) {
+                const float* kr = Ks + key * p.k_ld + (collapsed ? (h0 + h) / n_rep * D : 0);
+                const float* qr = Qs + group * RPT * q_ld + h * D;
+                if (D4) {
+#pragma unroll 4
+                    for (int d = 0; d < D; d += 4) {
+                        const float4 k4 = *reinterpret_cast<const float4*>(kr + d);
+#pragma unroll
+                        for (int r = 0; r < RPT; ++r) {
+                            const float4 q4 = *reinterpret_cast<const float4*>(qr + r * q_ld + d);
+                            acc[r] = fmaf(q4.w, k4.w, fmaf(q4.z, k4.z, fmaf(q4.y, k4.y, fmaf(q4.x, k4.x, acc[r]))));
                         }
                     }
-                    float y0 = x0, y1 = x1;
-                    if (p.apply_rope) {
-                        int i = ((qc0 + c) % D) / 2;
-                        float cos_angle = isq ? cq[lr][i] : ck[lr][i];
-                        float sin_angle = isq ? sq[lr][i] : sk[lr][i];
-                        y0 = x0 * cos_angle - x1 * sin_angle;
-                        y1 = x0 * sin_angle + x1 * cos_angle;
-                    }
-                    if (isq) { Qs[lr][2 * pr] = y0; Qs[lr][2 * pr + 1] = y1; }
-                    else { Ks[lr][2 * pr] = y0; Ks[lr][2 * pr + 1] = y1; }
-                }
-                __syncthreads();
+                } else {
+                    for (int d = 0; d < D; ++d)
 #pragma unroll
-                for (int kk = 0; kk < AF_BK; ++kk) {
-                    float a = Qs[r][kk];
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) s[j] = fmaf(a, Ks[cg + 16 * j][kk], s[j]);
+                        for (int r = 0; r < RPT; ++r) acc[r] = fmaf(qr[r * q_ld + d], kr[d], acc[r]);
                 }
             }
-            // scale (a separate fp32 multiply, as op_multiply does) and mask
-            bool ok[4];
+        }
+        // scale: a separate fp32 multiply, as op_multiply does
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                s[j] = s[j] * p.scale;
-                ok[j] = (j0 + cg + 16 * j) <= row_last;
+        for (int r = 0; r < RPT; ++r)
+            dst[(group * RPT + r) * p.p_ld + key] = j0 + key <= row_last(group * RPT + r) ? acc[r] * p.scale : -INFINITY;
+    };
+    // takes n scores of every row into its maximum and sum; a warp per row
+    auto take = [&](const float* src, int n) {
+        for (int r = warp; r < BM; r += THREADS / 32) {
+            float m = row_m[r], sum = 0.f;
+            for (int j = lane; j < n; j += 32) m = fmaxf(m, src[r * p.p_ld + j]);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+            if (m > -INFINITY)
+                for (int j = lane; j < n; j += 32) sum += expf(src[r * p.p_ld + j] - m);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            if (lane == 0 && m > -INFINITY) { row_l[r] = row_l[r] * expf(row_m[r] - m) + sum; row_m[r] = m; }
+            __syncwarp();
+        }
+    };
+    auto weights = [&](float* src, int j0, int n) {
+        for (int e = tid; e < BM * n; e += THREADS) {
+            const int r = e / n, j = e - r * n;
+            float& s = src[r * p.p_ld + j];
+            s = j0 + j <= row_last(r) ? expf(s - row_m[r]) / row_l[r] : 0.f;
+        }
+    };
+    float out[ROWS][CPT];
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i)
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) out[i][c] = 0.f;
+    const int col = tid % (PC / CPT), rg = tid / (PC / CPT);
+    // out += the weights of keys j0 .. j0 + n - 1 times their values, in key order
+    auto values = [&](const float* src, int j0, int n) {
+#pragma unroll 16
+        for (int j = 0; j < n; ++j) {
+            float v[CPT];
+#pragma unroll
+            for (int c = 0; c < CPT; ++c)
+                v[c] = col + c * (PC / CPT) < Wo ? __ldg(p.v + (int64_t)(j0 + j) * p.v_rs + (kv0 * D + col + c * (PC / CPT)) * p.v_cs) : 0.f;
+#pragma unroll
+            for (int i = 0; i < ROWS; ++i) {
+                const int r = rg + i * NG;
+                const float w = BM % NG == 0 || r < BM ? src[r * p.p_ld + j] : 0.f;
+#pragma unroll
+                for (int c = 0; c < CPT; ++c) out[i][c] = fmaf(w, v[c], out[i][c]);
             }
-            if (pass == 0) {
-                float tm = -INFINITY;
+        }
+    };
+
+    if (p.stored) {
+        for (int t = 0; t < n_tiles; ++t) scores(t, Ps + t * AF_KEYS);
+        __syncthreads();
+        take(Ps, n_keys);
+        __syncthreads();
+        weights(Ps, 0, n_keys);
+        __syncthreads();
+        values(Ps, 0, n_keys);
+    } else {
+        for (int t = 0; t < n_tiles; ++t) {
+            scores(t, Ps);
+            __syncthreads();
+            take(Ps, AF_KEYS);
+        }
+        for (int t = 0; t < n_tiles; ++t) {
+            const int n = min(AF_KEYS, n_keys - t * AF_KEYS);
+            scores(t, Ps);
+            __syncthreads();
+            weights(Ps, t * AF_KEYS, n);
+            __syncthreads();
+            values(Ps, t * AF_KEYS, n);
+        }
+    }
 #pragma unroll
-                for (int j = 0; j < 4; ++j) if (ok[j]) tm = fmaxf(tm, s[j]);
+    for (int i = 0; i < ROWS; ++i) {
+        const int r = rg + i * NG, g = row0 + r;
+        if (r >= BM || g >= p.S) continue;
 #pragma unroll
-                for (int o = 1; o < 16; o <<= 1) tm = fmaxf(tm, __shfl_xor_sync(0xffffffffu, tm, o));
-                float m_new = fmaxf(m_run, tm);
-                float ts = 0.0f;
-#pragma unroll
-                for (int j = 0; j < 4; ++j) if (ok[j]) ts += expf(s[j] - m_new);
-#pragma unroll
-                for (int o = 1; o < 16; o <<= 1) ts += __shfl_xor_sync(0xffffffffu, ts, o);
-                if (m_new > -INFINITY) {
-                    l_run = l_run * expf(m_run - m_new) + ts;
-                    m_run = m_new;
-                }
+        for (int c0 = 0; c0 < CPT; ++c0) {
+            const int c = col + c0 * (PC / CPT);
+            if (c >= Wo) continue;
+            if (collapsed) {
+                const int h = c / D, d = c - h * D;
+                for (int rep = 0; rep < n_rep; ++rep) p.out[g * p.o_rs + ((h * n_rep + rep) * D + d) * p.o_cs] = out[i][c0];
             } else {
-#pragma unroll
-                for (int j = 0; j < 4; ++j) Ps[r][cg + 16 * j] = ok[j] ? expf(s[j] - m_run) / l_run : 0.0f;
-                __syncthreads();
-                if (grow < p.S) {
-                    int jmax = min(AF_BN, p.S - j0);
-                    for (int jj = 0; jj < jmax; ++jj) {
-                        float pv = Ps[r][jj];
-                        const float* vrow = p.v + (int64_t)(j0 + jj) * p.v_rs;
-#pragma unroll
-                        for (int oc = 0; oc < AF_MAXOUT; ++oc) {
-                            int c = cg + 16 * oc;
-                            if (c < Wo) acc[oc] = fmaf(pv, vrow[(vc0 + c) * p.v_cs], acc[oc]);
-                        }
-                    }
-                }
+                p.out[g * p.o_rs + (prob * D + c) * p.o_cs] = out[i][c0];
             }
         }
     }
-    if (grow >= p.S) return;
-#pragma unroll
-    for (int oc = 0; oc < AF_MAXOUT; ++oc) {
-        int c = cg + 16 * oc;
-        if (c >= Wo) continue;
-        if (collapsed) {
-            int g = c / D, d = c % D;
-            for (int rep = 0; rep < n_rep; ++rep)
-                p.out[grow * p.o_rs + ((g * n_rep + rep) * D + d) * p.o_cs] = acc[oc];
-        } else {
-            p.out[grow * p.o_rs + (prob * D + c) * p.o_cs] = acc[oc];
-        }
-    }
+}
+
+template <int RPT, int GR, int PC, bool D4>
+static int attn_f32_run(AttnF32Params p, int problems, cudaStream_t st) {
+    constexpr int BM = RPT * GR;
+    const size_t fixed = (size_t)(AF_KEYS * p.k_ld + BM * p.heads_per_piece * p.D + (AF_KEYS + BM) * p.D) * sizeof(float);
+    const int all_keys = ceil_div(p.S, AF_KEYS) * AF_KEYS + 4;
+    p.stored = fixed + (size_t)BM * all_keys * sizeof(float) <= AF_SMEM;
+    p.p_ld = p.stored ? all_keys : AF_KEYS + 4;
+    const size_t smem = fixed + (size_t)BM * p.p_ld * sizeof(float);
+    if (int rc = allow_smem(attn_f32_kernel<RPT, GR, PC, D4>, smem, "bn_attn_prefill_f32")) return rc;
+    attn_f32_kernel<RPT, GR, PC, D4><<<dim3(ceil_div(p.S, BM), problems), AF_KEYS * GR, smem, st>>>(p);
+    return launch_status("bn_attn_prefill_f32");
+}
+
+template <int PC, bool D4>
+static int attn_f32_rows(const AttnF32Params& p, int problems, cudaStream_t st) {
+    // As many rows to a CTA as leave a CTA for every multiprocessor: rows share the keys' rotation and their reading from
+    // shared memory, CTAs share nothing.
+    const long long rows = (long long)p.S * problems, sms = sm_count();
+    if (rows > 16 * sms / 2) return attn_f32_run<4, 4, PC, D4>(p, problems, st);
+    if (rows > sms) return attn_f32_run<2, 2, PC, D4>(p, problems, st);
+    return attn_f32_run<1, 1, PC, D4>(p, problems, st);
 }
 
 }  // namespace bn
@@ -238,16 +305,20 @@ extern "C" int bn_attn_prefill_f32(const float* q, int64_t q_rs, int64_t q_cs, c
     if (Hq % Hkv != 0) return fail(BN_ERR_INVALID_ARG, "bn_attn_prefill_f32: Hq=%d not a multiple of Hkv=%d", Hq, Hkv);
     if (heads_mode != BN_HEADS_COLLAPSED && heads_mode != BN_HEADS_PER_HEAD)
         return fail(BN_ERR_INVALID_ARG, "bn_attn_prefill_f32: heads_mode=%d", heads_mode);
-    if (D % 2 || D > 2 * AF_MAXHALF)
-        return fail(BN_ERR_UNSUPPORTED, "bn_attn_prefill_f32: head_dim=%d (even, <= %d supported)", D, 2 * AF_MAXHALF);
-    int Wo = heads_mode == BN_HEADS_COLLAPSED ? Hkv * D : D;
-    if (Wo > 16 * AF_MAXOUT)
-        return fail(BN_ERR_UNSUPPORTED, "bn_attn_prefill_f32: Hkv*D=%d (<= %d supported)", Wo, 16 * AF_MAXOUT);
+    if (D % 2 || D > AF_MAXD)
+        return fail(BN_ERR_UNSUPPORTED, "bn_attn_prefill_f32: head_dim=%d (even, <= %d supported)", D, AF_MAXD);
+    const int Wo = heads_mode == BN_HEADS_COLLAPSED ? Hkv * D : D;
+    if (Wo > AF_MAXOUT)
+        return fail(BN_ERR_UNSUPPORTED, "bn_attn_prefill_f32: Hkv*D=%d (<= %d supported)", Wo, AF_MAXOUT);
     if (int rc = require_sm100()) return rc;
     if (S == 0) return BN_OK;
-    AttnF32Params p{q, k, v, out, q_rs, q_cs, k_rs, k_cs, v_rs, v_cs, o_rs, o_cs, S, Hq, Hkv, D,
-                    scale, theta, position_offset, causal, heads_mode, apply_rope};
-    dim3 grid(ceil_div(S, AF_BM), heads_mode == BN_HEADS_COLLAPSED ? 1 : Hq);
-    attn_f32_kernel<<<grid, 256, 0, as_stream(stream)>>>(p);
-    return launch_status("bn_attn_prefill_f32");
+    const int heads = heads_mode == BN_HEADS_COLLAPSED ? Hq : 1, problems = heads_mode == BN_HEADS_COLLAPSED ? 1 : Hq;
+    const int per_piece = AF_QCOLS / D < heads ? AF_QCOLS / D : heads;
+    // a row stride of 4 floats more than a multiple of 8 puts the 16-byte reads of eight neighbouring keys on different banks
+    const int k_ld = (Wo + 7) / 8 * 8 + 4;
+    const AttnF32Params p{q, k, v, out, q_rs, q_cs, k_rs, k_cs, v_rs, v_cs, o_rs, o_cs, S, Hq, Hkv, D,
+                          scale, theta, position_offset, causal, heads_mode, apply_rope, per_piece, k_ld, 0, 0};
+    cudaStream_t st = as_stream(stream);
+    if (D % 4) return Wo <= 64 ? attn_f32_rows<64, false>(p, problems, st) : attn_f32_rows<256, false>(p, problems, st);
+    return Wo <= 64 ? attn_f32_rows<64, true>(p, problems, st) : attn_f32_rows<256, true>(p, problems, st);
 }

@@ -27,7 +27,7 @@ def dev_inv_freq(T):
     """The device's own frequency table (CUDA powf), read back through bn_rope_f32:
     rotating (1, 0) pairs at position 1 yields (cos f_i, sin f_i)."""
     out = {}
-    for D in (32, 64):
+    for D in (6, 20, 32, 64):
         x = np.zeros((1, D), dtype=np.float32)
         x[0, 0::2] = 1.0
         t = T.TensorF(1, D)
@@ -118,6 +118,10 @@ CASES = [  # S, Hq, Hkv, D, offset, causal
     (17, 8, 2, 64, 3, True),
     (65, 8, 8, 32, 0, False),
     (130, 4, 1, 64, 0, True),
+    (149, 8, 4, 64, 0, True),      # from here on: other numbers of rows to a block, several key tiles, head sizes that are
+    (257, 5, 5, 20, 2, False),     # no multiple of 4, wide results
+    (300, 6, 3, 6, 0, True),
+    (1300, 4, 4, 64, 0, True),     # scores that do not fit beside the keys: computed twice
 ]
 
 
