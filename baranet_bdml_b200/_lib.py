@@ -26,6 +26,9 @@ SIGNATURES = {
     "bn_last_error": (C.c_char_p, []),
     "bn_version": (_i, []),
     "bn_mm_f32": (_i, [_p, _i64, _i64, _p, _i64, _i64, _p, _i64, _i64, _i, _i, _i, _p]),
+    "bn_split_f32": (_i, [_p, _i64, _p, _i, _i, _p]),
+    "bn_mm_f32_split": (_i, [_p, _p, _i, _p, _i64, _p, _i64, _p, _i, _p, _i, _i, _i, _p, _p]),
+    "bn_mm_f32_split_pays": (_i, [_i, _i, _i, _i]),
     "bn_rope_f32": (_i, [_p, _i64, _i64, _p, _i64, _i64, _i, _i, _i, _f, _i, _p]),
     "bn_embedding_gather_f32": (_i, [_p, _i64, _p, _p, _i64, _i, _i, _i, _p, _p]),
     "bn_argmax_rows_f32": (_i, [_p, _i64, _i64, _p, _i, _i, _p]),

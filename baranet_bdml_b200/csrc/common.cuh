@@ -74,6 +74,9 @@ inline void prefill_bf16_workspace_layout(int B, int S, int Hkv, size_t* table, 
     *total = *krot + up((size_t)B * S * Hkv * 64 * sizeof(__nv_bfloat16));
 }
 
+// The time of bn_mm_f32 in us, roughly (mm_f32.cu)
+float mm_f32_estimate(int M, int N, int K);
+
 // The RoPE frequency of pair i, with the reference's exact arithmetic
 // (src/ops/op_rope.cuh:82): fp32 exponent, fp32 pow, reciprocal taken in
 // double, rounded to fp32.

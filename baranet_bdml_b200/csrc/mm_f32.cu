@@ -203,18 +203,24 @@ static int mm_f32_copies(const MmParams& p, cudaStream_t st) {
 // that reading (8 x 4 outputs a thread: 12 16-byte reads, 4 cycles each, for 128 FMAs), 53 - 60 % of the FMA rate.
 // One 64 x 64 tile of 4 x 4 outputs a thread without copies in flight, before / after: 128 x 2048 x 2048 134 / 52 us,
 // 128 x 256 x 2048 134 / 24 us, 800 x 7424 x 2048 1470 / 610 us, 4 x 32000 x 2048 570 / 88 us.
-static int mm_f32_pick(const MmParams& p, cudaStream_t st) {
+static float mm_f32_times(int M, int N, int* best) {
     const int sms = sm_count();
     auto estimate = [&](int bm, int bn, float alone, float more) {
-        const long long tiles = (long long)ceil_div(p.M, bm) * ceil_div(p.N, bn);
-        if (ceil_div(p.M, bm) > 65535 && bm < 128) return INFINITY;      // the grid's limit
+        const long long tiles = (long long)ceil_div(M, bm) * ceil_div(N, bn);
+        if (ceil_div(M, bm) > 65535 && bm < 128) return INFINITY;        // the grid's limit
         return fmaxf(alone, (float)((tiles + sms - 1) / sms) * more);
     };
     const float t[5] = {estimate(128, 128, 221.f, 220.f), estimate(64, 64, 77.f, 62.f), estimate(32, 64, 52.f, 34.f),
                         estimate(16, 32, 33.f, 16.f), estimate(8, 32, 24.f, 10.4f)};
-    int best = 0;
+    *best = 0;
     for (int i = 1; i < 5; ++i)
-        if (t[i] < t[best]) best = i;
+        if (t[i] < t[*best]) *best = i;
+    return t[*best];
+}
+
+static int mm_f32_pick(const MmParams& p, cudaStream_t st) {
+    int best;
+    mm_f32_times(p.M, p.N, &best);
     switch (best) {
         case 0: return mm_f32_copies<128, 128, 8, 8>(p, st);
         case 1: return mm_f32_copies<64, 64, 8, 4>(p, st);
@@ -222,6 +228,11 @@ static int mm_f32_pick(const MmParams& p, cudaStream_t st) {
         case 3: return mm_f32_copies<16, 32, 4, 2>(p, st);
         default: return mm_f32_copies<8, 32, 2, 1>(p, st);
     }
+}
+
+float mm_f32_estimate(int M, int N, int K) {
+    int best;
+    return mm_f32_times(M, N, &best) * (float)K / 2048.f;
 }
 
 // x = act(x + bias) in place, fp32 rows (the unfused form of the products with a bias or an activation)

@@ -436,9 +436,17 @@ def _rows(t: torch.Tensor, what: str) -> torch.Tensor:
     return t
 
 
+def _bf16_parts(x: torch.Tensor) -> torch.Tensor:
+    """The three bf16 matrices whose sum fp32 x (rows, a multiple of 8) is"""
+    out = torch.empty((3,) + tuple(x.shape), dtype=torch.bfloat16, device=x.device)
+    _lib.check(_lib.load().bn_split_f32(x.data_ptr(), x.stride(0), out.data_ptr(), x.shape[0], x.shape[1], _stream()))
+    return out
+
+
 class Linear:
-    """y = act(x W^T + bias) for a weight (out, in), bias (out) and act optional: bf16 on the tensor cores, or true fp32
-    (`bn_mm_f32`).  Both sizes are rounded up to multiples of 8 with zeros, so x may be passed with its padding columns (which
+    """y = act(x W^T + bias) for a weight (out, in), bias (out) and act optional: bf16 on the tensor cores, or true fp32 (chains
+    of FMAs, `bn_mm_f32`, or for many rows `bn_mm_f32_split`, whose error is smaller).  The latter reads bf16 parts of the weight
+    that are laid out here: one where every weight is a bf16 number, else three, beside the weight itself.  Both sizes are rounded up to multiples of 8 with zeros, so x may be passed with its padding columns (which
     must be finite) and y has them."""
 
     def __init__(self, weight: torch.Tensor, dtype, device="cuda", bias: Optional[torch.Tensor] = None, act: str = "none"):
@@ -450,6 +458,13 @@ class Linear:
         self.n, self.k = round8(self.out_features), round8(self.in_features)
         self.weight = torch.zeros((self.n, self.k), dtype=dtype, device=device)
         self.weight[:self.out_features, :self.in_features] = weight.to(device)
+        self._parts = {}              # number of parts -> the parts of an fp32 weight (a copy: not among a model's parameters)
+        if dtype == torch.float32 and self.weight.is_cuda:
+            parts = _bf16_parts(self.weight)
+            if bool(parts[1:].any()):
+                self._parts[3] = parts
+            else:
+                self._parts[1] = parts[0].clone()
 
     def _operand(self, x: torch.Tensor) -> torch.Tensor:
         _rows(x, "linear(x)")
@@ -464,9 +479,18 @@ class Linear:
         return out
 
     def _mm_f32(self, x: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
-        w = self.weight
-        _lib.check(_lib.load().bn_mm_f32(x.data_ptr(), x.stride(0), 1, w.data_ptr(), 1, w.stride(0), out.data_ptr(),
-                                         out.stride(0), 1, x.shape[0], self.k, self.n, _stream()))
+        """x W^T with the bias and the activation, fp32"""
+        w, rows, lib, act = self.weight, x.shape[0], _lib.load(), ACTIVATIONS[self.act]
+        for n, parts in self._parts.items():
+            if x.data_ptr() % 16 == 0 and lib.bn_mm_f32_split_pays(rows, self.n, self.k, n):
+                _lib.check(lib.bn_mm_f32_split(_bf16_parts(x).data_ptr(), parts.data_ptr(), n, x.data_ptr(), x.stride(0), w.data_ptr(),
+                                               w.stride(0), _ptr(self.bias), act, out.data_ptr(), rows, self.n, self.k,
+                                               _gemm_error_ptr(x.device, None), _stream()))
+                return out
+        _lib.check(lib.bn_mm_f32(x.data_ptr(), x.stride(0), 1, w.data_ptr(), 1, w.stride(0), out.data_ptr(), out.stride(0), 1, rows,
+                                 self.k, self.n, _stream()))
+        if self.bias is not None or self.act != "none":
+            _lib.check(lib.bn_bias_act_f32(out.data_ptr(), self.n, _ptr(self.bias), rows, self.n, act, _stream()))
         return out
 
     def __call__(self, x: torch.Tensor, f32_out: bool = False) -> torch.Tensor:
@@ -475,11 +499,7 @@ class Linear:
         rows = x.shape[0]
         plain = self.bias is None and self.act == "none"
         if self.dtype == torch.float32:
-            out = self._mm_f32(x, torch.empty((rows, self.n), dtype=torch.float32, device=x.device))
-            if not plain:
-                _lib.check(_lib.load().bn_bias_act_f32(out.data_ptr(), self.n, _ptr(self.bias), rows, self.n, ACTIVATIONS[self.act],
-                                                       _stream()))
-            return out
+            return self._mm_f32(x, torch.empty((rows, self.n), dtype=torch.float32, device=x.device))
         if not f32_out:
             return linear_bf16(x, self.weight) if plain else self._bias_act(x)
         if not plain:

@@ -99,6 +99,20 @@ BN_API int bn_selftest_wait_timeout(void* workspace, unsigned limit_us, bn_strea
 BN_API int bn_mm_f32(const float* A, int64_t a_rs, int64_t a_cs, const float* B, int64_t b_rs, int64_t b_cs,
               float* C, int64_t c_rs, int64_t c_cs, int M, int K, int N, bn_stream_t stream);
 
+/* The products of many rows on the tensor cores, with the precision of an fp32 sum: C(M,N) = act(A(M,K) W(N,K)^T + bias),
+ * fp32, from the bf16 parts of both operands.
+ * bn_split_f32 writes x (rows, cols) as three bf16 matrices [3][rows][cols] whose sum it is; cols a multiple of 8, 16-byte
+ * aligned rows.
+ * bn_mm_f32_split takes A's three parts, and of W all three or (w_nparts = 1) the first, where the others are zeros, beside the
+ * operands themselves, from which results that are not finite are worked out as by bn_mm_f32.  N and K multiples of 8;
+ * bias (N) or null; act one of BN_ACT_*.
+ * bn_mm_f32_split_pays: whether both together take less time than bn_mm_f32 (an estimate). */
+BN_API int bn_mm_f32_split_pays(int M, int N, int K, int w_nparts);
+BN_API int bn_split_f32(const float* x, int64_t ld, void* parts, int rows, int cols, bn_stream_t stream);
+BN_API int bn_mm_f32_split(const void* a_parts, const void* w_parts, int w_nparts, const float* a, int64_t a_ld, const float* w,
+                           int64_t w_ld, const float* bias, int act, float* c, int M, int N, int K, int* error_word,
+                           bn_stream_t stream);
+
 /* y = RoPE(x): adjacent pairs (2i, 2i+1) inside every head_dim-wide column
  * block, row r at position r + position_offset, fp32 angles.
  * Replaces op_rope (src/ops/op_rope.cuh:101-126). */

@@ -84,6 +84,46 @@ def test_mm_tiles_and_copies(T, cref, M, K, N, layout):
     assert np.array_equal(got, ref)
 
 
+@pytest.mark.parametrize("M,K,N", [(1, 8, 8), (127, 72, 72), (129, 136, 136), (300, 2056, 264), (513, 64, 2056), (1300, 128, 4096)])
+@pytest.mark.parametrize("parts", [1, 3])
+def test_mm_of_bf16_parts(lib, M, K, N, parts):
+    import torch
+    from baranet_bdml_b200 import _lib, ops
+    gen = torch.Generator(device="cuda").manual_seed(M + parts)
+    x, w, bias = (torch.randn(s, generator=gen, device="cuda") for s in ((M, K), (N, K), (N,)))
+    if parts == 1:
+        w = w.bfloat16().float()
+    xp, wp = ops._bf16_parts(x), ops._bf16_parts(w)
+    assert torch.equal(xp.double().sum(0), x.double()) and torch.equal(wp.double().sum(0), w.double())
+    assert bool(wp[1:].any()) == (parts == 3)
+    # a bad row of x and a bad row of w touch their own results alone, and there the chain decides
+    x[M // 2, K // 2], w[N // 2, 0] = float("inf"), float("nan")
+    xp, wp = ops._bf16_parts(x), ops._bf16_parts(w)
+    L, st = lib, torch.cuda.current_stream().cuda_stream
+    chain, word = torch.empty((M, N), device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    _lib.check(L.bn_mm_f32(x.data_ptr(), K, 1, w.data_ptr(), 1, K, chain.data_ptr(), N, 1, M, K, N, st))
+    exact, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    fine = torch.isfinite(chain)
+    for b, act in ((None, 0), (bias, 3), (bias, 2)):
+        got = torch.empty((M, N), device="cuda")
+        _lib.check(L.bn_mm_f32_split(xp.data_ptr(), wp.data_ptr(), parts, x.data_ptr(), K, w.data_ptr(), K,
+                                    None if b is None else b.data_ptr(), act, got.data_ptr(), M, N, K, word.data_ptr(), st))
+        want = chain.clone()
+        if act:
+            _lib.check(L.bn_bias_act_f32(want.data_ptr(), N, b.data_ptr(), M, N, act, st))
+        assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isinf(got), torch.isinf(want))
+        if act == 0:
+            # in an accumulator 4 truncations at full size, each of 2 units of 2^-24, beside 8 at 2^-8 of it; K / 64 roundings
+            # of the sum; products left out and the bias: 1 more
+            bound = (4 * 2 + 1 + K / 64 + 1) * 2.0 ** -24 * size
+            assert ((got.double() - exact).abs() <= bound)[fine].all()
+        elif act == 2:
+            # the activation's slope is below 1.13; the chain itself is off by at most K roundings
+            bound = 1.13 * (K + K / 64 + 12) * 2.0 ** -24 * (size + b.double().abs())
+            assert ((got.double() - want.double()).abs() <= bound)[fine].all()
+    assert int(word.item()) == 0
+
+
 def test_mm_transposed_and_sliced_views(T):
     rng = np.random.default_rng(2)
     a = rng.standard_normal((40, 96), dtype=np.float32)
