@@ -20,6 +20,7 @@
 // and the product in one launch.
 // Every mbarrier wait is bounded; on expiry the kernel raises the caller's error word, frees TMEM and returns.
 #include "common.cuh"
+#include "gemm_rows.cuh"
 #include "hybrid.cuh"
 #include "ptx.cuh"
 #include "tcgen05.cuh"
@@ -125,11 +126,23 @@ gemm_bf16_nt_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     tc::fence_after_sync();
     const uint32_t tmem = s_tmem_base;
 
+    // A programmatic dependent: the set-up above runs while the kernel ahead finishes, and so does the fetch of the weights into
+    // L2 where they are what the launch waits for (EPI_PARTIAL).
+    if (warp == 5 && lane == 0) {
+        prefetch_tensormap(&tmap_a);
+        prefetch_tensormap(&tmap_b);
+        if (EPI == EPI_PARTIAL && (int)blockIdx.x < n_tiles) {
+            int ks0, ks1;
+            k_range(blockIdx.x, ks0, ks1);
+            for (int ks = ks0; ks < ks1; ++ks) tma_prefetch_2d(&tmap_b, ks * GM_BK, (blockIdx.x / tiles_m) % tiles_n * GM_BN);
+        }
+    }
+    grid_dependency_wait();
+    if (EPI == EPI_PARTIAL) grid_launch_dependents();
+
     if (warp == 5) {
         // ---------------------------------------------------------- TMA producer
         if (lane == 0) {
-            prefetch_tensormap(&tmap_a);
-            prefetch_tensormap(&tmap_b);
             uint32_t it = 0;      // ring steps issued
             bool ok = true;
             for (int t = blockIdx.x; ok && t < n_tiles; t += gridDim.x) {
@@ -444,8 +457,10 @@ using namespace bn;
 // activation times `mul`
 __global__ void __launch_bounds__(256)
 gemm_splitk_reduce_kernel(const float* __restrict__ partial, __nv_bfloat16* __restrict__ c, long long mn4, int splits,
-                          float* __restrict__ c32, const __nv_bfloat16* __restrict__ mul, long long mul_ld, int N, int act,
+                          float* __restrict__ c32, const __nv_bfloat16* mul, long long mul_ld, int N, int act,
                           const float* __restrict__ bias) {
+    grid_dependency_wait();
+    grid_launch_dependents();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;     // one group of 4 outputs
     if (i >= mn4) return;
     const float4* p4 = reinterpret_cast<const float4*>(partial);
@@ -523,6 +538,11 @@ static int gemm_launch(const void* a, const void* bt, void* c, int M, int N, int
                             : cudaMemsetAsync(c, 0, (size_t)M * n_out * 2, as_stream(stream));
         return e == cudaSuccess ? BN_OK : fail(BN_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
     }
+    if (epi != EPI_QKV && epi != EPI_PLAIN && gemm_rows_ok(M, n_out)) {
+        RowsGemm r{a, bt, static_cast<__nv_bfloat16*>(c), c32, static_cast<const __nv_bfloat16*>(mul), bias, error_word, mul_ld, M, N, K,
+                   n_out, epi >= EPI_GLU ? epi - EPI_GLU : act, epi >= EPI_GLU};
+        return gemm_rows(r, as_stream(stream), what);
+    }
     const int bn = epi == EPI_PARTIAL ? 64 : 256;
     CUtensorMap tmap_a, tmap_b;
     {
@@ -551,32 +571,32 @@ static int gemm_launch(const void* a, const void* bt, void* c, int M, int N, int
     cudaStream_t st = as_stream(stream);
     if (epi == EPI_PLAIN) {
         if (int rc = gemm_configure<EPI_PLAIN, 256>(dev)) return rc;
-        gemm_bf16_nt_kernel<EPI_PLAIN, 256><<<grid, GM_THREADS, GemmShape<256>::SMEM_BYTES, st>>>(tmap_a, tmap_b, p);
+        launch_dependent(gemm_bf16_nt_kernel<EPI_PLAIN, 256>, grid, GM_THREADS, GemmShape<256>::SMEM_BYTES, st, tmap_a, tmap_b, p);
     } else if (epi == EPI_GLU_SILU) {
         if (int rc = gemm_configure<EPI_GLU_SILU, 256>(dev)) return rc;
-        gemm_bf16_nt_kernel<EPI_GLU_SILU, 256><<<grid, GM_THREADS, GemmShape<256>::SMEM_BYTES, st>>>(tmap_a, tmap_b, p);
+        launch_dependent(gemm_bf16_nt_kernel<EPI_GLU_SILU, 256>, grid, GM_THREADS, GemmShape<256>::SMEM_BYTES, st, tmap_a, tmap_b, p);
     } else if (epi == EPI_GLU_GELU) {
         if (int rc = gemm_configure<EPI_GLU_GELU, 256>(dev)) return rc;
-        gemm_bf16_nt_kernel<EPI_GLU_GELU, 256><<<grid, GM_THREADS, GemmShape<256>::SMEM_BYTES, st>>>(tmap_a, tmap_b, p);
+        launch_dependent(gemm_bf16_nt_kernel<EPI_GLU_GELU, 256>, grid, GM_THREADS, GemmShape<256>::SMEM_BYTES, st, tmap_a, tmap_b, p);
     } else if (epi == EPI_F32) {
         if (int rc = gemm_configure<EPI_F32, 256>(dev)) return rc;
-        gemm_bf16_nt_kernel<EPI_F32, 256><<<grid, GM_THREADS, GemmShape<256>::SMEM_BYTES, st>>>(tmap_a, tmap_b, p);
+        launch_dependent(gemm_bf16_nt_kernel<EPI_F32, 256>, grid, GM_THREADS, GemmShape<256>::SMEM_BYTES, st, tmap_a, tmap_b, p);
     } else if (epi == EPI_ACTMUL) {
         if (int rc = gemm_configure<EPI_ACTMUL, 256>(dev)) return rc;
-        gemm_bf16_nt_kernel<EPI_ACTMUL, 256><<<grid, GM_THREADS, GemmShape<256>::SMEM_BYTES, st>>>(tmap_a, tmap_b, p);
+        launch_dependent(gemm_bf16_nt_kernel<EPI_ACTMUL, 256>, grid, GM_THREADS, GemmShape<256>::SMEM_BYTES, st, tmap_a, tmap_b, p);
     } else if (epi == EPI_BIAS) {
         if (int rc = gemm_configure<EPI_BIAS, 256>(dev)) return rc;
-        gemm_bf16_nt_kernel<EPI_BIAS, 256><<<grid, GM_THREADS, GemmShape<256>::SMEM_BYTES, st>>>(tmap_a, tmap_b, p);
+        launch_dependent(gemm_bf16_nt_kernel<EPI_BIAS, 256>, grid, GM_THREADS, GemmShape<256>::SMEM_BYTES, st, tmap_a, tmap_b, p);
     } else if (epi == EPI_QKV) {
         if (int rc = gemm_configure<EPI_QKV, 256>(dev)) return rc;
         gemm_bf16_nt_kernel<EPI_QKV, 256><<<grid, GM_THREADS, GemmShape<256>::SMEM_BYTES, st>>>(tmap_a, tmap_b, p);
     } else {
         if (int rc = gemm_configure<EPI_PARTIAL, 64>(dev)) return rc;
-        gemm_bf16_nt_kernel<EPI_PARTIAL, 64><<<grid, GM_THREADS, GemmShape<64>::SMEM_BYTES, st>>>(tmap_a, tmap_b, p);
+        launch_dependent(gemm_bf16_nt_kernel<EPI_PARTIAL, 64>, grid, GM_THREADS, GemmShape<64>::SMEM_BYTES, st, tmap_a, tmap_b, p);
         if (int rc = launch_status(what)) return rc;
         const long long mn4 = (long long)M * N / 4;
-        gemm_splitk_reduce_kernel<<<(unsigned)((mn4 + 255) / 256), 256, 0, st>>>(partial, static_cast<__nv_bfloat16*>(c),
-                                                                             mn4, splits, c32, p.mul, mul_ld, N, act, bias);
+        launch_dependent(gemm_splitk_reduce_kernel, (unsigned)((mn4 + 255) / 256), 256, 0, st, (const float*)partial,
+                         static_cast<__nv_bfloat16*>(c), mn4, splits, c32, p.mul, mul_ld, N, act, bias);
     }
     return launch_status(what);
 }

@@ -171,8 +171,8 @@ def _small_m_scratch(device, M: int, N: int, K: int):
 
 def gemm_bf16_nt_small_m(a: torch.Tensor, bt: torch.Tensor, *, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """a (M,K) @ bt (N,K)^T for few rows (a decode step: one token per sequence): the weight stream is spread over
-    all SMs (64-wide N tiles, K split, partial sums added in a fixed order).  The fp32 scratch is kept per
-    (device, size) and reused by later calls on the same stream."""
+    all SMs (K split, partial sums added in a fixed order).  The fp32 scratch, which products of more than 128 rows or of
+    many columns use, is kept per (device, size) and reused by later calls on the same stream."""
     _need(a, torch.bfloat16, "gemm_bf16_nt_small_m(a)")
     _need(bt, torch.bfloat16, "gemm_bf16_nt_small_m(bt)")
     if a.dim() != 2 or bt.dim() != 2 or a.shape[1] != bt.shape[1]:
@@ -198,9 +198,16 @@ def skinny_any_k(rows: int, n_out: int, k: int) -> bool:
     return 0 < rows <= 16 and n_out % 8 == 0 and k % 8 == 0 and 0 < k <= 8192
 
 
+def skinny_best(rows: int, n_out: int, k: int) -> bool:
+    """Those of them for which it is the fastest.  Its CTAs read the rows for every 8 columns of the weight, which shows with
+    many of both: us at 16 rows, 2048 -> 7424 11.2 (the kernel for up to 128 rows: 8.3), 2048 -> 8512 11.6 (8.8), 2048 -> 4608
+    6.4 (6.8); 2048 -> 32000 32.5 (128 x 256 tiles: 27.3), the same at 8 rows 27.0 (26.9)."""
+    return skinny_any_k(rows, n_out, k) and (rows <= 4 or n_out < 6144 or (rows <= 8 and n_out > 17000))
+
+
 def small_m_ok(rows: int, n_out: int) -> bool:
     """Few rows and too few 256-wide output tiles to occupy the GPU (measured cross-over: fewer than half as many tiles as
-    SMs): the split-K form."""
+    SMs): the form for up to 128 rows."""
     return rows <= 128 and (n_out + 255) // 256 < 74
 
 
@@ -262,9 +269,9 @@ def gemm_swiglu_bf16_nt_skinny(x: torch.Tensor, gate_t: torch.Tensor, up_t: torc
 
 def linear_bf16(x: torch.Tensor, weight_t: torch.Tensor) -> torch.Tensor:
     """x (rows, in) @ weight_t (out, in)^T, choosing the kernel by shape: at most 16 rows -> the weight-streaming
-    kernel; few rows and few output tiles -> the split-K small-M form; otherwise the large-tile kernel."""
+    kernel, mostly; few rows and few output tiles -> the small-M form; otherwise the large-tile kernel."""
     rows, n_out = x.shape[0], weight_t.shape[0]
-    if skinny_any_k(rows, n_out, x.shape[1]):
+    if skinny_best(rows, n_out, x.shape[1]):
         return gemm_bf16_nt_skinny(x, weight_t)
     if small_m_ok(rows, n_out):
         return gemm_bf16_nt_small_m(x, weight_t)
@@ -506,7 +513,7 @@ class Linear:
             raise RuntimeError("linear: the fp32 result has neither a bias nor an activation")
         out = torch.empty((rows, self.n), dtype=torch.float32, device=x.device)
         lib = _lib.load()
-        if skinny_any_k(rows, self.n, self.k):
+        if skinny_best(rows, self.n, self.k):
             _lib.check(lib.bn_gemm_bf16_nt_skinny_f32(x.data_ptr(), self.weight.data_ptr(), rows, self.n, self.k,
                                                       out.data_ptr(), _stream()))
         elif small_m_ok(rows, self.n):
@@ -521,7 +528,7 @@ class Linear:
     def _bias_act(self, x: torch.Tensor) -> torch.Tensor:
         rows, a, lib = x.shape[0], ACTIVATIONS[self.act], _lib.load()
         out = torch.empty((rows, self.n), dtype=self.dtype, device=x.device)
-        if skinny_any_k(rows, self.n, self.k):
+        if skinny_best(rows, self.n, self.k):
             _lib.check(lib.bn_gemm_bias_act_bf16_nt_skinny(x.data_ptr(), self.weight.data_ptr(), _ptr(self.bias), out.data_ptr(), rows,
                                                            self.n, self.k, a, _stream()))
         elif small_m_ok(rows, self.n):
@@ -549,7 +556,7 @@ class Linear:
             self._mm_f32(x, out)
             _lib.check(lib.bn_act_mul_f32(out.data_ptr(), self.n, mul.data_ptr(), mul.stride(0), out.data_ptr(), self.n, rows,
                                           self.n, a, _stream()))
-        elif skinny_any_k(rows, self.n, self.k):
+        elif skinny_best(rows, self.n, self.k):
             _lib.check(lib.bn_gemm_act_mul_bf16_nt_skinny(x.data_ptr(), self.weight.data_ptr(), mul.data_ptr(), mul.stride(0),
                                                           out.data_ptr(), rows, self.n, self.k, a, _stream()))
         elif small_m_ok(rows, self.n):

@@ -187,6 +187,43 @@ def test_graphed_decoder_layer_equals_eager(lib):
         assert torch.equal(res_e, res_g) and torch.equal(mlp_e, mlp_g)
 
 
+# rows around the widths of the narrow operand; K of one step, of less than five per CTA, ragged, and of full clusters; columns
+# of one 128-wide tile, of a part of one, and of so many tiles that a CTA has a tile to itself
+@pytest.mark.parametrize("M", [1, 17, 32, 33, 64, 65, 128])
+@pytest.mark.parametrize("N,K", [(8, 8), (136, 328), (256, 2120), (2048, 2048), (16896, 128)])
+def test_small_m_epilogues(lib, M, N, K):
+    from baranet_bdml_b200 import _lib, ops
+    gen = torch.Generator(device="cuda").manual_seed(M * 31 + N + K)
+    rnd = lambda *s: torch.randn(s, generator=gen, device="cuda")                                # noqa: E731
+    x, w, u = rnd(M, K).bfloat16(), (rnd(N, K) * 0.06).bfloat16(), (rnd(N, K) * 0.06).bfloat16()
+    bias, mul = rnd(N), rnd(M, N + 8).bfloat16()
+    prod, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    up, up_size = x.double() @ u.double().T, x.double().abs() @ u.double().abs().T
+    n = int(lib.bn_gemm_bf16_nt_small_m_workspace_bytes(M, N, K))
+    ws, word, st = torch.empty(n, dtype=torch.uint8, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda"), torch.cuda.current_stream().cuda_stream
+    tail = (ws.data_ptr(), n, word.data_ptr(), st)
+    c, c32 = torch.empty((M, N), dtype=torch.bfloat16, device="cuda"), torch.empty((M, N), device="cuda")
+    # fp32 sums of exact products: K roundings (or truncations of 2 units) of at most 2^-24 of the absolute sum
+    slack, bf = 2 * K * 2.0 ** -24, 2.0 ** -8
+    silu = torch.nn.functional.silu
+    _lib.check(lib.bn_gemm_bf16_nt_small_m_f32(x.data_ptr(), w.data_ptr(), c32.data_ptr(), M, N, K, *tail))
+    assert ((c32.double() - prod).abs() <= slack * size).all()
+    _lib.check(lib.bn_gemm_bf16_nt_small_m(x.data_ptr(), w.data_ptr(), c.data_ptr(), M, N, K, *tail))
+    assert torch.equal(c, c32.bfloat16())
+    _lib.check(lib.bn_gemm_bias_act_bf16_nt_small_m(x.data_ptr(), w.data_ptr(), bias.data_ptr(), c.data_ptr(), M, N, K, _lib.BN_ACT_RELU2, *tail))
+    assert torch.equal(c, (torch.relu(c32 + bias) ** 2).bfloat16())
+    # the fast exponential and quotient: within 2^-18 of the factor; the slope of silu is below 1.1
+    _lib.check(lib.bn_gemm_act_mul_bf16_nt_small_m(x.data_ptr(), w.data_ptr(), mul.data_ptr(), N + 8, c.data_ptr(), M, N, K, _lib.BN_ACT_SILU, *tail))
+    m = mul[:, :N].double()
+    assert ((c.double() - silu(prod) * m).abs() <= bf * (silu(prod) * m).abs() + (1.1 * slack * size + 2.0 ** -18 * prod.abs()) * m.abs() + 1e-30).all()
+    packed = ops.pack_gate_up(w, u)
+    _lib.check(lib.bn_gemm_glu_bf16_nt(x.data_ptr(), packed.data_ptr(), c.data_ptr(), M, N, K, _lib.BN_ACT_SILU, word.data_ptr(), st))
+    want = silu(prod) * up
+    bound = bf * want.abs() + (1.1 * slack * size + 2.0 ** -18 * prod.abs()) * up.abs() + slack * up_size * (silu(prod).abs() + slack * size) + 1e-30
+    assert ((c.double() - want).abs() <= bound).all()
+    assert int(word.item()) == 0
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 8, 8), (64, 2048, 2048), (64, 256, 2048), (17, 2048, 5632), (128, 1000, 520),
                                    (64, 32000, 2048), (130, 136, 264)])
 def test_small_m_gemm(lib, M, N, K):
