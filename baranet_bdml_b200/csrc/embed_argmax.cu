@@ -10,6 +10,7 @@
 //       it is element 0.  The reference runs ONE THREAD per row; here a CTA per row.
 // Both are HBM-bound copies / reductions: 16-byte accesses, consecutive threads on consecutive addresses.
 #include "common.cuh"
+#include "ptx.cuh"
 #include "hybrid.cuh"
 
 namespace bn {
@@ -79,27 +80,40 @@ __device__ __forceinline__ ArgMax better(ArgMax a, ArgMax b) {
     return a;
 }
 
-__global__ void __launch_bounds__(256)
-argmax_rows_kernel(const float* __restrict__ x, int64_t x_rs, int64_t x_cs, uint32_t* __restrict__ out, int rows,
-                   int cols) {
-    __shared__ float sv[8];
-    __shared__ int si[8];
+// A row is one block's: what bounds a step's few rows is how many of a row's loads are in flight.  64 rows of 32000: 256
+// threads with one 16-byte load each in turn 10.2 us, 1024 with up to eight 5.2 us; short rows keep the small block.
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS)
+argmax_rows_kernel(const float* x, int64_t x_rs, int64_t x_cs, uint32_t* out, int rows, int cols) {
+    constexpr int AHEAD = 8;
+    __shared__ float sv[THREADS / 32];
+    __shared__ int si[THREADS / 32];
+    ptx::grid_dependency_wait();
+    ptx::grid_launch_dependents();
     const int tid = threadIdx.x, lane = tid % 32, warp = tid / 32;
     for (int r = blockIdx.x; r < rows; r += gridDim.x) {
         const float* xr = x + (int64_t)r * x_rs;
         ArgMax best{-INFINITY, 0x7fffffff};
         if (x_cs == 1 && (reinterpret_cast<uintptr_t>(xr) & 15) == 0) {
             const float4* x4 = reinterpret_cast<const float4*>(xr);
-            for (int c = tid; c < cols / 4; c += blockDim.x) {
-                const float4 v = __ldg(x4 + c);
-                best = better(best, ArgMax{v.x, 4 * c});
-                best = better(best, ArgMax{v.y, 4 * c + 1});
-                best = better(best, ArgMax{v.z, 4 * c + 2});
-                best = better(best, ArgMax{v.w, 4 * c + 3});
+            for (int c0 = tid; c0 < cols / 4; c0 += AHEAD * THREADS) {
+                float4 v[AHEAD];
+#pragma unroll
+                for (int k = 0; k < AHEAD; ++k)
+                    if (c0 + k * THREADS < cols / 4) v[k] = x4[c0 + k * THREADS];
+#pragma unroll
+                for (int k = 0; k < AHEAD; ++k) {
+                    const int c = c0 + k * THREADS;
+                    if (c >= cols / 4) break;
+                    best = better(best, ArgMax{v[k].x, 4 * c});
+                    best = better(best, ArgMax{v[k].y, 4 * c + 1});
+                    best = better(best, ArgMax{v[k].z, 4 * c + 2});
+                    best = better(best, ArgMax{v[k].w, 4 * c + 3});
+                }
             }
-            for (int c = cols / 4 * 4 + tid; c < cols; c += blockDim.x) best = better(best, ArgMax{__ldg(xr + c), c});
+            for (int c = cols / 4 * 4 + tid; c < cols; c += THREADS) best = better(best, ArgMax{xr[c], c});
         } else {
-            for (int c = tid; c < cols; c += blockDim.x) best = better(best, ArgMax{__ldg(xr + (int64_t)c * x_cs), c});
+            for (int c = tid; c < cols; c += THREADS) best = better(best, ArgMax{xr[(int64_t)c * x_cs], c});
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
@@ -110,10 +124,10 @@ argmax_rows_kernel(const float* __restrict__ x, int64_t x_rs, int64_t x_cs, uint
         __syncthreads();
         if (tid == 0) {
             ArgMax b{sv[0], si[0]};
-            for (int w = 1; w < 8; ++w) b = better(b, ArgMax{sv[w], si[w]});
+            for (int w = 1; w < THREADS / 32; ++w) b = better(b, ArgMax{sv[w], si[w]});
             // the reference starts from element 0: it stays unless something is strictly greater; a NaN there
             // is never beaten, and if no element compares (all NaN or -inf) index 0 stands
-            const float x0 = __ldg(xr);
+            const float x0 = xr[0];
             out[r] = (x0 != x0 || !(b.v > x0)) ? 0u : (uint32_t)b.i;
         }
         __syncthreads();
@@ -169,6 +183,8 @@ extern "C" int bn_argmax_rows_f32(const float* x, int64_t x_rs, int64_t x_cs, ui
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const long long cap = (long long)sms * 8;
-    argmax_rows_kernel<<<(unsigned)(rows < cap ? rows : cap), 256, 0, as_stream(stream)>>>(x, x_rs, x_cs, out, rows, cols);
+    const unsigned grid = (unsigned)(rows < cap ? rows : cap);
+    if (cols >= 4096) launch_dependent(argmax_rows_kernel<1024>, grid, 1024, 0, as_stream(stream), x, x_rs, x_cs, out, rows, cols);
+    else launch_dependent(argmax_rows_kernel<256>, grid, 256, 0, as_stream(stream), x, x_rs, x_cs, out, rows, cols);
     return launch_status("bn_argmax_rows_f32");
 }

@@ -86,8 +86,8 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tmem = s_tmem_base;
-    grid_dependency_wait();
     grid_launch_dependents();
+    grid_dependency_wait();
 
     if (warp == 5) {
         if (lane == 0) {

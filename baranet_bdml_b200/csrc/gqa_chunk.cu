@@ -69,8 +69,8 @@ __device__ __forceinline__ void store8(__nv_bfloat16* p, const float (&v)[8]) { 
 template <typename T, int LANES>
 __global__ void __launch_bounds__(KP_THREADS)
 kv_prep_kernel(const KvPrepParams p) {
-    grid_dependency_wait();
     grid_launch_dependents();
+    grid_dependency_wait();
     constexpr int PER_BLOCK = KP_THREADS / LANES;
     const int lane = threadIdx.x % LANES;
     const unsigned n = (unsigned)p.B * p.S * p.G;
@@ -155,8 +155,8 @@ constexpr int GA_THREADS = 256, GA_BATCH = 4;
 __global__ void __launch_bounds__(GA_THREADS)
 kv_gather_kernel(const uint4* ring_k, const uint4* ring_v, int ring_tokens, int G, int k16, int v16, const int32_t* seq_ids,
                  const int32_t* positions, int chunk, int n_old, uint4* k_out, uint4* v_out, int rows_per_seq, int blocks) {
-    grid_dependency_wait();
     grid_launch_dependents();
+    grid_dependency_wait();
     const int part = blockIdx.x % blocks, g = blockIdx.x / blocks % G, b = blockIdx.x / (blocks * G);
     const int slot = seq_ids ? seq_ids[b] : b, n = min(min(n_old, positions[b] % chunk), ring_tokens);    // the host sized n_old by the same positions
     const uint4* ks = ring_k + ((int64_t)slot * G + g) * ring_tokens * k16;
@@ -270,8 +270,8 @@ gqa_step_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constan
         prefetch_tensormap(&tmap_v);
     }
     __syncthreads();
-    grid_dependency_wait();
     grid_launch_dependents();
+    grid_dependency_wait();
     const int pos = p.positions[b], slot = p.seq_ids ? p.seq_ids[b] : b;
     // This warp's part of the projection row is requested before the cache is streamed, or it would arrive behind the stream.
     // A lane has 8 columns of a head.  Queries as they are (zeros beyond the group's heads and their columns), their norms go

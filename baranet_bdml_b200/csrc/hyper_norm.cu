@@ -36,8 +36,8 @@ template <typename T, int NV, int NI, int NO>
 __global__ void __launch_bounds__(HY_THREADS)
 hyper_norm_regs_kernel(const __grid_constant__ HyperParams p) {
     __shared__ float sh[HY_THREADS / 32];
-    ptx::grid_dependency_wait();
     ptx::grid_launch_dependents();
+    ptx::grid_dependency_wait();
     const int pieces = p.hidden / 4;
     const float inv_n = 1.f / (float)p.hidden;
     for (int r = blockIdx.x; r < p.rows; r += gridDim.x) {
@@ -108,8 +108,8 @@ hyper_norm_any_kernel(const __grid_constant__ HyperParams p) {
     for (int i = threadIdx.x; i < p.n_in * p.n_out; i += HY_THREADS) s_mix[i] = p.mix[i];
     if (threadIdx.x < p.n_out) { s_out[threadIdx.x] = p.w_out[threadIdx.x]; s_in[threadIdx.x] = p.w_in[threadIdx.x]; }
     __syncthreads();
-    ptx::grid_dependency_wait();
     ptx::grid_launch_dependents();
+    ptx::grid_dependency_wait();
     for (int r = blockIdx.x; r < p.rows; r += gridDim.x) {
         const T* dr = p.delta ? static_cast<const T*>(p.delta) + (int64_t)r * p.delta_ld : nullptr;
         float ss = 0.f;

@@ -30,7 +30,7 @@ class CausalLM:
 
     def argmax(self, logits: torch.Tensor) -> torch.Tensor:
         rows, cols = logits.shape
-        out = torch.zeros((rows,), dtype=torch.int32, device="cuda")
+        out = torch.empty((rows,), dtype=torch.int32, device="cuda")
         _lib.check(_lib.load().bn_argmax_rows_f32(logits.data_ptr(), logits.stride(0), logits.stride(1), out.data_ptr(),
                                                   rows, cols, torch.cuda.current_stream().cuda_stream))
         return out
@@ -172,10 +172,17 @@ class SequenceLM(CausalLM):
     def decode_step(self, token_ids: torch.Tensor, check: bool = True, slots: Optional[Sequence[int]] = None) -> torch.Tensor:
         """One new token for the sequences in `slots` (None: the first B slots), whatever their lengths."""
         B = token_ids.numel()
-        seq_ids = self._all_slots[:B] if slots is None else torch.tensor(list(slots), dtype=torch.int32, device="cuda")
-        positions = self.seq_lens.index_select(0, seq_ids)
+        if slots is None:
+            seq_ids, lens = self._all_slots[:B], self.seq_lens[:B]
+            positions = lens.clone()
+        else:
+            seq_ids = torch.tensor(list(slots), dtype=torch.int32, device="cuda")
+            positions = self.seq_lens.index_select(0, seq_ids)
         state = self._forward(token_ids.reshape(-1).to(torch.int32).contiguous(), B, 1, seq_ids, positions, None)
-        self.seq_lens.index_add_(0, seq_ids, torch.ones_like(seq_ids))
+        if slots is None:
+            lens.add_(1)
+        else:
+            self.seq_lens.index_add_(0, seq_ids, torch.ones_like(seq_ids))
         if check:
             self._check_ids()
         return self._logits(state)
