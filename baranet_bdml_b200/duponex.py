@@ -14,6 +14,7 @@ import torch
 
 from . import ops
 from .checkpoint import Weights
+from .kv_cache import ZeroedTogether
 from .mixers import MLP, ChunkedAttention, ChunkedAttentionConfig
 from .model import SequenceLM
 
@@ -106,7 +107,10 @@ class DuponexModel(SequenceLM):
             warnings.warn(f"checkpoint tensors that this design does not have: {w.leftover()[:5]}")
 
     def new_states(self, num_seqs: int, max_tokens: Optional[int]):
-        return [layer.mixer.new_state(num_seqs, max_tokens) for layer in self.layers]
+        zeros = ZeroedTogether()
+        states = [layer.mixer.new_state(num_seqs, max_tokens, zeros) for layer in self.layers]
+        zeros.fill()
+        return states
 
     # -------------------------------------------------------------------- forward
     def _forward(self, ids: torch.Tensor, B: int, S: int, seq_ids, positions, n_old: Optional[int]):

@@ -22,14 +22,35 @@ from .ops import Workspace, _need, _stream
 PAGE_TOKENS = _lib.BN_PAGE_TOKENS
 
 
+class ZeroedTogether:
+    """Stands in for torch.zeros while the states of many layers are made: the tensors come from torch.empty, and `fill`
+    zeroes them in one launch per dtype (a launch for each took the host longer than a short prompt takes the GPU)."""
+
+    def __init__(self):
+        self.tensors = {}
+
+    def __call__(self, shape, dtype, device):
+        t = torch.empty(shape, dtype=dtype, device=device)
+        self.tensors.setdefault(dtype, []).append(t)
+        return t
+
+    def fill(self) -> None:
+        for group in self.tensors.values():
+            torch._foreach_zero_(group)
+
+
 class PagedKVCache:
+    """`storage`: pool, page table and lengths, made by the caller (of these shapes and dtypes); else they are made zeroed."""
+
     def __init__(self, num_pages: int, num_seqs: int, max_pages_per_seq: int, num_kv_heads: int = 4,
-                 head_dim: int = 64, theta: float = 10000.0, device="cuda"):
+                 head_dim: int = 64, theta: float = 10000.0, device="cuda", storage=None):
         self.num_pages, self.num_seqs, self.max_pages = int(num_pages), int(num_seqs), int(max_pages_per_seq)
         self.num_kv_heads, self.head_dim, self.theta = int(num_kv_heads), int(head_dim), float(theta)
-        self.pool = torch.zeros((num_pages, num_kv_heads, 2, PAGE_TOKENS, head_dim), dtype=torch.bfloat16, device=device)
-        self.page_table = torch.zeros((num_seqs, max_pages_per_seq), dtype=torch.int32, device=device)
-        self.seq_lens = torch.zeros((num_seqs,), dtype=torch.int32, device=device)
+        if storage is None:
+            storage = (torch.zeros((num_pages, num_kv_heads, 2, PAGE_TOKENS, head_dim), dtype=torch.bfloat16, device=device),
+                       torch.zeros((num_seqs, max_pages_per_seq), dtype=torch.int32, device=device),
+                       torch.zeros((num_seqs,), dtype=torch.int32, device=device))
+        self.pool, self.page_table, self.seq_lens = storage
         self._ws = {}          # decode scratch per (B, Hq, max_seq_len, chunk_tokens); kept while the cache lives
 
     @property
@@ -106,12 +127,12 @@ class LatentRingCache:
 
     ring[slot][ring_tokens][round8(kv_rank) | round8(rot_dim)], zeros behind the values of each part."""
 
-    def __init__(self, num_seqs: int, window: int, kv_rank: int, rot_dim: int, dtype=torch.bfloat16, device="cuda"):
+    def __init__(self, num_seqs: int, window: int, kv_rank: int, rot_dim: int, dtype=torch.bfloat16, device="cuda", zeros=torch.zeros):
         from .ops import round8
         self.num_seqs, self.window, self.kv_rank, self.rot_dim, self.dtype = num_seqs, window, kv_rank, rot_dim, dtype
         self.kv_ld, self.rot_ld = round8(kv_rank), round8(rot_dim)
         self.ring_tokens = (window + PAGE_TOKENS - 1) // PAGE_TOKENS * PAGE_TOKENS
-        self.ring = torch.zeros((num_seqs, self.ring_tokens, self.kv_ld + self.rot_ld), dtype=dtype, device=device)
+        self.ring = zeros((num_seqs, self.ring_tokens, self.kv_ld + self.rot_ld), dtype=dtype, device=device)
 
     def reset(self, slot: int) -> None:
         """Nothing to clear: a row is read only for positions that the sequence itself has written."""
@@ -135,14 +156,14 @@ class ChunkCache:
     k[slot][kv_head][ring_tokens][round8(dim)], v likewise, zeros behind the values."""
 
     def __init__(self, num_seqs: int, chunk: int, kv_heads: int, dim: int, vdim: int, dtype=torch.bfloat16,
-                 max_tokens: Optional[int] = None, groups: int = 1, device="cuda"):
+                 max_tokens: Optional[int] = None, groups: int = 1, device="cuda", zeros=torch.zeros):
         from .ops import round8
         self.num_seqs, self.chunk, self.kv_heads, self.dtype = num_seqs, chunk, kv_heads, dtype
         self.dim_ld, self.vdim_ld = round8(dim), round8(vdim)
         self.ring_tokens = chunk if max_tokens is None else max(1, min(chunk, max_tokens))
-        self.k = torch.zeros((num_seqs, kv_heads, self.ring_tokens, self.dim_ld), dtype=dtype, device=device)
-        self.v = torch.zeros((num_seqs, kv_heads, self.ring_tokens, self.vdim_ld), dtype=dtype, device=device)
-        self.tickets = torch.zeros(num_seqs * kv_heads * groups, dtype=torch.int32, device=device)   # of the one-token kernel, left zero by it
+        self.k = zeros((num_seqs, kv_heads, self.ring_tokens, self.dim_ld), dtype=dtype, device=device)
+        self.v = zeros((num_seqs, kv_heads, self.ring_tokens, self.vdim_ld), dtype=dtype, device=device)
+        self.tickets = zeros((num_seqs * kv_heads * groups,), dtype=torch.int32, device=device)   # of the one-token kernel, left zero by it
 
     def reset(self, slot: int) -> None:
         """Nothing to clear: a row is read only for positions that the sequence itself has written."""
@@ -164,10 +185,10 @@ class RecurrentState:
     (the input of position p in row p % taps)."""
 
     def __init__(self, num_seqs: int, heads: int, vdim: int, state: int, channels: int, taps: int, dtype=torch.bfloat16,
-                 device="cuda"):
+                 device="cuda", zeros=torch.zeros):
         self.num_seqs = num_seqs
-        self.state = torch.zeros((num_seqs, heads, vdim, state), dtype=torch.float32, device=device)
-        self.conv = torch.zeros((num_seqs, taps, channels), dtype=dtype, device=device)
+        self.state = zeros((num_seqs, heads, vdim, state), dtype=torch.float32, device=device)
+        self.conv = zeros((num_seqs, taps, channels), dtype=dtype, device=device)
 
     def reset(self, slot: int) -> None:
         self.state[slot].zero_()

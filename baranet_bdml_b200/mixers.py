@@ -53,9 +53,9 @@ class LatentAttention:
         self.freq = ops.rotation_frequencies(c.rot_dim, c.rope_base)
         self.kv_ld, self.rot_ld = round8(c.kv_rank), round8(c.rot_dim)
 
-    def new_state(self, num_seqs: int) -> LatentRingCache:
+    def new_state(self, num_seqs: int, zeros=torch.zeros) -> LatentRingCache:
         c = self.cfg
-        return LatentRingCache(num_seqs, c.window, c.kv_rank, c.rot_dim, self.dtype)
+        return LatentRingCache(num_seqs, c.window, c.kv_rank, c.rot_dim, self.dtype, zeros=zeros)
 
     def _prep(self, proj, B, S, cache, seq_ids, positions, latents, keys, rows_per_seq, row_offset):
         c = self.cfg
@@ -161,9 +161,9 @@ class ChunkedAttention:
         self.score_bound = 1.02 * c.dim * abs(c.scale)          # unit-RMS queries and keys, the keys rounded to bf16
         self.mix = float(weight("vmix").reshape(())) if c.mixes_values else 0.0      # one number
 
-    def new_state(self, num_seqs: int, max_tokens: Optional[int] = None) -> ChunkCache:
+    def new_state(self, num_seqs: int, max_tokens: Optional[int] = None, zeros=torch.zeros) -> ChunkCache:
         c = self.cfg
-        return ChunkCache(num_seqs, c.chunk, c.kv_heads, c.dim, c.vdim, self.dtype, max_tokens, self.head_groups)
+        return ChunkCache(num_seqs, c.chunk, c.kv_heads, c.dim, c.vdim, self.dtype, max_tokens, self.head_groups, zeros=zeros)
 
     def project(self, h: torch.Tensor) -> torch.Tensor:
         return self.proj(h)
@@ -252,9 +252,9 @@ class Mamba2Mixer:
         self.norm = f32("norm", c.inner)
         self.o = ops.Linear(weight("o", width, c.inner), dtype)
 
-    def new_state(self, num_seqs: int) -> RecurrentState:
+    def new_state(self, num_seqs: int, zeros=torch.zeros) -> RecurrentState:
         c = self.cfg
-        return RecurrentState(num_seqs, c.heads, c.vdim, c.state, c.channels, c.taps, self.dtype)
+        return RecurrentState(num_seqs, c.heads, c.vdim, c.state, c.channels, c.taps, self.dtype, zeros=zeros)
 
     def __call__(self, h: torch.Tensor, B: int, S: int, st: RecurrentState, seq_ids, positions, n_old: Optional[int]):
         c, dev, dt_code, lib, s = self.cfg, h.device, _dt(self.dtype), _lib.load(), _stream()

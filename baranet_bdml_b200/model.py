@@ -138,36 +138,64 @@ class SequenceLM(CausalLM):
     def extend(self, ids: torch.Tensor, slots: Sequence[int], want: Optional[torch.Tensor] = None) -> torch.Tensor:
         """The next S tokens of the sequences in `slots`, which all have seen equally many: ids (B, S) int32.  Returns the
         fp32 logits of the rows `want` (indices into the B * S rows; None: the last row of every sequence)."""
+        return self._extend(ids, list(slots), want, None)
+
+    def _extend(self, ids: torch.Tensor, slots: List[int], want: Optional[torch.Tensor], n_old: Optional[int]) -> torch.Tensor:
+        """`n_old`: how many tokens every one of them has, where the host knows; None: read from the GPU.  The token ids'
+        check, a synchronisation, comes last, so that the host is not waited for in between."""
         B, S = ids.shape
         flat = ids.reshape(-1).to(torch.int32).contiguous()
-        seq_ids = torch.tensor(list(slots), dtype=torch.int32, device="cuda")
-        positions = self.seq_lens.index_select(0, seq_ids)
-        seen = set(positions.tolist())
-        if len(seen) != 1:
-            raise RuntimeError("extend: the sequences of a portion must have equal lengths")
-        n_old = seen.pop()
+        whole = slots == list(range(B)) and B <= self.slots.num_seqs
+        if whole:
+            seq_ids, lens = self._all_slots[:B], self.seq_lens[:B]
+            positions = lens.clone()
+        else:
+            seq_ids = torch.tensor(slots, dtype=torch.int32, device="cuda")
+            positions = self.seq_lens.index_select(0, seq_ids)
+        if n_old is None:
+            seen = set(positions.tolist())
+            if len(seen) != 1:
+                raise RuntimeError("extend: the sequences of a portion must have equal lengths")
+            n_old = seen.pop()
         if self.max_tokens is not None and n_old + S > self.max_tokens:
             raise RuntimeError(f"extend: {n_old + S} tokens in a sequence; the caches were allocated for {self.max_tokens}")
+
+        def advance(n):
+            if whole:
+                lens.add_(n)
+            else:
+                self.seq_lens.index_add_(0, seq_ids, torch.full_like(seq_ids, n))
+
         state = self._forward(flat, B, S, seq_ids, positions, None if S == 1 else n_old)
-        self._check_ids()
-        self.seq_lens.index_add_(0, seq_ids, torch.full_like(seq_ids, S))
-        if want is None:
-            want = torch.arange(B, device="cuda") * S + S - 1
-        if want.numel() == 0:
-            return torch.empty((0, self.config.vocab_size), dtype=torch.float32, device="cuda")
-        if want.numel() != B * S or S > 1:
-            state = self._select(state, want)
-        return self._logits(state)
+        advance(S)
+        if want is None and S > 1:
+            want = torch.arange(S - 1, B * S, S, device="cuda")
+        if want is not None and want.numel() == 0:
+            logits = torch.empty((0, self.config.vocab_size), dtype=torch.float32, device="cuda")
+        else:
+            if want is not None and (want.numel() != B * S or S > 1):
+                state = self._select(state, want)
+            logits = self._logits(state)
+        try:
+            self._check_ids()
+        except IndexError:
+            advance(-S)
+            raise
+        return logits
 
     def prefill(self, input_ids, max_len: int) -> torch.Tensor:
         """Prompts, (B, S) ids or a list of id lists of any lengths -> logits of each one's last position, (B, vocab)."""
+        as_ids = lambda p: torch.as_tensor(p).to(device="cuda", dtype=torch.int32)     # noqa: E731
+        if isinstance(input_ids, torch.Tensor) and input_ids.dim() == 2 and input_ids.shape[0] > 0:
+            B, S = input_ids.shape
+            self.allocate(B, max(max_len, S))
+            return self._extend(as_ids(input_ids), [self.slots.acquire() for _ in range(B)], None, 0)
         prompts = list(input_ids)
         self.allocate(len(prompts), max(max_len, max(len(p) for p in prompts)))
         slots = [self.slots.acquire() for _ in prompts]
-        as_ids = lambda p: torch.as_tensor(p).to(device="cuda", dtype=torch.int32)     # noqa: E731
         if len({len(p) for p in prompts}) == 1:
-            return self.extend(torch.stack([as_ids(p) for p in prompts]), slots)
-        return torch.cat([self.extend(as_ids(p)[None], [s]) for p, s in zip(prompts, slots)])
+            return self._extend(torch.stack([as_ids(p) for p in prompts]), slots, None, 0)
+        return torch.cat([self._extend(as_ids(p)[None], [s], None, 0) for p, s in zip(prompts, slots)])
 
     def decode_step(self, token_ids: torch.Tensor, check: bool = True, slots: Optional[Sequence[int]] = None) -> torch.Tensor:
         """One new token for the sequences in `slots` (None: the first B slots), whatever their lengths."""
@@ -207,13 +235,14 @@ class LLaMAModelBF16(CausalLM):
         self.caches: Optional[List[PagedKVCache]] = None
 
     # ------------------------------------------------------------------ pieces
-    def embed(self, input_ids: torch.Tensor, check: bool = True) -> torch.Tensor:
+    def embed(self, input_ids: torch.Tensor, check: bool = True, error: Optional[torch.Tensor] = None) -> torch.Tensor:
         """(n,) int32 token ids on the device -> (n, hidden) bf16 (gather on the device).  `check=False` skips the
-        host read of the out-of-range flag (a synchronisation), for use inside a CUDA graph."""
+        host read of the out-of-range flag (a synchronisation), for use inside a CUDA graph, or where the caller reads
+        the flag, a zeroed int32 `error` of its own, later."""
         ids = input_ids.to(torch.int32).contiguous()
         n, H = ids.numel(), self.config.hidden_size
         out = torch.empty((n, H), dtype=torch.float32, device="cuda")
-        err = torch.zeros(1, dtype=torch.int32, device="cuda")
+        err = torch.zeros(1, dtype=torch.int32, device="cuda") if error is None else error
         _lib.check(_lib.load().bn_embedding_gather_f32(self.embed_tokens.data_ptr(), H, ids.data_ptr(), out.data_ptr(), H,
                                                        n, H, self.config.vocab_size, err.data_ptr(),
                                                        torch.cuda.current_stream().cuda_stream))
@@ -240,13 +269,14 @@ class LLaMAModelBF16(CausalLM):
     def _alloc_caches(self, B: int, max_len: int):
         cfg = self.config
         pages_per_seq = (max_len + PAGE_TOKENS - 1) // PAGE_TOKENS
-        self.caches = []
-        for _ in self.layers:
-            c = PagedKVCache(B * pages_per_seq, B, pages_per_seq, cfg.num_key_value_heads, cfg.head_dim, cfg.rope_theta)
-            c.page_table.copy_(torch.arange(B * pages_per_seq, dtype=torch.int32, device="cuda").view(B, pages_per_seq))
-            if self.caches:
-                c.seq_lens = self.caches[0].seq_lens      # every block holds the same tokens: ONE length vector, advanced once per step
-            self.caches.append(c)
+        # every block holds the same tokens: ONE length vector, advanced once per step; pools and page tables are parts of one
+        # tensor each, so that they are filled by one launch
+        n, pages = len(self.layers), B * pages_per_seq
+        pools = torch.zeros((n, pages, cfg.num_key_value_heads, 2, PAGE_TOKENS, cfg.head_dim), dtype=torch.bfloat16, device="cuda")
+        tables = torch.arange(pages, dtype=torch.int32, device="cuda").view(B, pages_per_seq).repeat(n, 1, 1)
+        lens = torch.zeros((B,), dtype=torch.int32, device="cuda")
+        self.caches = [PagedKVCache(pages, B, pages_per_seq, cfg.num_key_value_heads, cfg.head_dim, cfg.rope_theta,
+                                    storage=(pools[i], tables[i], lens)) for i in range(n)]
         self.seq_lens = self.caches[0].seq_lens
 
     def prefill(self, input_ids: torch.Tensor, max_len: int) -> torch.Tensor:
@@ -254,7 +284,8 @@ class LLaMAModelBF16(CausalLM):
         cfg = self.config
         B, S = input_ids.shape
         self._alloc_caches(B, max_len)
-        h = self.embed(input_ids.reshape(-1)).view(B, S, -1)
+        id_error = torch.zeros(1, dtype=torch.int32, device="cuda")
+        h = self.embed(input_ids.reshape(-1), check=False, error=id_error).view(B, S, -1)
         pending = None
         H = cfg.hidden_size
         # one scratch buffer for all blocks (they run one after the other): cos/sin table written once
@@ -271,7 +302,11 @@ class LLaMAModelBF16(CausalLM):
             residual, normed = ops.add_rmsnorm_bf16(residual, o, layer.post_attention_layernorm_weight, layer.eps)
             h, pending = residual.view(B, S, H), layer.mlp(normed).view(B, S, H)
         self.seq_lens.fill_(S)
-        return self._logits(h[:, -1].contiguous(), pending[:, -1].contiguous())
+        logits = self._logits(h[:, -1].contiguous(), pending[:, -1].contiguous())
+        if int(id_error.item()) != 0:             # read last, so that the host is not waited for in between
+            self.seq_lens.zero_()
+            raise IndexError("token id out of range")
+        return logits
 
     def decode_step(self, token_ids: torch.Tensor, check: bool = True) -> torch.Tensor:
         """One new token per sequence: (B,) ids -> (B, vocab) logits; appends to the caches."""

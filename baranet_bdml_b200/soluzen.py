@@ -13,6 +13,7 @@ import torch
 
 from . import ops
 from .checkpoint import Weights
+from .kv_cache import ZeroedTogether
 from .mixers import GatedMLP, LatentAttention, LatentAttentionConfig, Mamba2Config, Mamba2Mixer, TokenSide
 from .model import SequenceLM
 from .ops import Pending, round8
@@ -134,7 +135,10 @@ class SoluzenModel(SequenceLM):
     # ------------------------------------------------------------------ sequences
     def new_states(self, num_seqs: int, max_tokens: Optional[int]):
         """One per layer run, so each pass of the loop has its own; their size does not depend on a sequence's length."""
-        return [self.layers[i].mixer.new_state(num_seqs) for i, _ in self.runs]
+        zeros = ZeroedTogether()
+        states = [self.layers[i].mixer.new_state(num_seqs, zeros) for i, _ in self.runs]
+        zeros.fill()
+        return states
 
     # -------------------------------------------------------------------- forward
     def _embed(self, ids: torch.Tensor):
