@@ -28,6 +28,7 @@ SIGNATURES = {
     "bn_mm_f32": (_i, [_p, _i64, _i64, _p, _i64, _i64, _p, _i64, _i64, _i, _i, _i, _p]),
     "bn_split_f32": (_i, [_p, _i64, _p, _i, _i, _p]),
     "bn_mm_f32_split": (_i, [_p, _p, _i, _p, _i64, _p, _i64, _p, _i, _p, _i, _i, _i, _p, _p]),
+    "bn_mm_f32_each": (_i, [_p, _i64, _i64, _i, _p, _p, _p, _p, _p, _p, _i, _i, _p, _p]),
     "bn_mm_f32_split_pays": (_i, [_i, _i, _i, _i]),
     "bn_rope_f32": (_i, [_p, _i64, _i64, _p, _i64, _i64, _i, _i, _i, _f, _i, _p]),
     "bn_embedding_gather_f32": (_i, [_p, _i64, _p, _p, _i64, _i, _i, _i, _p, _p]),

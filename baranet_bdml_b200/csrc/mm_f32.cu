@@ -18,25 +18,37 @@ namespace bn {
 // ---------------------------------------------------------------------------
 constexpr int MM_K = 16, MM_LD = MM_K + 4, MM_STAGES = 4;
 
-struct MmParams {
-    const float *A, *B;
+// Up to three products of one A in a launch (q, k and v of the attention layer: the two narrow ones alone leave most of the chip
+// idle for as long as a chain takes): set s has the tile columns up to tile_end[s].
+constexpr int MM_SETS = 3;
+struct MmSet {
+    const float* B;
     float* C;
-    int64_t a_rs, a_cs, b_rs, b_cs, c_rs, c_cs;
-    int M, K, N;
+    int64_t b_rs, b_cs, c_rs, c_cs;
+    int N;
+};
+struct MmParams {
+    const float* A;
+    int64_t a_rs, a_cs;
+    int M, K, sets;
+    MmSet set[MM_SETS];
+    int tile_end[MM_SETS];
 };
 
 // VA / VB: 16-byte copies along the operand's contiguous dimension (K for A; K for B, or N with B_N).  B_N: B lies in shared
 // memory with N contiguous.
 template <int BM, int BN, int TM, int TN, bool VA, bool VB, bool B_N>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN))
-mm_f32_kernel(const MmParams p) {
+mm_f32_kernel(const __grid_constant__ MmParams p) {
     constexpr int THREADS = (BM / TM) * (BN / TN), ROWS_T = BM / TM, COLS_T = BN / TN;
     constexpr int A_FLOATS = BM * MM_LD, B_FLOATS = B_N ? MM_K * BN : BN * MM_LD, STAGE = A_FLOATS + B_FLOATS;
     constexpr bool B_N4 = B_N && TN % 4 == 0;              // a thread's columns in groups of four neighbours
     extern __shared__ __align__(16) float mm_smem[];
     const uint32_t smem = ptx::smem_u32(mm_smem);
     const int tid = threadIdx.x, tx = tid % COLS_T, ty = tid / COLS_T;
-    const int row0 = blockIdx.y * BM, col0 = blockIdx.x * BN;
+    const int tile = blockIdx.x, s = (tile >= p.tile_end[0]) + (tile >= p.tile_end[1]);
+    const MmSet& q = p.set[s];
+    const int row0 = blockIdx.y * BM, col0 = (tile - (s ? p.tile_end[s - 1] : 0)) * BN;
     const int steps = (p.K + MM_K - 1) / MM_K;
 
     // What lies outside the operands becomes zero: a chain's last links then add 0 * 0.  16-byte copies go from a source of the
@@ -59,12 +71,12 @@ mm_f32_kernel(const MmParams p) {
         for (int i = 0; i < NB; ++i) {
             const int e = tid + i * THREADS, c = B_N ? e % (BN / 4) * 4 : e / (MM_K / 4), k = B_N ? e / (BN / 4) : e % (MM_K / 4) * 4;
             const bool mine = e < BN * (MM_K / 4);
-            src_b[i] = mine && col0 + c < p.N ? p.B + (B_N ? k * p.b_rs + col0 + c : (col0 + c) * p.b_cs + k) : nullptr;
+            src_b[i] = mine && col0 + c < q.N ? q.B + (B_N ? k * q.b_rs + col0 + c : (col0 + c) * q.b_cs + k) : nullptr;
             dst_b[i] = mine ? smem + (A_FLOATS + (B_N ? k * BN + c : c * MM_LD + k)) * 4 : 0;
             k_b[i] = k;
         }
     }
-    const int64_t advance_b = B_N ? MM_K * p.b_rs : MM_K;
+    const int64_t advance_b = B_N ? MM_K * q.b_rs : MM_K;
     auto stage_in = [&](int step) {
         const uint32_t at = (step % MM_STAGES) * (STAGE * 4);
         const int k0 = step * MM_K;
@@ -88,14 +100,14 @@ mm_f32_kernel(const MmParams p) {
             for (int i = 0; i < NB; ++i)
                 if ((BN * (MM_K / 4)) % THREADS == 0 || dst_b[i]) {
                     const bool in = src_b[i] && k0 + k_b[i] < p.K;
-                    ptx::cp_async_16(dst_b[i] + at, in ? src_b[i] : p.B, in ? 16 : 0);
+                    ptx::cp_async_16(dst_b[i] + at, in ? src_b[i] : q.B, in ? 16 : 0);
                     if (src_b[i]) src_b[i] += advance_b;
                 }
         } else {
             for (int e = tid; e < BN * MM_K; e += THREADS) {
                 const int c = e / MM_K, k = e % MM_K;
-                const bool in = col0 + c < p.N && k0 + k < p.K;
-                ptx::cp_async_4(smem + at + (A_FLOATS + c * MM_LD + k) * 4, p.B + (in ? (k0 + k) * p.b_rs + (col0 + c) * p.b_cs : 0),
+                const bool in = col0 + c < q.N && k0 + k < p.K;
+                ptx::cp_async_4(smem + at + (A_FLOATS + c * MM_LD + k) * 4, q.B + (in ? (k0 + k) * q.b_rs + (col0 + c) * q.b_cs : 0),
                                 in ? 4 : 0);
             }
         }
@@ -170,16 +182,17 @@ mm_f32_kernel(const MmParams p) {
 #pragma unroll
         for (int j = 0; j < TN; ++j) {
             const int c = col0 + (B_N4 ? (tx + j / 4 * COLS_T) * 4 + j % 4 : tx + j * COLS_T);
-            if (c < p.N) p.C[r * p.c_rs + c * p.c_cs] = acc[i][j];
+            if (c < q.N) q.C[r * q.c_rs + c * q.c_cs] = acc[i][j];
         }
     }
 }
 
 template <int BM, int BN, int TM, int TN, bool VA, bool VB, bool B_N>
-static int mm_f32_run(const MmParams& p, cudaStream_t st) {
+static int mm_f32_run(MmParams p, cudaStream_t st) {
     constexpr size_t smem = (size_t)MM_STAGES * (BM * MM_LD + (B_N ? MM_K * BN : BN * MM_LD)) * sizeof(float);
     if (int rc = allow_smem(mm_f32_kernel<BM, BN, TM, TN, VA, VB, B_N>, smem, "bn_mm_f32")) return rc;
-    const dim3 grid(ceil_div(p.N, BN), ceil_div(p.M, BM));
+    for (int s = 0; s < MM_SETS; ++s) p.tile_end[s] = (s ? p.tile_end[s - 1] : 0) + (s < p.sets ? ceil_div(p.set[s].N, BN) : 0);
+    const dim3 grid(p.tile_end[MM_SETS - 1], ceil_div(p.M, BM));
     if (grid.y > 65535) return fail(BN_ERR_UNSUPPORTED, "bn_mm_f32: M=%d too large", p.M);
     mm_f32_kernel<BM, BN, TM, TN, VA, VB, B_N><<<grid, (BM / TM) * (BN / TN), smem, st>>>(p);
     return launch_status("bn_mm_f32");
@@ -192,8 +205,13 @@ static int mm_f32_copies(const MmParams& p, cudaStream_t st) {
         return contiguous == 1 && other % 4 == 0 && n % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
     };
     const bool va = fours(p.A, p.a_cs, p.a_rs, p.K);
-    if (va && fours(p.B, p.b_cs, p.b_rs, p.N)) return mm_f32_run<BM, BN, TM, TN, true, true, true>(p, st);
-    if (va && fours(p.B, p.b_rs, p.b_cs, p.K)) return mm_f32_run<BM, BN, TM, TN, true, true, false>(p, st);
+    bool along_n = va, along_k = va;                       // every set's B
+    for (int s = 0; s < p.sets; ++s) {
+        along_n = along_n && fours(p.set[s].B, p.set[s].b_cs, p.set[s].b_rs, p.set[s].N);
+        along_k = along_k && fours(p.set[s].B, p.set[s].b_rs, p.set[s].b_cs, p.K);
+    }
+    if (along_n) return mm_f32_run<BM, BN, TM, TN, true, true, true>(p, st);
+    if (along_k) return mm_f32_run<BM, BN, TM, TN, true, true, false>(p, st);
     return mm_f32_run<BM, BN, TM, TN, false, false, false>(p, st);
 }
 
@@ -203,10 +221,11 @@ static int mm_f32_copies(const MmParams& p, cudaStream_t st) {
 // that reading (8 x 4 outputs a thread: 12 16-byte reads, 4 cycles each, for 128 FMAs), 53 - 60 % of the FMA rate.
 // One 64 x 64 tile of 4 x 4 outputs a thread without copies in flight, before / after: 128 x 2048 x 2048 134 / 52 us,
 // 128 x 256 x 2048 134 / 24 us, 800 x 7424 x 2048 1470 / 610 us, 4 x 32000 x 2048 570 / 88 us.
-static float mm_f32_times(int M, int N, int* best) {
+static float mm_f32_times(int M, const int* N, int sets, int* best) {
     const int sms = sm_count();
     auto estimate = [&](int bm, int bn, float alone, float more) {
-        const long long tiles = (long long)ceil_div(M, bm) * ceil_div(N, bn);
+        long long tiles = 0;
+        for (int s = 0; s < sets; ++s) tiles += (long long)ceil_div(M, bm) * ceil_div(N[s], bn);
         if (ceil_div(M, bm) > 65535 && bm < 128) return INFINITY;        // the grid's limit
         return fmaxf(alone, (float)((tiles + sms - 1) / sms) * more);
     };
@@ -219,8 +238,9 @@ static float mm_f32_times(int M, int N, int* best) {
 }
 
 static int mm_f32_pick(const MmParams& p, cudaStream_t st) {
-    int best;
-    mm_f32_times(p.M, p.N, &best);
+    int best, n[MM_SETS];
+    for (int s = 0; s < p.sets; ++s) n[s] = p.set[s].N;
+    mm_f32_times(p.M, n, p.sets, &best);
     switch (best) {
         case 0: return mm_f32_copies<128, 128, 8, 8>(p, st);
         case 1: return mm_f32_copies<64, 64, 8, 4>(p, st);
@@ -232,7 +252,7 @@ static int mm_f32_pick(const MmParams& p, cudaStream_t st) {
 
 float mm_f32_estimate(int M, int N, int K) {
     int best;
-    return mm_f32_times(M, N, &best) * (float)K / 2048.f;
+    return mm_f32_times(M, &N, 1, &best) * (float)K / 2048.f;
 }
 
 // x = act(x + bias) in place, fp32 rows (the unfused form of the products with a bias or an activation)
@@ -254,7 +274,24 @@ extern "C" int bn_mm_f32(const float* A, int64_t a_rs, int64_t a_cs, const float
     if (M < 0 || K < 0 || N < 0) return fail(BN_ERR_INVALID_ARG, "bn_mm_f32: negative size");
     if (int rc = require_sm100()) return rc;
     if (M == 0 || N == 0) return BN_OK;
-    return mm_f32_pick(MmParams{A, B, C, a_rs, a_cs, b_rs, b_cs, c_rs, c_cs, M, K, N}, as_stream(stream));
+    MmParams p{A, a_rs, a_cs, M, K, 1, {{B, C, b_rs, b_cs, c_rs, c_cs, N}}, {}};
+    return mm_f32_pick(p, as_stream(stream));
+}
+
+extern "C" int bn_mm_f32_each(const float* A, int64_t a_rs, int64_t a_cs, int n, const float* const* B, const int64_t* b_rs,
+                              const int64_t* b_cs, float* const* C, const int64_t* c_rs, const int64_t* c_cs, int M, int K, const int* N,
+                              bn_stream_t stream) {
+    const char* what = "bn_mm_f32_each";
+    if (!A || !B || !b_rs || !b_cs || !C || !c_rs || !c_cs || !N) return fail(BN_ERR_INVALID_ARG, "%s: null pointer", what);
+    if (n < 0 || n > MM_SETS || M < 0 || K < 0) return fail(BN_ERR_INVALID_ARG, "%s: bad shape n=%d M=%d K=%d", what, n, M, K);
+    MmParams p{A, a_rs, a_cs, M, K, 0, {}, {}};
+    for (int s = 0; s < n; ++s) {
+        if (!B[s] || !C[s] || N[s] < 0) return fail(BN_ERR_INVALID_ARG, "%s: product %d", what, s);
+        if (N[s] > 0) p.set[p.sets++] = MmSet{B[s], C[s], b_rs[s], b_cs[s], c_rs[s], c_cs[s], N[s]};
+    }
+    if (int rc = require_sm100()) return rc;
+    if (M == 0 || p.sets == 0) return BN_OK;
+    return mm_f32_pick(p, as_stream(stream));
 }
 
 extern "C" int bn_bias_act_f32(float* x, int64_t ld, const float* bias, int rows, int cols, int act, bn_stream_t stream) {

@@ -118,9 +118,7 @@ class GroupedQueryAttention:
         return AGTensor(w, requires_grad=True, is_cuda=self.is_cuda)
 
     def __call__(self, hidden_states: AGTensor, position_offset: int = 0, use_causal_mask: bool = True) -> AGTensor:
-        query = hidden_states @ self.q_proj
-        key = hidden_states @ self.k_proj
-        value = hidden_states @ self.v_proj
+        query, key, value = hidden_states.matmul_each([self.q_proj, self.k_proj, self.v_proj])
         mode = _lib.BN_HEADS_COLLAPSED if self.heads_mode == "collapsed" else _lib.BN_HEADS_PER_HEAD
         attn = query.data.attention_fused(
             key.data, value.data, float(self.scale), causal=use_causal_mask, seq_offset=position_offset,

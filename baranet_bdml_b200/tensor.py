@@ -20,6 +20,7 @@ src/ops/op_mm_optimized.cuh:78-80).
 """
 from __future__ import annotations
 
+import ctypes as C
 from typing import Optional, Tuple, Union
 
 import numpy as np
@@ -143,6 +144,22 @@ class TensorF:
                                  other.stride_w, out._ptr(), out.stride_h, out.stride_w, self.h, self.w, other.w,
                                  _stream_ptr()))
         return out
+
+    def matmul_each(self, others) -> list:
+        """[self @ o for o in others], at most three, in one launch -> bn_mm_f32_each."""
+        for o in others:
+            if self.w != o.h:
+                raise RuntimeError(f"a,b,out tensor shape mismatch a:{self!r}, b:{o!r}")
+        for t in (self, *others):
+            t._require_device("Matrix multiply")
+        outs, n = [TensorF(self.h, o.w, True) for o in others], len(others)
+        array = lambda kind, values: (kind * n)(*values)                                      # noqa: E731
+        _lib.check(_lib.load().bn_mm_f32_each(
+            self._ptr(), self.stride_h, self.stride_w, n, array(C.c_void_p, [o._ptr() for o in others]),
+            array(C.c_int64, [o.stride_h for o in others]), array(C.c_int64, [o.stride_w for o in others]),
+            array(C.c_void_p, [o._ptr() for o in outs]), array(C.c_int64, [o.stride_h for o in outs]),
+            array(C.c_int64, [o.stride_w for o in outs]), self.h, self.w, array(C.c_int, [o.w for o in others]), _stream_ptr()))
+        return outs
 
     def rope(self, position_offset: int = 0, head_dim: int = 64, theta: float = 10000.0) -> "TensorF":
         """op_rope (src/ops/op_rope.cuh:101-126) -> bn_rope_f32."""
@@ -285,6 +302,10 @@ class AGTensor:
 
     def __matmul__(self, other: "AGTensor") -> "AGTensor":
         return AGTensor(self.data @ other.data, (self, other), "@", requires_grad=False)
+
+    def matmul_each(self, others) -> list:
+        """[self @ o for o in others], at most three, in one launch"""
+        return [AGTensor(d, (self, o), "@", requires_grad=False) for d, o in zip(self.data.matmul_each([o.data for o in others]), others)]
 
     def rope(self, position_offset: int = 0, head_dim: int = 64, theta: float = 10000.0) -> "AGTensor":
         return AGTensor(self.data.rope(position_offset, head_dim, theta), (self,), "rope", requires_grad=False)

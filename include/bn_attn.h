@@ -99,6 +99,11 @@ BN_API int bn_selftest_wait_timeout(void* workspace, unsigned limit_us, bn_strea
 BN_API int bn_mm_f32(const float* A, int64_t a_rs, int64_t a_cs, const float* B, int64_t b_rs, int64_t b_cs,
               float* C, int64_t c_rs, int64_t c_cs, int M, int K, int N, bn_stream_t stream);
 
+/* n (at most 3) products of one A, the same chains, in one launch: C[i](M,N[i]) = A(M,K) @ B[i](K,N[i]). */
+BN_API int bn_mm_f32_each(const float* A, int64_t a_rs, int64_t a_cs, int n, const float* const* B, const int64_t* b_rs,
+                          const int64_t* b_cs, float* const* C, const int64_t* c_rs, const int64_t* c_cs, int M, int K, const int* N,
+                          bn_stream_t stream);
+
 /* The products of many rows on the tensor cores, with the precision of an fp32 sum: C(M,N) = act(A(M,K) W(N,K)^T + bias),
  * fp32, from the bf16 parts of both operands.
  * bn_split_f32 writes x (rows, cols) as three bf16 matrices [3][rows][cols] whose sum it is; cols a multiple of 8, 16-byte

@@ -124,6 +124,24 @@ def test_mm_of_bf16_parts(lib, M, K, N, parts):
     assert int(word.item()) == 0
 
 
+@pytest.mark.parametrize("M,K,widths", [(128, 64, (2048, 256, 256)), (5, 20, (40, 8, 33)), (33, 16, (64, 1, 65)), (70, 36, (100, 260))])
+@pytest.mark.parametrize("transposed", [(), (1,), (0, 1, 2)])
+def test_mm_each_is_the_single_products(T, M, K, widths, transposed):
+    rng = np.random.default_rng(M + K + len(transposed))
+
+    def tensor(h, w):
+        t = T.TensorF(h, w)
+        t.copy_from_numpy(rng.standard_normal((h, w), dtype=np.float32))
+        return t
+
+    x = tensor(M, K)
+    ws = [tensor(n, K).T if i in transposed else tensor(K, n) for i, n in enumerate(widths)]
+    for got, w in zip(x.matmul_each(ws), ws):
+        assert np.array_equal(got.to_numpy(), (x @ w).to_numpy())
+    with pytest.raises(RuntimeError):
+        x.matmul_each([ws[0], tensor(K + 1, 4)])
+
+
 def test_mm_transposed_and_sliced_views(T):
     rng = np.random.default_rng(2)
     a = rng.standard_normal((40, 96), dtype=np.float32)
