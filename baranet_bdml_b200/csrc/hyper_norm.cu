@@ -32,13 +32,19 @@ struct HyperParams {
 };
 
 // NV = float4 pieces per thread: hidden <= 1024 * NV, hidden % 4 == 0, every row start 16-byte (bf16: 8-byte) aligned
-template <typename T, int NV, int NI, int NO>
+// FEW: one row per block (a step), whose weights are asked for in L2 while the kernel ahead finishes and read with the row
+template <typename T, int NV, int NI, int NO, bool FEW>
 __global__ void __launch_bounds__(HY_THREADS)
 hyper_norm_regs_kernel(const __grid_constant__ HyperParams p) {
     __shared__ float sh[HY_THREADS / 32];
-    ptx::grid_launch_dependents();
-    ptx::grid_dependency_wait();
     const int pieces = p.hidden / 4;
+    ptx::grid_launch_dependents();
+    if (FEW)
+        for (int c = threadIdx.x; c < pieces; c += HY_THREADS) {
+            if (p.delta_scale) ptx::prefetch_l2(p.delta_scale + 4 * c);
+            if (p.w) ptx::prefetch_l2(p.w + 4 * c);
+        }
+    ptx::grid_dependency_wait();
     const float inv_n = 1.f / (float)p.hidden;
     for (int r = blockIdx.x; r < p.rows; r += gridDim.x) {
         float xv[NV][NI][4], d[NV][4];
@@ -54,6 +60,14 @@ hyper_norm_regs_kernel(const __grid_constant__ HyperParams p) {
 #pragma unroll
                 for (int s = 0; s < NI; ++s) load4(xr + (int64_t)s * p.hidden + 4 * c, xv[k][s]);
                 if (p.delta) load4(dr + 4 * c, d[k]);
+            }
+        }
+        float early[FEW ? NV : 1][4];                      // the norm's weight
+        if (FEW && p.w) {
+#pragma unroll
+            for (int k = 0; k < NV; ++k) {
+                const int c = threadIdx.x + k * HY_THREADS;
+                if (c < pieces) load4(p.w + 4 * c, early[FEW ? k : 0]);
             }
         }
         float u[NV][4], ss = 0.f;
@@ -90,7 +104,12 @@ hyper_norm_regs_kernel(const __grid_constant__ HyperParams p) {
             const int c = threadIdx.x + k * HY_THREADS;
             if (c < pieces) {
                 float w4[4], o4[4];
-                load4(p.w + 4 * c, w4);
+                if (FEW) {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) w4[e] = early[FEW ? k : 0][e];
+                } else {
+                    load4(p.w + 4 * c, w4);
+                }
 #pragma unroll
                 for (int e = 0; e < 4; ++e) o4[e] = u[k][e] * inv * w4[e];
                 store4(yr + 4 * c, o4);
@@ -133,25 +152,27 @@ hyper_norm_any_kernel(const __grid_constant__ HyperParams p) {
     }
 }
 
-template <int NV, int NI, int NO>
+template <typename T, int NV, int NI, int NO>
 static void hyper_launch(unsigned grid, cudaStream_t st, const HyperParams& p) {
-    launch_dependent(hyper_norm_regs_kernel<__nv_bfloat16, NV, NI, NO>, grid, HY_THREADS, 0, st, p);
+    constexpr bool SHORT = NV <= 2;
+    if (SHORT && p.rows <= 2 * sm_count()) launch_dependent(hyper_norm_regs_kernel<T, NV, NI, NO, SHORT>, grid, HY_THREADS, 0, st, p);
+    else launch_dependent(hyper_norm_regs_kernel<T, NV, NI, NO, false>, grid, HY_THREADS, 0, st, p);
 }
 
 // the stream counts that have a register form; false: none
-template <int NV>
+template <typename T, int NV>
 static bool hyper_regs(unsigned grid, cudaStream_t st, const HyperParams& p) {
     switch (p.n_in * 8 + p.n_out) {
-        case 1 * 8 + 1: hyper_launch<NV, 1, 1>(grid, st, p); return true;
-        case 1 * 8 + 2: hyper_launch<NV, 1, 2>(grid, st, p); return true;
-        case 1 * 8 + 3: hyper_launch<NV, 1, 3>(grid, st, p); return true;
-        case 1 * 8 + 4: hyper_launch<NV, 1, 4>(grid, st, p); return true;
-        case 2 * 8 + 1: hyper_launch<NV, 2, 1>(grid, st, p); return true;
-        case 2 * 8 + 2: hyper_launch<NV, 2, 2>(grid, st, p); return true;
-        case 3 * 8 + 1: hyper_launch<NV, 3, 1>(grid, st, p); return true;
-        case 3 * 8 + 3: hyper_launch<NV, 3, 3>(grid, st, p); return true;
-        case 4 * 8 + 1: hyper_launch<NV, 4, 1>(grid, st, p); return true;
-        case 4 * 8 + 4: hyper_launch<NV, 4, 4>(grid, st, p); return true;
+        case 1 * 8 + 1: hyper_launch<T, NV, 1, 1>(grid, st, p); return true;
+        case 1 * 8 + 2: hyper_launch<T, NV, 1, 2>(grid, st, p); return true;
+        case 1 * 8 + 3: hyper_launch<T, NV, 1, 3>(grid, st, p); return true;
+        case 1 * 8 + 4: hyper_launch<T, NV, 1, 4>(grid, st, p); return true;
+        case 2 * 8 + 1: hyper_launch<T, NV, 2, 1>(grid, st, p); return true;
+        case 2 * 8 + 2: hyper_launch<T, NV, 2, 2>(grid, st, p); return true;
+        case 3 * 8 + 1: hyper_launch<T, NV, 3, 1>(grid, st, p); return true;
+        case 3 * 8 + 3: hyper_launch<T, NV, 3, 3>(grid, st, p); return true;
+        case 4 * 8 + 1: hyper_launch<T, NV, 4, 1>(grid, st, p); return true;
+        case 4 * 8 + 4: hyper_launch<T, NV, 4, 4>(grid, st, p); return true;
     }
     return false;
 }
@@ -196,11 +217,14 @@ extern "C" int bn_hyper_norm(const float* x, int n_in, int n_out, const float* m
     const unsigned grid = (unsigned)(rows < cap ? rows : cap);
     const uintptr_t all = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(delta) | reinterpret_cast<uintptr_t>(delta_scale) |
                           reinterpret_cast<uintptr_t>(x_out) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y);
-    const bool vec = dtype == 1 && hidden % 4 == 0 && hidden <= 4096 && delta_ld % 4 == 0 && y_ld % 4 == 0 && (all & 15) == 0 &&
+    const bool vec = hidden % 4 == 0 && hidden <= 4096 && delta_ld % 4 == 0 && y_ld % 4 == 0 && (all & 15) == 0 &&
                      n_in <= 4 && n_out <= 4;
     cudaStream_t st = as_stream(stream);
-    if (vec && hidden <= 1024 && hyper_regs<1>(grid, st, p)) return launch_status(what);
-    if (vec && hidden > 1024 && hidden <= 2048 && hyper_regs<2>(grid, st, p)) return launch_status(what);
-    if (vec && hidden > 2048 && hyper_regs<4>(grid, st, p)) return launch_status(what);
+    auto regs = [&](auto zero) {
+        using T = decltype(zero);
+        return hidden <= 1024 ? hyper_regs<T, 1>(grid, st, p) : hidden <= 2048 ? hyper_regs<T, 2>(grid, st, p) : hyper_regs<T, 4>(grid, st, p);
+    };
+    // fp32, 800 rows of 2 x 2048: 17 us by the form for any sizes, 8 by this one
+    if (vec && (dtype == 0 ? regs(0.f) : regs(__nv_bfloat16{}))) return launch_status(what);
     return dtype == 0 ? hyper_any<float>(grid, st, p) : hyper_any<__nv_bfloat16>(grid, st, p);
 }

@@ -143,6 +143,8 @@ latent_prep_regs_kernel(const LatentPrepParams p) {
     __shared__ float sh[2][LP_THREADS / 32];
     const int tid = threadIdx.x;
     const double freq = 2 * tid < p.rot ? p.freq[tid] : 0.0;
+    for (int i = tid * 4; i < p.q_rank; i += LP_THREADS * 4) ptx::prefetch_l2(p.q_norm + i);
+    for (int i = tid * 4; i < p.kv_rank; i += LP_THREADS * 4) ptx::prefetch_l2(p.kv_norm + i);
     ptx::grid_dependency_wait();
     ptx::grid_launch_dependents();
     for (int r = blockIdx.x; r < p.rows; r += gridDim.x) {

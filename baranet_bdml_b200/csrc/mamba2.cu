@@ -257,12 +257,21 @@ template <typename T, int R, int VEC, int TAPS>
 __global__ void __launch_bounds__(ST_WARPS * 32)
 mamba2_step_kernel(const StepParams p) {
     extern __shared__ float sm[];                      // B [N], C [N], x [p_per_block], silu(z) [p_per_block]
-    ptx::grid_dependency_wait();
-    ptx::grid_launch_dependents();
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const int p_tiles = (p.P + p.p_per_block - 1) / p.p_per_block;
     const int pt = blockIdx.x % p_tiles, h = (blockIdx.x / p_tiles) % p.H, b = blockIdx.x / (p_tiles * p.H);
-    const int g = h / (p.H / p.G), slot = p.seq_ids ? p.seq_ids[b] : b, pos = p.positions[b];
+    const int g = h / (p.H / p.G);
+    // the convolution's weights in L2 while the kernel ahead finishes: this block's x channels, its group's B and C
+    if (TAPS == 4)
+        for (int i = threadIdx.x; i < 2 * p.N + min(p.p_per_block, p.P - pt * p.p_per_block); i += ST_WARPS * 32) {
+            const int c = i < p.N ? p.H * p.P + g * p.N + i : i < 2 * p.N ? p.H * p.P + p.G * p.N + g * p.N + (i - p.N)
+                                                                        : h * p.P + pt * p.p_per_block + (i - 2 * p.N);
+            ptx::prefetch_l2(p.conv_w + (int64_t)c * 4);
+            if (i % 32 == 0) ptx::prefetch_l2(p.conv_b + c);
+        }
+    ptx::grid_dependency_wait();
+    ptx::grid_launch_dependents();
+    const int slot = p.seq_ids ? p.seq_ids[b] : b, pos = p.positions[b];
     const int inner = p.H * p.P, GN = p.G * p.N, C = inner + 2 * GN;
     const T* row = static_cast<const T*>(p.proj) + (int64_t)b * p.proj_ld;
     const T* in = row + inner;
@@ -372,32 +381,51 @@ __global__ void __launch_bounds__(GN_THREADS)
 gated_norm_kernel(const GatedNormParams p) {
     extern __shared__ float part_buf[];
     __shared__ float sh[GN_THREADS / 32];
+    constexpr bool STEP = RV && sizeof(TY) > sizeof(T);    // few rows: the weight is read along with them, not behind their sums
+    const int n = p.width / p.groups;
+    if (STEP)
+        for (int i = threadIdx.x * 4; i < p.width; i += GN_THREADS * 4) ptx::prefetch_l2(p.w + i);
     ptx::grid_dependency_wait();
     ptx::grid_launch_dependents();
-    const int n = p.width / p.groups;
     for (long long item = blockIdx.x; item < (long long)p.rows * p.groups; item += gridDim.x) {
         const int64_t r = item / p.groups;
         const int c0 = (int)(item % p.groups) * n;
         const TY* y = static_cast<const TY*>(p.y) + r * p.y_ld + c0;
         const T* z = p.z ? static_cast<const T*>(p.z) + r * p.z_ld + c0 : nullptr;
         float s = 0.f;
-        float v[RV ? RV : 1][4];
+        float v[RV ? RV : 1][4], w[STEP ? RV : 1][4];
         if (RV) {
+            // both operands' loads ahead of the arithmetic (a branch on z around each pair of them left one pair in flight)
+            float g[RV ? RV : 1][4];
 #pragma unroll
             for (int k = 0; k < RV; ++k) {
                 const int i = (threadIdx.x + k * GN_THREADS) * 4;
-                if (i < n) {
-                    load4(y + i, v[k]);
-                    if (z) {
-                        float z4[4];
-                        load4(z + i, z4);
+                v[k][0] = v[k][1] = v[k][2] = v[k][3] = 0.f;
+                if (i < n) load4(y + i, v[k]);
+            }
+            if (STEP) {
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) v[k][e] *= conv_silu_f<T>(z4[e]);
-                    }
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) s = fmaf(v[k][e], v[k][e], s);
+                for (int k = 0; k < RV; ++k) {
+                    const int i = (threadIdx.x + k * GN_THREADS) * 4;
+                    if (i < n) load4(p.w + c0 + i, w[STEP ? k : 0]);
                 }
             }
+            if (z) {
+#pragma unroll
+                for (int k = 0; k < RV; ++k) {
+                    const int i = (threadIdx.x + k * GN_THREADS) * 4;
+                    g[k][0] = g[k][1] = g[k][2] = g[k][3] = 0.f;
+                    if (i < n) load4(z + i, g[k]);
+                }
+#pragma unroll
+                for (int k = 0; k < RV; ++k)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) v[k][e] *= conv_silu_f<T>(g[k][e]);
+            }
+#pragma unroll
+            for (int k = 0; k < RV; ++k)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) s = fmaf(v[k][e], v[k][e], s);
         } else {
             for (int i = threadIdx.x; i < n; i += GN_THREADS) {
                 const float q = to_f(y[i]) * (z ? conv_silu_f<T>(to_f(z[i])) : 1.f);
@@ -412,7 +440,7 @@ gated_norm_kernel(const GatedNormParams p) {
         __syncthreads();
         s = 0.f;
 #pragma unroll
-        for (int w = 0; w < GN_THREADS / 32; ++w) s += sh[w];
+        for (int i = 0; i < GN_THREADS / 32; ++i) s += sh[i];
         const float inv = rsqrtf(s / (float)n + p.eps);
         T* o = static_cast<T*>(p.out) + r * p.out_ld + c0;
         if (RV) {
@@ -421,7 +449,12 @@ gated_norm_kernel(const GatedNormParams p) {
                 const int i = (threadIdx.x + k * GN_THREADS) * 4;
                 if (i < n) {
                     float w4[4], o4[4];
-                    load4(p.w + c0 + i, w4);
+                    if (STEP) {
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) w4[e] = w[STEP ? k : 0][e];
+                    } else {
+                        load4(p.w + c0 + i, w4);
+                    }
 #pragma unroll
                     for (int e = 0; e < 4; ++e) o4[e] = v[k][e] * inv * w4[e];
                     store4(o + i, o4);

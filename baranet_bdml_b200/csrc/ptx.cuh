@@ -180,6 +180,11 @@ __device__ __forceinline__ void tma_load_2d_hint(uint32_t smem_dst, const CUtens
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// asks for the line of an address in L2; null: nothing
+__device__ __forceinline__ void prefetch_l2(const void* p) {
+    if (p) asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+}
+
 // asks for a 2-D tile in L2 (the point of coherence: a tile that is written later is not stale)
 __device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* m, int x, int y) {
     asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"(reinterpret_cast<uint64_t>(m)), "r"(x), "r"(y) : "memory");

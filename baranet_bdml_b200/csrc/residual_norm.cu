@@ -31,13 +31,32 @@ struct ResidualNormParams {
 constexpr int RS_THREADS = 256;
 
 // NV = float4 pieces per thread: hidden <= 1024 * NV, hidden % 4 == 0, every row start 16-byte (T = bf16: 8-byte) aligned
-template <typename T, typename TD, int NV>
+// FEW: a block has one row, so its time is a chain of memory round trips.  The weights are asked for in L2 while the kernel ahead
+// finishes and read along with the row, not behind its sums (a step's weights come from HBM: its norms took 5 us, now 2.8).
+// With many rows the registers are worth more: they hold rows in flight.
+template <typename T, typename TD, int NV, bool FEW>
 __global__ void __launch_bounds__(RS_THREADS)
 residual_norm_regs_kernel(const ResidualNormParams p) {
     __shared__ float sh[RS_THREADS / 32];
+    const int pieces = p.hidden / 4;
+    float early[FEW ? 3 : 1][FEW ? NV : 1][4];             // delta_w, w, b
+    if (FEW)
+        for (int c = threadIdx.x; c < pieces; c += RS_THREADS) {
+            const int at = 4 * c;
+            if (p.delta_w) ptx::prefetch_l2(p.delta_w + at);
+            if (p.w) ptx::prefetch_l2(p.w + at);
+            if (p.b) ptx::prefetch_l2(p.b + at);
+        }
     ptx::grid_dependency_wait();
     ptx::grid_launch_dependents();
-    const int pieces = p.hidden / 4;
+    auto weight = [&](const float* w, int which, int k, int c, float (&w4)[4]) {
+        if (FEW) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) w4[e] = early[FEW ? which : 0][FEW ? k : 0][e];
+        } else {
+            load4(w + 4 * c, w4);
+        }
+    };
     const float inv_n = 1.f / (float)p.hidden;
     for (int r = blockIdx.x; r < p.rows; r += gridDim.x) {
         float v[NV][4];
@@ -60,6 +79,17 @@ residual_norm_regs_kernel(const ResidualNormParams p) {
                 if (c < pieces) load4(xr + 4 * c, xv[k]);
             }
         }
+        if (FEW) {
+#pragma unroll
+            for (int k = 0; k < NV; ++k) {
+                const int c = threadIdx.x + k * RS_THREADS;
+                if (c < pieces) {
+                    if (p.delta_w) load4(p.delta_w + 4 * c, early[0][FEW ? k : 0]);
+                    if (p.w) load4(p.w + 4 * c, early[FEW ? 1 : 0][FEW ? k : 0]);
+                    if (p.b) load4(p.b + 4 * c, early[FEW ? 2 : 0][FEW ? k : 0]);
+                }
+            }
+        }
         if (p.delta_w) {
             float s = 0.f;
 #pragma unroll
@@ -72,7 +102,7 @@ residual_norm_regs_kernel(const ResidualNormParams p) {
                 const int c = threadIdx.x + k * RS_THREADS;
                 if (c < pieces) {
                     float w4[4];
-                    load4(p.delta_w + 4 * c, w4);
+                    weight(p.delta_w, 0, k, c, w4);
 #pragma unroll
                     for (int e = 0; e < 4; ++e) v[k][e] = v[k][e] * inv * w4[e];
                 }
@@ -129,8 +159,8 @@ residual_norm_regs_kernel(const ResidualNormParams p) {
             const int c = threadIdx.x + k * RS_THREADS;
             if (c < pieces) {
                 float w4[4], b4[4] = {0.f, 0.f, 0.f, 0.f}, o4[4];
-                load4(p.w + 4 * c, w4);
-                if (p.b) load4(p.b + 4 * c, b4);
+                weight(p.w, 1, k, c, w4);
+                if (p.b) weight(p.b, 2, k, c, b4);
 #pragma unroll
                 for (int e = 0; e < 4; ++e) o4[e] = fmaf((v[k][e] - mean) * inv, w4[e], b4[e]);
                 store4(yr + 4 * c, o4);
@@ -203,9 +233,10 @@ static int residual_norm_launch(const ResidualNormParams& p, bn_stream_t stream)
     const bool vec = p.hidden % 4 == 0 && p.hidden <= 4096 && p.delta_ld % 4 == 0 && p.cast_ld % 4 == 0 && p.y_ld % 4 == 0 &&
                      p.lo_offset % 4 == 0 && ((f32s | others) & 15) == 0;
     cudaStream_t st = as_stream(stream);
-    if (vec && p.hidden <= 1024) launch_dependent(residual_norm_regs_kernel<T, TD, 1>, grid, RS_THREADS, 0, st, p);
-    else if (vec && p.hidden <= 2048) launch_dependent(residual_norm_regs_kernel<T, TD, 2>, grid, RS_THREADS, 0, st, p);
-    else if (vec) launch_dependent(residual_norm_regs_kernel<T, TD, 4>, grid, RS_THREADS, 0, st, p);
+    const bool few = p.rows <= 2 * sms;
+    if (vec && p.hidden <= 1024) launch_dependent(few ? residual_norm_regs_kernel<T, TD, 1, true> : residual_norm_regs_kernel<T, TD, 1, false>, grid, RS_THREADS, 0, st, p);
+    else if (vec && p.hidden <= 2048) launch_dependent(few ? residual_norm_regs_kernel<T, TD, 2, true> : residual_norm_regs_kernel<T, TD, 2, false>, grid, RS_THREADS, 0, st, p);
+    else if (vec) launch_dependent(residual_norm_regs_kernel<T, TD, 4, false>, grid, RS_THREADS, 0, st, p);
     else {
         const size_t smem = (size_t)p.hidden * sizeof(float);
         if (smem > 200 * 1024) return fail(BN_ERR_UNSUPPORTED, "%s: hidden=%d (at most 51200)", what, p.hidden);

@@ -206,6 +206,8 @@ rmsnorm_bf16_kernel(const RmsBf16Params p) {
     __shared__ float s_part[8];
     const int tid = threadIdx.x, lane = tid % 32, warp = tid / 32;
     const int pieces = p.hidden / 8;
+    // the weight is asked for in L2 meanwhile (a step's comes from HBM) and read along with the row
+    for (int c = tid; c < pieces; c += 256) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.w + c * 8));
     // Launched as a programmatic dependent: nothing is read before the kernel ahead of this one has completed.  The
     // kernel behind this one (a projection that first requests its weights into L2) may start now; it in turn waits
     // for this grid's completion before it reads anything written here.
@@ -216,7 +218,7 @@ rmsnorm_bf16_kernel(const RmsBf16Params p) {
         const uint4* br = p.b ? reinterpret_cast<const uint4*>(p.b + (size_t)row * p.hidden) : nullptr;
         uint4* sr = p.s ? reinterpret_cast<uint4*>(p.s + (size_t)row * p.hidden) : nullptr;
         uint4* yr = reinterpret_cast<uint4*>(p.y + (size_t)row * p.hidden);
-        uint4 v[RB_MAXV];
+        uint4 v[RB_MAXV], wv[RB_MAXV];
         float acc = 0.f;
         auto fetch = [&](int c) {
             uint4 x = __ldg(ar + c);
@@ -241,7 +243,11 @@ rmsnorm_bf16_kernel(const RmsBf16Params p) {
 #pragma unroll
         for (int k = 0; k < RB_MAXV; ++k) {
             const int c = tid + k * 256;
-            if (c < pieces) { v[k] = fetch(c); sq(v[k]); }
+            if (c < pieces) {
+                v[k] = fetch(c);
+                wv[k] = __ldg(reinterpret_cast<const uint4*>(p.w) + c);
+                sq(v[k]);
+            }
         }
         for (int c = tid + RB_MAXV * 256; c < pieces; c += 256) { const uint4 x = fetch(c); sq(x); }
 #pragma unroll
@@ -252,9 +258,8 @@ rmsnorm_bf16_kernel(const RmsBf16Params p) {
 #pragma unroll
         for (int w8 = 0; w8 < 8; ++w8) total += s_part[w8];
         const float inv = rsqrtf(total / (float)p.hidden + p.eps);
-        auto emit = [&](int c, const uint4& x) {
+        auto emit = [&](int c, const uint4& x, const uint4& w4) {
             if (sr) sr[c] = x;
-            const uint4 w4 = __ldg(reinterpret_cast<const uint4*>(p.w) + c);
             const uint32_t* xs = reinterpret_cast<const uint32_t*>(&x);
             const uint32_t* ws = reinterpret_cast<const uint32_t*>(&w4);
             uint4 o4;
@@ -267,9 +272,9 @@ rmsnorm_bf16_kernel(const RmsBf16Params p) {
 #pragma unroll
         for (int k = 0; k < RB_MAXV; ++k) {
             const int c = tid + k * 256;
-            if (c < pieces) emit(c, v[k]);
+            if (c < pieces) emit(c, v[k], wv[k]);
         }
-        for (int c = tid + RB_MAXV * 256; c < pieces; c += 256) emit(c, fetch(c));
+        for (int c = tid + RB_MAXV * 256; c < pieces; c += 256) emit(c, fetch(c), __ldg(reinterpret_cast<const uint4*>(p.w) + c));
         __syncthreads();     // s_part is rewritten by the next row
     }
 }
