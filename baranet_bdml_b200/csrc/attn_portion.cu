@@ -105,12 +105,14 @@ attn_any_kernel(const AttnPortionParams p) {
 // 64; a warp per row for the running maximum and sum; thread = (value column mod 64, group of rows) for the result, which
 // reads a value from global memory once for AT_RPT rows.  fp32 throughout, a score is one FMA chain over its columns.
 // The warp-per-row kernel reads every key for every row, 32 rows of a matrix at a time: 32 heads over 4 x 64 columns, 4 x 200
-// tokens, 873 us; this one 129 us.
+// tokens, 873 us; this one 129 us, with keys and values staged (fp32, whole rows of at most 64 columns) 84 us.
 // ---------------------------------------------------------------------------------------------------------------
 constexpr int AT_KEYS = 64, AT_RPT = 8, AT_ROWS = 32, AT_THREADS = AT_KEYS * AT_ROWS / AT_RPT, AT_E = 64, AT_KLD = AT_E + 4;
 
-template <typename T, int VB>      // VB: value columns in blocks of 64
-__global__ void __launch_bounds__(AT_THREADS)
+// VB: value columns in blocks of 64.  STAGED (fp32, one piece of columns and one block of values, 16-byte rows): keys and values
+// come in by cp.async, the next keys while the weights are worked out and applied, the next values under the next scores.
+template <typename T, int VB, bool STAGED>
+__global__ void __launch_bounds__(AT_THREADS, STAGED ? 3 : 1)
 attn_tiled_kernel(const AttnPortionParams p) {
     extern __shared__ __align__(16) float at_smem[];
     __shared__ __align__(16) float Ks[AT_KEYS * AT_KLD];
@@ -153,11 +155,40 @@ attn_tiled_kernel(const AttnPortionParams p) {
 #pragma unroll
         for (int v = 0; v < VB; ++v) acc[r][v] = 0.f;
 
+    float* Vs = Qs + AT_ROWS * q_ld;                           // STAGED: [key][64]
+    // rows k0 .. k0 + 63 of a matrix with `cols` columns; what lies outside becomes zero
+    auto stage_in = [&](float* dst, int ld, const T* src, int64_t src_ld, int cols, int k0) {
+        const uint32_t to = ptx::smem_u32(dst);
+        for (int i = tid; i < AT_KEYS * 16; i += AT_THREADS) {
+            const int kk = i / 16, c = i % 16 * 4;
+            const bool in = k0 + kk <= last && c < cols;
+            ptx::cp_async_16(to + (kk * ld + c) * 4, in ? src + (int64_t)(k0 + kk) * src_ld + c : src, in ? 16 : 0);
+        }
+        ptx::cp_async_commit();
+    };
+    if constexpr (STAGED) {
+        stage_in(Ks, AT_KLD, kseq, p.k_ld, E, first);
+        stage_in(Vs, 64, vseq, p.v_ld, p.vdim, first);
+    }
+
     for (int k0 = first; k0 <= last; k0 += AT_KEYS) {
         float s[AT_RPT];
 #pragma unroll
         for (int r = 0; r < AT_RPT; ++r) s[r] = 0.f;
-        for (int e0 = 0; e0 < E; e0 += AT_E) {
+        if (STAGED) {
+            ptx::cp_async_wait<1>();                           // the keys; the values may still be on their way
+            __syncthreads();
+#pragma unroll 2
+            for (int e = 0; e < E; e += 4) {
+                const float4 k4 = *reinterpret_cast<const float4*>(Ks + key * AT_KLD + e);
+#pragma unroll
+                for (int r = 0; r < AT_RPT; ++r) {
+                    const float4 q4 = *reinterpret_cast<const float4*>(Qs + (group * AT_RPT + r) * q_ld + e);
+                    s[r] = fmaf(q4.w, k4.w, fmaf(q4.z, k4.z, fmaf(q4.y, k4.y, fmaf(q4.x, k4.x, s[r]))));
+                }
+            }
+        }
+        for (int e0 = 0; e0 < E && !STAGED; e0 += AT_E) {
             __syncthreads();                                   // the piece before (and the weights) have been read
 #pragma unroll 8
             for (int i = tid; i < AT_KEYS * AT_E; i += AT_THREADS) {
@@ -184,6 +215,12 @@ attn_tiled_kernel(const AttnPortionParams p) {
             Ps[row][key] = seen ? s[r] * row_scale[row] : -INFINITY;
         }
         __syncthreads();
+        const bool more = k0 + AT_KEYS <= last;
+        if (STAGED) {
+            if (more) stage_in(Ks, AT_KLD, kseq, p.k_ld, E, k0 + AT_KEYS);
+            else ptx::cp_async_commit();
+            ptx::cp_async_wait<1>();                           // the values, visible to all behind the next barrier
+        }
         for (int r = warp; r < AT_ROWS; r += AT_THREADS / 32) {
             const float a = Ps[r][lane], c = Ps[r][lane + 32], m = row_m[r];
             float mx = fmaxf(a, c);
@@ -220,7 +257,8 @@ attn_tiled_kernel(const AttnPortionParams p) {
             for (int i = 0; i < 4; ++i)
 #pragma unroll
                 for (int v = 0; v < VB; ++v)
-                    val[i][v] = j + i < nk && v * 64 + key < p.vdim ? to_f(vseq[(int64_t)(k0 + j + i) * p.v_ld + v * 64 + key]) : 0.f;
+                    if (STAGED) val[i][v] = Vs[(j + i) * 64 + key];
+                    else val[i][v] = j + i < nk && v * 64 + key < p.vdim ? to_f(vseq[(int64_t)(k0 + j + i) * p.v_ld + v * 64 + key]) : 0.f;
 #pragma unroll
             for (int r = 0; r < AT_RPT; ++r) {
                 const float4 w = *reinterpret_cast<const float4*>(&Ps[group * AT_RPT + r][j]);
@@ -228,6 +266,10 @@ attn_tiled_kernel(const AttnPortionParams p) {
                 for (int v = 0; v < VB; ++v)
                     acc[r][v] = fmaf(w.w, val[3][v], fmaf(w.z, val[2][v], fmaf(w.y, val[1][v], fmaf(w.x, val[0][v], acc[r][v]))));
             }
+        }
+        if (STAGED && more) {
+            __syncthreads();                                   // these values have been read
+            stage_in(Vs, 64, vseq, p.v_ld, p.vdim, k0 + AT_KEYS);
         }
     }
 #pragma unroll
@@ -252,7 +294,7 @@ attn_tiled_kernel(const AttnPortionParams p) {
 
 template <typename T>
 static int attn_tiled(const AttnPortionParams& p, cudaStream_t st, const char* what) {
-    const size_t smem = (size_t)AT_ROWS * ((p.dim + p.rot + 3) / 4 * 4 + 4) * sizeof(float);
+    size_t smem = (size_t)AT_ROWS * ((p.dim + p.rot + 3) / 4 * 4 + 4) * sizeof(float);
     const long long tiles = ((long long)p.S * (p.H / p.kv_heads) + AT_ROWS - 1) / AT_ROWS, blocks = tiles * p.B * p.kv_heads;
     if (blocks > 0x7fffffffLL) return fail(BN_ERR_UNSUPPORTED, "%s: B=%d x S=%d too large", what, p.B, p.S);
     auto run = [&](auto kernel) {
@@ -260,9 +302,15 @@ static int attn_tiled(const AttnPortionParams& p, cudaStream_t st, const char* w
         launch_dependent(kernel, (unsigned)blocks, AT_THREADS, smem, st, p);
         return launch_status(what);
     };
-    if (p.vdim <= 64) return run(attn_tiled_kernel<T, 1>);
-    if (p.vdim <= 128) return run(attn_tiled_kernel<T, 2>);
-    return run(attn_tiled_kernel<T, 4>);
+    if (sizeof(T) == 4 && p.rot == 0 && p.dim <= AT_E && p.vdim <= 64 && (p.dim | p.vdim) % 4 == 0 &&
+        (p.k_ld | p.v_ld | p.k_seq | p.v_seq | p.k_head | p.v_head) % 4 == 0 &&
+        ((reinterpret_cast<uintptr_t>(p.k) | reinterpret_cast<uintptr_t>(p.v)) & 15) == 0) {
+        smem += AT_KEYS * 64 * sizeof(float);
+        return run(attn_tiled_kernel<float, 1, true>);
+    }
+    if (p.vdim <= 64) return run(attn_tiled_kernel<T, 1, false>);
+    if (p.vdim <= 128) return run(attn_tiled_kernel<T, 2, false>);
+    return run(attn_tiled_kernel<T, 4, false>);
 }
 
 int attn_any(const AttnPortionParams& p, int dtype, cudaStream_t st, const char* what) {

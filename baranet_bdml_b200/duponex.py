@@ -113,11 +113,13 @@ class DuponexModel(SequenceLM):
         return states
 
     # -------------------------------------------------------------------- forward
-    def _forward(self, ids: torch.Tensor, B: int, S: int, seq_ids, positions, n_old: Optional[int]):
+    def _forward(self, ids: torch.Tensor, B: int, S: int, seq_ids, positions, n_old: Optional[int], embedded=None):
         """All layers over B x S new tokens: (streams, the last sublayer's output and its scale, still pending)."""
         c, dt = self.config, self.dtype
         x = torch.empty((B * S, 1, c.width), dtype=torch.float32, device="cuda")
         ops.embedding_rows(self.embed_tokens, ids, out_f32=x.view(B * S, c.width), error_word=self._id_error)
+        if embedded is not None:
+            embedded()
         delta = scale = v_first = None
         steps = iter(self.steps)
 

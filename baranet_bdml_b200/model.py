@@ -20,6 +20,23 @@ from .kv_cache import PAGE_TOKENS, PagedKVCache, SequenceSlots
 from .layers import LLaMAConfig, LLaMADecoderLayerBF16
 
 
+class IdCheck:
+    """Whether a launch has raised an error word, read without a wait for what is launched behind it: called, it sends the word
+    to the host; `failed` waits for that copy alone."""
+
+    def __init__(self, word: torch.Tensor):
+        self.word = word
+
+    def __call__(self) -> None:
+        self.host = self.word.to("cpu", non_blocking=True)
+        self.event = torch.cuda.Event()
+        self.event.record()
+
+    def failed(self) -> bool:
+        self.event.synchronize()
+        return int(self.host) != 0
+
+
 class CausalLM:
     """Generation over a cached model: what every model family here shares.  A family supplies `config` (with
     eos_token_id, or None), `prefill(prompts, max_len)` and `decode_step(token_ids, check)`, both returning fp32 logits of
@@ -102,9 +119,10 @@ class SequenceLM(CausalLM):
     A family supplies
       new_states(num_seqs, max_tokens)   one state per layer run (reset(slot), tensors()); max_tokens: the most tokens a
                                          sequence will have, or None
-      _forward(ids, B, S, seq_ids, positions, n_old)   all layers over B x S new tokens -> whatever _logits takes.  `n_old`:
-                                         how many earlier tokens each of the B sequences has; None with S = 1 selects the
-                                         one-token kernels, for which the sequences' lengths may differ
+      _forward(ids, B, S, seq_ids, positions, n_old, embedded)   all layers over B x S new tokens -> whatever _logits takes.
+                                         `n_old`: how many earlier tokens each of the B sequences has; None with S = 1
+                                         selects the one-token kernels, for which the sequences' lengths may differ.
+                                         `embedded`, if given, is called once the ids have been looked up
       _select(state, rows)               the same for some of the B * S rows
       _logits(state)                     fp32 logits of those rows
     and raises the int32 `_id_error` on the GPU for a token id outside the vocabulary."""
@@ -141,8 +159,8 @@ class SequenceLM(CausalLM):
         return self._extend(ids, list(slots), want, None)
 
     def _extend(self, ids: torch.Tensor, slots: List[int], want: Optional[torch.Tensor], n_old: Optional[int]) -> torch.Tensor:
-        """`n_old`: how many tokens every one of them has, where the host knows; None: read from the GPU.  The token ids'
-        check, a synchronisation, comes last, so that the host is not waited for in between."""
+        """`n_old`: how many tokens every one of them has, where the host knows; None: read from the GPU.  The check of the
+        token ids is read last, when the layers have been launched."""
         B, S = ids.shape
         flat = ids.reshape(-1).to(torch.int32).contiguous()
         whole = slots == list(range(B)) and B <= self.slots.num_seqs
@@ -166,7 +184,8 @@ class SequenceLM(CausalLM):
             else:
                 self.seq_lens.index_add_(0, seq_ids, torch.full_like(seq_ids, n))
 
-        state = self._forward(flat, B, S, seq_ids, positions, None if S == 1 else n_old)
+        ids_ok = IdCheck(self._id_error)
+        state = self._forward(flat, B, S, seq_ids, positions, None if S == 1 else n_old, ids_ok)
         advance(S)
         if want is None and S > 1:
             want = torch.arange(S - 1, B * S, S, device="cuda")
@@ -176,11 +195,10 @@ class SequenceLM(CausalLM):
             if want is not None and (want.numel() != B * S or S > 1):
                 state = self._select(state, want)
             logits = self._logits(state)
-        try:
-            self._check_ids()
-        except IndexError:
+        if ids_ok.failed():
             advance(-S)
-            raise
+            self._id_error.zero_()
+            raise IndexError("token id out of range")
         return logits
 
     def prefill(self, input_ids, max_len: int) -> torch.Tensor:
@@ -286,6 +304,8 @@ class LLaMAModelBF16(CausalLM):
         self._alloc_caches(B, max_len)
         id_error = torch.zeros(1, dtype=torch.int32, device="cuda")
         h = self.embed(input_ids.reshape(-1), check=False, error=id_error).view(B, S, -1)
+        ids_ok = IdCheck(id_error)
+        ids_ok()
         pending = None
         H = cfg.hidden_size
         # one scratch buffer for all blocks (they run one after the other): cos/sin table written once
@@ -303,7 +323,7 @@ class LLaMAModelBF16(CausalLM):
             h, pending = residual.view(B, S, H), layer.mlp(normed).view(B, S, H)
         self.seq_lens.fill_(S)
         logits = self._logits(h[:, -1].contiguous(), pending[:, -1].contiguous())
-        if int(id_error.item()) != 0:             # read last, so that the host is not waited for in between
+        if ids_ok.failed():
             self.seq_lens.zero_()
             raise IndexError("token id out of range")
         return logits

@@ -160,10 +160,12 @@ class SoluzenModel(SequenceLM):
             ops.embedding_rows(self.side_embed, ids, out_f32=side)
         return x, side, cat
 
-    def _forward(self, ids: torch.Tensor, B: int, S: int, seq_ids, positions, n_old: Optional[int]):
+    def _forward(self, ids: torch.Tensor, B: int, S: int, seq_ids, positions, n_old: Optional[int], embedded=None):
         """All layers over B x S new tokens: (the residual stream, its last addend, still pending)."""
         c, dt, width, w8, s8 = self.config, self.dtype, self.config.width, round8(self.config.width), self.side8
         x, side, cat = self._embed(ids)
+        if embedded is not None:
+            embedded()
         pending, row = None, None
         for (i, start_of_pass), state in zip(self.runs, self.states):
             layer = self.layers[i]
