@@ -201,13 +201,16 @@ __device__ __forceinline__ uint32_t packbf(float lo, float hi) {
     return r;
 }
 
-__global__ void __launch_bounds__(256)
+// FEW: a block has one row (a step).  Its weight, which then comes from HBM, is asked for in L2 while the kernel ahead finishes
+// and read along with the row; with many rows the registers hold rows in flight (8192 x 2048: 21.5 us, 28 with the weight early).
+template <bool FEW>
+__global__ void __launch_bounds__(256, FEW ? 1 : 8)
 rmsnorm_bf16_kernel(const RmsBf16Params p) {
     __shared__ float s_part[8];
     const int tid = threadIdx.x, lane = tid % 32, warp = tid / 32;
     const int pieces = p.hidden / 8;
-    // the weight is asked for in L2 meanwhile (a step's comes from HBM) and read along with the row
-    for (int c = tid; c < pieces; c += 256) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.w + c * 8));
+    if (FEW)
+        for (int c = tid; c < pieces; c += 256) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.w + c * 8));
     // Launched as a programmatic dependent: nothing is read before the kernel ahead of this one has completed.  The
     // kernel behind this one (a projection that first requests its weights into L2) may start now; it in turn waits
     // for this grid's completion before it reads anything written here.
@@ -218,8 +221,9 @@ rmsnorm_bf16_kernel(const RmsBf16Params p) {
         const uint4* br = p.b ? reinterpret_cast<const uint4*>(p.b + (size_t)row * p.hidden) : nullptr;
         uint4* sr = p.s ? reinterpret_cast<uint4*>(p.s + (size_t)row * p.hidden) : nullptr;
         uint4* yr = reinterpret_cast<uint4*>(p.y + (size_t)row * p.hidden);
-        uint4 v[RB_MAXV], wv[RB_MAXV];
+        uint4 v[RB_MAXV], early[FEW ? RB_MAXV : 1];
         float acc = 0.f;
+        auto weight = [&](int c) { return __ldg(reinterpret_cast<const uint4*>(p.w) + c); };
         auto fetch = [&](int c) {
             uint4 x = __ldg(ar + c);
             if (br) {
@@ -245,7 +249,7 @@ rmsnorm_bf16_kernel(const RmsBf16Params p) {
             const int c = tid + k * 256;
             if (c < pieces) {
                 v[k] = fetch(c);
-                wv[k] = __ldg(reinterpret_cast<const uint4*>(p.w) + c);
+                if (FEW) early[FEW ? k : 0] = weight(c);
                 sq(v[k]);
             }
         }
@@ -272,9 +276,9 @@ rmsnorm_bf16_kernel(const RmsBf16Params p) {
 #pragma unroll
         for (int k = 0; k < RB_MAXV; ++k) {
             const int c = tid + k * 256;
-            if (c < pieces) emit(c, v[k], wv[k]);
+            if (c < pieces) emit(c, v[k], FEW ? early[FEW ? k : 0] : weight(c));
         }
-        for (int c = tid + RB_MAXV * 256; c < pieces; c += 256) emit(c, fetch(c), __ldg(reinterpret_cast<const uint4*>(p.w) + c));
+        for (int c = tid + RB_MAXV * 256; c < pieces; c += 256) emit(c, fetch(c), weight(c));
         __syncthreads();     // s_part is rewritten by the next row
     }
 }
@@ -299,6 +303,6 @@ extern "C" int bn_add_rmsnorm_bf16(const void* a, const void* b, const void* w, 
     RmsBf16Params p{static_cast<const __nv_bfloat16*>(a), static_cast<const __nv_bfloat16*>(b),
                     static_cast<const __nv_bfloat16*>(w), static_cast<__nv_bfloat16*>(sum),
                     static_cast<__nv_bfloat16*>(y), rows, hidden, eps};
-    launch_dependent(rmsnorm_bf16_kernel, (unsigned)(rows < cap ? rows : cap), 256, 0, as_stream(stream), p);
+    launch_dependent(rows <= 2 * sms ? rmsnorm_bf16_kernel<true> : rmsnorm_bf16_kernel<false>, (unsigned)(rows < cap ? rows : cap), 256, 0, as_stream(stream), p);
     return launch_status("bn_add_rmsnorm_bf16");
 }
