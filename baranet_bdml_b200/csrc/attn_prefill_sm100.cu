@@ -72,20 +72,22 @@ rope_table_kernel(float2* __restrict__ table, int S, float theta, int position_o
 // ---------------------------------------------------------------------------
 // launch 1: K rotation + cos/sin table
 // ---------------------------------------------------------------------------
-// One block per (batch element, 128-key tile) and `heads` KV heads: the block owns the tile's norm maxima, so they are plain
+// One block per (batch element, 128-key tile) and one or all KV heads: the block owns the tile's norm maxima, so they are plain
 // stores (no global atomics, nothing to clear first), and a cos/sin pair is computed once per position and block.  All heads
 // where such blocks fill the GPU, else one (1 x 333 tokens, 4 heads: 3 blocks 6.0 us, 12 blocks 5.3 us).
 constexpr int RK_THREADS = 512;
 constexpr int RK_UNROLL = 4;    // 16-byte pieces a thread has in flight
 
+template <bool ONE_HEAD>
 __global__ void __launch_bounds__(RK_THREADS)
 rope_k_kernel(const __nv_bfloat16* __restrict__ k, __nv_bfloat16* __restrict__ krot, float2* __restrict__ table,
-              int* __restrict__ kmax2, int B, int S, int Hkv, int heads, float theta, int position_offset,
+              int* __restrict__ kmax2, int B, int S, int Hkv, float theta, int position_offset,
               int* __restrict__ error_word) {
     __shared__ float2 cs[PF_BN][PF_D / 2];      // 32 KB
     __shared__ int s_kmax[64];                  // per KV head (up to 64): largest |k|^2 of the tile's keys, as float bits
     const int tile = blockIdx.x, b = blockIdx.y;
-    const int s0 = tile * PF_BN, npos = min(PF_BN, S - s0), h0 = blockIdx.z * heads;
+    const int s0 = tile * PF_BN, npos = min(PF_BN, S - s0);
+    const int heads = ONE_HEAD ? 1 : Hkv, h0 = ONE_HEAD ? blockIdx.z : 0;
     if (tile == 0 && b == 0 && h0 == 0 && threadIdx.x == 0) *error_word = 0;
     // 16-byte pieces (4 rotation pairs) of the tile's keys: the first loads are issued before the cos/sin work
     const int chunks_per_pos = heads * (PF_D / 8);
@@ -93,7 +95,7 @@ rope_k_kernel(const __nv_bfloat16* __restrict__ k, __nv_bfloat16* __restrict__ k
     const uint4* src = reinterpret_cast<const uint4*>(k + (((size_t)b * S + s0) * Hkv + h0) * PF_D);
     uint4* dst = reinterpret_cast<uint4*>(krot + (((size_t)b * S + s0) * Hkv + h0) * PF_D);
     // piece e of the block's keys; with all heads in the block they lie one behind the other
-    auto at = [&](int e) { return heads == Hkv ? e : e / chunks_per_pos * (Hkv * (PF_D / 8)) + e % chunks_per_pos; };
+    auto at = [&](int e) { return ONE_HEAD ? e / (PF_D / 8) * (Hkv * (PF_D / 8)) + e % (PF_D / 8) : e; };
     uint4 raw[RK_UNROLL];
 #pragma unroll
     for (int i = 0; i < RK_UNROLL; ++i) {
@@ -1274,9 +1276,11 @@ extern "C" int bn_attn_prefill_bf16(const void* q, const void* k, const void* v,
 
     int* kmax2 = reinterpret_cast<int*>(ws + L.kmax2);
     if (!(flags & BN_PREFILL_REUSE_ROTATED_K)) {
-        const int tiles = (S + PF_BN - 1) / PF_BN, heads = (long long)tiles * B * 2 <= sm_count() && Hkv <= 65535 ? 1 : Hkv;
-        rope_k_kernel<<<dim3(tiles, B, Hkv / heads), RK_THREADS, 0, st>>>(static_cast<const __nv_bfloat16*>(k), krot, table, kmax2, B, S, Hkv,
-                                                                         heads, theta, position_offset, error_word);
+        const int tiles = (S + PF_BN - 1) / PF_BN;
+        const bool one_head = (long long)tiles * B * 2 <= sm_count() && Hkv <= 65535;
+        auto kernel = one_head ? rope_k_kernel<true> : rope_k_kernel<false>;
+        kernel<<<dim3(tiles, B, one_head ? Hkv : 1), RK_THREADS, 0, st>>>(static_cast<const __nv_bfloat16*>(k), krot, table, kmax2, B, S,
+                                                                         Hkv, theta, position_offset, error_word);
         if (int rc = launch_status("bn_attn_prefill_bf16 (rope_k)")) return rc;
     }
 
