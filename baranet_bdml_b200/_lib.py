@@ -29,7 +29,9 @@ SIGNATURES = {
     "bn_split_f32": (_i, [_p, _i64, _p, _i, _i, _p]),
     "bn_mm_f32_split": (_i, [_p, _p, _i, _p, _i64, _p, _i64, _p, _i, _p, _i, _i, _i, _p, _p]),
     "bn_mm_f32_each": (_i, [_p, _i64, _i64, _i, _p, _p, _p, _p, _p, _p, _i, _i, _p, _p]),
-    "bn_mm_f32_split_pays": (_i, [_i, _i, _i, _i]),
+    "bn_linear_f32_workspace_bytes": (_sz, [_i, _i, _i]),
+    "bn_linear_f32_pays": (_i, [_i, _i, _i, _i]),
+    "bn_linear_f32": (_i, [_p, _i64, _p, _i64, _p, _i, _p, _i, _i, _i, _p, _sz, _p, _p]),
     "bn_rope_f32": (_i, [_p, _i64, _i64, _p, _i64, _i64, _i, _i, _i, _f, _i, _p]),
     "bn_embedding_gather_f32": (_i, [_p, _i64, _p, _p, _i64, _i, _i, _i, _p, _p]),
     "bn_argmax_rows_f32": (_i, [_p, _i64, _i64, _p, _i, _i, _p]),

@@ -452,9 +452,9 @@ def _bf16_parts(x: torch.Tensor) -> torch.Tensor:
 
 class Linear:
     """y = act(x W^T + bias) for a weight (out, in), bias (out) and act optional: bf16 on the tensor cores, or true fp32 (chains
-    of FMAs, `bn_mm_f32`, or for many rows `bn_mm_f32_split`, whose error is smaller).  The latter reads bf16 parts of the weight
-    that are laid out here: one where every weight is a bf16 number, else three, beside the weight itself.  Both sizes are rounded up to multiples of 8 with zeros, so x may be passed with its padding columns (which
-    must be finite) and y has them."""
+    of FMAs, `bn_mm_f32`, or for many rows `bn_linear_f32`, whose error is smaller; both read `weight` as it is at the call).
+    Both sizes are rounded up to multiples of 8 with zeros, so x may be passed with its padding columns (which must be finite)
+    and y has them."""
 
     def __init__(self, weight: torch.Tensor, dtype, device="cuda", bias: Optional[torch.Tensor] = None, act: str = "none"):
         self.out_features, self.in_features = weight.shape
@@ -465,13 +465,8 @@ class Linear:
         self.n, self.k = round8(self.out_features), round8(self.in_features)
         self.weight = torch.zeros((self.n, self.k), dtype=dtype, device=device)
         self.weight[:self.out_features, :self.in_features] = weight.to(device)
-        self._parts = {}              # number of parts -> the parts of an fp32 weight (a copy: not among a model's parameters)
-        if dtype == torch.float32 and self.weight.is_cuda:
-            parts = _bf16_parts(self.weight)
-            if bool(parts[1:].any()):
-                self._parts[3] = parts
-            else:
-                self._parts[1] = parts[0].clone()
+        # bf16 numbers in fp32 have one bf16 part, others three: what the choice of a kernel goes by, and all that does
+        self.parts_hint = 1 if weight.dtype == torch.bfloat16 else 3
 
     def _operand(self, x: torch.Tensor) -> torch.Tensor:
         _rows(x, "linear(x)")
@@ -488,12 +483,12 @@ class Linear:
     def _mm_f32(self, x: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
         """x W^T with the bias and the activation, fp32"""
         w, rows, lib, act = self.weight, x.shape[0], _lib.load(), ACTIVATIONS[self.act]
-        for n, parts in self._parts.items():
-            if x.data_ptr() % 16 == 0 and lib.bn_mm_f32_split_pays(rows, self.n, self.k, n):
-                _lib.check(lib.bn_mm_f32_split(_bf16_parts(x).data_ptr(), parts.data_ptr(), n, x.data_ptr(), x.stride(0), w.data_ptr(),
-                                               w.stride(0), _ptr(self.bias), act, out.data_ptr(), rows, self.n, self.k,
-                                               _gemm_error_ptr(x.device, None), _stream()))
-                return out
+        if (x.data_ptr() | w.data_ptr()) % 16 == 0 and w.stride(0) % 4 == 0 and lib.bn_linear_f32_pays(rows, self.n, self.k, self.parts_hint):
+            scratch = torch.empty(lib.bn_linear_f32_workspace_bytes(rows, self.n, self.k), dtype=torch.uint8, device=x.device)
+            _lib.check(lib.bn_linear_f32(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), _ptr(self.bias), act,
+                                         out.data_ptr(), rows, self.n, self.k, scratch.data_ptr(), scratch.numel(),
+                                         _gemm_error_ptr(x.device, None), _stream()))
+            return out
         _lib.check(lib.bn_mm_f32(x.data_ptr(), x.stride(0), 1, w.data_ptr(), 1, w.stride(0), out.data_ptr(), out.stride(0), 1, rows,
                                  self.k, self.n, _stream()))
         if self.bias is not None or self.act != "none":

@@ -105,14 +105,22 @@ BN_API int bn_mm_f32_each(const float* A, int64_t a_rs, int64_t a_cs, int n, con
                           bn_stream_t stream);
 
 /* The products of many rows on the tensor cores, with the precision of an fp32 sum: C(M,N) = act(A(M,K) W(N,K)^T + bias),
- * fp32, from the bf16 parts of both operands.
+ * fp32, from the bf16 parts of both operands.  N and K multiples of 8; 16-byte aligned rows; bias (N) or null; act one of
+ * BN_ACT_*.  Results that are not finite are worked out as by bn_mm_f32.
+ * bn_linear_f32 cuts the operands itself, in `workspace` (bn_linear_f32_workspace_bytes, 16-byte aligned; contents need not be
+ * kept).
+ * bn_linear_f32_pays: whether it takes less time than bn_mm_f32 (an estimate), w_nparts being 1 where the weights are mostly bf16
+ * numbers, else 3. */
+BN_API size_t bn_linear_f32_workspace_bytes(int M, int N, int K);
+BN_API int bn_linear_f32_pays(int M, int N, int K, int w_nparts);
+BN_API int bn_linear_f32(const float* a, int64_t a_ld, const float* w, int64_t w_ld, const float* bias, int act, float* c, int M,
+                         int N, int K, void* workspace, size_t workspace_bytes, int* error_word, bn_stream_t stream);
+
+/* The same in two calls, for a weight whose parts the caller keeps and cuts again whenever it changes.
  * bn_split_f32 writes x (rows, cols) as three bf16 matrices [3][rows][cols] whose sum it is; cols a multiple of 8, 16-byte
  * aligned rows.
  * bn_mm_f32_split takes A's three parts, and of W all three or (w_nparts = 1) the first, where the others are zeros, beside the
- * operands themselves, from which results that are not finite are worked out as by bn_mm_f32.  N and K multiples of 8;
- * bias (N) or null; act one of BN_ACT_*.
- * bn_mm_f32_split_pays: whether both together take less time than bn_mm_f32 (an estimate). */
-BN_API int bn_mm_f32_split_pays(int M, int N, int K, int w_nparts);
+ * operands themselves. */
 BN_API int bn_split_f32(const float* x, int64_t ld, void* parts, int rows, int cols, bn_stream_t stream);
 BN_API int bn_mm_f32_split(const void* a_parts, const void* w_parts, int w_nparts, const float* a, int64_t a_ld, const float* w,
                            int64_t w_ld, const float* bias, int act, float* c, int M, int N, int K, int* error_word,

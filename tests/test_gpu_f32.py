@@ -124,6 +124,58 @@ def test_mm_of_bf16_parts(lib, M, K, N, parts):
     assert int(word.item()) == 0
 
 
+@pytest.mark.parametrize("M,K,N", [(1, 8, 8), (127, 72, 72), (129, 136, 136), (300, 2056, 264), (513, 64, 2056), (1300, 128, 4096)])
+@pytest.mark.parametrize("weights", ["bf16", "fp32", "mixed"])
+def test_linear_f32_cuts_its_operands(lib, M, K, N, weights):
+    """Tiles of one part beside tiles of three; what is not written in the scratch is not read."""
+    from baranet_bdml_b200 import _lib
+    gen = torch.Generator(device="cuda").manual_seed(M + K)
+    x, w, bias = (torch.randn(s, generator=gen, device="cuda") for s in ((M, K), (N, K), (N,)))
+    if weights == "bf16":
+        w = w.bfloat16().float()
+    elif weights == "mixed":
+        whole = torch.rand(((N + 63) // 64, (K + 63) // 64), generator=gen, device="cuda") < 0.5
+        whole = whole.repeat_interleave(64, 0)[:N].repeat_interleave(64, 1)[:, :K]
+        w = torch.where(whole, w.bfloat16().float(), w)
+    n = lib.bn_linear_f32_workspace_bytes(M, N, K)
+    scratch, word = torch.full((n,), 0xff, dtype=torch.uint8, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    got = torch.empty((M, N), device="cuda")
+    args = (x.data_ptr(), K, w.data_ptr(), K, bias.data_ptr(), 0, got.data_ptr(), M, N, K, scratch.data_ptr())
+    st = torch.cuda.current_stream().cuda_stream
+    _lib.check(lib.bn_linear_f32(*args, n, word.data_ptr(), st))
+    exact = x.double() @ w.double().T + bias.double()
+    # per 64 k: 4 truncations at full size, each of 2 units of 2^-24, beside 8 at 2^-8 of it; K / 64 roundings of the sum; products
+    # left out and the bias: 2 more
+    bound = (4 * 2 + 1 + K / 64 + 2) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T + bias.double().abs())
+    assert ((got.double() - exact).abs() <= bound).all() and int(word.item()) == 0
+    assert lib.bn_linear_f32(*args, n - 1, word.data_ptr(), st) != 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("write", ["data", "in_place", "replaced"])
+def test_linear_f32_reads_the_weight_of_the_call(lib, dtype, write):
+    """A weight that is written to, by whatever way, is the one that many rows are multiplied with as well as few."""
+    from baranet_bdml_b200 import ops
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    N, K, rows = 2048, 2048, 512
+    x, w0, w1 = (torch.randn(s, generator=gen, device="cuda") for s in ((rows, K), (N, K), (N, K)))
+    lin = ops.Linear(w0.to(dtype), torch.float32)
+    assert torch.equal(lin.weight, w0.to(dtype).float())
+    lin(x)
+    if write == "data":
+        lin.weight.data.copy_(w1)
+    elif write == "in_place":
+        lin.weight.mul_(0).add_(w1)
+    else:
+        lin.weight = w1.clone()
+    many, few = lin(x), torch.cat([lin(x[i:i + 4]) for i in range(0, rows, 4)])
+    exact, size = x.double() @ w1.double().T, x.double().abs() @ w1.double().abs().T
+    for got in (many, few):
+        assert ((got.double() - exact).abs() <= K * 2.0 ** -24 * size).all()
+    # the two are the two routes
+    assert lib.bn_linear_f32_pays(rows, N, K, lin.parts_hint) and not lib.bn_linear_f32_pays(4, N, K, lin.parts_hint)
+
+
 @pytest.mark.parametrize("M,K,widths", [(128, 64, (2048, 256, 256)), (5, 20, (40, 8, 33)), (33, 16, (64, 1, 65)), (70, 36, (100, 260))])
 @pytest.mark.parametrize("transposed", [(), (1,), (0, 1, 2)])
 def test_mm_each_is_the_single_products(T, M, K, widths, transposed):
