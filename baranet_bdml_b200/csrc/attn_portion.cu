@@ -1,6 +1,8 @@
 // Attention of a prompt portion (bn_attn_window: a sliding window and a rotated key part shared by the heads;
 // bn_attn_chunked: grouped-query heads, chunks of positions, unit-RMS queries, a gate on the result) for any sizes, in fp32
 // and in bf16, and the choice of the tensor-core form (attn_portion_sm100.cu).
+#include <type_traits>
+
 #include "attn_portion.cuh"
 #include "common.cuh"
 #include "hybrid.cuh"
@@ -106,6 +108,8 @@ attn_any_kernel(const AttnPortionParams p) {
 // reads a value from global memory once for AT_RPT rows.  fp32 throughout, a score is one FMA chain over its columns.
 // The warp-per-row kernel reads every key for every row, 32 rows of a matrix at a time: 32 heads over 4 x 64 columns, 4 x 200
 // tokens, 873 us; this one 129 us, with keys and values staged (fp32, whole rows of at most 64 columns) 84 us.
+// A tile of keys where the mask of some row cuts leaves the masked (row, key) pairs out of the result, as that kernel does: their
+// weight is no zero to multiply by, or a value that is not finite would reach rows that do not see it.
 // ---------------------------------------------------------------------------------------------------------------
 constexpr int AT_KEYS = 64, AT_RPT = 8, AT_ROWS = 32, AT_THREADS = AT_KEYS * AT_ROWS / AT_RPT, AT_E = 64, AT_KLD = AT_E + 4;
 
@@ -216,6 +220,8 @@ attn_tiled_kernel(const AttnPortionParams p) {
         }
         __syncthreads();
         const bool more = k0 + AT_KEYS <= last;
+        // whether some row does not see some key of the tile
+        const bool cut = k0 + AT_KEYS - 1 > p.n_old + position(0) || k0 < mask_oldest(p.mask, p.span, p.n_old + position(n_rows - 1));
         if (STAGED) {
             if (more) stage_in(Ks, AT_KLD, kseq, p.k_ld, E, k0 + AT_KEYS);
             else ptx::cp_async_commit();
@@ -233,8 +239,14 @@ attn_tiled_kernel(const AttnPortionParams p) {
             float sum = wa + wc;
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-            Ps[r][lane] = wa;
-            Ps[r][lane + 32] = wc;
+            if (cut) {                                         // a masked pair's weight: -1
+                const int own = p.n_old + position(r), oldest = mask_oldest(p.mask, p.span, own), k = k0 + lane;
+                Ps[r][lane] = k <= own && k >= oldest ? wa : -1.f;
+                Ps[r][lane + 32] = k + 32 <= own && k + 32 >= oldest ? wc : -1.f;
+            } else {
+                Ps[r][lane] = wa;
+                Ps[r][lane + 32] = wc;
+            }
             if (lane == 0) {
                 const float shrink = none ? 1.f : expf(m - m_new);
                 row_shrink[r] = shrink;
@@ -250,23 +262,28 @@ attn_tiled_kernel(const AttnPortionParams p) {
             for (int v = 0; v < VB; ++v) acc[r][v] *= shrink;
         }
         const int nk = min(AT_KEYS, last - k0 + 1);
+        auto apply = [&](auto masked) {
+            auto add = [&](float w, float v, float sum) { return decltype(masked)::value && w < 0.f ? sum : fmaf(w, v, sum); };
 #pragma unroll 2
-        for (int j = 0; j < nk; j += 4) {
-            float val[4][VB];
+            for (int j = 0; j < nk; j += 4) {
+                float val[4][VB];
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+                for (int i = 0; i < 4; ++i)
 #pragma unroll
-                for (int v = 0; v < VB; ++v)
-                    if (STAGED) val[i][v] = Vs[(j + i) * 64 + key];
-                    else val[i][v] = j + i < nk && v * 64 + key < p.vdim ? to_f(vseq[(int64_t)(k0 + j + i) * p.v_ld + v * 64 + key]) : 0.f;
+                    for (int v = 0; v < VB; ++v)
+                        if (STAGED) val[i][v] = Vs[(j + i) * 64 + key];
+                        else val[i][v] = j + i < nk && v * 64 + key < p.vdim ? to_f(vseq[(int64_t)(k0 + j + i) * p.v_ld + v * 64 + key]) : 0.f;
 #pragma unroll
-            for (int r = 0; r < AT_RPT; ++r) {
-                const float4 w = *reinterpret_cast<const float4*>(&Ps[group * AT_RPT + r][j]);
+                for (int r = 0; r < AT_RPT; ++r) {
+                    const float4 w = *reinterpret_cast<const float4*>(&Ps[group * AT_RPT + r][j]);
 #pragma unroll
-                for (int v = 0; v < VB; ++v)
-                    acc[r][v] = fmaf(w.w, val[3][v], fmaf(w.z, val[2][v], fmaf(w.y, val[1][v], fmaf(w.x, val[0][v], acc[r][v]))));
+                    for (int v = 0; v < VB; ++v)
+                        acc[r][v] = add(w.w, val[3][v], add(w.z, val[2][v], add(w.y, val[1][v], add(w.x, val[0][v], acc[r][v]))));
+                }
             }
-        }
+        };
+        if (cut) apply(std::true_type{});
+        else apply(std::false_type{});
         if (STAGED && more) {
             __syncthreads();                                   // these values have been read
             stage_in(Vs, 64, vseq, p.v_ld, p.vdim, k0 + AT_KEYS);

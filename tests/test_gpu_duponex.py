@@ -324,6 +324,26 @@ def test_chunked_attention(lib, dtype, H, G, E, V, S, n_old, chunk):
         assert np.abs(got - want).max() <= (2e-5 if dtype == torch.float32 else 3e-2), bound
 
 
+@pytest.mark.parametrize("H,G,E,V", [(4, 2, 64, 64), (3, 3, 40, 72), (6, 1, 10, 11), (4, 2, 48, 136)])
+@pytest.mark.parametrize("S,n_old,chunk", [(300, 0, 1000), (129, 63, 64), (257, 126, 150), (40, 0, 7)])
+@pytest.mark.parametrize("bad", [np.inf, np.nan])
+def test_a_token_that_is_not_finite_stays_with_those_that_see_it(lib, H, G, E, V, S, n_old, chunk, bad):
+    """fp32: key and value of a position do not reach positions before it, or those of later chunks."""
+    rng = np.random.default_rng(S + chunk + E)
+    n = S + n_old
+    q, k = rng.standard_normal((S, H, E)), R.unit_rms(rng.standard_normal((n, G, E)), 1e-5)
+    v, g, scale = rng.standard_normal((n, G, V)), rng.standard_normal((S, H, V)), E ** -0.5
+    clean, _ = _chunked_attention(q, k, v, g, n_old, chunk, scale, 1e-5, torch.float32)
+    own = n_old + np.arange(S)
+    for t in (0, n // 2, n - 2):
+        v2, k2 = v.copy(), k.copy()
+        v2[t], k2[t] = bad, np.nan
+        sees = (t <= own) & (own - own % chunk <= t)
+        for keys, values in ((k, v2), (k2, v2)):
+            got, _ = _chunked_attention(q, keys, values, g, n_old, chunk, scale, 1e-5, torch.float32)
+            assert np.array_equal(got[~sees], clean[~sees]) and not np.isfinite(got[sees]).any(), t
+
+
 @DTYPES
 @pytest.mark.parametrize("B,H,G,E,V", [(16, 32, 4, 64, 64), (9, 40, 8, 128, 128), (20, 16, 2, 40, 136)])
 @pytest.mark.parametrize("S,n_old,chunk", [(40, 0, 16), (130, 0, 500), (2, 9, 12), (300, 63, 64), (257, 0, 1)])

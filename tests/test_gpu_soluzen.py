@@ -333,6 +333,26 @@ def test_window_attention(lib, dtype, H, dim, rot, vd, S, n_old, window):
     assert np.abs(got - want).max() <= (2e-5 if dtype == torch.float32 else 3e-2)
 
 
+@pytest.mark.parametrize("H,dim,rot,vd,dtype", [(2, 128, 64, 128, torch.float32), (3, 64, 32, 64, torch.float32), (2, 10, 6, 11, torch.bfloat16)])
+@pytest.mark.parametrize("S,n_old,window", [(300, 0, 1000), (129, 63, 64), (200, 9, 10), (70, 0, 1)])
+def test_a_token_that_is_not_finite_stays_with_those_that_see_it(lib, H, dim, rot, vd, dtype, S, n_old, window):
+    """Sizes that the kernel for any sizes takes: key and value of a position do not reach rows that do not see it."""
+    rng = np.random.default_rng(S + window + dim)
+    n = S + n_old
+    q, kn = rng.standard_normal((S, H, dim + rot)), rng.standard_normal((n, H, dim))
+    kr, v = rng.standard_normal((n, rot)), rng.standard_normal((n, H, vd))
+    args = (n_old, window, (dim + rot) ** -0.5, dtype)
+    clean, _ = _window_attention(q, kn, kr, v, *args)
+    own = n_old + np.arange(S)
+    for t in (0, n // 2, n - 2):
+        v2, kn2, kr2 = v.copy(), kn.copy(), kr.copy()
+        v2[t], kn2[t], kr2[t] = np.inf, np.nan, np.nan
+        sees = (t <= own) & (t > own - window)
+        for k1, k2 in ((kn, kr), (kn2, kr2)):
+            got, _ = _window_attention(q, k1, k2, v2, *args)
+            assert np.array_equal(got[~sees], clean[~sees]) and not np.isfinite(got[sees]).any(), t
+
+
 @pytest.mark.parametrize("H,dim,rot,vd", [(20, 128, 64, 128), (32, 40, 16, 72), (16, 128, 64, 192)])
 @pytest.mark.parametrize("S,window", [(70, 30), (130, 500), (300, 64)])
 def test_window_attention_many_short_units(lib, H, dim, rot, vd, S, window):
