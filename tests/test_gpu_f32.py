@@ -151,6 +151,51 @@ def test_linear_f32_cuts_its_operands(lib, M, K, N, weights):
     assert lib.bn_linear_f32(*args, n - 1, word.data_ptr(), st) != 0
 
 
+@pytest.mark.parametrize("bad", ["row", "rows", "nan", "weight"])
+@pytest.mark.parametrize("act", [0, 1, 2, 3])
+def test_linear_f32_of_values_that_are_not_finite(lib, bad, act):
+    """Results that are not finite are the chain's and the others stay within their bound; a long K takes a few ms at worst, and
+    no wait runs out."""
+    from baranet_bdml_b200 import _lib
+    M, K, N = 300, 7424, 1032
+    gen = torch.Generator(device="cuda").manual_seed(act)
+    x, w, bias = (torch.randn(s, generator=gen, device="cuda") for s in ((M, K), (N, K), (N,)))
+    if bad == "row":
+        x[7, 5], x[129, K - 1] = float("inf"), -float("inf")
+    elif bad == "rows":
+        x[:, 3] = float("inf")                              # every result infinite, none a NaN
+    elif bad == "nan":
+        x[40:200, 0] = float("nan")
+    else:
+        w[1031, 77], w[12] = float("inf"), 3e38
+    chain, got = torch.empty((M, N), device="cuda"), torch.empty((M, N), device="cuda")
+    st, word = torch.cuda.current_stream().cuda_stream, torch.zeros(1, dtype=torch.int32, device="cuda")
+    _lib.check(lib.bn_mm_f32(x.data_ptr(), K, 1, w.data_ptr(), 1, K, chain.data_ptr(), N, 1, M, K, N, st))
+    fine = torch.isfinite(chain)
+    _lib.check(lib.bn_bias_act_f32(chain.data_ptr(), N, bias.data_ptr(), M, N, act, st))
+    n = lib.bn_linear_f32_workspace_bytes(M, N, K)
+    scratch = torch.empty(n, dtype=torch.uint8, device="cuda")
+    times = []
+    for _ in range(3):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        _lib.check(lib.bn_linear_f32(x.data_ptr(), K, w.data_ptr(), K, bias.data_ptr(), act, got.data_ptr(), M, N, K, scratch.data_ptr(), n,
+                                     word.data_ptr(), st))
+        b.record()
+        b.synchronize()
+        times.append(a.elapsed_time(b))
+    assert int(word.item()) == 0 and min(times) < 10.0, times
+    assert torch.equal(got[~fine].view(torch.int32), chain[~fine].view(torch.int32)) or \
+        (torch.equal(torch.isnan(got[~fine]), torch.isnan(chain[~fine])) and torch.equal(got[~fine].nan_to_num(5.0), chain[~fine].nan_to_num(5.0)))
+    ok = fine & torch.isfinite(chain)
+    xd, wd = x.double().nan_to_num(0.0, 0.0, 0.0), w.double().nan_to_num(0.0, 0.0, 0.0)
+    size = xd.abs() @ wd.abs().T + bias.double().abs()
+    err = (K + K / 64 + 12) * 2.0 ** -24 * size             # of the chain and of the product, before the activation
+    # slopes: 1.1 for SiLU, 1.13 for GELU; a square's 2 z, and the roundings of the square itself
+    bound = err if act == 0 else 2 * (size + err) * err + 2.0 ** -22 * size ** 2 if act == 3 else 1.13 * err + 2.0 ** -20 * size
+    assert ((got.double() - chain.double()).abs() <= bound)[ok].all()
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("write", ["data", "in_place", "replaced"])
 def test_linear_f32_reads_the_weight_of_the_call(lib, dtype, write):
