@@ -456,9 +456,8 @@ using namespace bn;
 // sum of the split-K partials, in split order (deterministic), rounded once to bf16, or kept in fp32 (c32), or its
 // activation times `mul`
 __global__ void __launch_bounds__(256)
-gemm_splitk_reduce_kernel(const float* __restrict__ partial, __nv_bfloat16* __restrict__ c, long long mn4, int splits,
-                          float* __restrict__ c32, const __nv_bfloat16* mul, long long mul_ld, int N, int act,
-                          const float* __restrict__ bias) {
+gemm_splitk_reduce_kernel(const float* partial, __nv_bfloat16* c, long long mn4, int splits, float* c32, const __nv_bfloat16* mul,
+                          long long mul_ld, int N, int act, const float* bias) {
     grid_dependency_wait();
     grid_launch_dependents();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;     // one group of 4 outputs

@@ -74,7 +74,7 @@ gemm_skinny_kernel(const SkinnyParams p) {
     // Loads first, arithmetic after: for a batch of K steps the lane requests its pieces of the weight rows (evict-first:
     // each weight byte is read once per launch) AND of the two activation rows (read by every CTA, so they stay in L2)
     // before it uses any of them - a launch of this kernel is one or two memory round trips long, and a load issued after
-    // a wait would add its whole latency to that.
+    // a wait would add its whole latency to that.  The activations by ordinary loads (see grid_dependency_wait).
     const uint4 z = make_uint4(0, 0, 0, 0);
     // whether this lane's 8 elements of step s lie inside K
     auto inside = [&](int s) { return !RAGGED || kbase + (size_t)s * 32 < (size_t)p.K; };
@@ -105,8 +105,8 @@ gemm_skinny_kernel(const SkinnyParams p) {
 #pragma unroll
         for (int s = 0; s < CH; ++s)
             if (s0 + s < p.steps) {
-                al[s] = lo_ok && inside(s0 + s) ? __ldg(a_lo + (size_t)(s0 + s) * 4) : z;
-                ah[s] = hi_ok && inside(s0 + s) ? __ldg(a_hi + (size_t)(s0 + s) * 4) : z;
+                al[s] = lo_ok && inside(s0 + s) ? a_lo[(size_t)(s0 + s) * 4] : z;
+                ah[s] = hi_ok && inside(s0 + s) ? a_hi[(size_t)(s0 + s) * 4] : z;
             }
 #pragma unroll
         for (int s = 0; s < CH; ++s)

@@ -21,15 +21,14 @@ __device__ __forceinline__ float load_as_float<__nv_bfloat16>(const __nv_bfloat1
 
 // one thread per (token, kv head, pair)
 template <typename T>
-__global__ void kv_append_kernel(__nv_bfloat16* __restrict__ pool, int64_t pool_pages,
-                                 const int32_t* __restrict__ page_table, int max_pages,
-                                 const int32_t* __restrict__ seq_ids, const int32_t* __restrict__ positions, int T_,
-                                 const T* __restrict__ k_new, const T* __restrict__ v_new, int64_t row_stride, int Hkv,
-                                 int D, float theta) {
+__global__ void kv_append_kernel(__nv_bfloat16* pool, int64_t pool_pages, const int32_t* page_table, int max_pages,
+                                 const int32_t* seq_ids, const int32_t* positions, int T_, const T* k_new, const T* v_new,
+                                 int64_t row_stride, int Hkv, int D, float theta) {
     const int half = D / 2;
     const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     // launched as a programmatic dependent: the projections that produce k_new / v_new have completed after the wait;
-    // the decode kernel behind this one may begin its set-up and waits for this grid before it reads the pool
+    // the decode kernel behind this one may begin its set-up and waits for this grid before it reads the pool.  No pointer is
+    // __restrict__: see grid_dependency_wait
     ptx::grid_dependency_wait();
     ptx::grid_launch_dependents();
     if (idx >= (int64_t)T_ * Hkv * half) return;

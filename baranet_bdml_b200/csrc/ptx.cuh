@@ -174,9 +174,10 @@ __device__ __forceinline__ void tma_load_2d_hint(uint32_t smem_dst, const CUtens
 // Either order is sound.  With launch_dependents first, the kernel behind may be resident, and ask for its weights, before the
 // kernel ahead has finished; it waits for this grid, which ends only after its own wait, so all that came earlier has completed
 // when a wait returns.  Then every block has to wait, and what an earlier kernel wrote is read behind the wait by ordinary loads
-// or TMA, never by __ldg, whose lines may be as old as the block.  Where the next kernel's weights are worth it that order is
-// taken (gemm_rows, gqa_step, hyper_norm: a step of 64 sequences 283 -> 268 us); with it in all kernels the steps of 16 went from
-// 320 to 367 us, their waiting blocks being in the way of the streaming kernels' own.
+// or TMA, never by __ldg or a const __restrict__ pointer, whose lines may be as old as the block (test_dependent_launches.py).
+// Where the next kernel's weights are worth it that order is taken (gemm_rows, gqa_step, hyper_norm: a step of 64 sequences 283 ->
+// 268 us); with it in all kernels the steps of 16 went from 320 to 367 us, their waiting blocks being in the way of the streaming
+// kernels' own.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

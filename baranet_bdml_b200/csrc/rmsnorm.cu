@@ -225,9 +225,9 @@ rmsnorm_bf16_kernel(const RmsBf16Params p) {
         float acc = 0.f;
         auto weight = [&](int c) { return __ldg(reinterpret_cast<const uint4*>(p.w) + c); };
         auto fetch = [&](int c) {
-            uint4 x = __ldg(ar + c);
+            uint4 x = ar[c];                                    // ordinary loads: see grid_dependency_wait
             if (br) {
-                const uint4 y4 = __ldg(br + c);
+                const uint4 y4 = br[c];
                 uint32_t* xs = reinterpret_cast<uint32_t*>(&x);
                 const uint32_t* ys = reinterpret_cast<const uint32_t*>(&y4);
 #pragma unroll
