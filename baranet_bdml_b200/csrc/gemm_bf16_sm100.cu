@@ -537,7 +537,7 @@ static int gemm_launch(const void* a, const void* bt, void* c, int M, int N, int
                             : cudaMemsetAsync(c, 0, (size_t)M * n_out * 2, as_stream(stream));
         return e == cudaSuccess ? BN_OK : fail(BN_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
     }
-    if (epi != EPI_QKV && epi != EPI_PLAIN && gemm_rows_ok(M, n_out)) {
+    if (epi != EPI_QKV && epi != EPI_PLAIN && gemm_rows_ok(M, n_out, K, epi >= EPI_GLU)) {
         RowsGemm r{a, bt, static_cast<__nv_bfloat16*>(c), c32, static_cast<const __nv_bfloat16*>(mul), bias, error_word, mul_ld, M, N, K,
                    n_out, epi >= EPI_GLU ? epi - EPI_GLU : act, epi >= EPI_GLU};
         return gemm_rows(r, as_stream(stream), what);

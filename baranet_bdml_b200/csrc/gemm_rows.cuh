@@ -19,8 +19,8 @@ struct RowsGemm {
     bool glu;
 };
 
-// whether gemm_rows is the kernel for a product of M rows with n_out columns
-bool gemm_rows_ok(int M, int n_out);
+// whether gemm_rows is the kernel for a product of M rows with n_out columns (glu: of gate and up each)
+bool gemm_rows_ok(int M, int n_out, int K, bool glu);
 int gemm_rows(const RowsGemm& p, cudaStream_t st, const char* what);
 
 }  // namespace bn

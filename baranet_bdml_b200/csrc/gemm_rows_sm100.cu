@@ -4,7 +4,8 @@
 // start, and nothing else should pass through memory.  The weights are the MMA's 128-row operand and the rows of A its narrow
 // one (N = 32, 64 or 128): a stage of 64 k holds 16 KB of weights beside 4 - 16 KB of A.  A cluster of up to eight CTAs shares
 // an output tile, each with a range of K, and adds up through distributed shared memory in rank order; no partial sum goes to
-// global memory and there is no second launch.  Two CTAs fit on a multiprocessor, so that most shapes are one wave.
+// global memory and there is no second launch.  Two CTAs fit on a multiprocessor (of gate and up of more than 64 rows one), so that
+// most shapes are one wave.
 // A programmatic dependent: while the kernel ahead finishes, every CTA asks for all of its weights in L2.
 //
 // Epilogues: bf16, the fp32 sum, act(sum + bias), act(sum) * factor, act(gate) * up (two weight tiles, two accumulators).
@@ -28,6 +29,7 @@ template <int MT, int NW> struct RowsShape {
     static constexpr int LDP = GR_BN + 4;                                  // row stride of the sums, floats
     static constexpr int RING = NSTAGE * STAGE_BYTES, SUMS = NW * MT * LDP * 4;
     static constexpr int SMEM_BYTES = 1024 + (RING > SUMS ? RING : SUMS);
+    static constexpr int PER_SM = SMEM_BYTES <= 113 * 1024 ? 2 : 1;        // of 228 KB, 1 of them the system's for each CTA
     static constexpr uint32_t TMEM_COLS = NW * MT < 32 ? 32 : NW * MT;
 };
 
@@ -200,20 +202,37 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     }
 }
 
-// CTAs per output tile: the most, an even number, of which the GPU runs all at the same time - two per multiprocessor, less what
-// whole clusters do not fill (measured: 252 to 268 CTAs run together, 288 do not) - and that have 5 steps of 64 k each.
+// How many CTAs run together: one or two per multiprocessor, as their shared memory fits (gate and up of more than 64 rows: one),
+// less what whole clusters do not fill (measured with two: 252 to 268 CTAs run together, 288 do not).
+static int rows_resident(int per_sm) { return per_sm == 2 ? sm_count() * 9 / 5 + 2 : sm_count() * 9 / 10; }
+
+// CTAs per output tile: the most, an even number, of which the GPU runs all at the same time and that have 5 steps of 64 k each
+// (gemm_rows_ok: two of them always are).
 // 64 rows, us by ranks (2, 4, 6, 8): 2048 -> 4608 11.0, 9.1, 8.5, 12.8; 2048 -> 7424 13.0, 9.9, 14.4, 15.8; 2048 -> 2048 8.8, 6.2,
 // 5.9, 6.8; 7424 -> 2048 19.6, 13.6, 12.3, 12.1.
 // 64-wide tiles of 128 rows of A, K over single CTAs and a second launch for the sums took 12.7, 15.1, 9.7, 17.3 us (a weight of
-// 30 MB alone 4.7 us); gate and up of 5632 as 256-wide tiles 18.1, here 15.0 us.
-static int rows_ranks(int tiles, int steps, int sms) {
+// 30 MB alone 4.7 us).
+static int rows_ranks(int tiles, int steps, int resident) {
     int r = GR_MAX_CLUSTER;
-    while (r > 1 && (tiles * r > sms * 9 / 5 + 2 || steps < 5 * r)) r -= 2;
-    return r < 1 ? 1 : r;
+    while (r > 2 && (tiles * r > resident || steps < 5 * r)) r -= 2;
+    return r;
 }
 
-// With more tiles than that (half of what runs together) 128 x 256 tiles do as well: 2048 -> 32000 28.7 us there, 30.6 us here
-bool gemm_rows_ok(int M, int n_out) { return M <= GR_MAX_ROWS && ceil_div(n_out, GR_BN) * 2 <= sm_count() * 9 / 5 + 2; }
+// - With more tiles than half of what runs together 128 x 256 tiles do as well: 2048 -> 32000, 64 rows, 28.7 us there, 30.6 here.
+// - A short K leaves a tile to one or two CTAs, and the time is that of the sums' way, which grows with the rows: 256 -> 2048, 17 /
+//   64 / 128 rows, 4.2 / 6.7 / 10.2 us here, 4.5 / 4.7 / 5.9 as 128 x 256 tiles; 512 -> 8192 5.7 / 8.2 / 11.9, there 5.9 / 6.1 /
+//   7.2; 640 -> 2048 4.3 / 6.1 / 8.0, there 6.3 / 6.4 / 7.6, and with K over single CTAs 6.2 / 6.5 / 7.1; 1024 -> 2048 4.9 / 6.8 /
+//   8.8, that form 7.1 / 6.9 / 7.5; 2048 -> 2048 128 rows 8.8, that form 9.7.
+// - Gate and up take twice the shared memory and twice that way, and are faster than 256-wide tiles of both where four CTAs share a
+//   tile, or two and the rows are few: 2048 -> 5632, four CTAs, 17 / 64 rows 12.0 / 15.0 us, there 18.1, and two CTAs, 65 / 128 rows,
+//   18.4 / 20.7; 2048 -> 2816 65 / 128 rows 10.8 / 12.8, there 17.1; 2048 -> 8704, two CTAs, 17 / 64 rows 22.1 / 24.2, there 20.1;
+//   1024 -> 4096, two CTAs, 17 / 48 / 64 / 128 rows 9.6 / 11.2 / 12.1 / 13.7, there 11.4.
+bool gemm_rows_ok(int M, int n_out, int K, bool glu) {
+    if (M > GR_MAX_ROWS || K < 640) return false;
+    const int tiles = ceil_div(n_out, GR_BN);
+    if (!glu) return tiles * 2 <= rows_resident(2) && (M <= 64 || K >= 1280);
+    return tiles * 4 <= rows_resident(M <= 64 ? 2 : 1) && (M <= 48 || K >= 1280);
+}
 
 template <int MT, int NW>
 static int rows_launch(const RowsGemm& p, cudaStream_t st, const char* what) {
@@ -232,7 +251,7 @@ static int rows_launch(const RowsGemm& p, cudaStream_t st, const char* what) {
     if (int rc = make_tensor_map(&mw, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, p.w, dims_w, stride, box_w, CU_TENSOR_MAP_SWIZZLE_128B)) return rc;
     if (int rc = make_tensor_map(&ma, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, p.a, dims_a, stride, box_a, CU_TENSOR_MAP_SWIZZLE_128B)) return rc;
     const int tiles = (p.n_out + GR_BN - 1) / GR_BN, steps = (p.K + GR_BK - 1) / GR_BK;
-    const int ranks = rows_ranks(tiles, steps, sm_count());
+    const int ranks = rows_ranks(tiles, steps, rows_resident(Sh::PER_SM));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(tiles * ranks));
     cfg.blockDim = dim3(GR_THREADS);

@@ -205,10 +205,10 @@ def skinny_best(rows: int, n_out: int, k: int) -> bool:
     return skinny_any_k(rows, n_out, k) and (rows <= 4 or n_out < 6144 or (rows <= 8 and n_out > 17000))
 
 
-def small_m_ok(rows: int, n_out: int) -> bool:
-    """Few rows and too few 256-wide output tiles to occupy the GPU (measured cross-over: fewer than half as many tiles as
-    SMs): the form for up to 128 rows."""
-    return rows <= 128 and (n_out + 255) // 256 < 74
+def small_m_ok(rows: int, n_out: int, k: int) -> bool:
+    """Shapes for which the form for up to 128 rows is the fastest: a K long enough to be shared by CTAs, and too few 128-wide
+    output tiles to occupy the GPU (us at 64 rows: 512 -> 8192 8.2, in 128 x 256 tiles 6.1; 2048 -> 32000 30.6 and 28.7)."""
+    return rows <= 128 and k >= 640 and n_out <= 134 * 128
 
 
 def gemm_bf16_nt_skinny(x: torch.Tensor, weight_t: torch.Tensor, splits: Optional[Tuple[int, ...]] = None):
@@ -273,7 +273,7 @@ def linear_bf16(x: torch.Tensor, weight_t: torch.Tensor) -> torch.Tensor:
     rows, n_out = x.shape[0], weight_t.shape[0]
     if skinny_best(rows, n_out, x.shape[1]):
         return gemm_bf16_nt_skinny(x, weight_t)
-    if small_m_ok(rows, n_out):
+    if small_m_ok(rows, n_out, x.shape[1]):
         return gemm_bf16_nt_small_m(x, weight_t)
     return gemm_bf16_nt(x, weight_t)
 
@@ -511,7 +511,7 @@ class Linear:
         if skinny_best(rows, self.n, self.k):
             _lib.check(lib.bn_gemm_bf16_nt_skinny_f32(x.data_ptr(), self.weight.data_ptr(), rows, self.n, self.k,
                                                       out.data_ptr(), _stream()))
-        elif small_m_ok(rows, self.n):
+        elif small_m_ok(rows, self.n, self.k):
             ws, n = _small_m_scratch(x.device, rows, self.n, self.k)
             _lib.check(lib.bn_gemm_bf16_nt_small_m_f32(x.data_ptr(), self.weight.data_ptr(), out.data_ptr(), rows, self.n,
                                                        self.k, ws.data_ptr(), n, _gemm_error_ptr(x.device, None), _stream()))
@@ -526,7 +526,7 @@ class Linear:
         if skinny_best(rows, self.n, self.k):
             _lib.check(lib.bn_gemm_bias_act_bf16_nt_skinny(x.data_ptr(), self.weight.data_ptr(), _ptr(self.bias), out.data_ptr(), rows,
                                                            self.n, self.k, a, _stream()))
-        elif small_m_ok(rows, self.n):
+        elif small_m_ok(rows, self.n, self.k):
             ws, n = _small_m_scratch(x.device, rows, self.n, self.k)
             _lib.check(lib.bn_gemm_bias_act_bf16_nt_small_m(x.data_ptr(), self.weight.data_ptr(), _ptr(self.bias), out.data_ptr(), rows,
                                                             self.n, self.k, a, ws.data_ptr(), n, _gemm_error_ptr(x.device, None),
@@ -554,7 +554,7 @@ class Linear:
         elif skinny_best(rows, self.n, self.k):
             _lib.check(lib.bn_gemm_act_mul_bf16_nt_skinny(x.data_ptr(), self.weight.data_ptr(), mul.data_ptr(), mul.stride(0),
                                                           out.data_ptr(), rows, self.n, self.k, a, _stream()))
-        elif small_m_ok(rows, self.n):
+        elif small_m_ok(rows, self.n, self.k):
             ws, n = _small_m_scratch(x.device, rows, self.n, self.k)
             _lib.check(lib.bn_gemm_act_mul_bf16_nt_small_m(x.data_ptr(), self.weight.data_ptr(), mul.data_ptr(), mul.stride(0),
                                                            out.data_ptr(), rows, self.n, self.k, a, ws.data_ptr(), n,

@@ -187,10 +187,12 @@ def test_graphed_decoder_layer_equals_eager(lib):
         assert torch.equal(res_e, res_g) and torch.equal(mlp_e, mlp_g)
 
 
-# rows around the widths of the narrow operand; K of one step, of less than five per CTA, ragged, and of full clusters; columns
-# of one 128-wide tile, of a part of one, and of so many tiles that a CTA has a tile to itself
-@pytest.mark.parametrize("M", [1, 17, 32, 33, 64, 65, 128])
-@pytest.mark.parametrize("N,K", [(8, 8), (136, 328), (256, 2120), (2048, 2048), (16896, 128)])
+# rows around the widths of the narrow operand and at the lines of the dispatch; K on both sides of its lines (640, 1280), ragged,
+# and of full clusters; columns of one 128-wide tile, of a part of one, and on both sides of the most that clusters of two (17152)
+# and gate and up in clusters of four (4224, 8576) are for
+@pytest.mark.parametrize("M", [1, 17, 32, 33, 48, 49, 64, 65, 128])
+@pytest.mark.parametrize("N,K", [(8, 8), (136, 328), (256, 2120), (2048, 2048), (16896, 128), (8, 632), (136, 648), (264, 1272), (264, 1288),
+                                 (17152, 640), (17160, 640), (4224, 1280), (4232, 1280), (8576, 640), (8584, 640)])
 def test_small_m_epilogues(lib, M, N, K):
     from baranet_bdml_b200 import _lib, ops
     gen = torch.Generator(device="cuda").manual_seed(M * 31 + N + K)
