@@ -199,10 +199,12 @@ def skinny_any_k(rows: int, n_out: int, k: int) -> bool:
 
 
 def skinny_best(rows: int, n_out: int, k: int) -> bool:
-    """Those of them for which it is the fastest.  Its CTAs read the rows for every 8 columns of the weight, which shows with
-    many of both: us at 16 rows, 2048 -> 7424 11.2 (the kernel for up to 128 rows: 8.3), 2048 -> 8512 11.6 (8.8), 2048 -> 4608
-    6.4 (6.8); 2048 -> 32000 32.5 (128 x 256 tiles: 27.3), the same at 8 rows 27.0 (26.9)."""
-    return skinny_any_k(rows, n_out, k) and (rows <= 4 or n_out < 6144 or (rows <= 8 and n_out > 17000))
+    """Those of them for which it is the fastest, by whole steps of 1 to 16 sequences.  Its CTAs read the rows for every 8 columns
+    of the weight, which shows with many rows and a wide or a long weight: us at 16 rows, 2048 -> 2048 4.2 (the kernel for up to
+    128 rows: 4.8), 4096 -> 2048 6.4 (6.4), 7424 -> 2048 9.9 (9.6), 2048 -> 4608 7.1 (6.6), 2048 -> 7424 12.0 (8.2), 512 -> 7424
+    5.0 (128 x 256 tiles: 5.7).  A Duponex step of 16 / 12 / 9 sequences, 2 layers, takes 127 / 125 / 122 us, with every product
+    here 152 / 140 / 126; of 5 sequences 117, with the wide ones in the other kernel 119."""
+    return skinny_any_k(rows, n_out, k) and (rows <= 8 or (n_out < 4096 and k <= 4096) or k < 640)
 
 
 def small_m_ok(rows: int, n_out: int, k: int) -> bool:
