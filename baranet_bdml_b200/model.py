@@ -16,7 +16,7 @@ import numpy as np
 import torch
 
 from . import _lib, ops
-from .kv_cache import PAGE_TOKENS, PagedKVCache, SequenceSlots
+from .kv_cache import PAGE_TOKENS, PagedKVCache, SequenceSlots, ZeroedTogether
 from .layers import LLaMAConfig, LLaMADecoderLayerBF16
 
 
@@ -287,10 +287,13 @@ class LLaMAModelBF16(CausalLM):
     def _alloc_caches(self, B: int, max_len: int):
         cfg = self.config
         pages_per_seq = (max_len + PAGE_TOKENS - 1) // PAGE_TOKENS
-        # every block holds the same tokens: ONE length vector, advanced once per step; pools and page tables are parts of one
-        # tensor each, so that they are filled by one launch
+        self.caches = []              # those of an earlier prompt make room first
+        # every block holds the same tokens: ONE length vector, advanced once per step; the pools are zeroed by one launch, and the
+        # page tables are parts of one tensor
         n, pages = len(self.layers), B * pages_per_seq
-        pools = torch.zeros((n, pages, cfg.num_key_value_heads, 2, PAGE_TOKENS, cfg.head_dim), dtype=torch.bfloat16, device="cuda")
+        zeros = ZeroedTogether()
+        pools = [zeros((pages, cfg.num_key_value_heads, 2, PAGE_TOKENS, cfg.head_dim), dtype=torch.bfloat16, device="cuda") for _ in range(n)]
+        zeros.fill()
         tables = torch.arange(pages, dtype=torch.int32, device="cuda").view(B, pages_per_seq).repeat(n, 1, 1)
         lens = torch.zeros((B,), dtype=torch.int32, device="cuda")
         self.caches = [PagedKVCache(pages, B, pages_per_seq, cfg.num_key_value_heads, cfg.head_dim, cfg.rope_theta,

@@ -140,3 +140,18 @@ def test_model_status_reads_the_gemm_error_word(lib):
         model.status()
     model.status()
     assert int(word.item()) == 0
+
+
+def test_a_prompt_takes_the_place_of_the_one_before(lib):
+    """The caches of an earlier prompt are given back before those of the next are allocated, and a block's pool is a tensor of
+    its own (kept or saved alone, it takes no more than its own bytes)."""
+    model = tiny_model(1)
+    ids = torch.ones((2, 8), dtype=torch.int32, device="cuda")
+    model.prefill(ids, 1 << 16)
+    pool = sum(c.pool.numel() * 2 for c in model.caches)
+    assert all(c.pool.untyped_storage().nbytes() == c.pool.numel() * 2 for c in model.caches)
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    model.prefill(ids, 1 << 16)
+    assert pool > 1 << 26 and torch.cuda.max_memory_allocated() < before + pool // 4
