@@ -58,7 +58,7 @@ struct SkinnyParams {
 // registers for more CTAs per SM (8: two, 2: four), which matters when the grid would otherwise need a second, nearly
 // empty wave.
 template <bool SWIGLU, int CH, bool APPEND = false, bool RAGGED = false>
-__global__ void __launch_bounds__(SK_WARPS * 32)
+__global__ void __launch_bounds__(SK_WARPS * 32, CH == 8 ? 2 : SWIGLU ? 3 : 4)
 gemm_skinny_kernel(const SkinnyParams p) {
     __shared__ float s_part[SK_WARPS][2][16][8 + 1];
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
@@ -100,26 +100,47 @@ gemm_skinny_kernel(const SkinnyParams p) {
     }
     grid_dependency_wait();
     grid_launch_dependents();
-    for (int s0 = 0; s0 < p.steps; s0 += CH) {
-        load_weights(s0);
+    auto load_rows = [&](int s0, uint4 (&lo)[CH], uint4 (&hi)[CH]) {
 #pragma unroll
         for (int s = 0; s < CH; ++s)
             if (s0 + s < p.steps) {
-                al[s] = lo_ok && inside(s0 + s) ? a_lo[(size_t)(s0 + s) * 4] : z;
-                ah[s] = hi_ok && inside(s0 + s) ? a_hi[(size_t)(s0 + s) * 4] : z;
+                lo[s] = lo_ok && inside(s0 + s) ? a_lo[(size_t)(s0 + s) * 4] : z;
+                hi[s] = hi_ok && inside(s0 + s) ? a_hi[(size_t)(s0 + s) * 4] : z;
             }
+    };
+    auto multiply = [&](int s0, const uint4 (&lo)[CH], const uint4 (&hi)[CH]) {
 #pragma unroll
         for (int s = 0; s < CH; ++s)
             if (s0 + s < p.steps) {
                 // two k16 MMAs per step: the lane's first four K positions play (2j, 2j+1, 2j+8, 2j+9) of the first,
                 // its last four of the second, in A and B alike
-                mma_bf16_16816(acc, al[s].x, ah[s].x, al[s].y, ah[s].y, wv[s].x, wv[s].y);
-                mma_bf16_16816(acc, al[s].z, ah[s].z, al[s].w, ah[s].w, wv[s].z, wv[s].w);
+                mma_bf16_16816(acc, lo[s].x, hi[s].x, lo[s].y, hi[s].y, wv[s].x, wv[s].y);
+                mma_bf16_16816(acc, lo[s].z, hi[s].z, lo[s].w, hi[s].w, wv[s].z, wv[s].w);
                 if (SWIGLU) {
-                    mma_bf16_16816(acc2, al[s].x, ah[s].x, al[s].y, ah[s].y, wv2[s].x, wv2[s].y);
-                    mma_bf16_16816(acc2, al[s].z, ah[s].z, al[s].w, ah[s].w, wv2[s].z, wv2[s].w);
+                    mma_bf16_16816(acc2, lo[s].x, hi[s].x, lo[s].y, hi[s].y, wv2[s].x, wv2[s].y);
+                    mma_bf16_16816(acc2, lo[s].z, hi[s].z, lo[s].w, hi[s].w, wv2[s].z, wv2[s].w);
                 }
             }
+    };
+    if (CH == 2 && !RAGGED && p.M > 4) {
+        // short batches: the next batch's activations are requested ahead of this one's arithmetic, too (a LLaMA step of 16
+        // sequences, 4 blocks, 300 us; without 314; a single row has little to wait for: a Soluzen step 254.5 us, with it 255.5)
+        uint4 nl[CH], nh[CH];
+        load_rows(0, al, ah);
+        for (int s0 = 0; s0 < p.steps; s0 += 2 * CH) {
+            load_weights(s0);
+            load_rows(s0 + CH, nl, nh);
+            multiply(s0, al, ah);
+            load_weights(s0 + CH);
+            load_rows(s0 + 2 * CH, al, ah);
+            multiply(s0 + CH, nl, nh);
+        }
+    } else {
+        for (int s0 = 0; s0 < p.steps; s0 += CH) {
+            load_weights(s0);
+            load_rows(s0, al, ah);
+            multiply(s0, al, ah);
+        }
     }
     // C fragment: acc[0], acc[1] = row g, columns 2j, 2j+1; acc[2], acc[3] = row g + 8
     s_part[warp][0][g][2 * j] = acc[0];
