@@ -18,6 +18,7 @@ BN_OK, BN_ERR_INVALID_ARG, BN_ERR_UNSUPPORTED, BN_ERR_CUDA, BN_ERR_ARCH, BN_ERR_
 BN_HEADS_COLLAPSED, BN_HEADS_PER_HEAD = 0, 1
 BN_PAGE_TOKENS = 16
 BN_ACT_NONE, BN_ACT_SILU, BN_ACT_GELU_TANH, BN_ACT_RELU2 = range(4)
+BN_LINEAR_F32_CHAINS, BN_LINEAR_F32_SUMS, BN_LINEAR_F32_PARTS = 0, 1, 2
 
 _i, _i64, _f, _p, _sz = C.c_int, C.c_int64, C.c_float, C.c_void_p, C.c_size_t
 
@@ -26,11 +27,12 @@ SIGNATURES = {
     "bn_last_error": (C.c_char_p, []),
     "bn_version": (_i, []),
     "bn_mm_f32": (_i, [_p, _i64, _i64, _p, _i64, _i64, _p, _i64, _i64, _i, _i, _i, _p]),
+    "bn_mm_f32_sums": (_i, [_p, _i64, _p, _i64, _p, _i64, _i, _i, _i, _p]),
     "bn_split_f32": (_i, [_p, _i64, _p, _i, _i, _p]),
     "bn_mm_f32_split": (_i, [_p, _p, _i, _p, _i64, _p, _i64, _p, _i, _p, _i, _i, _i, _p, _p]),
     "bn_mm_f32_each": (_i, [_p, _i64, _i64, _i, _p, _p, _p, _p, _p, _p, _i, _i, _p, _p]),
     "bn_linear_f32_workspace_bytes": (_sz, [_i, _i, _i]),
-    "bn_linear_f32_pays": (_i, [_i, _i, _i, _i]),
+    "bn_linear_f32_form": (_i, [_i, _i, _i, _i]),
     "bn_linear_f32": (_i, [_p, _i64, _p, _i64, _p, _i, _p, _i, _i, _i, _p, _sz, _p, _p]),
     "bn_rope_f32": (_i, [_p, _i64, _i64, _p, _i64, _i64, _i, _i, _i, _f, _i, _p]),
     "bn_embedding_gather_f32": (_i, [_p, _i64, _p, _p, _i64, _i, _i, _i, _p, _p]),

@@ -37,7 +37,11 @@ struct MmParams {
 
 // VA / VB: 16-byte copies along the operand's contiguous dimension (K for A; K for B, or N with B_N).  B_N: B lies in shared
 // memory with N contiguous.
-template <int BM, int BN, int TM, int TN, bool VA, bool VB, bool B_N>
+// SUMS: not one chain, but chains of 16 k, added up by eights, and these in a third sum: the error of K = 2048 falls from 8.1e-7 to
+// 1.2e-7, of K = 7424 from 1.5e-6 to 1.7e-7 (2-norms, against 64 bits).  4 x 2048 -> 32000 86.5 us either way; where the time is the
+// latency of few tiles the additions show: 1 x 2048 -> 2048 23.0 us, sums 27.1; 4 x 7424 -> 2048 108.9 and 115.3.  (Chains of 16 in
+// one sum 24.9 us and 2.2e-7, chains of 64 27.7 us and 1.8e-7.)
+template <int BM, int BN, int TM, int TN, bool VA, bool VB, bool B_N, bool SUMS>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN))
 mm_f32_kernel(const __grid_constant__ MmParams p) {
     constexpr int THREADS = (BM / TM) * (BN / TN), ROWS_T = BM / TM, COLS_T = BN / TN;
@@ -113,11 +117,21 @@ mm_f32_kernel(const __grid_constant__ MmParams p) {
         }
     };
 
-    float acc[TM][TN];
+    float acc[TM][TN], eights[TM][TN], total[TM][TN];
+    // SUMS: takes a sum into the next one
+    auto fold = [](float (&from)[TM][TN], float (&into)[TM][TN]) {
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+            for (int j = 0; j < TN; ++j) {
+                into[i][j] += from[i][j];
+                from[i][j] = 0.f;
+            }
+    };
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+        for (int j = 0; j < TN; ++j) acc[i][j] = eights[i][j] = total[i][j] = 0.f;
 
     // the operands of four k: b[column][k], or with B_N4 b[column group * 4 + k][column of the group]
     struct Frag { float a[TM][4], b[TN][4]; };
@@ -174,7 +188,12 @@ mm_f32_kernel(const __grid_constant__ MmParams p) {
                     for (int j = 0; j < TN; ++j)
                         acc[i][j] = fmaf(c.a[i][e], B_N4 ? c.b[j / 4 * 4 + e][j % 4] : c.b[j][e], acc[i][j]);
         }
+        if (SUMS) {
+            fold(acc, eights);
+            if (step % 8 == 7) fold(eights, total);
+        }
     }
+    if (SUMS) fold(eights, total);
 #pragma unroll
     for (int i = 0; i < TM; ++i) {
         const int r = row0 + ty + i * ROWS_T;
@@ -182,24 +201,24 @@ mm_f32_kernel(const __grid_constant__ MmParams p) {
 #pragma unroll
         for (int j = 0; j < TN; ++j) {
             const int c = col0 + (B_N4 ? (tx + j / 4 * COLS_T) * 4 + j % 4 : tx + j * COLS_T);
-            if (c < q.N) q.C[r * q.c_rs + c * q.c_cs] = acc[i][j];
+            if (c < q.N) q.C[r * q.c_rs + c * q.c_cs] = SUMS ? total[i][j] : acc[i][j];
         }
     }
 }
 
-template <int BM, int BN, int TM, int TN, bool VA, bool VB, bool B_N>
+template <int BM, int BN, int TM, int TN, bool VA, bool VB, bool B_N, bool SUMS>
 static int mm_f32_run(MmParams p, cudaStream_t st) {
     constexpr size_t smem = (size_t)MM_STAGES * (BM * MM_LD + (B_N ? MM_K * BN : BN * MM_LD)) * sizeof(float);
-    if (int rc = allow_smem(mm_f32_kernel<BM, BN, TM, TN, VA, VB, B_N>, smem, "bn_mm_f32")) return rc;
+    if (int rc = allow_smem(mm_f32_kernel<BM, BN, TM, TN, VA, VB, B_N, SUMS>, smem, "bn_mm_f32")) return rc;
     for (int s = 0; s < MM_SETS; ++s) p.tile_end[s] = (s ? p.tile_end[s - 1] : 0) + (s < p.sets ? ceil_div(p.set[s].N, BN) : 0);
     const dim3 grid(p.tile_end[MM_SETS - 1], ceil_div(p.M, BM));
     if (grid.y > 65535) return fail(BN_ERR_UNSUPPORTED, "bn_mm_f32: M=%d too large", p.M);
-    mm_f32_kernel<BM, BN, TM, TN, VA, VB, B_N><<<grid, (BM / TM) * (BN / TN), smem, st>>>(p);
+    mm_f32_kernel<BM, BN, TM, TN, VA, VB, B_N, SUMS><<<grid, (BM / TM) * (BN / TN), smem, st>>>(p);
     return launch_status("bn_mm_f32");
 }
 
 // How the operands can be copied: A and B along K, B along N, 16 bytes at a time where the strides and addresses allow it.
-template <int BM, int BN, int TM, int TN>
+template <int BM, int BN, int TM, int TN, bool SUMS>
 static int mm_f32_copies(const MmParams& p, cudaStream_t st) {
     auto fours = [](const float* x, int64_t contiguous, int64_t other, int n) {
         return contiguous == 1 && other % 4 == 0 && n % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
@@ -210,9 +229,10 @@ static int mm_f32_copies(const MmParams& p, cudaStream_t st) {
         along_n = along_n && fours(p.set[s].B, p.set[s].b_cs, p.set[s].b_rs, p.set[s].N);
         along_k = along_k && fours(p.set[s].B, p.set[s].b_rs, p.set[s].b_cs, p.K);
     }
-    if (along_n) return mm_f32_run<BM, BN, TM, TN, true, true, true>(p, st);
-    if (along_k) return mm_f32_run<BM, BN, TM, TN, true, true, false>(p, st);
-    return mm_f32_run<BM, BN, TM, TN, false, false, false>(p, st);
+    if constexpr (!SUMS)
+        if (along_n) return mm_f32_run<BM, BN, TM, TN, true, true, true, SUMS>(p, st);
+    if (along_k) return mm_f32_run<BM, BN, TM, TN, true, true, false, SUMS>(p, st);
+    return mm_f32_run<BM, BN, TM, TN, false, false, false, SUMS>(p, st);
 }
 
 // The tile by an estimate of the time: a tile alone on a multiprocessor takes `alone` (its chains' latency), several there take
@@ -221,7 +241,8 @@ static int mm_f32_copies(const MmParams& p, cudaStream_t st) {
 // that reading (8 x 4 outputs a thread: 12 16-byte reads, 4 cycles each, for 128 FMAs), 53 - 60 % of the FMA rate.
 // One 64 x 64 tile of 4 x 4 outputs a thread without copies in flight, before / after: 128 x 2048 x 2048 134 / 52 us,
 // 128 x 256 x 2048 134 / 24 us, 800 x 7424 x 2048 1470 / 610 us, 4 x 32000 x 2048 570 / 88 us.
-static float mm_f32_times(int M, const int* N, int sets, int* best) {
+// sums: without the largest tile, whose threads have no registers for three sums
+static float mm_f32_times(int M, const int* N, int sets, bool sums, int* best) {
     const int sms = sm_count();
     auto estimate = [&](int bm, int bn, float alone, float more) {
         long long tiles = 0;
@@ -231,28 +252,30 @@ static float mm_f32_times(int M, const int* N, int sets, int* best) {
     };
     const float t[5] = {estimate(128, 128, 221.f, 220.f), estimate(64, 64, 77.f, 62.f), estimate(32, 64, 52.f, 34.f),
                         estimate(16, 32, 33.f, 16.f), estimate(8, 32, 24.f, 10.4f)};
-    *best = 0;
-    for (int i = 1; i < 5; ++i)
+    *best = sums ? 1 : 0;
+    for (int i = *best + 1; i < 5; ++i)
         if (t[i] < t[*best]) *best = i;
     return t[*best];
 }
 
+template <bool SUMS>
 static int mm_f32_pick(const MmParams& p, cudaStream_t st) {
     int best, n[MM_SETS];
     for (int s = 0; s < p.sets; ++s) n[s] = p.set[s].N;
-    mm_f32_times(p.M, n, p.sets, &best);
+    mm_f32_times(p.M, n, p.sets, SUMS, &best);
     switch (best) {
-        case 0: return mm_f32_copies<128, 128, 8, 8>(p, st);
-        case 1: return mm_f32_copies<64, 64, 8, 4>(p, st);
-        case 2: return mm_f32_copies<32, 64, 4, 4>(p, st);
-        case 3: return mm_f32_copies<16, 32, 4, 2>(p, st);
-        default: return mm_f32_copies<8, 32, 2, 1>(p, st);
+        case 0:
+            if constexpr (!SUMS) return mm_f32_copies<128, 128, 8, 8, false>(p, st);
+        case 1: return mm_f32_copies<64, 64, 8, 4, SUMS>(p, st);
+        case 2: return mm_f32_copies<32, 64, 4, 4, SUMS>(p, st);
+        case 3: return mm_f32_copies<16, 32, 4, 2, SUMS>(p, st);
+        default: return mm_f32_copies<8, 32, 2, 1, SUMS>(p, st);
     }
 }
 
 float mm_f32_estimate(int M, int N, int K) {
     int best;
-    return mm_f32_times(M, &N, 1, &best) * (float)K / 2048.f;
+    return mm_f32_times(M, &N, 1, false, &best) * (float)K / 2048.f;
 }
 
 // x = act(x + bias) in place, fp32 rows (the unfused form of the products with a bias or an activation)
@@ -275,7 +298,18 @@ extern "C" int bn_mm_f32(const float* A, int64_t a_rs, int64_t a_cs, const float
     if (int rc = require_sm100()) return rc;
     if (M == 0 || N == 0) return BN_OK;
     MmParams p{A, a_rs, a_cs, M, K, 1, {{B, C, b_rs, b_cs, c_rs, c_cs, N}}, {}};
-    return mm_f32_pick(p, as_stream(stream));
+    return mm_f32_pick<false>(p, as_stream(stream));
+}
+
+extern "C" int bn_mm_f32_sums(const float* a, int64_t a_ld, const float* w, int64_t w_ld, float* c, int64_t c_ld, int M, int N, int K,
+                              bn_stream_t stream) {
+    if (!a || !w || !c) return fail(BN_ERR_INVALID_ARG, "bn_mm_f32_sums: null pointer");
+    if (M < 0 || K < 0 || N < 0) return fail(BN_ERR_INVALID_ARG, "bn_mm_f32_sums: negative size");
+    if (int rc = require_sm100()) return rc;
+    if (M == 0 || N == 0) return BN_OK;
+    MmParams p{a, a_ld, 1, M, K, 1, {{w, c, 1, w_ld, c_ld, 1, N}}, {}};
+    if (ceil_div(M, 64) > 65535) return mm_f32_pick<false>(p, as_stream(stream));      // the grid's limit
+    return mm_f32_pick<true>(p, as_stream(stream));
 }
 
 extern "C" int bn_mm_f32_each(const float* A, int64_t a_rs, int64_t a_cs, int n, const float* const* B, const int64_t* b_rs,
@@ -291,7 +325,7 @@ extern "C" int bn_mm_f32_each(const float* A, int64_t a_rs, int64_t a_cs, int n,
     }
     if (int rc = require_sm100()) return rc;
     if (M == 0 || p.sets == 0) return BN_OK;
-    return mm_f32_pick(p, as_stream(stream));
+    return mm_f32_pick<false>(p, as_stream(stream));
 }
 
 extern "C" int bn_bias_act_f32(float* x, int64_t ld, const float* bias, int rows, int cols, int act, bn_stream_t stream) {

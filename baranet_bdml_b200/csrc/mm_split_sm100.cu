@@ -132,6 +132,7 @@ mm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tmem = s_tmem_base;
+    grid_dependency_wait();                                    // a programmatic dependent, as the cut in front of it
 
     if (warp == 9) {
         if (lane == 0) {
@@ -308,6 +309,8 @@ struct CutParams {
 template <int BN>
 __global__ void __launch_bounds__(BN * 4)
 cut_operands_kernel(const CutParams p) {
+    grid_dependency_wait();
+    grid_launch_dependents();
     if ((int)blockIdx.x >= p.w_blocks) {
         cut_rows(p.a, p.a_ld, p.a_parts, p.M, p.K, (long long)(blockIdx.x - p.w_blocks) * (BN * 4) + threadIdx.x,
                  (long long)(gridDim.x - p.w_blocks) * (BN * 4));
@@ -362,7 +365,7 @@ static int split_launch(const void* a_parts, const void* w_parts, const SplitPar
     if (int rc = make_tensor_map(&mw, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, w_parts, dims_w, stride, box_w, CU_TENSOR_MAP_SWIZZLE_128B)) return rc;
     const long long tiles = (long long)ceil_div(p.M, MS_BM) * ceil_div(p.N, BN);
     const int sms = sm_count();
-    mm_split_kernel<BN><<<(unsigned)(tiles < sms ? tiles : sms), MS_THREADS, Sh::SMEM_BYTES, st>>>(ma, mw, p);
+    launch_dependent(mm_split_kernel<BN>, (unsigned)(tiles < sms ? tiles : sms), MS_THREADS, Sh::SMEM_BYTES, st, ma, mw, p);
     return launch_status(what);
 }
 
@@ -443,12 +446,19 @@ static bool split_fits(int M, int N, int K) {
 
 extern "C" size_t bn_linear_f32_workspace_bytes(int M, int N, int K) { return M <= 0 || N <= 0 || K <= 0 ? 0 : cut_layout(M, N, K).total; }
 
-extern "C" int bn_linear_f32_pays(int M, int N, int K, int w_nparts) {
-    if (M <= 0 || N <= 0 || K <= 0 || N % 8 || K % 8 || !split_fits(M, N, K)) return 0;
+// How a product is taken, by estimates in us (measured, one part / three): operands cut, where that takes less time than bn_mm_f32;
+// with up to 16 rows it does not, the weight being cut for them alone (2048 -> 32000, 4 / 16 / 32 rows: 169, 115, 114 / 251, 192,
+// 192 us, chains 87, 100, 153).  Where the parts alone would have been faster (4 rows 108 us with the cut elsewhere, 16 rows 59), the
+// weight is wide enough for bn_mm_f32_sums to hide its additions (4 / 12 rows 86.5 / 94.7 us, chains 86.5 / 91.9), and the error is
+// the smaller one again; narrower weights, whose time is a chain's latency, keep the chains (1 x 2048 -> 2048 23.0 us, sums 27.1).
+extern "C" int bn_linear_f32_form(int M, int N, int K, int w_nparts) {
+    if (M <= 0 || N <= 0 || K <= 0 || N % 8 || K % 8 || !split_fits(M, N, K)) return BN_LINEAR_F32_CHAINS;
     int bn;
+    const float product = split_estimate(M, N, K, w_nparts, &bn), chains = mm_f32_estimate(M, N, K);
     // starts, the cut of the weight (6 or 10 bytes each) and of A
     const float cut = 6.f + (float)N * (float)K * (w_nparts == 1 ? 0.8e-6f : 1.4e-6f) + (float)M * (float)K * 1.0e-6f;
-    return cut + split_estimate(M, N, K, w_nparts, &bn) < mm_f32_estimate(M, N, K);
+    if (M > 16 && cut + product < chains) return BN_LINEAR_F32_PARTS;
+    return 11.f + (float)M * (float)K * 1.2e-6f + product < chains ? BN_LINEAR_F32_SUMS : BN_LINEAR_F32_CHAINS;
 }
 
 extern "C" int bn_linear_f32(const float* a, int64_t a_ld, const float* w, int64_t w_ld, const float* bias, int act, float* c, int M,
@@ -473,8 +483,8 @@ extern "C" int bn_linear_f32(const float* a, int64_t a_ld, const float* w, int64
     const CutParams cp{a, w, reinterpret_cast<__nv_bfloat16*>(ws), reinterpret_cast<__nv_bfloat16*>(ws + l.w_parts), ws + l.counts, a_ld, w_ld, M, N,
                        K, ceil_div(N, bn) * ceil_div(K, MS_BK)};
     const unsigned grid = (unsigned)(cp.w_blocks + (blocks_a < 4096 ? blocks_a : 4096));
-    if (bn == 64) cut_operands_kernel<64><<<grid, 256, 0, st>>>(cp);
-    else cut_operands_kernel<128><<<grid, 512, 0, st>>>(cp);
+    if (bn == 64) launch_dependent(cut_operands_kernel<64>, grid, 256, 0, st, cp);
+    else launch_dependent(cut_operands_kernel<128>, grid, 512, 0, st, cp);
     if (int rc = launch_status(what)) return rc;
     const SplitParams p{a, w, bias, c, error_word, cp.counts, a_ld, w_ld, M, N, K, act, 0};
     return split_run(bn, cp.a_parts, cp.w_parts, p, st, what);

@@ -454,7 +454,8 @@ def _bf16_parts(x: torch.Tensor) -> torch.Tensor:
 
 class Linear:
     """y = act(x W^T + bias) for a weight (out, in), bias (out) and act optional: bf16 on the tensor cores, or true fp32 (chains
-    of FMAs, `bn_mm_f32`, or for many rows `bn_linear_f32`, whose error is smaller; both read `weight` as it is at the call).
+    of FMAs or sums of chains, `bn_mm_f32` and `bn_mm_f32_sums`, or for many rows `bn_linear_f32`, whose error is as small as that
+    of the sums; all read `weight` as it is at the call).
     Both sizes are rounded up to multiples of 8 with zeros, so x may be passed with its padding columns (which must be finite)
     and y has them."""
 
@@ -485,14 +486,19 @@ class Linear:
     def _mm_f32(self, x: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
         """x W^T with the bias and the activation, fp32"""
         w, rows, lib, act = self.weight, x.shape[0], _lib.load(), ACTIVATIONS[self.act]
-        if (x.data_ptr() | w.data_ptr()) % 16 == 0 and w.stride(0) % 4 == 0 and lib.bn_linear_f32_pays(rows, self.n, self.k, self.parts_hint):
+        form = lib.bn_linear_f32_form(rows, self.n, self.k, self.parts_hint)
+        if form == _lib.BN_LINEAR_F32_PARTS and (x.data_ptr() | w.data_ptr()) % 16 == 0 and w.stride(0) % 4 == 0:
             scratch = torch.empty(lib.bn_linear_f32_workspace_bytes(rows, self.n, self.k), dtype=torch.uint8, device=x.device)
             _lib.check(lib.bn_linear_f32(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), _ptr(self.bias), act,
                                          out.data_ptr(), rows, self.n, self.k, scratch.data_ptr(), scratch.numel(),
                                          _gemm_error_ptr(x.device, None), _stream()))
             return out
-        _lib.check(lib.bn_mm_f32(x.data_ptr(), x.stride(0), 1, w.data_ptr(), 1, w.stride(0), out.data_ptr(), out.stride(0), 1, rows,
-                                 self.k, self.n, _stream()))
+        if form == _lib.BN_LINEAR_F32_CHAINS:
+            _lib.check(lib.bn_mm_f32(x.data_ptr(), x.stride(0), 1, w.data_ptr(), 1, w.stride(0), out.data_ptr(), out.stride(0), 1, rows,
+                                     self.k, self.n, _stream()))
+        else:
+            _lib.check(lib.bn_mm_f32_sums(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0), rows, self.n,
+                                          self.k, _stream()))
         if self.bias is not None or self.act != "none":
             _lib.check(lib.bn_bias_act_f32(out.data_ptr(), self.n, _ptr(self.bias), rows, self.n, act, _stream()))
         return out

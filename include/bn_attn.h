@@ -99,6 +99,10 @@ BN_API int bn_selftest_wait_timeout(void* workspace, unsigned limit_us, bn_strea
 BN_API int bn_mm_f32(const float* A, int64_t a_rs, int64_t a_cs, const float* B, int64_t b_rs, int64_t b_cs,
               float* C, int64_t c_rs, int64_t c_cs, int M, int K, int N, bn_stream_t stream);
 
+/* C(M,N) = A(M,K) W(N,K)^T, rows of contiguous elements, with sums of sums in place of the one chain: a smaller error. */
+BN_API int bn_mm_f32_sums(const float* a, int64_t a_ld, const float* w, int64_t w_ld, float* c, int64_t c_ld, int M, int N, int K,
+                          bn_stream_t stream);
+
 /* n (at most 3) products of one A, the same chains, in one launch: C[i](M,N[i]) = A(M,K) @ B[i](K,N[i]). */
 BN_API int bn_mm_f32_each(const float* A, int64_t a_rs, int64_t a_cs, int n, const float* const* B, const int64_t* b_rs,
                           const int64_t* b_cs, float* const* C, const int64_t* c_rs, const int64_t* c_cs, int M, int K, const int* N,
@@ -109,10 +113,11 @@ BN_API int bn_mm_f32_each(const float* A, int64_t a_rs, int64_t a_cs, int n, con
  * BN_ACT_*.  Results that are not finite are worked out as by bn_mm_f32.
  * bn_linear_f32 cuts the operands itself, in `workspace` (bn_linear_f32_workspace_bytes, 16-byte aligned; contents need not be
  * kept).
- * bn_linear_f32_pays: whether it takes less time than bn_mm_f32 (an estimate), w_nparts being 1 where the weights are mostly bf16
- * numbers, else 3. */
+ * bn_linear_f32_form: which call such a product is for by time and error (an estimate): bn_mm_f32, bn_mm_f32_sums or bn_linear_f32.
+ * w_nparts: 1 where the weights are mostly bf16 numbers, else 3. */
+enum { BN_LINEAR_F32_CHAINS = 0, BN_LINEAR_F32_SUMS = 1, BN_LINEAR_F32_PARTS = 2 };
 BN_API size_t bn_linear_f32_workspace_bytes(int M, int N, int K);
-BN_API int bn_linear_f32_pays(int M, int N, int K, int w_nparts);
+BN_API int bn_linear_f32_form(int M, int N, int K, int w_nparts);
 BN_API int bn_linear_f32(const float* a, int64_t a_ld, const float* w, int64_t w_ld, const float* bias, int act, float* c, int M,
                          int N, int K, void* workspace, size_t workspace_bytes, int* error_word, bn_stream_t stream);
 

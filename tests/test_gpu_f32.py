@@ -200,7 +200,7 @@ def test_linear_f32_of_values_that_are_not_finite(lib, bad, act):
 @pytest.mark.parametrize("write", ["data", "in_place", "replaced"])
 def test_linear_f32_reads_the_weight_of_the_call(lib, dtype, write):
     """A weight that is written to, by whatever way, is the one that many rows are multiplied with as well as few."""
-    from baranet_bdml_b200 import ops
+    from baranet_bdml_b200 import _lib, ops
     gen = torch.Generator(device="cuda").manual_seed(7)
     N, K, rows = 2048, 2048, 512
     x, w0, w1 = (torch.randn(s, generator=gen, device="cuda") for s in ((rows, K), (N, K), (N, K)))
@@ -217,8 +217,26 @@ def test_linear_f32_reads_the_weight_of_the_call(lib, dtype, write):
     exact, size = x.double() @ w1.double().T, x.double().abs() @ w1.double().abs().T
     for got in (many, few):
         assert ((got.double() - exact).abs() <= K * 2.0 ** -24 * size).all()
-    # the two are the two routes
-    assert lib.bn_linear_f32_pays(rows, N, K, lin.parts_hint) and not lib.bn_linear_f32_pays(4, N, K, lin.parts_hint)
+    # the two are two routes; a wide weight takes few rows by the third
+    form = lambda r, n: lib.bn_linear_f32_form(r, n, K, lin.parts_hint)                          # noqa: E731
+    assert form(rows, N) == _lib.BN_LINEAR_F32_PARTS and form(4, N) == _lib.BN_LINEAR_F32_CHAINS
+    assert form(16, 32000) == _lib.BN_LINEAR_F32_SUMS
+
+
+@pytest.mark.parametrize("M,K,N", [(1, 4, 32), (8, 16, 33), (9, 20, 33), (17, 52, 1000), (33, 144, 4736), (65, 128, 9473), (1151, 272, 2052), (3, 2056, 8)])
+@pytest.mark.parametrize("odd", [False, True])
+def test_mm_sums(lib, M, K, N, odd):
+    """Every tile, both ways the operands are copied, K of less than a step, ragged, and on both sides of eight steps."""
+    from baranet_bdml_b200 import _lib
+    gen = torch.Generator(device="cuda").manual_seed(M + K + N)
+    x, w = (torch.randn((r, K + (3 if odd else 0)), generator=gen, device="cuda")[:, :K] for r in (M, N))
+    out = torch.full((M, N + 5), 7.0, device="cuda")
+    _lib.check(lib.bn_mm_f32_sums(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), N + 5, M, N, K,
+                                  torch.cuda.current_stream().cuda_stream))
+    exact, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    # 16 links, 8 additions, and one more for every 128 k
+    bound = (min(K, 16) + 8 + K / 128 + 1) * 2.0 ** -24 * size
+    assert ((out[:, :N].double() - exact).abs() <= bound).all() and bool((out[:, N:] == 7.0).all())
 
 
 @pytest.mark.parametrize("M,K,widths", [(128, 64, (2048, 256, 256)), (5, 20, (40, 8, 33)), (33, 16, (64, 1, 65)), (70, 36, (100, 260))])
