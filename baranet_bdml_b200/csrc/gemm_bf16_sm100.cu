@@ -640,6 +640,7 @@ extern "C" int bn_gemm_bias_act_bf16_nt(const void* a, const void* bt, const flo
 
 extern "C" size_t bn_gemm_bf16_nt_small_m_workspace_bytes(int M, int N, int K) {
     if (M <= 0 || N <= 0 || K <= 0) return 0;
+    if (gemm_rows_ok(M, N, K, false)) return 16;              // unused, but asked for
     int dev = 0, sms = 0, splits = 1, per = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -659,7 +660,7 @@ static int small_m_launch(const void* a, const void* bt, void* c, float* c32, co
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         splitk_plan(M, N, K, sms, &splits, &per);
-        if (workspace_bytes < (size_t)splits * M * N * sizeof(float))
+        if (workspace_bytes < bn_gemm_bf16_nt_small_m_workspace_bytes(M, N, K))
             return fail(BN_ERR_WORKSPACE, "%s: workspace of %zu bytes is too small", what, workspace_bytes);
     }
     return gemm_launch(a, bt, c, M, N, K, N, EPI_PARTIAL, error_word, stream, what, static_cast<float*>(workspace), splits, per,

@@ -1,6 +1,7 @@
 // fp32 products of many rows on the tensor cores: C (M,N) = act(A (M,K) W (N,K)^T + bias), both operands cut into bf16 parts.
 //
-// A 24-bit significand is three bf16 numbers: x1 = bf16(x), x2 = bf16(x - x1), x3 = x - x1 - x2, exactly.  Of the nine products
+// (The method: G. Henry, P. T. P. Tang, A. Heinecke, Leveraging the bfloat16 artificial intelligence datatype for higher-precision
+// computations, ARITH 2019.)  A 24-bit significand is three bf16 numbers: x1 = bf16(x), x2 = bf16(x - x1), x3 = x - x1 - x2, exactly.  Of the nine products
 // of parts the six down to 2^-18 of the largest are taken; the three left out are below 2^-26 of |a b|, less than the rounding
 // of a partial sum of an fp32 chain.  A weight that is a bf16 number (a bf16 checkpoint run in fp32) has one part, and three
 // products are all there are.  (Exactly from 2^-109 on: below that x3, from 2^-117 on x2 as well, falls out of bf16's range, and

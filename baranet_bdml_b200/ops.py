@@ -171,8 +171,8 @@ def _small_m_scratch(device, M: int, N: int, K: int):
 
 def gemm_bf16_nt_small_m(a: torch.Tensor, bt: torch.Tensor, *, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """a (M,K) @ bt (N,K)^T for few rows (a decode step: one token per sequence): the weight stream is spread over
-    all SMs (K split, partial sums added in a fixed order).  The fp32 scratch, which products of more than 128 rows or of
-    many columns use, is kept per (device, size) and reused by later calls on the same stream."""
+    all SMs (K split, partial sums added in a fixed order).  The fp32 scratch of products of more than 128 rows, of many
+    columns or of a short K is kept per (device, size) and reused by later calls on the same stream."""
     _need(a, torch.bfloat16, "gemm_bf16_nt_small_m(a)")
     _need(bt, torch.bfloat16, "gemm_bf16_nt_small_m(bt)")
     if a.dim() != 2 or bt.dim() != 2 or a.shape[1] != bt.shape[1]:

@@ -165,9 +165,9 @@ BN_API int bn_gemm_bf16_nt(const void* a, const void* bt, void* c, int M, int N,
 
 /* The same product for FEW rows (M <= 128 is where it pays: one token per sequence in a decode step), where the
  * weight matrix has to be streamed by all SMs: tiles of 128 columns, K cut over a cluster of up to 8 CTAs that add
- * their sums up through distributed shared memory; with M > 128 or more than half as many such tiles as run together,
- * 64-wide tiles and fp32 partial sums in `workspace`, added by a second kernel.  The order is fixed either way (results
- * do not depend on timing).
+ * their sums up through distributed shared memory; with M > 128, more than half as many such tiles as run together, or
+ * a K below 640 (of more than 64 rows 1280), 64-wide tiles and fp32 partial sums in `workspace`, added by a second
+ * kernel.  The order is fixed either way (results do not depend on timing).
  * workspace: bn_gemm_bf16_nt_small_m_workspace_bytes(M, N, K) bytes, 16-byte aligned; contents need not be kept. */
 BN_API size_t bn_gemm_bf16_nt_small_m_workspace_bytes(int M, int N, int K);
 BN_API int bn_gemm_bf16_nt_small_m(const void* a, const void* bt, void* c, int M, int N, int K, void* workspace,
