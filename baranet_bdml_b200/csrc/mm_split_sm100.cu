@@ -371,7 +371,8 @@ static int split_launch(const void* a_parts, const void* w_parts, const SplitPar
 }
 
 // The tile width by an estimate of the time, in us: what 64 k of a tile take, measured with one tile per multiprocessor and with
-// several (the same: a tile's loads and MMAs both read or write shared memory, 96 - 192 KB in this time).
+// several (the same).  The tensor pipe is active 69 % of the time with three parts, 50 % with one, whose two stages do not cover
+// the loads; L2 throughput a third of its peak.
 // Products of 800 rows, chain (bn_mm_f32) / with operands cut, three parts / the same, one part: 2048 -> 7424 691 / 152 / 96 us,
 // 2048 -> 2048 189 / 50 / 33 us, 7424 -> 2048 679 / 168 / 121 us; 64 rows 2048 -> 7424 81 / 60 / 38 us, 2048 -> 2048 34 / 39 / 26 us.
 // (A stage with room for one part of the weight, three of them in flight or 256 columns wide, is no faster for one part - 107, 38,
