@@ -1,15 +1,15 @@
 // fp32 products of many rows on the tensor cores: C (M,N) = act(A (M,K) W (N,K)^T + bias), both operands cut into bf16 parts.
 //
-// (The method: G. Henry, P. T. P. Tang, A. Heinecke, Leveraging the bfloat16 artificial intelligence datatype for higher-precision
-// computations, ARITH 2019.)  A 24-bit significand is three bf16 numbers: x1 = bf16(x), x2 = bf16(x - x1), x3 = x - x1 - x2, exactly.  Of the nine products
-// of parts the six down to 2^-18 of the largest are taken; the three left out are below 2^-26 of |a b|, less than the rounding
-// of a partial sum of an fp32 chain.  A weight that is a bf16 number (a bf16 checkpoint run in fp32) has one part, and three
-// products are all there are.  (Exactly from 2^-109 on: below that x3, from 2^-117 on x2 as well, falls out of bf16's range, and
-// what is lost stays below 2^-134.)
+// A 24-bit significand is three bf16 numbers: x1 = bf16(x), x2 = bf16(x - x1), x3 = x - x1 - x2, exactly (G. Henry, P. T. P. Tang,
+// A. Heinecke, Leveraging the bfloat16 artificial intelligence datatype for higher-precision computations, ARITH 2019).  Of the nine
+// products of parts the six down to 2^-18 of the largest are taken; the three left out are below 2^-26 of |a b|, less than the
+// rounding of a partial sum of an fp32 chain.  A weight that is a bf16 number (a bf16 checkpoint run in fp32) has one part, and
+// three products are all there are.  (Exactly from 2^-109 on: below that x3, from 2^-117 on x2 as well, falls out of bf16's range,
+// and what is lost stays below 2^-134.)
 //
 // bn_linear_f32 cuts both operands anew in every call, so that a weight may be written to at any time, and by anything, between
-// two calls; which tiles of the weight have one part and which three is found out on the way.  Cutting a
-// weight of 2048 x 7424 takes 21 us with three parts and 12 us with one.
+// two calls; which tiles of the weight have one part and which three is found out on the way.  Cutting a weight of 2048 x 7424 takes
+// 21 us with three parts and 12 us with one.
 //
 // The tensor cores add into fp32 accumulators with truncation, which over a long K would cost more than a chain of FMAs does.
 // So an accumulator takes 64 k only, the small products first and x1 w1 last, and these sums are added up in registers, rounded
@@ -51,6 +51,7 @@ struct SplitParams {
     const uint8_t* counts;         // how many parts the weight has, 1 or 3, in every tile of BN rows x 64 k; null: w_parts everywhere
     int64_t a_ld, w_ld;
     int M, N, K, act, w_parts;
+    bool aligned;                  // a's and w's rows start on 16-byte boundaries
 };
 
 // The rows m0 + i of the set bits i of `rows`, as chains: a warp, a lane per column (n the lane's), four rows at a time and 8 k of
@@ -60,6 +61,12 @@ __device__ __noinline__ void redo_rows(const SplitParams& p, uint32_t rows, int 
     constexpr int ROWS = 4, AHEAD = 2;           // K is a multiple of 8
     const bool in = n < p.N;
     const float* w = p.w + (in ? n : 0) * p.w_ld;
+    auto load = [&](const float* from, float (&v)[4]) {
+        if (p.aligned) load4(from, v);
+        else
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[e] = from[e];
+    };
     while (rows) {
         int m[ROWS];
         const float* a[ROWS];
@@ -75,9 +82,9 @@ __device__ __noinline__ void redo_rows(const SplitParams& p, uint32_t rows, int 
             float y[AHEAD][4], x[ROWS][AHEAD][4];
 #pragma unroll
             for (int j = 0; j < AHEAD; ++j) {
-                load4(w + k0 + 4 * j, y[j]);
+                load(w + k0 + 4 * j, y[j]);
 #pragma unroll
-                for (int r = 0; r < ROWS; ++r) load4(a[r] + k0 + 4 * j, x[r][j]);
+                for (int r = 0; r < ROWS; ++r) load(a[r] + k0 + 4 * j, x[r][j]);
             }
 #pragma unroll
             for (int j = 0; j < AHEAD; ++j)
@@ -425,7 +432,8 @@ extern "C" int bn_mm_f32_split(const void* a_parts, const void* w_parts, int w_n
     if ((long long)M * MS_PARTS > INT32_MAX || (long long)N * MS_PARTS > INT32_MAX) return fail(BN_ERR_UNSUPPORTED, "%s: M=%d N=%d too large", what, M, N);
     if (int rc = require_sm100()) return rc;
     if (M == 0 || N == 0) return BN_OK;
-    const SplitParams p{a, w, bias, c, error_word, nullptr, a_ld, w_ld, M, N, K, act, w_nparts};
+    const bool aligned = ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w)) & 15) == 0 && a_ld % 4 == 0 && w_ld % 4 == 0;
+    const SplitParams p{a, w, bias, c, error_word, nullptr, a_ld, w_ld, M, N, K, act, w_nparts, aligned};
     int bn;
     split_estimate(M, N, K, w_nparts, &bn);
     return split_run(bn, a_parts, w_parts, p, as_stream(stream), what);
@@ -488,6 +496,6 @@ extern "C" int bn_linear_f32(const float* a, int64_t a_ld, const float* w, int64
     if (bn == 64) launch_dependent(cut_operands_kernel<64>, grid, 256, 0, st, cp);
     else launch_dependent(cut_operands_kernel<128>, grid, 512, 0, st, cp);
     if (int rc = launch_status(what)) return rc;
-    const SplitParams p{a, w, bias, c, error_word, cp.counts, a_ld, w_ld, M, N, K, act, 0};
+    const SplitParams p{a, w, bias, c, error_word, cp.counts, a_ld, w_ld, M, N, K, act, 0, true};
     return split_run(bn, cp.a_parts, cp.w_parts, p, st, what);
 }

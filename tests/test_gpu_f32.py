@@ -124,6 +124,28 @@ def test_mm_of_bf16_parts(lib, M, K, N, parts):
     assert int(word.item()) == 0
 
 
+@pytest.mark.parametrize("shift_x,shift_w", [(1, 0), (0, 3), (2, 1)])
+def test_mm_of_bf16_parts_reads_operands_at_any_address(lib, shift_x, shift_w):
+    """The operands themselves, which results that are not finite are worked out from, need no alignment."""
+    from baranet_bdml_b200 import _lib, ops
+    M, K, N = 140, 264, 200
+    gen = torch.Generator(device="cuda").manual_seed(shift_x)
+    x, w = torch.randn((M, K), generator=gen, device="cuda"), torch.randn((N, K), generator=gen, device="cuda")
+    x[3], x[130, 7], w[70, 5] = float("inf"), -float("inf"), float("nan")
+    xp, wp = ops._bf16_parts(x), ops._bf16_parts(w)
+    xs, ws = (torch.zeros((r, K + s), device="cuda")[:, s:] for r, s in ((M, shift_x), (N, shift_w)))
+    xs.copy_(x)
+    ws.copy_(w)
+    got, chain, word = torch.empty((M, N), device="cuda"), torch.empty((M, N), device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    st = torch.cuda.current_stream().cuda_stream
+    _lib.check(lib.bn_mm_f32(x.data_ptr(), K, 1, w.data_ptr(), 1, K, chain.data_ptr(), N, 1, M, K, N, st))
+    _lib.check(lib.bn_mm_f32_split(xp.data_ptr(), wp.data_ptr(), 3, xs.data_ptr(), xs.stride(0), ws.data_ptr(), ws.stride(0), None, 0,
+                                   got.data_ptr(), M, N, K, word.data_ptr(), st))
+    assert torch.equal(torch.isnan(got), torch.isnan(chain)) and torch.equal(torch.isposinf(got), torch.isposinf(chain))
+    fine = torch.isfinite(chain)
+    assert ((got - chain).abs()[fine] <= 2e-4).all() and int(word.item()) == 0
+
+
 @pytest.mark.parametrize("M,K,N", [(1, 8, 8), (127, 72, 72), (129, 136, 136), (300, 2056, 264), (513, 64, 2056), (1300, 128, 4096)])
 @pytest.mark.parametrize("weights", ["bf16", "fp32", "mixed"])
 def test_linear_f32_cuts_its_operands(lib, M, K, N, weights):
