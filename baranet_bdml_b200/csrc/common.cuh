@@ -30,9 +30,9 @@ inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 // kernel's own prologue, hidden under the predecessor's tail - the decode step is a chain of ~180 short kernels.
 // Falls back to an ordinary launch if the attribute is refused.
 template <typename... P, typename... A>
-inline void launch_dependent(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, A... args) {
+inline void launch_dependent(void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t st, A... args) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
+    cfg.gridDim = grid;
     cfg.blockDim = dim3(block);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
@@ -49,9 +49,10 @@ inline void launch_dependent(void (*kernel)(P...), unsigned grid, unsigned block
 
 // SMs of the current device
 inline int sm_count() {
-    int dev = 0, sms = 148;
+    static thread_local int known_dev = -1, sms = 148;
+    int dev = 0;
     cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (dev != known_dev && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess) known_dev = dev;
     return sms;
 }
 

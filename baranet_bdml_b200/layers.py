@@ -118,8 +118,14 @@ class GroupedQueryAttention:
         return AGTensor(w, requires_grad=True, is_cuda=self.is_cuda)
 
     def __call__(self, hidden_states: AGTensor, position_offset: int = 0, use_causal_mask: bool = True) -> AGTensor:
-        query, key, value = hidden_states.matmul_each([self.q_proj, self.k_proj, self.v_proj])
         mode = _lib.BN_HEADS_COLLAPSED if self.heads_mode == "collapsed" else _lib.BN_HEADS_PER_HEAD
+        weights = (self.q_proj, self.k_proj, self.v_proj, self.o_proj)
+        whole = hidden_states.data.attention_layer(
+            *(w.data for w in weights), float(self.scale), use_causal_mask, position_offset, num_heads=self.num_heads,
+            num_kv_heads=self.num_kv_heads, head_dim=self.head_dim, theta=self.rotary_emb.base, heads_mode=mode)
+        if whole is not None:
+            return AGTensor(whole, (hidden_states, *weights), "attention_layer", requires_grad=False)
+        query, key, value = hidden_states.matmul_each([self.q_proj, self.k_proj, self.v_proj])
         attn = query.data.attention_fused(
             key.data, value.data, float(self.scale), causal=use_causal_mask, seq_offset=position_offset,
             num_heads=self.num_heads, num_kv_heads=self.num_kv_heads, head_dim=self.head_dim,

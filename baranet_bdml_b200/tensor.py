@@ -230,6 +230,29 @@ class TensorF:
             out.stride_w, self.h, self.w, float(eps), _stream_ptr()))
         return total, out
 
+    def attention_layer(self, wq: "TensorF", wk: "TensorF", wv: "TensorF", wo: "TensorF", scale: float, causal: bool, seq_offset: int, *,
+                        num_heads: int, num_kv_heads: int, head_dim: int, theta: float, heads_mode: int) -> Optional["TensorF"]:
+        """((self @ wq).attention_fused(self @ wk, self @ wv, ...)) @ wo in one call -> bn_attn_layer_f32; None where the shapes,
+        strides or addresses are none that it takes (then the single operators say what is wrong, or do it)."""
+        hidden, kv = self.w, num_kv_heads * head_dim
+        weights = (wq, wk, wv, wo)
+        if [(t.h, t.w) for t in weights] != [(hidden, num_heads * head_dim), (hidden, kv), (hidden, kv), (num_heads * head_dim, hidden)]:
+            return None
+        for t in (self, *weights):
+            if not t.on_device or t.stride_w != 1 or t.stride_h % 4 or t._ptr() % 16:
+                return None
+        lib = _lib.load()
+        n = lib.bn_attn_layer_f32_workspace_bytes(self.h, hidden, num_heads, num_kv_heads, head_dim, int(heads_mode)) if seq_offset >= 0 else 0
+        if n == 0:
+            return None
+        out = TensorF(self.h, hidden, True)
+        scratch = torch.empty(n, dtype=torch.uint8, device=self.base.device)
+        _lib.check(lib.bn_attn_layer_f32(
+            self._ptr(), self.stride_h, wq._ptr(), wq.stride_h, wk._ptr(), wk.stride_h, wv._ptr(), wv.stride_h, wo._ptr(), wo.stride_h,
+            out._ptr(), out.stride_h, self.h, hidden, num_heads, num_kv_heads, head_dim, float(scale), float(theta), int(seq_offset),
+            int(bool(causal)), int(heads_mode), scratch.data_ptr(), n, _stream_ptr()))
+        return out
+
     def attention_fused(self, key: "TensorF", value: "TensorF", scale: float, causal: bool = False,
                         seq_offset: int = 0, *, num_heads: int, num_kv_heads: int, head_dim: int,
                         theta: float = 10000.0, heads_mode: int = _lib.BN_HEADS_COLLAPSED,

@@ -108,6 +108,16 @@ BN_API int bn_mm_f32_each(const float* A, int64_t a_rs, int64_t a_cs, int n, con
                           const int64_t* b_cs, float* const* C, const int64_t* c_rs, const int64_t* c_cs, int M, int K, const int* N,
                           bn_stream_t stream);
 
+/* The whole attention layer: x (S, hidden) -> softmax attention of rotated q = x wq, k = x wk, v = x wv -> @ wo, fp32, rows of
+ * contiguous elements: wq (hidden, Hq D), wk and wv (hidden, Hkv D), wo (Hq D, hidden).  Heads, scale, positions and mask as in
+ * bn_attn_prefill_f32; sums are shorter and in another order than those of the single operators.  16-byte aligned pointers and
+ * strides; `workspace` of bn_attn_layer_f32_workspace_bytes, which is 0 for sizes that this call does not take. */
+BN_API size_t bn_attn_layer_f32_workspace_bytes(int S, int hidden, int Hq, int Hkv, int D, int heads_mode);
+BN_API int bn_attn_layer_f32(const float* x, int64_t x_rs, const float* wq, int64_t wq_rs, const float* wk, int64_t wk_rs,
+                             const float* wv, int64_t wv_rs, const float* wo, int64_t wo_rs, float* out, int64_t out_rs, int S,
+                             int hidden, int Hq, int Hkv, int D, float scale, float theta, int position_offset, int causal,
+                             int heads_mode, void* workspace, size_t workspace_bytes, bn_stream_t stream);
+
 /* The products of many rows on the tensor cores, with the precision of an fp32 sum: C(M,N) = act(A(M,K) W(N,K)^T + bias),
  * fp32, from the bf16 parts of both operands.  N and K multiples of 8; 16-byte aligned rows; bias (N) or null; act one of
  * BN_ACT_*.  Results that are not finite are worked out as by bn_mm_f32.

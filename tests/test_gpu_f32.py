@@ -374,6 +374,65 @@ def test_layer_config1_matches_oracle(T, cref, dev_inv_freq):
     assert nerr(out, ref64) < 2e-5
 
 
+LAYERS = [  # S, hidden, Hq, Hkv, D, offset, causal: rows to a block 1 .. 16, tiles of 64 keys, groups of 1, 3, 5, 8 and 12 heads
+    (1, 128, 4, 2, 32, 0, True),
+    (16, 2048, 32, 4, 64, 0, True),
+    (65, 100, 5, 5, 20, 3, False),
+    (129, 192, 12, 4, 16, 0, True),
+    (200, 260, 5, 1, 12, 2, True),
+    (333, 768, 12, 1, 64, 0, True),
+    (512, 256, 32, 4, 64, 0, False),
+    (600, 128, 8, 2, 4, 0, True),
+]
+
+
+@pytest.mark.parametrize("S,hid,Hq,Hkv,D,off,causal", LAYERS)
+@pytest.mark.parametrize("mode", ["collapsed", "per_head"])
+def test_layer_in_one_call(T, dev_inv_freq, S, hid, Hq, Hkv, D, off, causal, mode):
+    """bn_attn_layer_f32 against 64 bits (the gate of the layer's other tests) and against the single operators; a row that is not
+    finite is seen by the rows behind it alone."""
+    import torch
+    from baranet_bdml_b200 import _lib
+    rng = np.random.default_rng(S + Hq)
+    x = rng.standard_normal((S, hid), dtype=np.float32)
+    ws = [(rng.standard_normal(s) * hid ** -0.5).astype(np.float32) for s in ((hid, Hq * D), (hid, Hkv * D), (hid, Hkv * D), (Hq * D, hid))]
+    scale, hm = D ** -0.5, _lib.BN_HEADS_COLLAPSED if mode == "collapsed" else _lib.BN_HEADS_PER_HEAD
+    tx, *tw = (T.TensorF.from_torch(torch.from_numpy(a).cuda()) for a in (x, *ws))
+    sizes = dict(num_heads=Hq, num_kv_heads=Hkv, head_dim=D, theta=10000.0, heads_mode=hm)
+    layer = lambda t: t.attention_layer(*tw, scale, causal, off, **sizes)                         # noqa: E731
+    got = layer(tx).to_numpy()
+    inv = np.array([np.float32(1.0 / float(np.float32(10000.0) ** (np.float32(2 * i) / np.float32(D)))) for i in range(D // 2)], dtype=np.float32)
+    inv = dev_inv_freq[D].astype(np.float32) if D in dev_inv_freq else inv
+    q, k, v = (x.astype(np.float64) @ w.astype(np.float64) for w in ws[:3])
+    core = R.attention_collapsed if mode == "collapsed" else R.attention_per_head
+    want = core(q, k, v, num_heads=Hq, num_kv_heads=Hkv, head_dim=D, position_offset=off, causal=causal, dtype=np.float64,
+                inv_freq=inv) @ ws[3].astype(np.float64)
+    single = tx @ tw[0]
+    single = single.attention_fused(tx @ tw[1], tx @ tw[2], scale, causal, off, **sizes) @ tw[3]
+    assert nerr(got, want) < 2e-5 and nerr(got, single.to_numpy()) < 2 * GATE, (nerr(got, want), nerr(got, single.to_numpy()))
+    if causal and S > 2:
+        x[S // 2, 0] = np.inf
+        bad = layer(T.TensorF.from_torch(torch.from_numpy(x).cuda())).to_numpy()
+        before = S // 2 - off
+        assert before <= 0 or np.array_equal(bad[:before], got[:before])
+        assert not np.isfinite(bad[S // 2:]).any()
+
+
+def test_layer_in_one_call_refuses_what_it_does_not_take(T):
+    import torch
+    from baranet_bdml_b200 import _lib
+    x = torch.randn(8, 64, device="cuda")
+    w = [torch.randn(s, device="cuda") for s in ((64, 48), (64, 12), (64, 12), (48, 64))]
+    sizes = dict(num_heads=4, num_kv_heads=1, head_dim=12, theta=10000.0, heads_mode=_lib.BN_HEADS_COLLAPSED)
+    run = lambda x, w, off=0, **kw: T.TensorF.from_torch(x).attention_layer(*(T.TensorF.from_torch(t) for t in w), 1.0, True, off, **{**sizes, **kw})   # noqa: E731
+    assert run(x, w) is not None
+    assert run(x, [w[0].t().contiguous().t()] + w[1:]) is None                       # columns that are not contiguous
+    assert run(torch.randn(8, 65, device="cuda")[:, 1:], w) is None                  # rows that do not start on 16 bytes
+    assert run(x, w, num_heads=2) is None and run(x, w, -1) is None
+    assert run(x, [torch.randn(64, 24, device="cuda"), *(torch.randn(64, 6, device="cuda") for _ in "kv"), torch.randn(24, 64, device="cuda")],
+               head_dim=6) is None                                                    # heads that are no multiple of 4
+
+
 def test_layer_matches_reference_cuda_ops(T, cref):
     """Same inputs through the reference's OWN CUDA operators (compiled from the
     reference tree into oracle/_ref) and through the fused layer."""
