@@ -107,16 +107,15 @@ attn_any_kernel(const AttnPortionParams p) {
 // 64; a warp per row for the running maximum and sum; thread = (value column mod 64, group of rows) for the result, which
 // reads a value from global memory once for AT_RPT rows.  fp32 throughout, a score is one FMA chain over its columns.
 // The warp-per-row kernel reads every key for every row, 32 rows of a matrix at a time: 32 heads over 4 x 64 columns, 4 x 200
-// tokens, 873 us; this one 129 us, with keys and values staged (fp32, whole rows of at most 64 columns) 84 us.
+// tokens, 873 us; this one 129 us.
 // A tile of keys where the mask of some row cuts leaves the masked (row, key) pairs out of the result, as that kernel does: their
 // weight is no zero to multiply by, or a value that is not finite would reach rows that do not see it.
 // ---------------------------------------------------------------------------------------------------------------
 constexpr int AT_KEYS = 64, AT_RPT = 8, AT_ROWS = 32, AT_THREADS = AT_KEYS * AT_ROWS / AT_RPT, AT_E = 64, AT_KLD = AT_E + 4;
 
-// VB: value columns in blocks of 64.  STAGED (fp32, one piece of columns and one block of values, 16-byte rows): keys and values
-// come in by cp.async, the next keys while the weights are worked out and applied, the next values under the next scores.
-template <typename T, int VB, bool STAGED>
-__global__ void __launch_bounds__(AT_THREADS, STAGED ? 3 : 1)
+// VB: value columns in blocks of 64.
+template <typename T, int VB>
+__global__ void __launch_bounds__(AT_THREADS, 1)
 attn_tiled_kernel(const AttnPortionParams p) {
     extern __shared__ __align__(16) float at_smem[];
     __shared__ __align__(16) float Ks[AT_KEYS * AT_KLD];
@@ -159,40 +158,11 @@ attn_tiled_kernel(const AttnPortionParams p) {
 #pragma unroll
         for (int v = 0; v < VB; ++v) acc[r][v] = 0.f;
 
-    float* Vs = Qs + AT_ROWS * q_ld;                           // STAGED: [key][64]
-    // rows k0 .. k0 + 63 of a matrix with `cols` columns; what lies outside becomes zero
-    auto stage_in = [&](float* dst, int ld, const T* src, int64_t src_ld, int cols, int k0) {
-        const uint32_t to = ptx::smem_u32(dst);
-        for (int i = tid; i < AT_KEYS * 16; i += AT_THREADS) {
-            const int kk = i / 16, c = i % 16 * 4;
-            const bool in = k0 + kk <= last && c < cols;
-            ptx::cp_async_16(to + (kk * ld + c) * 4, in ? src + (int64_t)(k0 + kk) * src_ld + c : src, in ? 16 : 0);
-        }
-        ptx::cp_async_commit();
-    };
-    if constexpr (STAGED) {
-        stage_in(Ks, AT_KLD, kseq, p.k_ld, E, first);
-        stage_in(Vs, 64, vseq, p.v_ld, p.vdim, first);
-    }
-
     for (int k0 = first; k0 <= last; k0 += AT_KEYS) {
         float s[AT_RPT];
 #pragma unroll
         for (int r = 0; r < AT_RPT; ++r) s[r] = 0.f;
-        if (STAGED) {
-            ptx::cp_async_wait<1>();                           // the keys; the values may still be on their way
-            __syncthreads();
-#pragma unroll 2
-            for (int e = 0; e < E; e += 4) {
-                const float4 k4 = *reinterpret_cast<const float4*>(Ks + key * AT_KLD + e);
-#pragma unroll
-                for (int r = 0; r < AT_RPT; ++r) {
-                    const float4 q4 = *reinterpret_cast<const float4*>(Qs + (group * AT_RPT + r) * q_ld + e);
-                    s[r] = fmaf(q4.w, k4.w, fmaf(q4.z, k4.z, fmaf(q4.y, k4.y, fmaf(q4.x, k4.x, s[r]))));
-                }
-            }
-        }
-        for (int e0 = 0; e0 < E && !STAGED; e0 += AT_E) {
+        for (int e0 = 0; e0 < E; e0 += AT_E) {
             __syncthreads();                                   // the piece before (and the weights) have been read
 #pragma unroll 8
             for (int i = tid; i < AT_KEYS * AT_E; i += AT_THREADS) {
@@ -219,14 +189,8 @@ attn_tiled_kernel(const AttnPortionParams p) {
             Ps[row][key] = seen ? s[r] * row_scale[row] : -INFINITY;
         }
         __syncthreads();
-        const bool more = k0 + AT_KEYS <= last;
         // whether some row does not see some key of the tile
         const bool cut = k0 + AT_KEYS - 1 > p.n_old + position(0) || k0 < mask_oldest(p.mask, p.span, p.n_old + position(n_rows - 1));
-        if (STAGED) {
-            if (more) stage_in(Ks, AT_KLD, kseq, p.k_ld, E, k0 + AT_KEYS);
-            else ptx::cp_async_commit();
-            ptx::cp_async_wait<1>();                           // the values, visible to all behind the next barrier
-        }
         for (int r = warp; r < AT_ROWS; r += AT_THREADS / 32) {
             const float a = Ps[r][lane], c = Ps[r][lane + 32], m = row_m[r];
             float mx = fmaxf(a, c);
@@ -271,8 +235,7 @@ attn_tiled_kernel(const AttnPortionParams p) {
                 for (int i = 0; i < 4; ++i)
 #pragma unroll
                     for (int v = 0; v < VB; ++v)
-                        if (STAGED) val[i][v] = Vs[(j + i) * 64 + key];
-                        else val[i][v] = j + i < nk && v * 64 + key < p.vdim ? to_f(vseq[(int64_t)(k0 + j + i) * p.v_ld + v * 64 + key]) : 0.f;
+                        val[i][v] = j + i < nk && v * 64 + key < p.vdim ? to_f(vseq[(int64_t)(k0 + j + i) * p.v_ld + v * 64 + key]) : 0.f;
 #pragma unroll
                 for (int r = 0; r < AT_RPT; ++r) {
                     const float4 w = *reinterpret_cast<const float4*>(&Ps[group * AT_RPT + r][j]);
@@ -284,10 +247,6 @@ attn_tiled_kernel(const AttnPortionParams p) {
         };
         if (cut) apply(std::true_type{});
         else apply(std::false_type{});
-        if (STAGED && more) {
-            __syncthreads();                                   // these values have been read
-            stage_in(Vs, 64, vseq, p.v_ld, p.vdim, k0 + AT_KEYS);
-        }
     }
 #pragma unroll
     for (int r = 0; r < AT_RPT; ++r) {
@@ -309,9 +268,233 @@ attn_tiled_kernel(const AttnPortionParams p) {
     }
 }
 
+// ---------------------------------------------------------------------------------------------------------------
+// The same in fp32 for rows of whole 16-byte pieces: a CTA owns 64 rows, and a thread 8 rows x 4 keys of the scores and 8 rows x 4
+// columns (of each 64) of the result, 12 16-byte reads of shared memory for 128 FMAs; those reads bind (the kernel above has 9 for
+// 32).  Keys come in pieces of 64 columns by cp.async, one ahead, values under the scores; maximum, sum and weights of a row stay
+// with the 16 threads that have it.  Scores and results are the same chains as above.
+// 32 heads over 4 x 64 columns, 4 x 200 tokens, 63 us; with 8 rows x 1 key a thread 96 us, with 8 x 4 in 128 threads (two warps a
+// scheduler, which show every latency) 97 us, with the tiles of one sequence one behind the other 68 us.
+// ---------------------------------------------------------------------------------------------------------------
+constexpr int AP_ROWS = 64, AP_KEYS = 64, AP_THREADS = 256, AP_LD = 68;
+
+template <int VB>
+__global__ void __launch_bounds__(AP_THREADS, VB == 1 ? 3 : 2)
+attn_tiles_f32_kernel(const AttnPortionParams p) {
+    extern __shared__ __align__(16) float at_smem[];
+    ptx::grid_dependency_wait();
+    ptx::grid_launch_dependents();
+    const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32, tx = tid % 16, ty = tid / 16;
+    const int E = p.dim + p.rot, pieces = (E + 63) / 64, q_ld = pieces * 64 + 4, n_rep = p.H / p.kv_heads;
+    constexpr int V_LD = VB * 64;
+    float* Ks = at_smem;                                       // [64][68]
+    float* Vs = Ks + AP_KEYS * AP_LD;                      // [64][V_LD]
+    float* Ps = Vs + AP_KEYS * V_LD;                           // [64][68]
+    float* Qs = Ps + AP_ROWS * AP_LD;                          // [64][q_ld], zeros behind the columns
+    float* row_scale = Qs + AP_ROWS * q_ld;
+    const int tiles_per_seq = (int)(((long long)p.S * n_rep + AP_ROWS - 1) / AP_ROWS);
+    // the tiles with most keys first, of all sequences and heads: a multiprocessor then gets a long, a middle and a short one
+    const int bgs = p.B * p.kv_heads, tile = tiles_per_seq - 1 - (int)(blockIdx.x / bgs), bg = (int)(blockIdx.x % bgs);
+    const int b = bg / p.kv_heads, g = bg % p.kv_heads, t0 = tile * AP_ROWS, n_rows = min(AP_ROWS, p.S * n_rep - t0);
+    auto position = [&](int r) { return (t0 + r) / n_rep; };   // of the portion
+    auto head = [&](int r) { return g * n_rep + (t0 + r) % n_rep; };
+    const int first = max(0, mask_oldest(p.mask, p.span, p.n_old + position(0))), last = p.n_old + position(n_rows - 1);
+    const int key_tiles = (last - first) / AP_KEYS + 1;
+    const float* kseq = static_cast<const float*>(p.k) + b * p.k_seq + g * p.k_head;
+    const float* vseq = static_cast<const float*>(p.v) + b * p.v_seq + g * p.v_head;
+    const float* kr_seq = static_cast<const float*>(p.krot) + (int64_t)b * p.rows_per_seq * p.krot_ld;
+    const uint32_t uK = ptx::smem_u32(Ks), uV = ptx::smem_u32(Vs);
+
+    // piece n of the keys: columns 64 (n % pieces) .. of key tile n / pieces; what lies outside becomes zero
+    auto ask_keys = [&](int n) {
+        if (n < key_tiles * pieces) {
+            const int k0 = first + n / pieces * AP_KEYS, e0 = n % pieces * 64;
+#pragma unroll
+            for (int i = 0; i < AP_KEYS * 16 / AP_THREADS; ++i) {
+                const int kk = ty + i * (AP_THREADS / 16), e = e0 + tx * 4, k = k0 + kk;
+                const bool in = k <= last && e < E;
+                const float* at = e < p.dim ? kseq + (int64_t)k * p.k_ld + e : kr_seq + (int64_t)k * p.krot_ld + e - p.dim;
+                ptx::cp_async_16(uK + (kk * AP_LD + tx * 4) * 4, in ? at : kseq, in ? 16 : 0);
+            }
+        }
+        ptx::cp_async_commit();
+    };
+    auto ask_values = [&](int t) {
+        const int k0 = first + t * AP_KEYS;
+#pragma unroll
+        for (int i = 0; i < AP_KEYS * 16 / AP_THREADS; ++i) {
+            const int kk = ty + i * (AP_THREADS / 16);
+#pragma unroll
+            for (int v = 0; v < VB; ++v) {
+                const int c = v * 64 + tx * 4;
+                const bool in = k0 + kk <= last && c < p.vdim;
+                ptx::cp_async_16(uV + (kk * V_LD + c) * 4, in ? vseq + (int64_t)(k0 + kk) * p.v_ld + c : vseq, in ? 16 : 0);
+            }
+        }
+        ptx::cp_async_commit();
+    };
+    ask_keys(0);
+    for (int r = warp; r < AP_ROWS; r += AP_THREADS / 32) {
+        float ss = 0.f;
+        const float* q = static_cast<const float*>(p.q) + ((int64_t)b * p.S + position(r)) * p.q_ld + head(r) * E;
+        for (int e = lane; e < pieces * 64; e += 32) {
+            const float v = r < n_rows && e < E ? q[e] : 0.f;
+            Qs[r * q_ld + e] = v;
+            ss = fmaf(v, v, ss);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        if (lane == 0) row_scale[r] = p.rms_dim ? p.scale * rsqrtf(ss / (float)p.rms_dim + p.rms_eps) : p.scale;
+    }
+    // this thread's rows: ty + 16 i
+    float acc[4][VB][4], m[4], l[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        m[i] = -INFINITY;
+        l[i] = 0.f;
+#pragma unroll
+        for (int v = 0; v < VB; ++v) acc[i][v][0] = acc[i][v][1] = acc[i][v][2] = acc[i][v][3] = 0.f;
+    }
+    for (int t = 0, n = 0; t < key_tiles; ++t) {
+        const int k0 = first + t * AP_KEYS;
+        float s[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) s[i][0] = s[i][1] = s[i][2] = s[i][3] = 0.f;
+        for (int piece = 0; piece < pieces; ++piece, ++n) {
+            ptx::cp_async_wait<0>();                           // these keys (and the values before the last piece)
+            __syncthreads();
+            if (piece == 0) ask_values(t);
+            const float* ks = Ks + tx * AP_LD;
+            const float* qs = Qs + ty * q_ld + piece * 64;
+#pragma unroll 2
+            for (int e = 0; e < 64; e += 4) {                  // (the last columns may be zeros on both sides)
+                float4 k4[4], q4[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) k4[j] = *reinterpret_cast<const float4*>(ks + j * 16 * AP_LD + e);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) q4[i] = *reinterpret_cast<const float4*>(qs + i * 16 * q_ld + e);
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        s[i][j] = fmaf(q4[i].w, k4[j].w, fmaf(q4[i].z, k4[j].z, fmaf(q4[i].y, k4[j].y, fmaf(q4[i].x, k4[j].x, s[i][j]))));
+            }
+            __syncthreads();                                   // the piece has been read
+            ask_keys(n + 1);
+        }
+        // whether some row does not see some key of the tile
+        const bool cut = k0 + AP_KEYS - 1 > p.n_old + position(0) || k0 < mask_oldest(p.mask, p.span, p.n_old + position(n_rows - 1)) || n_rows < AP_ROWS;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int r = ty + i * 16, own = p.n_old + position(r), oldest = mask_oldest(p.mask, p.span, own);
+            const float scale = row_scale[r];
+            bool seen[4];
+            float mx = -INFINITY;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int k = k0 + tx + j * 16;
+                seen[j] = !cut || (r < n_rows && k <= own && k >= oldest);
+                s[i][j] = seen[j] ? s[i][j] * scale : -INFINITY;
+                mx = fmaxf(mx, s[i][j]);
+            }
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            const float m_new = fmaxf(m[i], mx);
+            // nothing of the row seen yet: no weight, whatever the (masked) scores; a NaN score is seen and stays one
+            const bool none = m_new == -INFINITY;
+            float sum = 0.f;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float w = none && s[i][j] == -INFINITY ? 0.f : expf(s[i][j] - m_new);
+                sum += w;
+                Ps[r * AP_LD + tx + j * 16] = seen[j] ? w : -1.f;          // a masked pair's weight: -1
+            }
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            const float shrink = none ? 1.f : expf(m[i] - m_new);
+            l[i] = l[i] * shrink + sum;
+            m[i] = m_new;
+#pragma unroll
+            for (int v = 0; v < VB; ++v)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) acc[i][v][c] *= shrink;
+        }
+        ptx::cp_async_wait<1>();                               // the values; the next keys are on their way
+        __syncthreads();
+        const int nk = min(AP_KEYS, last - k0 + 1);
+        auto apply = [&](auto masked) {
+            auto add = [&](float w, float v, float sum) { return decltype(masked)::value && w < 0.f ? sum : fmaf(w, v, sum); };
+#pragma unroll 2
+            for (int j = 0; j < nk; j += 4) {                  // (weights beyond the last key are -1 or, uncut, there are none)
+                float4 w4[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) w4[i] = *reinterpret_cast<const float4*>(Ps + (ty + i * 16) * AP_LD + j);
+#pragma unroll
+                for (int v = 0; v < VB; ++v) {
+                    float4 x[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) x[e] = *reinterpret_cast<const float4*>(Vs + (j + e) * V_LD + v * 64 + tx * 4);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        float(&a)[4] = acc[i][v];
+                        a[0] = add(w4[i].w, x[3].x, add(w4[i].z, x[2].x, add(w4[i].y, x[1].x, add(w4[i].x, x[0].x, a[0]))));
+                        a[1] = add(w4[i].w, x[3].y, add(w4[i].z, x[2].y, add(w4[i].y, x[1].y, add(w4[i].x, x[0].y, a[1]))));
+                        a[2] = add(w4[i].w, x[3].z, add(w4[i].z, x[2].z, add(w4[i].y, x[1].z, add(w4[i].x, x[0].z, a[2]))));
+                        a[3] = add(w4[i].w, x[3].w, add(w4[i].z, x[2].w, add(w4[i].y, x[1].w, add(w4[i].x, x[0].w, a[3]))));
+                    }
+                }
+            }
+        };
+        if (cut) apply(std::true_type{});
+        else apply(std::false_type{});
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int r = ty + i * 16;
+        if (r >= n_rows) continue;
+        const int64_t at = (int64_t)b * p.S + position(r);
+        const int h = head(r);
+        float* out = static_cast<float*>(p.out) + at * p.out_ld;
+#pragma unroll
+        for (int v = 0; v < VB; ++v)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const int col = v * 64 + tx * 4 + c;
+                if (col >= p.vdim) continue;
+                float o = acc[i][v][c] / l[i];
+                if (p.gate) o *= sigmoid_exact(static_cast<const float*>(p.gate)[at * p.gate_ld + h * p.vdim + col]);
+                out[h * p.vdim + col] = o;
+            }
+        if (h == p.H - 1)                                      // the padding columns behind the last head
+            for (int c = p.H * p.vdim + tx; c < p.out_ld; c += 16) out[c] = 0.f;
+    }
+}
+
+static size_t attn_tiles_f32_smem(const AttnPortionParams& p) {
+    const int pieces = (p.dim + p.rot + 63) / 64, blocks = (p.vdim + 63) / 64;
+    return (size_t)(AP_KEYS * AP_LD + AP_KEYS * blocks * 64 + AP_ROWS * (AP_LD + pieces * 64 + 4 + 1)) * sizeof(float);
+}
+
+// Whole 16-byte pieces of keys and values at 16-byte addresses, at most 128 value columns, and room for the queries
+static bool attn_tiles_f32_ok(const AttnPortionParams& p) {
+    const uintptr_t at = reinterpret_cast<uintptr_t>(p.k) | reinterpret_cast<uintptr_t>(p.v) | (p.rot ? reinterpret_cast<uintptr_t>(p.krot) : 0);
+    return p.vdim <= 128 && (p.dim | p.rot | p.vdim) % 4 == 0 && (p.k_ld | p.v_ld | p.k_seq | p.v_seq | p.k_head | p.v_head) % 4 == 0 &&
+           (p.rot == 0 || p.krot_ld % 4 == 0) && (at & 15) == 0 && attn_tiles_f32_smem(p) <= 200 * 1024;
+}
+
+template <int VB>
+static int attn_tiles_f32(const AttnPortionParams& p, cudaStream_t st, const char* what) {
+    const long long tiles = ((long long)p.S * (p.H / p.kv_heads) + AP_ROWS - 1) / AP_ROWS, blocks = tiles * p.B * p.kv_heads;
+    if (blocks > 0x7fffffffLL) return fail(BN_ERR_UNSUPPORTED, "%s: B=%d x S=%d too large", what, p.B, p.S);
+    const size_t smem = attn_tiles_f32_smem(p);
+    if (int rc = allow_smem(attn_tiles_f32_kernel<VB>, smem, what)) return rc;
+    launch_dependent(attn_tiles_f32_kernel<VB>, (unsigned)blocks, AP_THREADS, smem, st, p);
+    return launch_status(what);
+}
+
 template <typename T>
 static int attn_tiled(const AttnPortionParams& p, cudaStream_t st, const char* what) {
-    size_t smem = (size_t)AT_ROWS * ((p.dim + p.rot + 3) / 4 * 4 + 4) * sizeof(float);
+    const size_t smem = (size_t)AT_ROWS * ((p.dim + p.rot + 3) / 4 * 4 + 4) * sizeof(float);
     const long long tiles = ((long long)p.S * (p.H / p.kv_heads) + AT_ROWS - 1) / AT_ROWS, blocks = tiles * p.B * p.kv_heads;
     if (blocks > 0x7fffffffLL) return fail(BN_ERR_UNSUPPORTED, "%s: B=%d x S=%d too large", what, p.B, p.S);
     auto run = [&](auto kernel) {
@@ -319,20 +502,15 @@ static int attn_tiled(const AttnPortionParams& p, cudaStream_t st, const char* w
         launch_dependent(kernel, (unsigned)blocks, AT_THREADS, smem, st, p);
         return launch_status(what);
     };
-    if (sizeof(T) == 4 && p.rot == 0 && p.dim <= AT_E && p.vdim <= 64 && (p.dim | p.vdim) % 4 == 0 &&
-        (p.k_ld | p.v_ld | p.k_seq | p.v_seq | p.k_head | p.v_head) % 4 == 0 &&
-        ((reinterpret_cast<uintptr_t>(p.k) | reinterpret_cast<uintptr_t>(p.v)) & 15) == 0) {
-        smem += AT_KEYS * 64 * sizeof(float);
-        return run(attn_tiled_kernel<float, 1, true>);
-    }
-    if (p.vdim <= 64) return run(attn_tiled_kernel<T, 1, false>);
-    if (p.vdim <= 128) return run(attn_tiled_kernel<T, 2, false>);
-    return run(attn_tiled_kernel<T, 4, false>);
+    if (p.vdim <= 64) return run(attn_tiled_kernel<T, 1>);
+    if (p.vdim <= 128) return run(attn_tiled_kernel<T, 2>);
+    return run(attn_tiled_kernel<T, 4>);
 }
 
 int attn_any(const AttnPortionParams& p, int dtype, cudaStream_t st, const char* what) {
     // Portions go through tiles where the rows' queries and the values' columns fit; one-token rows over a cache (a row per
     // head and sequence) and wider heads take a warp per row.
+    if (dtype == 0 && !p.positions && attn_tiles_f32_ok(p)) return p.vdim <= 64 ? attn_tiles_f32<1>(p, st, what) : attn_tiles_f32<2>(p, st, what);
     if (!p.positions && p.vdim <= 256 && p.dim + p.rot <= 1024)
         return dtype == 0 ? attn_tiled<float>(p, st, what) : attn_tiled<__nv_bfloat16>(p, st, what);
     if (p.vdim > AW_MAXV * 32) return fail(BN_ERR_UNSUPPORTED, "%s: vdim=%d (at most %d)", what, p.vdim, AW_MAXV * 32);
