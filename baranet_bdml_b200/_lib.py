@@ -35,6 +35,8 @@ SIGNATURES = {
     "bn_attn_layer_f32": (_i, [_p, _i64, _p, _i64, _p, _i64, _p, _i64, _p, _i64, _p, _i64, _i, _i, _i, _i, _i, _f, _f, _i, _i, _i, _p,
                                _sz, _p]),
     "bn_linear_f32_workspace_bytes": (_sz, [_i, _i, _i]),
+    "bn_linear_f32_streams": (_i, [_i, _i, _i, _i]),
+    "bn_linear_f32_stream": (_i, [_p, _i64, _p, _i64, _p, _i, _p, _i64, _i, _i, _i, _p]),
     "bn_linear_f32_form": (_i, [_i, _i, _i, _i]),
     "bn_linear_f32": (_i, [_p, _i64, _p, _i64, _p, _i, _p, _i, _i, _i, _p, _sz, _p, _p]),
     "bn_rope_f32": (_i, [_p, _i64, _i64, _p, _i64, _i64, _i, _i, _i, _f, _i, _p]),

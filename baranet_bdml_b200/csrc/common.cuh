@@ -75,8 +75,9 @@ inline void prefill_bf16_workspace_layout(int B, int S, int Hkv, size_t* table, 
     *total = *krot + up((size_t)B * S * Hkv * 64 * sizeof(__nv_bfloat16));
 }
 
-// The time of bn_mm_f32 in us, roughly (mm_f32.cu)
+// The times of bn_mm_f32 and of bn_linear_f32_stream in us, roughly (mm_f32.cu, mm_stream_f32.cu)
 float mm_f32_estimate(int M, int N, int K);
+float mm_stream_estimate(int M, int N, int K);
 
 // The RoPE frequency of pair i, with the reference's exact arithmetic
 // (src/ops/op_rope.cuh:82): fp32 exponent, fp32 pow, reciprocal taken in

@@ -461,14 +461,27 @@ extern "C" size_t bn_linear_f32_workspace_bytes(int M, int N, int K) { return M 
 // 192 us, chains 87, 100, 153).  Where the parts alone would have been faster (4 rows 108 us with the cut elsewhere, 16 rows 59), the
 // weight is wide enough for bn_mm_f32_sums to hide its additions (4 / 12 rows 86.5 / 94.7 us, chains 86.5 / 91.9), and the error is
 // the smaller one again; narrower weights, whose time is a chain's latency, keep the chains (1 x 2048 -> 2048 23.0 us, sums 27.1).
+// The time of bn_linear_f32: starts, the cut of the weight (6 or 10 bytes each) and of A, the product
+static float parts_estimate(int M, int N, int K, int w_nparts, float product) {
+    return 6.f + (float)N * (float)K * (w_nparts == 1 ? 0.8e-6f : 1.4e-6f) + (float)M * (float)K * 1.0e-6f + product;
+}
+
 extern "C" int bn_linear_f32_form(int M, int N, int K, int w_nparts) {
     if (M <= 0 || N <= 0 || K <= 0 || N % 8 || K % 8 || !split_fits(M, N, K)) return BN_LINEAR_F32_CHAINS;
     int bn;
     const float product = split_estimate(M, N, K, w_nparts, &bn), chains = mm_f32_estimate(M, N, K);
-    // starts, the cut of the weight (6 or 10 bytes each) and of A
-    const float cut = 6.f + (float)N * (float)K * (w_nparts == 1 ? 0.8e-6f : 1.4e-6f) + (float)M * (float)K * 1.0e-6f;
-    if (M > 16 && cut + product < chains) return BN_LINEAR_F32_PARTS;
+    if (M > 16 && parts_estimate(M, N, K, w_nparts, product) < chains) return BN_LINEAR_F32_PARTS;
     return 11.f + (float)M * (float)K * 1.2e-6f + product < chains ? BN_LINEAR_F32_SUMS : BN_LINEAR_F32_CHAINS;
+}
+
+extern "C" int bn_linear_f32_streams(int M, int N, int K, int w_nparts) {
+    if (M <= 0 || M > 48 || N <= 0 || K <= 0 || N % 8 || K % 8) return 0;      // (64 rows 2048 -> 2048: 32.3 us, chains 25.7)
+    float other = mm_f32_estimate(M, N, K);
+    if (M > 16 && split_fits(M, N, K)) {
+        int bn;
+        other = fminf(other, parts_estimate(M, N, K, w_nparts, split_estimate(M, N, K, w_nparts, &bn)));
+    }
+    return mm_stream_estimate(M, N, K) < other;
 }
 
 extern "C" int bn_linear_f32(const float* a, int64_t a_ld, const float* w, int64_t w_ld, const float* bias, int act, float* c, int M,

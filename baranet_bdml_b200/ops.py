@@ -453,9 +453,9 @@ def _bf16_parts(x: torch.Tensor) -> torch.Tensor:
 
 
 class Linear:
-    """y = act(x W^T + bias) for a weight (out, in), bias (out) and act optional: bf16 on the tensor cores, or true fp32 (chains
-    of FMAs or sums of chains, `bn_mm_f32` and `bn_mm_f32_sums`, or for many rows `bn_linear_f32`, whose error is as small as that
-    of the sums; all read `weight` as it is at the call).
+    """y = act(x W^T + bias) for a weight (out, in), bias (out) and act optional: bf16 on the tensor cores, or true fp32 (for
+    few rows a stream of the weight, `bn_linear_f32_stream`; chains of FMAs or sums of chains, `bn_mm_f32` and `bn_mm_f32_sums`; for
+    many rows `bn_linear_f32`; all read `weight` as it is at the call).
     Both sizes are rounded up to multiples of 8 with zeros, so x may be passed with its padding columns (which must be finite)
     and y has them."""
 
@@ -486,8 +486,13 @@ class Linear:
     def _mm_f32(self, x: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
         """x W^T with the bias and the activation, fp32"""
         w, rows, lib, act = self.weight, x.shape[0], _lib.load(), ACTIVATIONS[self.act]
+        aligned = (x.data_ptr() | w.data_ptr()) % 16 == 0 and w.stride(0) % 4 == 0 and x.stride(0) % 4 == 0
+        if aligned and lib.bn_linear_f32_streams(rows, self.n, self.k, self.parts_hint):
+            _lib.check(lib.bn_linear_f32_stream(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), _ptr(self.bias), act, out.data_ptr(),
+                                                out.stride(0), rows, self.n, self.k, _stream()))
+            return out
         form = lib.bn_linear_f32_form(rows, self.n, self.k, self.parts_hint)
-        if form == _lib.BN_LINEAR_F32_PARTS and (x.data_ptr() | w.data_ptr()) % 16 == 0 and w.stride(0) % 4 == 0:
+        if form == _lib.BN_LINEAR_F32_PARTS and aligned:
             scratch = torch.empty(lib.bn_linear_f32_workspace_bytes(rows, self.n, self.k), dtype=torch.uint8, device=x.device)
             _lib.check(lib.bn_linear_f32(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), _ptr(self.bias), act,
                                          out.data_ptr(), rows, self.n, self.k, scratch.data_ptr(), scratch.numel(),

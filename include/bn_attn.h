@@ -131,6 +131,13 @@ BN_API int bn_linear_f32_form(int M, int N, int K, int w_nparts);
 BN_API int bn_linear_f32(const float* a, int64_t a_ld, const float* w, int64_t w_ld, const float* bias, int act, float* c, int M,
                          int N, int K, void* workspace, size_t workspace_bytes, int* error_word, bn_stream_t stream);
 
+/* The same for few rows (more than 16: 16 at a time), as a stream of the weight: K spread over lanes and warps, sums of pairs.
+ * N a multiple of 8, K of 4; 16-byte aligned rows of a and w.  bn_linear_f32_streams: whether it is the fastest of the ways for
+ * such a product (an estimate). */
+BN_API int bn_linear_f32_streams(int M, int N, int K, int w_nparts);
+BN_API int bn_linear_f32_stream(const float* a, int64_t a_ld, const float* w, int64_t w_ld, const float* bias, int act, float* c,
+                                int64_t c_ld, int M, int N, int K, bn_stream_t stream);
+
 /* The same in two calls, for a weight whose parts the caller keeps and cuts again whenever it changes.
  * bn_split_f32 writes x (rows, cols) as three bf16 matrices [3][rows][cols] whose sum it is; cols a multiple of 8, 16-byte
  * aligned rows.

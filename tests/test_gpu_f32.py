@@ -245,6 +245,41 @@ def test_linear_f32_reads_the_weight_of_the_call(lib, dtype, write):
     assert form(16, 32000) == _lib.BN_LINEAR_F32_SUMS
 
 
+@pytest.mark.parametrize("M", [1, 2, 3, 4, 5, 8, 9, 16, 17, 40])
+@pytest.mark.parametrize("K,N,odd", [(4, 8, 0), (128, 24, 0), (132, 2056, 4), (1028, 4744, 0), (2048, 19000, 0), (7424, 64, 8)])
+def test_linear_stream(lib, M, K, N, odd):
+    """Every number of rows a warp has sums for, one to four slices of K, rounds that are not full, columns that fill no block."""
+    from baranet_bdml_b200 import _lib, ops
+    gen = torch.Generator(device="cuda").manual_seed(M + K + N)
+    x, w = (torch.randn((r, K + odd), generator=gen, device="cuda")[:, :K] for r in (M, N))
+    bias = torch.randn(N, generator=gen, device="cuda")
+    st = torch.cuda.current_stream().cuda_stream
+    run = lambda x, bias, act, out: _lib.check(lib.bn_linear_f32_stream(                         # noqa: E731
+        x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), None if bias is None else bias.data_ptr(), ops.ACTIVATIONS[act],
+        out.data_ptr(), out.stride(0), M, N, K, st))
+    out = torch.full((M, N + 5), 7.0, device="cuda")
+    run(x, None, "none", out)
+    exact, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    # a lane's links (K in 128 lanes at the least), five additions of lanes, four of slices
+    bound = (4 * (K // 128 + 1) + 9) * 2.0 ** -24 * size
+    assert ((out[:, :N].double() - exact).abs() <= bound).all() and bool((out[:, N:] == 7.0).all())
+    run(x, bias, "relu2", out)
+    exact = exact + bias.double()
+    size = size + bias.double().abs()
+    bound = (4 * (K // 128 + 1) + 10) * 2.0 ** -24 * size
+    want = exact.clamp(min=0).square()
+    assert ((out[:, :N].double() - want).abs() <= 2 * bound * (exact.abs() + bound) + 2.0 ** -23 * want).all()
+    if M > 1:                                      # a row that is not finite stays alone
+        y = x.clone()
+        y[M - 1, K - 1] = float("inf")
+        again = torch.empty((M, N), device="cuda")
+        run(y, None, "none", again)
+        chain = torch.empty((1, N), device="cuda")
+        _lib.check(lib.bn_mm_f32(y[M - 1:].data_ptr(), y.stride(0), 1, w.data_ptr(), 1, w.stride(0), chain.data_ptr(), N, 1, 1, K, N, st))
+        run(x, None, "none", out)
+        assert torch.equal(again[:M - 1], out[:M - 1, :N]) and torch.equal(again[M - 1].nan_to_num(5.0), chain[0].nan_to_num(5.0))
+
+
 @pytest.mark.parametrize("M,K,N", [(1, 4, 32), (8, 16, 33), (9, 20, 33), (17, 52, 1000), (33, 144, 4736), (65, 128, 9473), (1151, 272, 2052), (3, 2056, 8)])
 @pytest.mark.parametrize("odd", [False, True])
 def test_mm_sums(lib, M, K, N, odd):
