@@ -49,7 +49,7 @@ class CausalLM:
         rows, cols = logits.shape
         out = torch.empty((rows,), dtype=torch.int32, device="cuda")
         _lib.check(_lib.load().bn_argmax_rows_f32(logits.data_ptr(), logits.stride(0), logits.stride(1), out.data_ptr(),
-                                                  rows, cols, torch.cuda.current_stream().cuda_stream))
+                                                  rows, cols, ops._stream()))
         return out
 
     def capture_decode_step(self):
@@ -263,7 +263,7 @@ class LLaMAModelBF16(CausalLM):
         err = torch.zeros(1, dtype=torch.int32, device="cuda") if error is None else error
         _lib.check(_lib.load().bn_embedding_gather_f32(self.embed_tokens.data_ptr(), H, ids.data_ptr(), out.data_ptr(), H,
                                                        n, H, self.config.vocab_size, err.data_ptr(),
-                                                       torch.cuda.current_stream().cuda_stream))
+                                                       ops._stream()))
         if check and int(err.item()) != 0:
             raise IndexError("token id out of range")
         return out.to(torch.bfloat16)

@@ -12,7 +12,8 @@ from . import _lib
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """The current device's current stream, as the C ABI takes it (a torch.cuda.Stream object for it costs 3 us a call)"""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def _need(t: torch.Tensor, dtype, what: str):

@@ -32,7 +32,7 @@ from . import _lib
 def _stream_ptr() -> int:
     # The reference launches everything on the legacy default stream; torch's
     # current stream is that stream unless the caller changed it.
-    return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 class TensorF:
