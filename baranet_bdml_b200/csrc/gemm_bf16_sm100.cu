@@ -9,6 +9,9 @@
 //   warps 0-3  epilogue: TMEM -> registers -> bf16 -> global (thread = output row = TMEM lane)
 //   warp 4     MMA issuer: tcgen05.mma.cta_group::1.kind::f16, 128 x 256 x 16 per instruction
 //   warp 5     TMA producer: A tile 128 x 64 and Bt tile 256 x 64 per stage (48 KB), 4-stage mbarrier ring
+// (PAIR: a cluster of two CTAs shares a tile of 256 x 256, tcgen05.mma.cta_group::2 issued by the first of them; each loads its 128 rows
+// of A and half of the tile's rows of Bt, 32 KB a stage, 6 stages, and has its 128 rows of the result in its own tensor memory.  Both
+// CTAs' copies are counted on the first one's barriers, commits arrive in both, and both epilogues release an accumulator there.)
 // Output tile 128 x 256; the fp32 accumulator (256 TMEM columns) is double buffered, so the epilogue of one tile
 // runs under the main loop of the next.  Tiles are walked N-panel by N-panel with M fastest, so the CTAs that run
 // together share their Bt panel in L2.  Edges: TMA zero-fills loads beyond M, N, K; stores are bounds-checked.
@@ -35,9 +38,10 @@ constexpr int GM_A_BYTES = GM_BM * GM_BK * 2;          // 16384
 constexpr int GM_THREADS = 192;
 // per N-tile width BN (256: the throughput shape; 64: many small tiles for M <= 128, where the weight stream has to
 // be spread over all SMs): ring depth, bytes, TMEM columns (two accumulators of BN columns, a power of two >= 32)
-template <int BN> struct GemmShape {
-    static constexpr int NSTAGE = BN == 256 ? 4 : 8;
-    static constexpr int B_BYTES = BN * GM_BK * 2;
+// PAIR: two CTAs share a tile of 256 x 256, each with its 128 rows of A and half of the tile of Bt
+template <int BN, bool PAIR = false> struct GemmShape {
+    static constexpr int NSTAGE = PAIR ? 6 : BN == 256 ? 4 : 8;
+    static constexpr int B_BYTES = (PAIR ? BN / 2 : BN) * GM_BK * 2;
     static constexpr int STAGE_BYTES = GM_A_BYTES + B_BYTES;
     static constexpr int SMEM_BYTES = 1024 + NSTAGE * STAGE_BYTES;
     static constexpr uint32_t TMEM_COLS = 2 * BN;
@@ -76,12 +80,14 @@ struct GemmParams {
 };
 
 
-template <int EPI, int GM_BN>
+template <int EPI, int GM_BN, bool PAIR = false>
 __global__ void __launch_bounds__(GM_THREADS, 1)
 gemm_bf16_nt_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                     const GemmParams p) {
-    constexpr int GM_NSTAGE = GemmShape<GM_BN>::NSTAGE, GM_STAGE_BYTES = GemmShape<GM_BN>::STAGE_BYTES;
-    constexpr uint32_t GM_TMEM_COLS = GemmShape<GM_BN>::TMEM_COLS;
+    using Shape = GemmShape<GM_BN, PAIR>;
+    constexpr int GM_NSTAGE = Shape::NSTAGE, GM_STAGE_BYTES = Shape::STAGE_BYTES;
+    constexpr uint32_t GM_TMEM_COLS = Shape::TMEM_COLS;
+    constexpr int TILE_M = PAIR ? 2 * GM_BM : GM_BM;
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t bar_full[GM_NSTAGE], bar_empty[GM_NSTAGE], bar_acc_full[2], bar_acc_empty[2];
     __shared__ uint32_t s_tmem_base;
@@ -90,7 +96,9 @@ gemm_bf16_nt_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
 
     const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
     const uint32_t smem0 = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    const int tiles_m = (p.M + GM_BM - 1) / GM_BM, tiles_n = (p.N + GM_BN - 1) / GM_BN;
+    const uint32_t rank = PAIR ? cluster_rank() : 0;          // the pair's first CTA issues the MMAs
+    const int first = PAIR ? blockIdx.x / 2 : blockIdx.x, stride = PAIR ? gridDim.x / 2 : gridDim.x;
+    const int tiles_m = (p.M + TILE_M - 1) / TILE_M, tiles_n = (p.N + GM_BN - 1) / GM_BN;
     const int k_steps_all = (p.K + GM_BK - 1) / GM_BK;
     // a work item is an output tile, or (EPI_PARTIAL) a tile and one range of the K steps
     const int splits = EPI == EPI_PARTIAL ? p.splits : 1;
@@ -112,17 +120,23 @@ gemm_bf16_nt_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         }
         for (int i = 0; i < 2; ++i) {
             mbar_init(smem_u32(&bar_acc_full[i]), 1);
-            mbar_init(smem_u32(&bar_acc_empty[i]), 4);      // one arrive per epilogue warp
+            mbar_init(smem_u32(&bar_acc_empty[i]), PAIR ? 8 : 4);      // one arrive per epilogue warp
         }
         s_abort = 0;
         fence_mbar_init();
     }
     if (warp == 4) {
-        tc::tmem_alloc(smem_u32(&s_tmem_base), GM_TMEM_COLS);
-        tc::tmem_relinquish();
+        if (PAIR) {
+            tc::pair_tmem_alloc(smem_u32(&s_tmem_base), GM_TMEM_COLS);
+            tc::pair_tmem_relinquish();
+        } else {
+            tc::tmem_alloc(smem_u32(&s_tmem_base), GM_TMEM_COLS);
+            tc::tmem_relinquish();
+        }
     }
     tc::fence_before_sync();
     __syncthreads();
+    if (PAIR) cluster_sync();                                  // the other CTA's barriers are there
     tc::fence_after_sync();
     const uint32_t tmem = s_tmem_base;
 
@@ -131,10 +145,10 @@ gemm_bf16_nt_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     if (warp == 5 && lane == 0) {
         prefetch_tensormap(&tmap_a);
         prefetch_tensormap(&tmap_b);
-        if (EPI == EPI_PARTIAL && (int)blockIdx.x < n_tiles) {
+        if (EPI == EPI_PARTIAL && first < n_tiles) {
             int ks0, ks1;
-            k_range(blockIdx.x, ks0, ks1);
-            for (int ks = ks0; ks < ks1; ++ks) tma_prefetch_2d(&tmap_b, ks * GM_BK, (blockIdx.x / tiles_m) % tiles_n * GM_BN);
+            k_range(first, ks0, ks1);
+            for (int ks = ks0; ks < ks1; ++ks) tma_prefetch_2d(&tmap_b, ks * GM_BK, first / tiles_m % tiles_n * GM_BN);
         }
     }
     grid_dependency_wait();
@@ -145,8 +159,8 @@ gemm_bf16_nt_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         if (lane == 0) {
             uint32_t it = 0;      // ring steps issued
             bool ok = true;
-            for (int t = blockIdx.x; ok && t < n_tiles; t += gridDim.x) {
-                const int m0 = (t % tiles_m) * GM_BM, n0 = ((t / tiles_m) % tiles_n) * GM_BN;
+            for (int t = first; ok && t < n_tiles; t += stride) {
+                const int m0 = (t % tiles_m) * TILE_M + rank * GM_BM, n0 = ((t / tiles_m) % tiles_n) * GM_BN + rank * (GM_BN / 2);
                 int ks0, ks1;
                 k_range(t, ks0, ks1);
                 for (int ks = ks0; ks < ks1; ++ks, ++it) {
@@ -154,6 +168,13 @@ gemm_bf16_nt_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                     ok = mbar_wait(smem_u32(&bar_empty[stage]), ((it / GM_NSTAGE) & 1u) ^ 1u, &s_abort);
                     if (!ok) break;
                     const uint32_t sA = smem0 + stage * GM_STAGE_BYTES, sB = sA + GM_A_BYTES;
+                    if (PAIR) {                                // both CTAs' tiles are counted on the first one's barrier
+                        const uint32_t full = in_rank(smem_u32(&bar_full[stage]), 0);
+                        if (rank == 0) mbar_arrive_expect_tx(smem_u32(&bar_full[stage]), 2 * GM_STAGE_BYTES);
+                        tma_load_2d_pair(sA, &tmap_a, ks * GM_BK, m0, full);
+                        tma_load_2d_pair(sB, &tmap_b, ks * GM_BK, n0, full);
+                        continue;
+                    }
                     mbar_arrive_expect_tx(smem_u32(&bar_full[stage]), GM_STAGE_BYTES);
                     tma_load_2d(sA, &tmap_a, ks * GM_BK, m0, smem_u32(&bar_full[stage]));
                     tma_load_2d(sB, &tmap_b, ks * GM_BK, n0, smem_u32(&bar_full[stage]));
@@ -162,11 +183,11 @@ gemm_bf16_nt_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         }
     } else if (warp == 4) {
         // ------------------------------------------------------------ MMA issuer
-        constexpr uint32_t IDESC = tc::idesc_bf16(GM_BM, GM_BN, 0);
+        constexpr uint32_t IDESC = tc::idesc_bf16(TILE_M, GM_BN, 0);
         const uint64_t dZero = tc::smem_desc_sw128(0);   // descriptor = this + (address >> 4)
         uint32_t it = 0, local = 0;
-        bool ok = true;
-        for (int t = blockIdx.x; ok && t < n_tiles; t += gridDim.x, ++local) {
+        bool ok = rank == 0;
+        for (int t = first; ok && t < n_tiles; t += stride, ++local) {
             const uint32_t acc = local & 1u;
             // the epilogue must have drained this accumulator (two tiles ago)
             ok = mbar_wait(smem_u32(&bar_acc_empty[acc]), ((local >> 1) & 1u) ^ 1u, &s_abort);
@@ -182,11 +203,19 @@ gemm_bf16_nt_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                     tc::fence_after_sync();
                     const uint32_t sA = smem0 + stage * GM_STAGE_BYTES, sB = sA + GM_A_BYTES;
 #pragma unroll
-                    for (int kk = 0; kk < GM_BK / 16; ++kk)
-                        tc::mma_ss(tmem + acc * GM_BN, dZero + (uint64_t)((sA >> 4) + kk * 2),
-                                   dZero + (uint64_t)((sB >> 4) + kk * 2), IDESC, (ks > ks0) || (kk > 0));
-                    tc::commit(smem_u32(&bar_empty[stage]));                       // the stage may be refilled
-                    if (ks == ks1 - 1) tc::commit(smem_u32(&bar_acc_full[acc]));  // the tile is complete
+                    for (int kk = 0; kk < GM_BK / 16; ++kk) {
+                        const uint64_t da = dZero + (uint64_t)((sA >> 4) + kk * 2), db = dZero + (uint64_t)((sB >> 4) + kk * 2);
+                        if (PAIR) tc::pair_mma_ss(tmem + acc * GM_BN, da, db, IDESC, (ks > ks0) || (kk > 0));
+                        else tc::mma_ss(tmem + acc * GM_BN, da, db, IDESC, (ks > ks0) || (kk > 0));
+                    }
+                    const uint32_t empty = smem_u32(&bar_empty[stage]), full = smem_u32(&bar_acc_full[acc]);
+                    if (PAIR) {
+                        tc::pair_commit(empty);                                    // the stage may be refilled, in both CTAs
+                        if (ks == ks1 - 1) tc::pair_commit(full);                  // the tile is complete
+                    } else {
+                        tc::commit(empty);
+                        if (ks == ks1 - 1) tc::commit(full);
+                    }
                 }
                 __syncwarp();
             }
@@ -197,9 +226,9 @@ gemm_bf16_nt_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         const uint32_t lane_base = ((uint32_t)(warp * 32)) << 16;
         uint32_t local = 0;
         bool ok = true;
-        for (int t = blockIdx.x; ok && t < n_tiles; t += gridDim.x, ++local) {
+        for (int t = first; ok && t < n_tiles; t += stride, ++local) {
             const uint32_t acc = local & 1u;
-            const int m0 = (t % tiles_m) * GM_BM, n0 = ((t / tiles_m) % tiles_n) * GM_BN;
+            const int m0 = (t % tiles_m) * TILE_M + rank * GM_BM, n0 = ((t / tiles_m) % tiles_n) * GM_BN;
             if (EPI == EPI_BIAS) {                // the tile's bias, fetched while its products run
                 __syncwarp();
                 for (int c = lane; c < GM_BN; c += 32) s_bias[warp][c] = p.bias && n0 + c < p.n_out ? __ldg(p.bias + n0 + c) : 0.f;
@@ -435,17 +464,22 @@ gemm_bf16_nt_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             // this warp has read its lanes of the accumulator
             tc::fence_before_sync();
             __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&bar_acc_empty[acc]));
+            if (lane == 0) {
+                if (PAIR) mbar_arrive_cluster(in_rank(smem_u32(&bar_acc_empty[acc]), 0));
+                else mbar_arrive(smem_u32(&bar_acc_empty[acc]));
+            }
         }
     }
 
     // common exit: everybody arrives here (all waits are bounded), then TMEM is freed
     tc::fence_before_sync();
     __syncthreads();
+    if (PAIR) cluster_sync();                                  // nothing more is on its way from one CTA to the other
     if (tid == 0 && s_abort && p.error_word) atomicExch(p.error_word, BN_ERR_TIMEOUT);
     if (warp == 4) {
         tc::fence_after_sync();
-        tc::tmem_dealloc(tmem, GM_TMEM_COLS);
+        if (PAIR) tc::pair_tmem_dealloc(tmem, GM_TMEM_COLS);
+        else tc::tmem_dealloc(tmem, GM_TMEM_COLS);
     }
 }
 
@@ -505,15 +539,62 @@ static void splitk_plan(int M, int N, int K, int sms, int* splits, int* k_per_sp
     *splits = (k_steps + per - 1) / per;
 }
 
-template <int EPI, int BN>
-static int gemm_configure(int dev) {
+// Launches the kernel on `grid` CTAs (PAIR: clusters of two), as a programmatic dependent unless what is ahead has to be complete
+template <int EPI, int BN, bool PAIR = false>
+static int gemm_run(const CUtensorMap& a, const CUtensorMap& b, const GemmParams& p, unsigned grid, cudaStream_t st) {
+    constexpr size_t smem = GemmShape<BN, PAIR>::SMEM_BYTES;
     static thread_local int configured_dev = -1;
-    if (configured_dev == dev) return BN_OK;
-    cudaError_t e = cudaFuncSetAttribute(gemm_bf16_nt_kernel<EPI, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         GemmShape<BN>::SMEM_BYTES);
-    if (e != cudaSuccess) return fail(BN_ERR_CUDA, "cudaFuncSetAttribute(gemm): %s", cudaGetErrorString(e));
-    configured_dev = dev;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (configured_dev != dev) {
+        cudaError_t e = cudaFuncSetAttribute(gemm_bf16_nt_kernel<EPI, BN, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return fail(BN_ERR_CUDA, "cudaFuncSetAttribute(gemm): %s", cudaGetErrorString(e));
+        configured_dev = dev;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(GM_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (PAIR) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = 2;
+        attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+        ++n;
+    }
+    if (EPI != EPI_QKV) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n].val.programmaticStreamSerializationAllowed = 1;
+        ++n;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = n;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_bf16_nt_kernel<EPI, BN, PAIR>, a, b, p);
+    if (e != cudaSuccess) {
+        (void)cudaGetLastError();
+        return fail(BN_ERR_CUDA, "gemm: %s", cudaGetErrorString(e));
+    }
     return BN_OK;
+}
+
+// Whether two CTAs share a tile.  A lone CTA moves 96 KB through its shared memory for every 64 k (48 in, 48 to the tensor core),
+// 750 cycles at 128 bytes a cycle beside 512 of MMAs; one of a pair 64 KB, since each holds half of the tile of Bt: 8192 x 11264 x 2048
+// 276 -> 246 us, 8192 x 2048 x 5632 157 -> 138, 2568 x 7424 x 2048 66 -> 60, 4096 x 2048 x 2048 32.4 -> 27.1, 16384 x 2112 x 2048
+// 118 -> 101.  Not where a single wave of tiles leaves nothing to gain on the start of a cluster (16384 x 256 x 2048 18.5, pairs 21.1;
+// 1545 x 2048 x 2048 15.5, pairs 17.1), where a K of less than 1024 leaves the epilogue the longest (16384 x 4096 x 512 83, pairs 99),
+// nor where tiles of twice the rows make a wave more than they save (an eighth).
+static bool gemm_pairs(int M, int N, int K) {
+    const long long sms = sm_count(), columns = (N + 255) / 256, single = ((M + GM_BM - 1) / GM_BM) * columns,
+                    pairs = ((M + 2 * GM_BM - 1) / (2 * GM_BM)) * columns;
+    const long long waves = (single + sms - 1) / sms, waves_of_pairs = (pairs + sms / 2 - 1) / (sms / 2);
+    return K >= 1024 && waves > 1 && waves_of_pairs * 7 <= waves * 8;
+}
+
+template <int EPI>
+static int gemm_run256(bool pairs, const CUtensorMap& a, const CUtensorMap& b, const GemmParams& p, unsigned grid, cudaStream_t st) {
+    return pairs ? gemm_run<EPI, 256, true>(a, b, p, grid, st) : gemm_run<EPI, 256>(a, b, p, grid, st);
 }
 
 static int gemm_launch(const void* a, const void* bt, void* c, int M, int N, int K, int n_out, int epi, int* error_word,
@@ -542,7 +623,8 @@ static int gemm_launch(const void* a, const void* bt, void* c, int M, int N, int
                    n_out, epi >= EPI_GLU ? epi - EPI_GLU : act, epi >= EPI_GLU};
         return gemm_rows(r, as_stream(stream), what);
     }
-    const int bn = epi == EPI_PARTIAL ? 64 : 256;
+    const int bn = epi == EPI_PARTIAL ? 64 : 256, sms = sm_count();
+    const bool pairs = epi != EPI_PARTIAL && gemm_pairs(M, N, K);
     CUtensorMap tmap_a, tmap_b;
     {
         const uint64_t dims[2] = {(uint64_t)K, (uint64_t)M}, strides[1] = {(uint64_t)K * 2};
@@ -553,45 +635,30 @@ static int gemm_launch(const void* a, const void* bt, void* c, int M, int N, int
     }
     {
         const uint64_t dims[2] = {(uint64_t)K, (uint64_t)N}, strides[1] = {(uint64_t)K * 2};
-        const uint32_t box[2] = {GM_BK, (uint32_t)bn};
+        const uint32_t box[2] = {GM_BK, (uint32_t)(pairs ? bn / 2 : bn)};
         if (int rc = make_tensor_map(&tmap_b, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, bt, dims, strides, box,
                                      CU_TENSOR_MAP_SWIZZLE_128B))
             return rc;
     }
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const long long n_items = (long long)((M + GM_BM - 1) / GM_BM) * ((N + bn - 1) / bn) * splits;
+    const int tile_m = pairs ? 2 * GM_BM : GM_BM, places = pairs ? sms / 2 : sms;
+    const long long n_items = (long long)((M + tile_m - 1) / tile_m) * ((N + bn - 1) / bn) * splits;
     GemmParams p{static_cast<__nv_bfloat16*>(c), error_word, M, N, K, n_out, partial, splits, k_per_split, QkvEpilogue{},
                  static_cast<const __nv_bfloat16*>(mul), mul_ld, act, bias};
     if (epi == EPI_F32) p.partial = c32;
     if (qkv) p.qkv = *qkv;
-    const unsigned grid = (unsigned)(n_items < sms ? n_items : sms);
+    const unsigned grid = (unsigned)(n_items < places ? n_items : places) * (pairs ? 2 : 1);
     cudaStream_t st = as_stream(stream);
-    if (epi == EPI_PLAIN) {
-        if (int rc = gemm_configure<EPI_PLAIN, 256>(dev)) return rc;
-        launch_dependent(gemm_bf16_nt_kernel<EPI_PLAIN, 256>, grid, GM_THREADS, GemmShape<256>::SMEM_BYTES, st, tmap_a, tmap_b, p);
-    } else if (epi == EPI_GLU_SILU) {
-        if (int rc = gemm_configure<EPI_GLU_SILU, 256>(dev)) return rc;
-        launch_dependent(gemm_bf16_nt_kernel<EPI_GLU_SILU, 256>, grid, GM_THREADS, GemmShape<256>::SMEM_BYTES, st, tmap_a, tmap_b, p);
-    } else if (epi == EPI_GLU_GELU) {
-        if (int rc = gemm_configure<EPI_GLU_GELU, 256>(dev)) return rc;
-        launch_dependent(gemm_bf16_nt_kernel<EPI_GLU_GELU, 256>, grid, GM_THREADS, GemmShape<256>::SMEM_BYTES, st, tmap_a, tmap_b, p);
-    } else if (epi == EPI_F32) {
-        if (int rc = gemm_configure<EPI_F32, 256>(dev)) return rc;
-        launch_dependent(gemm_bf16_nt_kernel<EPI_F32, 256>, grid, GM_THREADS, GemmShape<256>::SMEM_BYTES, st, tmap_a, tmap_b, p);
-    } else if (epi == EPI_ACTMUL) {
-        if (int rc = gemm_configure<EPI_ACTMUL, 256>(dev)) return rc;
-        launch_dependent(gemm_bf16_nt_kernel<EPI_ACTMUL, 256>, grid, GM_THREADS, GemmShape<256>::SMEM_BYTES, st, tmap_a, tmap_b, p);
-    } else if (epi == EPI_BIAS) {
-        if (int rc = gemm_configure<EPI_BIAS, 256>(dev)) return rc;
-        launch_dependent(gemm_bf16_nt_kernel<EPI_BIAS, 256>, grid, GM_THREADS, GemmShape<256>::SMEM_BYTES, st, tmap_a, tmap_b, p);
-    } else if (epi == EPI_QKV) {
-        if (int rc = gemm_configure<EPI_QKV, 256>(dev)) return rc;
-        gemm_bf16_nt_kernel<EPI_QKV, 256><<<grid, GM_THREADS, GemmShape<256>::SMEM_BYTES, st>>>(tmap_a, tmap_b, p);
-    } else {
-        if (int rc = gemm_configure<EPI_PARTIAL, 64>(dev)) return rc;
-        launch_dependent(gemm_bf16_nt_kernel<EPI_PARTIAL, 64>, grid, GM_THREADS, GemmShape<64>::SMEM_BYTES, st, tmap_a, tmap_b, p);
+    int rc = BN_OK;
+    if (epi == EPI_PLAIN) rc = gemm_run256<EPI_PLAIN>(pairs, tmap_a, tmap_b, p, grid, st);
+    else if (epi == EPI_GLU_SILU) rc = gemm_run256<EPI_GLU_SILU>(pairs, tmap_a, tmap_b, p, grid, st);
+    else if (epi == EPI_GLU_GELU) rc = gemm_run256<EPI_GLU_GELU>(pairs, tmap_a, tmap_b, p, grid, st);
+    else if (epi == EPI_F32) rc = gemm_run256<EPI_F32>(pairs, tmap_a, tmap_b, p, grid, st);
+    else if (epi == EPI_ACTMUL) rc = gemm_run256<EPI_ACTMUL>(pairs, tmap_a, tmap_b, p, grid, st);
+    else if (epi == EPI_BIAS) rc = gemm_run256<EPI_BIAS>(pairs, tmap_a, tmap_b, p, grid, st);
+    else if (epi == EPI_QKV) rc = gemm_run256<EPI_QKV>(pairs, tmap_a, tmap_b, p, grid, st);
+    else rc = gemm_run<EPI_PARTIAL, 64>(tmap_a, tmap_b, p, grid, st);
+    if (rc) return rc;
+    if (epi == EPI_PARTIAL) {
         if (int rc = launch_status(what)) return rc;
         const long long mn4 = (long long)M * N / 4;
         launch_dependent(gemm_splitk_reduce_kernel, (unsigned)((mn4 + 255) / 256), 256, 0, st, (const float*)partial,

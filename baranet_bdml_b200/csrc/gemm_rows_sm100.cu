@@ -33,9 +33,6 @@ template <int MT, int NW> struct RowsShape {
     static constexpr uint32_t TMEM_COLS = NW * MT < 32 ? 32 : NW * MT;
 };
 
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
-}
 __device__ __forceinline__ float4 ld_cluster(uint32_t addr, uint32_t rank) {
     float4 v;
     asm volatile(

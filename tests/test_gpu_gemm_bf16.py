@@ -49,6 +49,56 @@ def test_gemm_projection_shapes_of_the_layer(lib):
         assert float((y.double() - ref).abs().max()) <= float(ref.abs().max()) * 2.0 ** -8
 
 
+# more tiles than multiprocessors and a long K: two CTAs share a tile of 256 x 256.  Odd numbers of 128-row tiles, rows and columns
+# that fill no tile, K that fills no step, one pair more than run together
+PAIRED = [(2569, 2048, 1024), (300, 19000, 1032), (1290, 4616, 1096), (256 * 75, 256, 1024), (4097, 1544, 2040)]
+
+
+@pytest.mark.parametrize("M,N,K", PAIRED)
+def test_paired_tiles_are_the_single_ones(lib, M, N, K):
+    """Every epilogue on rows that come in one call (pairs) and in calls of few enough rows for single tiles: the same sums over the
+    same k in the same order, so the same bits; and against fp64."""
+    from baranet_bdml_b200 import _lib, ops
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    x = torch.randn((M, K), generator=g, device="cuda").bfloat16()
+    w, u = ((torch.randn((N, K), generator=g, device="cuda") * K ** -0.5).bfloat16() for _ in "wu")
+    bias = torch.randn(N, generator=g, device="cuda")
+    mul = torch.randn((M, N), generator=g, device="cuda").bfloat16()
+    packed = ops.pack_gate_up(w, u)
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    st = torch.cuda.current_stream().cuda_stream
+
+    def run(kind, r0, r1):
+        a, m, rows = x[r0:r1], mul[r0:r1], r1 - r0
+        out = torch.full((rows, N), 7.0, dtype=torch.float32 if kind == "f32" else torch.bfloat16, device="cuda")
+        head, tail = (a.data_ptr(), w.data_ptr()), (rows, N, K, err.data_ptr(), st)
+        if kind == "plain":
+            rc = lib.bn_gemm_bf16_nt(*head, out.data_ptr(), *tail)
+        elif kind == "f32":
+            rc = lib.bn_gemm_bf16_nt_f32(*head, out.data_ptr(), *tail)
+        elif kind == "bias":
+            rc = lib.bn_gemm_bias_act_bf16_nt(*head, bias.data_ptr(), out.data_ptr(), rows, N, K, _lib.BN_ACT_RELU2, err.data_ptr(), st)
+        elif kind == "mul":
+            rc = lib.bn_gemm_act_mul_bf16_nt(*head, m.data_ptr(), m.stride(0), out.data_ptr(), rows, N, K, _lib.BN_ACT_SILU, err.data_ptr(), st)
+        else:
+            act = _lib.BN_ACT_SILU if kind == "silu" else _lib.BN_ACT_GELU_TANH
+            rc = lib.bn_gemm_glu_bf16_nt(a.data_ptr(), packed.data_ptr(), out.data_ptr(), rows, N, K, act, err.data_ptr(), st)
+        _lib.check(rc)
+        return out
+
+    few = max(1, 148 // (-(-2 * N // 256))) * 128
+    for kind in ("plain", "f32", "bias", "mul", "silu", "gelu"):
+        whole, parts = run(kind, 0, M), torch.cat([run(kind, r, min(M, r + few)) for r in range(0, M, few)])
+        if few > 128:                       # (up to 128 rows some of them take other forms)
+            assert torch.equal(whole, parts), kind
+        if kind == "f32":
+            exact = x.double() @ w.double().T
+            assert ((whole.double() - exact).abs() <= K * 2.0 ** -23 * (x.double().abs() @ w.double().abs().T)).all()
+        else:
+            assert ((whole.double() - parts.double()).abs() <= 2.0 ** -7 * parts.double().abs() + 2.0 ** -8).all(), kind
+    assert int(err.item()) == 0
+
+
 def test_gemm_rejects_bad_arguments(lib):
     from baranet_bdml_b200 import ops
     a = torch.zeros((16, 12), dtype=torch.bfloat16, device="cuda")
@@ -245,6 +295,39 @@ def test_small_m_gemm(lib, M, N, K):
     scale = max(np.abs(ref).max(), 1e-30)
     assert np.abs(got.float().cpu().numpy() - ref).max() <= scale * 2.0 ** -8
     assert float((got.float() - big.float()).abs().max()) <= scale * 2.0 ** -7
+
+
+@pytest.mark.parametrize("B,S,off", [(3, 803, 0), (2, 1300, 5)])
+def test_fused_qkv_projection_in_paired_tiles(lib, B, S, off):
+    """The fused projection where two CTAs share a tile: its parts are those of the plain products, the cache holds what it returns."""
+    from baranet_bdml_b200 import ops
+    from baranet_bdml_b200.kv_cache import PagedKVCache, PAGE_TOKENS
+    Hq, Hkv, D, hidden = 32, 4, 64, 1024
+    g = torch.Generator(device="cuda").manual_seed(S)
+    x = torch.randn((B * S, hidden), generator=g, device="cuda").bfloat16()
+    w = (torch.randn(((Hq + 2 * Hkv) * D, hidden), generator=g, device="cuda") * 0.03).bfloat16()
+    pages = -(-(S + off) // PAGE_TOKENS)
+    cache = PagedKVCache(B * pages, B, pages, Hkv, D)
+    cache.page_table.copy_(torch.arange(B * pages, dtype=torch.int32).view(B, pages).flip(1))
+    ws = ops.prefill_workspace(B, S, Hq, Hkv, D)
+    ops.prefill_table(ws, B, S, Hkv, D, 10000.0, off)
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    q, v = ops.gemm_qkv_rope_bf16(x, w, B, S, Hq, Hkv, D, ws, position_offset=off, cache=cache, error_word=err)
+    wq, wk, wv = w.split([Hq * D, Hkv * D, Hkv * D])
+    assert torch.equal(q.view(B * S, -1), ops.gemm_bf16_nt(x, wq.contiguous())) and torch.equal(v.view(B * S, -1), ops.gemm_bf16_nt(x, wv.contiguous()))
+    rows = cache.pool[cache.page_table.long()].permute(0, 1, 4, 2, 3, 5).reshape(B, pages * PAGE_TOKENS, Hkv, 2, D)[:, off:off + S]
+    assert torch.equal(rows[:, :, :, 1], v.view(B, S, Hkv, D))
+    k = (x.double() @ wk.double().T).view(B, S, Hkv, D // 2, 2)
+    i = torch.arange(D // 2, device="cuda", dtype=torch.float32)
+    freq = (1.0 / torch.pow(torch.tensor(10000.0, device="cuda"), 2 * i / D)).float()
+    a = ((torch.arange(S, device="cuda", dtype=torch.float32) + off)[:, None] * freq).double()[:, None]
+    want = torch.stack([k[..., 0] * a.cos() - k[..., 1] * a.sin(), k[..., 0] * a.sin() + k[..., 1] * a.cos()], -1).flatten(-2)
+    assert float((rows[:, :, :, 0].double() - want).abs().max()) <= float(want.abs().max()) * 2.0 ** -8
+    out = ops.attn_prefill_bf16(q, None, v, position_offset=off, workspace=ws, reuse_rotated_k=True)
+    ref = ops.attn_prefill_bf16(q, ops.gemm_bf16_nt(x, wk.contiguous()).view(B, S, Hkv, D), v, position_offset=off)
+    assert float((out.float() - ref.float()).abs().max()) <= 2e-2
+    ws.status()
+    assert int(err.item()) == 0
 
 
 @pytest.mark.parametrize("B,S,off", [(2, 200, 0), (1, 128, 0), (3, 77, 5)])
