@@ -99,6 +99,7 @@ SIGNATURES = {
     "bn_latent_expand_out": (_i, [_p, _p, _i, _p, _p, _i64, _i, _i, _i, _i, _i, _p]),
     "bn_mamba2_conv": (_i, [_p, _i64, _p, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _p, _i64, _p, _p, _i,
                             _p]),
+    "bn_ssm_scan_checked": (_i, [_p, _i64, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _p, _i64, _p, _i, _p]),
     "bn_ssm_scan": (_i, [_p, _i64, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _p, _i64, _i, _p]),
     "bn_mamba2_step": (_i, [_p, _i64, _p, _p, _p, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _p, _i, _p]),
     "bn_gemm_bias_act_bf16_nt": (_i, [_p, _p, _p, _p, _i, _i, _i, _i, _p, _p]),

@@ -567,19 +567,32 @@ extern "C" int bn_mamba2_conv(const void* proj, int64_t proj_ld, const float* co
     return launch_status(what);
 }
 
-extern "C" int bn_ssm_scan(const void* xbc, int64_t xbc_ld, const float* dt, const float* a, const float* D, float* state,
-                           const int32_t* seq_ids, int B, int S, int H, int P, int G, int N, void* y, int64_t y_ld, int dtype,
-                           bn_stream_t stream) {
-    const char* what = "bn_ssm_scan";
+static int ssm_scan(const char* what, const void* xbc, int64_t xbc_ld, const float* dt, const float* a, const float* D, float* state,
+                    const int32_t* seq_ids, int B, int S, int H, int P, int G, int N, void* y, int64_t y_ld, int* error_word, int dtype,
+                    bn_stream_t stream) {
     if (!xbc || !dt || !a || !D || !state || !y) return fail(BN_ERR_INVALID_ARG, "%s: null pointer", what);
     if (int rc = mamba2_shape(what, B, S, H, P, G, N, 1, dtype)) return rc;
     if (B == 0 || S == 0) return BN_OK;
     SsmScanParams p{xbc, dt, a, D, state, seq_ids, y, xbc_ld, y_ld, B, S, H, P, G, N};
+    if (dtype == 1 && error_word && ssd_scan_tc_ok(p)) return ssd_scan_tc(p, error_word, as_stream(stream));
     if (dtype == 1 && ssd_scan_ok(p)) return ssd_scan(p, as_stream(stream));
     const unsigned grid = (unsigned)((long long)B * H * ((P + SC_WARPS - 1) / SC_WARPS));
     if (dtype == 0) launch_dependent(ssm_scan_any_kernel<float>, grid, SC_WARPS * 32, 0, as_stream(stream), p);
     else launch_dependent(ssm_scan_any_kernel<__nv_bfloat16>, grid, SC_WARPS * 32, 0, as_stream(stream), p);
     return launch_status(what);
+}
+
+extern "C" int bn_ssm_scan(const void* xbc, int64_t xbc_ld, const float* dt, const float* a, const float* D, float* state,
+                           const int32_t* seq_ids, int B, int S, int H, int P, int G, int N, void* y, int64_t y_ld, int dtype,
+                           bn_stream_t stream) {
+    return ssm_scan("bn_ssm_scan", xbc, xbc_ld, dt, a, D, state, seq_ids, B, S, H, P, G, N, y, y_ld, nullptr, dtype, stream);
+}
+
+extern "C" int bn_ssm_scan_checked(const void* xbc, int64_t xbc_ld, const float* dt, const float* a, const float* D, float* state,
+                                   const int32_t* seq_ids, int B, int S, int H, int P, int G, int N, void* y, int64_t y_ld, int* error_word,
+                                   int dtype, bn_stream_t stream) {
+    if (!error_word) return fail(BN_ERR_INVALID_ARG, "bn_ssm_scan_checked: null pointer");
+    return ssm_scan("bn_ssm_scan_checked", xbc, xbc_ld, dt, a, D, state, seq_ids, B, S, H, P, G, N, y, y_ld, error_word, dtype, stream);
 }
 
 extern "C" int bn_mamba2_step(const void* proj, int64_t proj_ld, const float* conv_w, const float* conv_b, const float* dt_bias,

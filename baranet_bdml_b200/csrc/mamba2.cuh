@@ -17,5 +17,8 @@ struct SsmScanParams {
 
 bool ssd_scan_ok(const SsmScanParams& p);
 int ssd_scan(const SsmScanParams& p, cudaStream_t stream);
+// the same in chunks of 128 tokens on tcgen05 (ssd_scan_sm100.cu); error_word is set when a bounded wait ran out
+bool ssd_scan_tc_ok(const SsmScanParams& p);
+int ssd_scan_tc(const SsmScanParams& p, int* error_word, cudaStream_t stream);
 
 }  // namespace bn

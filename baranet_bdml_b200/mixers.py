@@ -277,9 +277,9 @@ class Mamba2Mixer:
                 self.a_log.data_ptr(), st.conv.data_ptr(), seq_ids.data_ptr(), positions.data_ptr(), B, S, c.heads, c.vdim,
                 c.groups, c.state, c.taps, xbc.data_ptr(), xbc.stride(0), dt.data_ptr(), a.data_ptr(), dt_code, s))
             y = torch.empty((rows, round8(c.inner)), dtype=self.dtype, device=dev)
-            _lib.check(lib.bn_ssm_scan(xbc.data_ptr(), xbc.stride(0), dt.data_ptr(), a.data_ptr(), self.d.data_ptr(),
-                                       st.state.data_ptr(), seq_ids.data_ptr(), B, S, c.heads, c.vdim, c.groups, c.state,
-                                       y.data_ptr(), y.stride(0), dt_code, s))
+            _lib.check(lib.bn_ssm_scan_checked(xbc.data_ptr(), xbc.stride(0), dt.data_ptr(), a.data_ptr(), self.d.data_ptr(),
+                                               st.state.data_ptr(), seq_ids.data_ptr(), B, S, c.heads, c.vdim, c.groups, c.state,
+                                               y.data_ptr(), y.stride(0), ops.status_word(dev).data_ptr(), dt_code, s))
             y_dt, z, z_ld = dt_code, proj, proj.stride(0)
         _lib.check(lib.bn_gated_group_norm(y.data_ptr(), y.stride(0), y_dt, _ptr(z), z_ld, self.norm.data_ptr(), out.data_ptr(),
                                            out.stride(0), rows, c.inner, c.norm_groups, self.eps, dt_code, s))

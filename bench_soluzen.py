@@ -160,13 +160,14 @@ def prompt_kernels(pk, B=8, S=2048, window=1024):
                                       m.state, m.taps, xbc.data_ptr(), xbc.stride(0), dt.data_ptr(), a.data_ptr(), 1, st()))
 
     def scan(i):
-        _lib.check(lib.bn_ssm_scan(xbc.data_ptr(), xbc.stride(0), dt.data_ptr(), a.data_ptr(), mb.d.data_ptr(), rs.state.data_ptr(), seq.data_ptr(),
-                                   B, S, m.heads, m.vdim, m.groups, m.state, y.data_ptr(), y.stride(0), 1, st()))
+        _lib.check(lib.bn_ssm_scan_checked(xbc.data_ptr(), xbc.stride(0), dt.data_ptr(), a.data_ptr(), mb.d.data_ptr(), rs.state.data_ptr(),
+                                           seq.data_ptr(), B, S, m.heads, m.vdim, m.groups, m.state, y.data_ptr(), y.stride(0),
+                                           ops.status_word("cuda").data_ptr(), 1, st()))
     K.hbm("mamba2 conv + steps", timed(conv), T * (2 * m.channels * 2 + m.heads * (2 + 8)))
     ms = timed(scan)
     K.hbm("ssd_scan", ms, T * ((m.channels + m.inner) * 2 + m.heads * 8) + 2 * B * m.heads * m.vdim * m.state * 4)
-    # products of a chunk of 64 tokens and a head: C B^T, M x, C S, w x B (the last three with two-part operands)
-    K.out["ssd_scan"]["TFLOP_per_s"] = 2.0 * T * m.heads * (64 * m.state + 2 * 64 * m.vdim + 4 * m.state * m.vdim) / ms * 1e-9
+    # products of a chunk of 128 tokens and a head: C B^T, M x, C S, w x B (the last three with two-part operands)
+    K.out["ssd_scan"]["TFLOP_per_s"] = 2.0 * T * m.heads * (128 * m.state + 2 * 128 * m.vdim + 4 * m.state * m.vdim) / ms * 1e-9
     og = rnd(T, m.inner)
     K.hbm("gated_group_norm", timed(lambda i: lib.bn_gated_group_norm(y.data_ptr(), y.stride(0), 1, pin.data_ptr(), pin.stride(0), mb.norm.data_ptr(),
                                                                       og.data_ptr(), og.stride(0), T, m.inner, 1, 1e-5, 1, st())), 3 * T * m.inner * 2)

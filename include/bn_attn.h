@@ -517,6 +517,11 @@ BN_API int bn_mamba2_conv(const void* proj, int64_t proj_ld, const float* conv_w
 BN_API int bn_ssm_scan(const void* xbc, int64_t xbc_ld, const float* dt, const float* a, const float* D, float* state,
                        const int32_t* seq_ids, int B, int S, int H, int P, int G, int N, void* y, int64_t y_ld, int dtype,
                        bn_stream_t stream);
+/* The same; heads of 64 values with a state of 128 go to a kernel whose waits are bounded, and *error_word (an int32 on the GPU) becomes
+ * BN_ERR_TIMEOUT when one of them ran out. */
+BN_API int bn_ssm_scan_checked(const void* xbc, int64_t xbc_ld, const float* dt, const float* a, const float* D, float* state,
+                               const int32_t* seq_ids, int B, int S, int H, int P, int G, int N, void* y, int64_t y_ld, int* error_word,
+                               int dtype, bn_stream_t stream);
 /* one new token per row, everything between the two products but the norm: gated (B, H*P) = (y + D x) silu(z) */
 BN_API int bn_mamba2_step(const void* proj, int64_t proj_ld, const float* conv_w, const float* conv_b,
                           const float* dt_bias, const float* a_log, const float* D, void* ring, float* state,

@@ -481,6 +481,75 @@ def test_scan_carries_its_state(lib, dtype, H, P, G, N):
     assert np.array_equal(state[1].double().cpu().numpy(), start[1])
 
 
+@pytest.mark.parametrize("S", [1, 15, 16, 17, 31, 32, 33, 64, 96, 97, 127, 128, 129, 255, 256, 257, 700])
+@pytest.mark.parametrize("H,G,pad", [(4, 2, 0), (3, 1, 8)])
+def test_scan_in_chunks_of_128(lib, S, H, G, pad):
+    """Heads of 64 values with a state of 128 on tcgen05: every way a portion ends inside a chunk, rows with padding, steps of 0,
+    heads that decay within a token, against fp64 and (the state, to two parts' 16 bits) in a slot of their own."""
+    from baranet_bdml_b200 import _lib, ops
+    rng = np.random.default_rng(S + H)
+    B, P, N = 2, 64, 128
+    inner = H * P
+    C = inner + 2 * G * N
+    ld = C + pad
+    xbc = torch.full((B, S, ld), float("nan"), dtype=torch.bfloat16, device="cuda")
+    xbc[:, :, :C] = gpu(rng.standard_normal((B, S, C)), torch.bfloat16)
+    step = np.logaddexp(0, rng.standard_normal((B, S, H)))
+    step[:, ::7] = 0.0
+    dt = gpu(step)
+    A = gpu(-np.exp(np.linspace(-6.0, 3.0, H)))
+    a, D = (dt * A).contiguous(), gpu(rng.standard_normal(H))
+    state = gpu(rng.standard_normal((3, H, P, N)))
+    start = state.double().cpu().numpy()
+    slots = torch.tensor([2, 0], dtype=torch.int32, device="cuda")
+    y = torch.full((B, S, inner + pad), 7.0, dtype=torch.bfloat16, device="cuda")
+    word = torch.zeros(1, dtype=torch.int32, device="cuda")
+    _lib.check(_lib.load().bn_ssm_scan_checked(xbc.data_ptr(), ld, dt.data_ptr(), a.data_ptr(), D.data_ptr(), state.data_ptr(), slots.data_ptr(),
+                                               B, S, H, P, G, N, y.data_ptr(), y.stride(1), word.data_ptr(), 1,
+                                               torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    assert int(word.item()) == 0 and bool((y[:, :, inner:] == 7.0).all())
+    X, dn, an, Dn = xbc[:, :, :C].double().cpu().numpy(), dt.double().cpu().numpy(), a.double().cpu().numpy(), D.double().cpu().numpy()
+    grp = np.arange(H) // (H // G)
+    for b, slot in enumerate((2, 0)):
+        St = start[slot].copy()
+        want = np.empty((S, H, P))
+        for t in range(S):
+            x, Bt, Ct = X[b, t, :inner].reshape(H, P), X[b, t, inner:inner + G * N].reshape(G, N)[grp], X[b, t, inner + G * N:].reshape(G, N)[grp]
+            St = np.exp(an[b, t])[:, None, None] * St + dn[b, t][:, None, None] * x[:, :, None] * Bt[:, None, :]
+            want[t] = np.einsum("hpn,hn->hp", St, Ct) + Dn[:, None] * x
+        got = y[b, :, :inner].double().cpu().numpy().reshape(S, H, P)
+        assert np.abs(got - want).max() <= 2.0 ** -8 * np.abs(want).max()
+        assert np.abs(state[slot].double().cpu().numpy() - St).max() <= 1e-4 * np.abs(St).max()
+    assert np.array_equal(state[1].double().cpu().numpy(), start[1])
+
+
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+@pytest.mark.parametrize("t", [0, 16, 40, 127, 128, 200])
+def test_scan_of_a_token_that_is_not_finite(lib, bad, t):
+    """It reaches no token before its sixteen, no other value's output, and all tokens behind it."""
+    from baranet_bdml_b200 import _lib
+    rng = np.random.default_rng(t)
+    S, H, P, N = 250, 2, 64, 128
+    C = H * P + 2 * N
+    xbc = gpu(rng.standard_normal((1, S, C)), torch.bfloat16)
+    dt = gpu(np.full((1, S, H), 0.1))
+    a, D = -dt, gpu(rng.standard_normal(H))
+    word = torch.zeros(1, dtype=torch.int32, device="cuda")
+
+    def run(x):
+        state, y = torch.zeros((1, H, P, N), device="cuda"), torch.empty((1, S, H * P), dtype=torch.bfloat16, device="cuda")
+        _lib.check(_lib.load().bn_ssm_scan_checked(x.data_ptr(), C, dt.data_ptr(), a.data_ptr(), D.data_ptr(), state.data_ptr(), None, 1, S, H, P, 1,
+                                                   N, y.data_ptr(), H * P, word.data_ptr(), 1, torch.cuda.current_stream().cuda_stream))
+        return y[0]
+    clean = run(xbc)
+    xbc[0, t, 5] = bad
+    got = run(xbc)
+    others = [c for c in range(H * P) if c != 5]
+    assert torch.equal(got[:, others], clean[:, others]) and torch.equal(got[:t // 16 * 16], clean[:t // 16 * 16])
+    assert not torch.isfinite(got[t:, 5]).any() and int(word.item()) == 0
+
+
 @DTYPES
 @pytest.mark.parametrize("sizes", [dict(), dict(heads=2, vdim=64, state=128, groups=1, conv=4, norm_groups=1),
                                    dict(heads=4, vdim=12, state=256, groups=2, conv=1, norm_groups=2),
