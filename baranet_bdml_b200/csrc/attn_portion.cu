@@ -492,6 +492,255 @@ static int attn_tiles_f32(const AttnPortionParams& p, cudaStream_t st, const cha
     return launch_status(what);
 }
 
+// ---------------------------------------------------------------------------------------------------------------
+// One new fp32 token a sequence over its cached keys.  A cluster of up to eight CTAs per (sequence, key head, group of eight of
+// its query heads): block j of 32 keys belongs to warp j / ranks of CTA j % ranks, so that short and long sequences both spread
+// over all warps, and a key or value is read once for eight heads.  A warp has all keys and values of its block on their way
+// into shared memory at once; a lane = (head, every fourth key) for the scores and weights, VC value columns of all eight
+// heads for the result.  Warps keep their own maxima and meet in shared memory, CTAs in each other's (the entry has no scratch
+// memory to give).
+// What bounds it is latency: 1024 keys of 64 columns are one pass of a cluster's 32 warps.  The loops are unrolled no further
+// than loads need: a step meets this code cold, and the same work in 2500 instructions in a row took 28 us however short the
+// sequence was.  A warp per head that walks the keys by itself (attn_any_kernel) is a chain of rounds: 32 heads over 4 x 64
+// columns, 4 sequences of 400 tokens, 580 us; this 13.
+// ---------------------------------------------------------------------------------------------------------------
+constexpr int SA_WARPS = 4, SA_HEADS = 8, SA_MAXRANKS = 8, SA_THREADS = SA_WARPS * 32;
+
+// E, V: columns of keys and values in shared memory (64 or 128 each)
+template <int E, int V>
+struct SaShape {
+    static constexpr int LD = E + 4;
+    static constexpr int SMEM_BYTES = SA_WARPS * 32 * (LD + V) * 4;
+};
+
+template <int E, int V>
+__global__ void __launch_bounds__(SA_THREADS)
+attn_step_f32_kernel(const AttnPortionParams p, int ranks) {
+    constexpr int LD = SaShape<E, V>::LD, VC = V / 32;
+    extern __shared__ __align__(16) float sa_smem[];
+    __shared__ __align__(16) float qs[SA_HEADS][LD];                           // zeros behind the columns and the heads
+    __shared__ __align__(16) float ws[SA_WARPS][32][SA_HEADS], part[SA_WARPS][SA_HEADS][V], cta[SA_HEADS][V];
+    __shared__ float shr[SA_WARPS][SA_HEADS], wm[SA_WARPS][SA_HEADS], wl[SA_WARPS][SA_HEADS], cm[SA_HEADS], cl[SA_HEADS], hs[SA_HEADS],
+        share[SA_MAXRANKS][SA_HEADS];
+    ptx::grid_dependency_wait();
+    ptx::grid_launch_dependents();
+    const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32, rank = (int)ptx::cluster_rank();
+    const int n_rep = p.H / p.kv_heads, hgs = (n_rep + SA_HEADS - 1) / SA_HEADS, item = blockIdx.x / ranks;
+    const int hg = item % hgs, g = item / hgs % p.kv_heads, b = item / (hgs * p.kv_heads);
+    const int h0 = g * n_rep + hg * SA_HEADS, heads = min(SA_HEADS, n_rep - hg * SA_HEADS);
+    const int block = p.seq_ids ? p.seq_ids[b] : b, last = p.positions[b] % p.span, first = max(0, mask_oldest(p.mask, p.span, last));
+    const bool room = last < p.rows_per_seq;                                   // else the cache has no room for this token
+    const float* kseq = static_cast<const float*>(p.k) + block * p.k_seq + g * p.k_head;
+    const float* vseq = static_cast<const float*>(p.v) + block * p.v_seq + g * p.v_head;
+    float* Ks = sa_smem + warp * 32 * (LD + V);
+    float* Vs = Ks + 32 * LD;
+    auto fetch = [&](int k0) {                                                 // two groups: keys, values
+#pragma unroll 4
+        for (int i = lane; i < 32 * (E / 4); i += 32) {
+            const int k = i / (E / 4), e = i % (E / 4) * 4;
+            const bool in = k0 + k <= last && e < p.dim;
+            ptx::cp_async_16(ptx::smem_u32(Ks + k * LD + e), kseq + (in ? (k0 + k) * p.k_ld + e : 0), in ? 16 : 0);
+        }
+        ptx::cp_async_commit();
+#pragma unroll 4
+        for (int i = lane; i < 32 * (V / 4); i += 32) {
+            const int k = i / (V / 4), c = i % (V / 4) * 4;
+            const bool in = k0 + k <= last && c < p.vdim;
+            ptx::cp_async_16(ptx::smem_u32(Vs + k * V + c), vseq + (in ? (k0 + k) * p.v_ld + c : 0), in ? 16 : 0);
+        }
+        ptx::cp_async_commit();
+    };
+    int k0 = room ? first + (warp * ranks + rank) * 32 : last + 1;
+    if (k0 <= last) fetch(k0);
+#pragma unroll 1
+    for (int h = warp; h < SA_HEADS; h += SA_WARPS) {
+        const float* q = static_cast<const float*>(p.q) + b * p.q_ld + (int64_t)(h0 + h) * p.dim;
+        float ss = 0.f;
+#pragma unroll
+        for (int e = lane; e < E; e += 32) {
+            const float x = h < heads && e < p.dim ? q[e] : 0.f;
+            qs[h][e] = x;
+            ss = fmaf(x, x, ss);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        if (lane == 0) hs[h] = p.rms_dim ? p.scale * rsqrtf(ss / (float)p.rms_dim + p.rms_eps) : p.scale;
+    }
+    __syncthreads();
+    const int hw = lane / 4, kw = lane % 4, c0 = lane * VC;
+    float m = -INFINITY, l = 0.f, acc[SA_HEADS][VC];
+#pragma unroll
+    for (int h = 0; h < SA_HEADS; ++h)
+#pragma unroll
+        for (int c = 0; c < VC; ++c) acc[h][c] = 0.f;
+#pragma unroll 1
+    for (; k0 <= last; ) {
+        ptx::cp_async_wait<1>();
+        __syncwarp();
+        float mx = m;
+#pragma unroll 1
+        for (int i = 0; i < 8; i += 2) {                                       // two keys a lane at a time
+            float d0 = 0.f, d1 = 0.f;
+#pragma unroll 8
+            for (int e = 0; e < E; e += 4) {
+                float qv[4], ka[4], kb[4];
+                load4(&qs[hw][e], qv);
+                load4(Ks + (i * 4 + kw) * LD + e, ka);
+                load4(Ks + (i * 4 + 4 + kw) * LD + e, kb);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    d0 = fmaf(qv[j], ka[j], d0);
+                    d1 = fmaf(qv[j], kb[j], d1);
+                }
+            }
+            d0 = k0 + i * 4 + kw <= last ? d0 * hs[hw] : -INFINITY;
+            d1 = k0 + i * 4 + 4 + kw <= last ? d1 * hs[hw] : -INFINITY;
+            ws[warp][i * 4 + kw][hw] = d0;
+            ws[warp][i * 4 + 4 + kw][hw] = d1;
+            mx = fmaxf(mx, fmaxf(d0, d1));
+        }
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+        const float base = mx == -INFINITY ? 0.f : mx, shrink = expf(m - base);          // 0 at the first keys (m = -inf)
+        float sum = 0.f;
+#pragma unroll 2
+        for (int i = 0; i < 8; ++i) {
+            const float w = expf(ws[warp][i * 4 + kw][hw] - base);
+            sum += w;
+            ws[warp][i * 4 + kw][hw] = w;
+        }
+        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+        l = l * shrink + sum;
+        m = mx;
+        if (kw == 0) shr[warp][hw] = shrink;
+        ptx::cp_async_wait<0>();
+        __syncwarp();
+#pragma unroll
+        for (int h = 0; h < SA_HEADS; ++h)
+#pragma unroll
+            for (int c = 0; c < VC; ++c) acc[h][c] *= shr[warp][h];
+        const int nk = min(32, last - k0 + 1);
+#pragma unroll 4
+        for (int j = 0; j < nk; ++j) {
+            float vx[VC], w8[SA_HEADS];
+            if (VC == 4) load4(Vs + j * V + c0, *reinterpret_cast<float(*)[4]>(vx));
+            else { const float2 t = *reinterpret_cast<const float2*>(Vs + j * V + c0); vx[0] = t.x; vx[1] = t.y; }
+            load4(&ws[warp][j][0], *reinterpret_cast<float(*)[4]>(w8));
+            load4(&ws[warp][j][4], *reinterpret_cast<float(*)[4]>(w8 + 4));
+#pragma unroll
+            for (int h = 0; h < SA_HEADS; ++h)
+#pragma unroll
+                for (int c = 0; c < VC; ++c) acc[h][c] = fmaf(w8[h], vx[c], acc[h][c]);
+        }
+        __syncwarp();
+        k0 += 32 * SA_WARPS * ranks;
+        if (k0 <= last) fetch(k0);
+    }
+#pragma unroll
+    for (int h = 0; h < SA_HEADS; ++h)
+#pragma unroll
+        for (int c = 0; c < VC; ++c) part[warp][h][c0 + c] = acc[h][c];
+    if (kw == 0) { wm[warp][hw] = m; wl[warp][hw] = l; }
+    __syncthreads();
+    if (tid < SA_HEADS) {                                                      // the CTA's warps
+        float top = -INFINITY, sum = 0.f;
+        for (int w = 0; w < SA_WARPS; ++w) top = fmaxf(top, wm[w][tid]);
+        const float base = top == -INFINITY ? 0.f : top;
+#pragma unroll 1
+        for (int w = 0; w < SA_WARPS; ++w) {
+            const float f = expf(wm[w][tid] - base);
+            shr[w][tid] = f;
+            sum = fmaf(wl[w][tid], f, sum);
+        }
+        cm[tid] = top;
+        cl[tid] = sum;
+    }
+    __syncthreads();
+    for (int i = tid; i < SA_HEADS * V; i += SA_THREADS) {
+        const int h = i / V, c = i % V;
+        float o = 0.f;
+#pragma unroll
+        for (int w = 0; w < SA_WARPS; ++w) o = fmaf(part[w][h][c], shr[w][h], o);
+        cta[h][c] = o;
+    }
+    ptx::cluster_sync();
+    if (tid < SA_HEADS) {                                                      // the cluster's CTAs
+        float ms[SA_MAXRANKS], ls[SA_MAXRANKS], top = -INFINITY, sum = 0.f;
+#pragma unroll
+        for (int r = 0; r < SA_MAXRANKS; ++r) {
+            ms[r] = r < ranks ? ptx::ld_cluster(ptx::in_rank(ptx::smem_u32(&cm[tid]), r)) : -INFINITY;
+            ls[r] = r < ranks ? ptx::ld_cluster(ptx::in_rank(ptx::smem_u32(&cl[tid]), r)) : 0.f;
+        }
+#pragma unroll
+        for (int r = 0; r < SA_MAXRANKS; ++r) top = fmaxf(top, ms[r]);
+        const float base = top == -INFINITY ? 0.f : top;
+#pragma unroll
+        for (int r = 0; r < SA_MAXRANKS; ++r) {
+            ms[r] = expf(ms[r] - base);
+            sum = fmaf(ls[r], ms[r], sum);
+        }
+#pragma unroll
+        for (int r = 0; r < SA_MAXRANKS; ++r) share[r][tid] = ms[r] / sum;
+    }
+    __syncthreads();
+    for (int i = rank * SA_THREADS + tid; i < heads * p.vdim; i += ranks * SA_THREADS) {
+        const int h = i / p.vdim, c = i % p.vdim;
+        float part_of[SA_MAXRANKS], o = 0.f;
+#pragma unroll
+        for (int r = 0; r < SA_MAXRANKS; ++r) part_of[r] = r < ranks ? ptx::ld_cluster(ptx::in_rank(ptx::smem_u32(&cta[h][c]), r)) : 0.f;
+#pragma unroll
+        for (int r = 0; r < SA_MAXRANKS; ++r) o = fmaf(part_of[r], share[r][h], o);
+        const int at = (h0 + h) * p.vdim + c;
+        if (p.gate) o *= sigmoid_exact(static_cast<const float*>(p.gate)[b * p.gate_ld + at]);
+        static_cast<float*>(p.out)[b * p.out_ld + at] = room ? o : __int_as_float(0x7fc00000);
+    }
+    if (room && rank == 0 && h0 + heads == p.H)                                // the padding columns behind the last head
+        for (int64_t i = (int64_t)p.H * p.vdim + tid; i < p.out_ld; i += SA_THREADS) static_cast<float*>(p.out)[b * p.out_ld + i] = 0.f;
+    ptx::cluster_sync();                                                       // nobody leaves while its sums are being read
+}
+
+// Whole 16-byte pieces of keys and values at 16-byte addresses, at most 128 columns of each, keys of their own for each head
+static bool attn_step_f32_ok(const AttnPortionParams& p) {
+    return p.positions && p.S == 1 && p.rot == 0 && p.dim <= 128 && p.vdim <= 128 && (p.dim | p.vdim) % 4 == 0 &&
+           (p.k_ld | p.v_ld | p.k_seq | p.v_seq | p.k_head | p.v_head) % 4 == 0 &&
+           ((reinterpret_cast<uintptr_t>(p.k) | reinterpret_cast<uintptr_t>(p.v)) & 15) == 0;
+}
+
+static int attn_step_f32(const AttnPortionParams& p, cudaStream_t st, const char* what) {
+    const int n_rep = p.H / p.kv_heads;
+    const long long items = (long long)p.B * p.kv_heads * ((n_rep + SA_HEADS - 1) / SA_HEADS), keys = p.span < p.rows_per_seq ? p.span : p.rows_per_seq;
+    // as many ranks as the longest sequence has passes of a CTA's warps for, while about two CTAs a multiprocessor hold them all
+    // (one where both heads are wider than 64)
+    int ranks = SA_MAXRANKS;
+    while (ranks > 1 && (items * ranks > 2LL * sm_count() || (ranks / 2) * 32LL * SA_WARPS >= keys)) ranks /= 2;
+    if (items * ranks > 0x7fffffffLL) return fail(BN_ERR_UNSUPPORTED, "%s: B=%d too large", what, p.B);
+    auto run = [&](auto kernel, size_t smem) {
+        if (int rc = allow_smem(kernel, smem, what)) return rc;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)(items * ranks));
+        cfg.blockDim = dim3(SA_THREADS);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = st;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)ranks;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 2;
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, p, ranks);
+        if (e == cudaSuccess) return launch_status(what);
+        (void)cudaGetLastError();
+        return fail(BN_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
+    };
+    if (p.dim <= 64 && p.vdim <= 64) return run(attn_step_f32_kernel<64, 64>, SaShape<64, 64>::SMEM_BYTES);
+    if (p.dim <= 64) return run(attn_step_f32_kernel<64, 128>, SaShape<64, 128>::SMEM_BYTES);
+    if (p.vdim <= 64) return run(attn_step_f32_kernel<128, 64>, SaShape<128, 64>::SMEM_BYTES);
+    return run(attn_step_f32_kernel<128, 128>, SaShape<128, 128>::SMEM_BYTES);
+}
+
 template <typename T>
 static int attn_tiled(const AttnPortionParams& p, cudaStream_t st, const char* what) {
     const size_t smem = (size_t)AT_ROWS * ((p.dim + p.rot + 3) / 4 * 4 + 4) * sizeof(float);
@@ -508,9 +757,10 @@ static int attn_tiled(const AttnPortionParams& p, cudaStream_t st, const char* w
 }
 
 int attn_any(const AttnPortionParams& p, int dtype, cudaStream_t st, const char* what) {
-    // Portions go through tiles where the rows' queries and the values' columns fit; one-token rows over a cache (a row per
-    // head and sequence) and wider heads take a warp per row.
+    // Portions go through tiles where the rows' queries and the values' columns fit, fp32 rows of one token over a cache through a
+    // cluster per key head; other one-token rows and wider heads take a warp per row.
     if (dtype == 0 && !p.positions && attn_tiles_f32_ok(p)) return p.vdim <= 64 ? attn_tiles_f32<1>(p, st, what) : attn_tiles_f32<2>(p, st, what);
+    if (dtype == 0 && attn_step_f32_ok(p)) return attn_step_f32(p, st, what);
     if (!p.positions && p.vdim <= 256 && p.dim + p.rot <= 1024)
         return dtype == 0 ? attn_tiled<float>(p, st, what) : attn_tiled<__nv_bfloat16>(p, st, what);
     if (p.vdim > AW_MAXV * 32) return fail(BN_ERR_UNSUPPORTED, "%s: vdim=%d (at most %d)", what, p.vdim, AW_MAXV * 32);

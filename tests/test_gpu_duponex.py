@@ -534,6 +534,43 @@ def test_one_token_over_the_cache(lib, dtype, H, G, E, V, chunk):
             assert (f64(cache.k[int(s), :, m + 1:]) == 9.0).all()
 
 
+# The fp32 step's cluster: one rank or several, a group of eight heads full, short by some or followed by a second, columns in one
+# block of 64 or two, sequences that end inside a block of 32 keys, at its end, and in a cluster's second pass
+@pytest.mark.parametrize("H,G,E,V,chunk", [(32, 4, 64, 64, 2200), (9, 1, 72, 128, 257), (16, 2, 128, 40, 512), (7, 7, 4, 100, 33), (1, 1, 64, 64, 4200)])
+@pytest.mark.parametrize("n", [0, 31, 32, 255, 256, 2047, 4199])
+def test_one_fp32_token_in_a_cluster(lib, H, G, E, V, chunk, n):
+    """Against all scores at once in fp64: a result is a mean of values of 1, off by the rounding of a score of about 10 and of
+    sums of n terms, 2^-24 * (E + 10 + n / 32 in a chain)"""
+    from baranet_bdml_b200 import _lib
+    from baranet_bdml_b200.kv_cache import ChunkCache
+    g, n, eps, scale = torch.Generator(device="cuda").manual_seed(H + n), n % chunk, 1e-4, 2.0 * E ** -0.5
+    B, dev = 3, "cuda"
+    cache = ChunkCache(B, chunk, G, E, V, torch.float32)
+    cache.k.normal_(generator=g)
+    cache.v.normal_(generator=g)
+    el, vl = cache.dim_ld, cache.vdim_ld
+    cache.k[..., E:], cache.v[..., V:] = 0, 0
+    widths = [H * el, G * el, G * vl, H * vl]
+    proj = torch.randn(B, sum(widths), generator=g, device=dev)
+    q, k, v, gate = (t.view(B, -1, d) for t, d in zip(proj.split(widths, 1), (el, el, vl, vl)))
+    q[..., E:], k[..., E:], v[..., V:], gate[..., V:] = 0, 0, 0, 0
+    out, word = torch.full((B, H * vl + 8), 7.0, device=dev), torch.zeros(1, dtype=torch.int32, device=dev)
+    sl, at = ints([2, 0, 1]), ints([n, n // 2, n + chunk])
+    _lib.check(_lib.load().bn_gqa_step(
+        q.data_ptr(), k.data_ptr(), v.data_ptr(), gate.data_ptr(), proj.stride(0), None, 0, 0.0, cache.k.data_ptr(), cache.v.data_ptr(),
+        cache.num_seqs, cache.ring_tokens, chunk, sl.data_ptr(), at.data_ptr(), None, cache.tickets.data_ptr(), 1, out.data_ptr(), out.stride(0),
+        B, H, G, el, vl, E, eps, scale, word.data_ptr(), 0, stream()))
+    assert bool((out[:, H * vl:] == 0).all()) and int(word.item()) == 0
+    for b, slot in enumerate((2, 0, 1)):
+        m = int(at[b]) % chunk
+        keys, values = (t[slot, :, :m + 1].double().repeat_interleave(H // G, 0) for t in (cache.k, cache.v))
+        query = q[b].double()
+        query = query * (query.square().sum(1, keepdim=True) / E + eps).rsqrt()
+        want = (torch.softmax((keys @ query[:, :, None])[:, :, 0] * scale, 1)[:, None] @ values)[:, 0] * torch.sigmoid(gate[b].double())
+        err = float((out[b, :H * vl].view(H, vl).double() - want).abs().max())
+        assert err <= 2.0 ** -24 * 4 * (E + 10 + n / 32), (b, m, err)
+
+
 @DTYPES
 def test_a_token_behind_the_cache_gives_nan_and_touches_nothing(lib, dtype):
     from baranet_bdml_b200.mixers import ChunkedAttention, ChunkedAttentionConfig
