@@ -11,8 +11,8 @@
 //
 // One new token: ONE launch does convolution, step, recurrence and gate (bn_mamba2_step).  It writes row p % taps of the
 // ring, the only row that no other block of the launch reads.  A prompt portion: convolution and step over all rows, the
-// ring update, the scan, the gated norm.  The scan of this file goes token by token and takes any sizes in fp32 and bf16;
-// the chunked tensor-core scan is in ssd_scan.cu.
+// ring update, the scan, the gated norm.  The scans of this file go token by token: one takes any sizes in fp32 and bf16, one
+// fp32 rows of the usual sizes; the chunked tensor-core scans are in ssd_scan.cu and ssd_scan_sm100.cu.
 #include "common.cuh"
 #include "hybrid.cuh"
 #include "mamba2.cuh"
@@ -204,6 +204,167 @@ ssm_scan_any_kernel(const SsmScanParams p) {
 #pragma unroll
     for (int i = 0; i < SC_MAXN; ++i)
         if (i * 32 + lane < p.N) state[i * 32 + lane] = s[i];
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// The same for fp32 rows of N = 64 or 128: a warp holds eight values of one head, sixteen lanes four values each, a lane every
+// sixteenth group of four of the N state elements.  Tokens come through shared memory, SF_TOK a stage, the next stage on its way
+// while one is worked on; the sums over N of four tokens and four values are folded over the sixteen lanes together.
+// What bounds it: three operations an element and token on pairs (FFMA2: 48 issues where single ones took 96; 4 x 128 tokens
+// 67 -> 55 us), with the shared-memory reads of B and C close behind; with one warp a scheduler (one sequence of 64 heads), the
+// chain of a token, 160 ns.  The warp-per-value form above waits for a token's loads before it asks for the next ones:
+// 64 heads of 64 x 128, 2 x 256 tokens 783 -> 62 us, 1 x 512 about 1600 -> 81.
+// ---------------------------------------------------------------------------------------------------------------
+constexpr int SF_TOK = 16;
+
+using Pair = unsigned long long;                        // two fp32 in a register pair
+__device__ __forceinline__ Pair pair(float a, float b) {
+    Pair r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ Pair pair_mul(Pair a, Pair b) {
+    Pair r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ Pair pair_fma(Pair a, Pair b, Pair c) {
+    Pair r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ float pair_sum(Pair a) {
+    float lo, hi;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a));
+    return lo + hi;
+}
+__device__ __forceinline__ void load_pairs(const float* p, Pair (&v)[2]) {
+    const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(p);
+    v[0] = t.x;
+    v[1] = t.y;
+}
+
+template <int NR, int WARPS>                            // NR: groups of four state elements a lane (N = 64 NR)
+__global__ void __launch_bounds__(WARPS * 32)
+ssm_scan_f32_kernel(const SsmScanParams p) {
+    constexpr int N = NR * 64, VALS = WARPS * 8, THREADS = WARPS * 32;
+    __shared__ __align__(16) float bc[2][SF_TOK][2 * N], xs[2][SF_TOK][VALS];
+    __shared__ float2 step[2][SF_TOK];                  // step size and decay
+    ptx::grid_dependency_wait();
+    ptx::grid_launch_dependents();
+    const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32, in = lane % 16, vw = warp * 8 + lane / 16 * 4;
+    const int tiles = (p.P + VALS - 1) / VALS, pt = blockIdx.x % tiles, h = blockIdx.x / tiles % p.H, b = blockIdx.x / (tiles * p.H);
+    const int v0 = pt * VALS, g = h / (p.H / p.G), slot = p.seq_ids ? p.seq_ids[b] : b;
+    const float* rows = static_cast<const float*>(p.xbc) + (int64_t)b * p.S * p.xbc_ld;
+    const float* dts = p.dt + (int64_t)b * p.S * p.H + h;
+    const float* as = p.a + (int64_t)b * p.S * p.H + h;
+    const int b_col = p.H * p.P + g * N, c_col = b_col + p.G * N, x_col = h * p.P + v0;
+    const bool mine = v0 + vw < p.P;                    // P is a multiple of four
+    // Tokens behind the portion: a decay of one and zeros, which leave the state as it is
+    float dt_next, a_next;                              // not waited for before the stage in hand is done
+    auto fetch = [&](int t0, int buf) {
+        for (int i = tid; i < SF_TOK * (N / 2); i += THREADS) {
+            const int t = i / (N / 2), e = i % (N / 2) * 4;
+            const bool ok = t0 + t < p.S;
+            ptx::cp_async_16(ptx::smem_u32(&bc[buf][t][e]), rows + (ok ? (t0 + t) * p.xbc_ld + (e < N ? b_col + e : c_col + e - N) : 0), ok ? 16 : 0);
+        }
+        for (int i = tid; i < SF_TOK * (VALS / 4); i += THREADS) {
+            const int t = i / (VALS / 4), e = i % (VALS / 4) * 4;
+            const bool ok = t0 + t < p.S && v0 + e < p.P;
+            ptx::cp_async_16(ptx::smem_u32(&xs[buf][t][e]), rows + (ok ? (t0 + t) * p.xbc_ld + x_col + e : 0), ok ? 16 : 0);
+        }
+        ptx::cp_async_commit();
+        const bool ok = tid < SF_TOK && t0 + tid < p.S;
+        dt_next = ok ? dts[(int64_t)(t0 + tid) * p.H] : 0.f;
+        a_next = ok ? as[(int64_t)(t0 + tid) * p.H] : 0.f;
+    };
+    float* state = p.state + (((int64_t)slot * p.H + h) * p.P + v0 + vw) * N + in * 4;
+    Pair s[4][NR][2];
+#pragma unroll
+    for (int v = 0; v < 4; ++v)
+#pragma unroll
+        for (int r = 0; r < NR; ++r) {
+            if (mine) load_pairs(state + v * N + r * 64, s[v][r]);
+            else s[v][r][0] = s[v][r][1] = pair(0.f, 0.f);
+        }
+    const float D = p.D[h];
+    float* y = static_cast<float*>(p.y) + (int64_t)b * p.S * p.y_ld + x_col + vw + in % 4;
+    fetch(0, 0);
+    if (tid < SF_TOK) step[0][tid] = make_float2(dt_next, expf(a_next));
+    for (int t0 = 0, buf = 0; t0 < p.S; t0 += SF_TOK, buf ^= 1) {
+        if (t0 + SF_TOK < p.S) {
+            fetch(t0 + SF_TOK, buf ^ 1);
+            ptx::cp_async_wait<1>();
+        } else {
+            ptx::cp_async_wait<0>();
+        }
+        __syncthreads();
+        const int n = min(SF_TOK, p.S - t0);
+#pragma unroll 2
+        for (int q = 0; q < n; q += 4) {
+            Pair sum2[16];                              // [token][value], even and odd elements apart
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float2 dd = step[buf][q + j];
+                float x[4];
+                load4(&xs[buf][q + j][vw], x);
+#pragma unroll
+                for (int v = 0; v < 4; ++v) x[v] *= dd.x;
+#pragma unroll
+                for (int r = 0; r < NR; ++r) {
+                    Pair bt[2], ct[2];
+                    load_pairs(&bc[buf][q + j][r * 64 + in * 4], bt);
+                    load_pairs(&bc[buf][q + j][N + r * 64 + in * 4], ct);
+#pragma unroll
+                    for (int v = 0; v < 4; ++v)
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            s[v][r][e] = pair_fma(pair(dd.y, dd.y), s[v][r][e], pair_mul(bt[e], pair(x[v], x[v])));
+                            sum2[j * 4 + v] = r || e ? pair_fma(s[v][r][e], ct[e], sum2[j * 4 + v]) : pair_mul(s[v][r][e], ct[e]);
+                        }
+                }
+            }
+            float sum[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) sum[i] = pair_sum(sum2[i]);
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    if (i < o) {
+                        const float keep = in & o ? sum[i + o] : sum[i], give = in & o ? sum[i] : sum[i + o];
+                        sum[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+                    }
+            // lane `in` is left with token in / 4 and value in % 4
+            const int t = q + in / 4;
+            if (mine && t0 + t < p.S) y[(int64_t)(t0 + t) * p.y_ld] = fmaf(D, xs[buf][t][vw + in % 4], sum[0]);
+        }
+        if (tid < SF_TOK) step[buf ^ 1][tid] = make_float2(dt_next, expf(a_next));
+        __syncthreads();
+    }
+    if (mine)
+#pragma unroll
+        for (int v = 0; v < 4; ++v)
+#pragma unroll
+            for (int r = 0; r < NR; ++r)
+                *reinterpret_cast<ulonglong2*>(state + v * N + r * 64) = make_ulonglong2(s[v][r][0], s[v][r][1]);
+}
+
+// Rows that 16-byte loads can take, and the two sizes of state
+static bool ssm_scan_f32_ok(const SsmScanParams& p) {
+    return (p.N == 64 || p.N == 128) && p.P % 4 == 0 && p.xbc_ld % 4 == 0 &&
+           ((reinterpret_cast<uintptr_t>(p.xbc) | reinterpret_cast<uintptr_t>(p.state)) & 15) == 0;
+}
+
+template <int NR>
+static void ssm_scan_f32(const SsmScanParams& p, cudaStream_t st) {
+    // the largest blocks that still reach every multiprocessor: each stages B and C for itself.  2 x 256 tokens of 64 heads: blocks
+    // of 32 values 62 us, of 16 (twice as many) 87
+    const long long heads = (long long)p.B * p.H;
+    auto blocks = [&](int vals) { return heads * ((p.P + vals - 1) / vals); };
+    if (blocks(64) >= sm_count()) launch_dependent(ssm_scan_f32_kernel<NR, 8>, (unsigned)blocks(64), 256, 0, st, p);
+    else if (blocks(32) >= sm_count()) launch_dependent(ssm_scan_f32_kernel<NR, 4>, (unsigned)blocks(32), 128, 0, st, p);
+    else launch_dependent(ssm_scan_f32_kernel<NR, 2>, (unsigned)blocks(16), 64, 0, st, p);
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -576,6 +737,11 @@ static int ssm_scan(const char* what, const void* xbc, int64_t xbc_ld, const flo
     SsmScanParams p{xbc, dt, a, D, state, seq_ids, y, xbc_ld, y_ld, B, S, H, P, G, N};
     if (dtype == 1 && error_word && ssd_scan_tc_ok(p)) return ssd_scan_tc(p, error_word, as_stream(stream));
     if (dtype == 1 && ssd_scan_ok(p)) return ssd_scan(p, as_stream(stream));
+    if (dtype == 0 && ssm_scan_f32_ok(p)) {
+        if (N == 64) ssm_scan_f32<1>(p, as_stream(stream));
+        else ssm_scan_f32<2>(p, as_stream(stream));
+        return launch_status(what);
+    }
     const unsigned grid = (unsigned)((long long)B * H * ((P + SC_WARPS - 1) / SC_WARPS));
     if (dtype == 0) launch_dependent(ssm_scan_any_kernel<float>, grid, SC_WARPS * 32, 0, as_stream(stream), p);
     else launch_dependent(ssm_scan_any_kernel<__nv_bfloat16>, grid, SC_WARPS * 32, 0, as_stream(stream), p);

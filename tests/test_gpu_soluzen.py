@@ -524,6 +524,40 @@ def test_scan_in_chunks_of_128(lib, S, H, G, pad):
     assert np.array_equal(state[1].double().cpu().numpy(), start[1])
 
 
+# blocks of 16, 32 and 64 values, values that end inside a block, both sizes of state, groups, portions that end inside a stage of 16
+# tokens and inside four
+@pytest.mark.parametrize("B,H,P,G,N", [(2, 4, 64, 2, 128), (2, 40, 36, 1, 128), (10, 30, 64, 3, 128), (1, 6, 12, 2, 64), (160, 1, 64, 1, 64),
+                                       (75, 4, 100, 1, 64)])
+@pytest.mark.parametrize("S", [1, 3, 4, 15, 16, 17, 33, 70])
+def test_scan_of_fp32_rows(lib, B, H, P, G, N, S):
+    """Against fp64: an output is a sum over N of elements that fade from token to token, S roundings in a chain at most and a
+    tree over N behind it"""
+    from baranet_bdml_b200 import _lib
+    g = torch.Generator(device="cuda").manual_seed(S + H)
+    inner, dev = H * P, "cuda"
+    C = inner + 2 * G * N
+    xbc = torch.full((B, S, C + 4), float("nan"), device=dev)
+    xbc[:, :, :C] = torch.randn(B, S, C, generator=g, device=dev)
+    dt = torch.nn.functional.softplus(torch.randn(B, S, H, generator=g, device=dev))
+    a = dt * -torch.exp(torch.linspace(-6.0, 3.0, H, device=dev))
+    D, state = torch.randn(H, generator=g, device=dev), torch.randn(B + 1, H, P, N, generator=g, device=dev)
+    slots = torch.randperm(B + 1, generator=g, device=dev).to(torch.int32)
+    St, untouched = state[slots[:B].long()].double(), state[slots[B].long()].clone()
+    y = torch.full((B, S, inner + 3), 7.0, device=dev)
+    _lib.check(_lib.load().bn_ssm_scan(xbc.data_ptr(), C + 4, dt.data_ptr(), a.data_ptr(), D.data_ptr(), state.data_ptr(), slots.data_ptr(), B, S, H, P,
+                                       G, N, y.data_ptr(), y.stride(1), 0, torch.cuda.current_stream().cuda_stream))
+    x = xbc[:, :, :inner].double().view(B, S, H, P)
+    Bt, Ct = (t.double().view(B, S, G, N).repeat_interleave(H // G, 2) for t in xbc[:, :, inner:C].split(G * N, 2))
+    want = torch.empty_like(x)
+    for t in range(S):
+        St = torch.exp(a[:, t].double())[..., None, None] * St + dt[:, t].double()[..., None, None] * x[:, t, :, :, None] * Bt[:, t, :, None]
+        want[:, t] = (St @ Ct[:, t, :, :, None])[..., 0] + D.double()[:, None] * x[:, t]
+    tol = 2.0 ** -24 * (2 * min(S, 64) + 16)
+    assert float((y[:, :, :inner].double().view_as(want) - want).abs().max()) <= tol * float(want.abs().max())
+    assert float((state[slots[:B].long()].double() - St).abs().max()) <= tol * float(St.abs().max())
+    assert torch.equal(state[slots[B].long()], untouched) and bool((y[:, :, inner:] == 7.0).all())
+
+
 @pytest.mark.parametrize("bad", [float("inf"), float("nan")])
 @pytest.mark.parametrize("t", [0, 16, 40, 127, 128, 200])
 def test_scan_of_a_token_that_is_not_finite(lib, bad, t):
