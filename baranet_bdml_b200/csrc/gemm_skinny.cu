@@ -54,6 +54,52 @@ struct SkinnyParams {
     float theta;
 };
 
+// Where a finished sum of row `row`, column n goes, and what is done to it on the way
+template <bool GLU>
+__device__ __forceinline__ void skinny_store(const SkinnyParams& p, int row, int n, float v) {
+    if (p.out32) {
+        p.out32[(size_t)row * p.N + n] = v;
+        return;
+    }
+    if (p.bias) v += __ldg(p.bias + n);
+    if (!GLU) v = activation_fast(p.act, v);
+    if (p.mul) v *= __bfloat162float(p.mul[row * p.mul_ld + n]);
+    // selects, not indexed parameter arrays (an index known only at run time would copy them to local memory)
+    __nv_bfloat16* o = p.out[0];
+    int ld = p.ld[0], first = 0;
+    if (n >= p.n_end[1]) { o = p.out[2]; ld = p.ld[2]; first = p.n_end[1]; }
+    else if (n >= p.n_end[0]) { o = p.out[1]; ld = p.ld[1]; first = p.n_end[0]; }
+    o[(size_t)row * ld + (n - first)] = __float2bfloat16(v);
+}
+
+// APPEND: what bn_kv_append does with the bf16 row the plain kernel would have written: the value is rounded to bf16 first, a K pair
+// (2i, 2i+1) = (this column, its neighbour's lane) is rotated at the row's position in fp32 and rounded again, V is stored as it
+// is - the cache ends up with the bits of the two-launch path.  Whole warps call it.
+__device__ __forceinline__ void skinny_append(const SkinnyParams& p, int row, int n, float v) {
+    const float vb = __bfloat162float(__float2bfloat16(v));
+    const float other = __shfl_xor_sync(0xffffffffu, vb, 1);
+    if (row < p.M) {
+        const bool is_k = n < p.n_end[1];
+        const int local = n - (is_k ? p.n_end[0] : p.n_end[1]);
+        const int g = local / p.D, d = local - g * p.D;
+        const int pos = p.positions[row];
+        const int lp = pos / BN_PAGE_TOKENS;
+        if (pos >= 0 && lp < p.max_pages) {
+            const int page = p.page_table[(int64_t)p.seq_ids[row] * p.max_pages + lp];
+            if (page >= 0 && page < p.pool_pages) {
+                float y = vb;
+                if (is_k) {
+                    const float angle = pos * rope_inv_freq(d / 2, p.D, p.theta);
+                    const float c = cosf(angle), sn = sinf(angle);
+                    y = (d & 1) ? other * sn + vb * c : vb * c - other * sn;
+                }
+                p.pool[((((int64_t)page * p.Hkv + g) * 2 + (is_k ? 0 : 1)) * BN_PAGE_TOKENS + pos % BN_PAGE_TOKENS) * p.D + d] =
+                    __float2bfloat16(y);
+            }
+        }
+    }
+}
+
 // CH = K steps whose loads a lane keeps in flight at once.  More of them cover more latency per warp; fewer leave
 // registers for more CTAs per SM (8: two, 2: four), which matters when the grid would otherwise need a second, nearly
 // empty wave.
@@ -167,45 +213,132 @@ gemm_skinny_kernel(const SkinnyParams p) {
         }
         const int n = n0 + col;
         if (APPEND && n >= p.n_end[0]) {       // the same for the CTA's 8 columns: the ranges are multiples of 8
-            // What bn_kv_append does with the bf16 row the plain kernel would have written: the value is rounded to
-            // bf16 first, a K pair (2i, 2i+1) = (this column, its neighbour) is rotated at the row's position in fp32
-            // and rounded again, V is stored as it is - the cache ends up with the bits of the two-launch path.
-            const float vb = __bfloat162float(__float2bfloat16(v));
-            const float other = __shfl_xor_sync(0xffffffffu, vb, 1);
-            if (row < p.M) {
-                const bool is_k = n < p.n_end[1];
-                const int local = n - (is_k ? p.n_end[0] : p.n_end[1]);
-                const int g = local / p.D, d = local - g * p.D;
-                const int pos = p.positions[row];
-                const int lp = pos / BN_PAGE_TOKENS;
-                if (pos >= 0 && lp < p.max_pages) {
-                    const int page = p.page_table[(int64_t)p.seq_ids[row] * p.max_pages + lp];
-                    if (page >= 0 && page < p.pool_pages) {
-                        float y = vb;
-                        if (is_k) {
-                            const float angle = pos * rope_inv_freq(d / 2, p.D, p.theta);
-                            const float c = cosf(angle), sn = sinf(angle);
-                            y = (d & 1) ? other * sn + vb * c : vb * c - other * sn;
-                        }
-                        p.pool[((((int64_t)page * p.Hkv + g) * 2 + (is_k ? 0 : 1)) * BN_PAGE_TOKENS + pos % BN_PAGE_TOKENS) * p.D + d] =
-                            __float2bfloat16(y);
-                    }
-                }
-            }
-        } else if (row < p.M && p.out32) {
-            p.out32[(size_t)row * p.N + n] = v;
+            skinny_append(p, row, n, v);
         } else if (row < p.M) {
-            if (p.bias) v += __ldg(p.bias + n);
-            if (!SWIGLU) v = activation_fast(p.act, v);
-            if (p.mul) v *= __bfloat162float(p.mul[row * p.mul_ld + n]);
-            // selects, not indexed parameter arrays (an index known only at run time would copy them to local memory)
-            __nv_bfloat16* o = p.out[0];
-            int ld = p.ld[0], first = 0;
-            if (n >= p.n_end[1]) { o = p.out[2]; ld = p.ld[2]; first = p.n_end[1]; }
-            else if (n >= p.n_end[0]) { o = p.out[1]; ld = p.ld[1]; first = p.n_end[0]; }
-            o[(size_t)row * ld + (n - first)] = __float2bfloat16(v);
+            skinny_store<SWIGLU>(p, row, n, v);
         }
     }
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// The same for K a multiple of 256: CTAs that stay, two a multiprocessor, and take the groups of eight columns in turn.  A warp
+// keeps its eighth of the activation rows in registers for all of them (the kernel above reads all rows again for every eight
+// columns: with 16 rows that is as much as a weight) and has the next slice of its weight rows on the way into shared memory
+// of its own while it multiplies one: 512 contiguous bytes of a row an instruction, where a fragment's own load is 64 bytes of
+// eight rows each.  No warp waits for another but in the sum over warps, whose buffer alternates.
+// What bounds it is HBM, after the few us until the first rows are there.  us with 1 / 16 rows, before and now, and what
+// the weight takes at the copy bandwidth: 2048 -> 32000 26.0 / 33.9, 20.2 / 22.8 (20.1); 2048 -> 8512 9.6 / 11.6, 6.7 / 8.4
+// (5.4); gated pair 2048 -> 5632 11.7 / 12.8, 9.0 / 10.0 (7.1); 2048 -> 2560 4.5 / 5.7, 3.5 / 5.0 (1.6).  Three slices of
+// room instead of two: the same for the widest, 10 % slower for 2048 -> 4608; one CTA a multiprocessor with six: 12 - 40 %
+// slower; slices asked for in L2 further ahead: 2 - 10 % slower.
+// MULTI: K above 2048, in parts of which a warp holds one at a time.
+// ---------------------------------------------------------------------------------------------------------------
+constexpr int WD_STAGES = 2, WD_STEPS = 8, WD_SLICE = 8 * WD_STEPS * 64;
+constexpr int WD_SMEM = SK_WARPS * WD_STAGES * WD_SLICE, WD_CTAS = 2;
+
+// HI: more than eight rows
+template <bool GLU, bool HI, bool MULTI, bool APPEND>
+__global__ void __launch_bounds__(SK_WARPS * 32, WD_CTAS)
+gemm_wide_kernel(const SkinnyParams p) {
+    constexpr int UNITS = GLU ? 2 : 1;                    // weights of a group: gate and up
+    extern __shared__ __align__(128) uint8_t wd_smem[];
+    __shared__ __align__(8) float s_part[2][UNITS][SK_WARPS][16][8];
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, g = lane / 4, j = lane % 4;
+    const int groups = p.N / 8, mine = (groups - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+    const int parts = MULTI ? (p.steps + WD_STEPS - 1) / WD_STEPS : 1, n_slices = mine * parts * UNITS;
+    const size_t kbase = (size_t)warp * p.steps * 32;
+    auto steps_of = [&](int part) { return MULTI ? min(WD_STEPS, p.steps - part * WD_STEPS) : p.steps; };
+    // Slices in the order group, part, weight: where slice u starts
+    auto slice = [&](int u) {
+        const int part = MULTI ? u / UNITS % parts : 0, i = u / UNITS / parts;
+        const int n0 = ((int)blockIdx.x + i * (int)gridDim.x) * 8;
+        return (GLU && u % 2 ? p.bt2 : p.bt) + (size_t)n0 * p.K + kbase + part * (WD_STEPS * 32);
+    };
+    const uint32_t ring = smem_u32(wd_smem) + warp * (WD_STAGES * WD_SLICE);
+    // Row r's piece c lies at piece c ^ (4 for odd r): the eight lanes of a phase (two rows, four pieces) meet different banks
+    auto fetch = [&](int u) {
+        if (u < n_slices && lane < steps_of(MULTI ? u / UNITS % parts : 0) * 4) {
+            const __nv_bfloat16* w = slice(u) + lane * 8;
+            const uint32_t to = ring + u % WD_STAGES * WD_SLICE;
+#pragma unroll
+            for (int r = 0; r < 8; ++r) cp_async_16(to + r * 512 + ((lane ^ (r & 1) * 4) * 16), w + (size_t)r * p.K, 16);
+        }
+        cp_async_commit();
+    };
+    // The first slices are asked for in L2 beside the kernel ahead: the weights do not depend on it, and nothing is READ before the
+    // wait.  A lane has a line of 64 elements of a row.
+#pragma unroll
+    for (int u = 0; u < WD_STAGES; ++u)
+        if (u < n_slices && j * 64 < steps_of(MULTI ? u / UNITS % parts : 0) * 32) prefetch_l2(slice(u) + (size_t)g * p.K + j * 64);
+    grid_dependency_wait();
+    grid_launch_dependents();
+#pragma unroll
+    for (int u = 0; u < WD_STAGES - 1; ++u) fetch(u);
+    const uint4 z = make_uint4(0, 0, 0, 0);
+    const uint4* a_lo = reinterpret_cast<const uint4*>(p.a + (size_t)g * p.K + kbase) + j;
+    const uint4* a_hi = reinterpret_cast<const uint4*>(p.a + (size_t)(g + 8) * p.K + kbase) + j;
+    uint4 al[WD_STEPS], ah[HI ? WD_STEPS : 1];
+    ah[0] = z;
+    auto load_rows = [&](int part) {
+        const int n = steps_of(part);
+#pragma unroll
+        for (int s = 0; s < WD_STEPS; ++s) {
+            al[s] = s < n && g < p.M ? a_lo[(part * WD_STEPS + s) * 4] : z;
+            if (HI) ah[HI ? s : 0] = s < n && g + 8 < p.M ? a_hi[(part * WD_STEPS + s) * 4] : z;
+        }
+    };
+    load_rows(0);
+    for (int i = 0, u = 0; i < mine; ++i) {
+        const int buf = i & 1;
+        float acc[UNITS][2][4];                           // two chains of MMAs each
+#pragma unroll
+        for (int k = 0; k < UNITS; ++k)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) acc[k][0][c] = acc[k][1][c] = 0.f;
+        for (int part = 0; part < parts; ++part) {
+            const int n = steps_of(part);
+#pragma unroll
+            for (int k = 0; k < UNITS; ++k, ++u) {
+                fetch(u + WD_STAGES - 1);
+                cp_async_wait<WD_STAGES - 1>();
+                __syncwarp();
+                const uint8_t* at = wd_smem + warp * (WD_STAGES * WD_SLICE) + u % WD_STAGES * WD_SLICE + g * 512;
+#pragma unroll
+                for (int s = 0; s < WD_STEPS; ++s)
+                    if (s < n) {
+                        const uint4 w = *reinterpret_cast<const uint4*>(at + ((s * 4 + j) ^ (g & 1) * 4) * 16);
+                        mma_bf16_16816(acc[k][0], al[s].x, ah[HI ? s : 0].x, al[s].y, ah[HI ? s : 0].y, w.x, w.y);
+                        mma_bf16_16816(acc[k][1], al[s].z, ah[HI ? s : 0].z, al[s].w, ah[HI ? s : 0].w, w.z, w.w);
+                    }
+                __syncwarp();                             // the slice is read before the next fetch overwrites it
+            }
+            if (MULTI && (part + 1 < parts || i + 1 < mine)) load_rows(part + 1 < parts ? part + 1 : 0);
+        }
+#pragma unroll
+        for (int k = 0; k < UNITS; ++k) {
+            float (*sums)[8] = s_part[buf][k][warp];
+            *reinterpret_cast<float2*>(&sums[g][2 * j]) = make_float2(acc[k][0][0] + acc[k][1][0], acc[k][0][1] + acc[k][1][1]);
+            if (HI) *reinterpret_cast<float2*>(&sums[g + 8][2 * j]) = make_float2(acc[k][0][2] + acc[k][1][2], acc[k][0][3] + acc[k][1][3]);
+        }
+        __syncthreads();
+        // four of the warps, in turn; the others go on, as far as the next sum
+        const int t = (int)threadIdx.x - buf * 128;
+        if (t >= 0 && t < 128) {
+            const int row = t / 8, n = ((int)blockIdx.x + i * (int)gridDim.x) * 8 + t % 8;
+            float v = 0.f, up = 0.f;
+            if (row < p.M) {
+#pragma unroll
+                for (int w = 0; w < SK_WARPS; ++w) {
+                    v += s_part[buf][0][w][row][t % 8];
+                    if (GLU) up += s_part[buf][UNITS - 1][w][row][t % 8];
+                }
+                if (GLU) v = activation_fast(p.act, v) * up;
+            }
+            if (APPEND && n >= p.n_end[0]) skinny_append(p, row, n, v);
+            else if (row < p.M) skinny_store<GLU>(p, row, n, v);
+        }
+    }
+    cp_async_wait<0>();
 }
 
 static int skinny_check(const char* what, const void* a, const void* bt, int M, int N, int K) {
@@ -219,13 +352,29 @@ static int skinny_check(const char* what, const void* a, const void* bt, int M, 
     return require_sm100();
 }
 
-// Measured on the decode step's shapes: 256 CTAs (o, down) run fastest two per SM with 8 steps in flight, 320 (q/k/v in
-// one launch) four per SM with 2; the gated pair holds two weights and runs with 2.
+// Which kernel.  Of the first: up to two CTAs per SM run fastest with 8 steps in flight, more with four per SM and 2; the gated pair
+// holds two weights and runs with 2.
 template <bool GLU, bool APPEND>
 static int skinny_launch(const SkinnyParams& p, cudaStream_t st, const char* what) {
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    // us before and now, the kernel that stays second.  Gated pairs: 2048 -> 2048 5.4, 4.1, -> 3072 6.0, 6.4 (three CTAs a multiprocessor
+    // hold all groups at once), -> 5632 11.7, 9.0.  Others with 8 rows: 2048 -> 256 2.2, 2.1, -> 4608 5.4, 4.9, 4096 -> 2048 5.4, 4.6,
+    // 7424 -> 2048 8.6, 7.3, but 1024 -> 4608 3.3, 3.5 (1024 -> 6144, in two waves, 5.0, 4.1); with 16 rows the groups have
+    // to share CTAs before the rows kept pay: 2048 -> 512 2.6, 3.0, -> 2048 4.0, 4.1, -> 2560 5.7, 5.0
+    const int groups = p.N / 8;
+    const bool wide = GLU ? groups <= 2 * sms || groups > 3 * sms
+                          : groups > 4 * sms || (p.K >= 1280 && (p.M <= 8 || p.K > 2048 || groups > 2 * sms));
+    if (wide && p.K % (SK_WARPS * 32) == 0) {
+        auto run = [&](auto kernel) {
+            if (int rc = allow_smem(kernel, WD_SMEM, what)) return rc;
+            launch_dependent(kernel, (unsigned)(groups < WD_CTAS * sms ? groups : WD_CTAS * sms), SK_WARPS * 32, WD_SMEM, st, p);
+            return launch_status(what);
+        };
+        if (p.steps > WD_STEPS) return p.M > 8 ? run(gemm_wide_kernel<GLU, true, true, APPEND>) : run(gemm_wide_kernel<GLU, false, true, APPEND>);
+        return p.M > 8 ? run(gemm_wide_kernel<GLU, true, false, APPEND>) : run(gemm_wide_kernel<GLU, false, false, APPEND>);
+    }
     const bool deep = !GLU && p.N / 8 <= 2 * sms;
     if (p.K % (SK_WARPS * 32)) launch_dependent(gemm_skinny_kernel<GLU, 2, APPEND, true>, p.N / 8, SK_WARPS * 32, 0, st, p);
     else if (deep) launch_dependent(gemm_skinny_kernel<GLU, GLU ? 2 : 8, APPEND>, p.N / 8, SK_WARPS * 32, 0, st, p);

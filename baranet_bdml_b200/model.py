@@ -271,7 +271,7 @@ class LLaMAModelBF16(CausalLM):
     def _logits(self, residual: torch.Tensor, pending: torch.Tensor) -> torch.Tensor:
         """final norm of (residual + pending), lm_head: (rows, hidden) -> (rows, vocab) fp32"""
         _, normed = ops.add_rmsnorm_bf16(residual, pending, self.norm_weight, self.config.rms_norm_eps, want_sum=False)
-        return ops.gemm_bf16_nt(normed, self.lm_head).float()
+        return ops.linear_bf16(normed, self.lm_head).float()
 
     # ----------------------------------------------------------------- forward
     def __call__(self, input_ids: torch.Tensor, position_offset: int = 0, use_causal_mask: bool = True) -> torch.Tensor:

@@ -200,12 +200,10 @@ def skinny_any_k(rows: int, n_out: int, k: int) -> bool:
 
 
 def skinny_best(rows: int, n_out: int, k: int) -> bool:
-    """Those of them for which it is the fastest, by whole steps of 1 to 16 sequences.  Its CTAs read the rows for every 8 columns
-    of the weight, which shows with many rows and a wide or a long weight: us at 16 rows, 2048 -> 2048 4.2 (the kernel for up to
-    128 rows: 4.8), 4096 -> 2048 6.4 (6.4), 7424 -> 2048 9.9 (9.6), 2048 -> 4608 7.1 (6.6), 2048 -> 7424 12.0 (8.2), 512 -> 7424
-    5.0 (128 x 256 tiles: 5.7).  A Duponex step of 16 / 12 / 9 sequences, 2 layers, takes 127 / 125 / 122 us, with every product
-    here 152 / 140 / 126; of 5 sequences 117, with the wide ones in the other kernel 119."""
-    return skinny_any_k(rows, n_out, k) and (rows <= 8 or (n_out < 4096 and k <= 4096) or k < 640)
+    """Those of them for which it is the fastest.  Where K is no multiple of 256 its CTAs read the rows for every 8 columns of the
+    weight, which shows with many rows and a wide or a long weight.  With one, us at 16 rows and in the kernel for up to 128 rows:
+    2048 -> 2048 4.1, 4.8, 4096 -> 2048 5.8, 6.4, 7424 -> 2048 9.0, 9.6, 2048 -> 4608 5.9, 6.6, 2048 -> 7424 7.9, 8.2."""
+    return skinny_any_k(rows, n_out, k) and (rows <= 8 or k % 256 == 0 or (n_out < 4096 and k <= 4096) or k < 640)
 
 
 def small_m_ok(rows: int, n_out: int, k: int) -> bool:
@@ -272,7 +270,7 @@ def gemm_swiglu_bf16_nt_skinny(x: torch.Tensor, gate_t: torch.Tensor, up_t: torc
 
 def linear_bf16(x: torch.Tensor, weight_t: torch.Tensor) -> torch.Tensor:
     """x (rows, in) @ weight_t (out, in)^T, choosing the kernel by shape: at most 16 rows -> the weight-streaming
-    kernel, mostly; few rows and few output tiles -> the small-M form; otherwise the large-tile kernel."""
+    kernels, mostly; few rows and few output tiles -> the small-M form; otherwise the large-tile kernel."""
     rows, n_out = x.shape[0], weight_t.shape[0]
     if skinny_best(rows, n_out, x.shape[1]):
         return gemm_bf16_nt_skinny(x, weight_t)

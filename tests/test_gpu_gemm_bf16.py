@@ -414,6 +414,46 @@ def test_skinny_gemm(lib, M, N, K):
         assert torch.equal(torch.cat(parts, dim=1), got)
 
 
+# Wide products of few rows: one column group more than three a multiprocessor, a number of groups that the CTAs do not share evenly,
+# K of one, two, seven and eight steps a warp, rows in the low half of a fragment and in both
+@pytest.mark.parametrize("N,K", [(3560, 256), (4608, 512), (3704, 1792), (8520, 2048)])
+@pytest.mark.parametrize("M", [1, 8, 9, 16])
+def test_wide_products_of_few_rows(lib, M, N, K):
+    """Every output form against fp64: bf16's rounding (2^-9 of the result) and fp32 sums of K terms"""
+    from baranet_bdml_b200 import _lib
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    x = torch.randn(M, K, generator=g, device="cuda").bfloat16()
+    w, u = ((torch.randn(N, K, generator=g, device="cuda") * 0.05).bfloat16() for _ in range(2))
+    bias, mul = torch.randn(N, generator=g, device="cuda"), torch.randn(M, N + 8, generator=g, device="cuda").bfloat16()
+    st = torch.cuda.current_stream().cuda_stream
+    ref = x.double() @ w.double().T
+    up = x.double() @ u.double().T
+    terms = 2.0 ** -24 * (K / 16 + 24) * float((x.double().abs() @ w.double().abs().T).max())
+
+    def out(dtype=torch.bfloat16, cols=N):
+        return torch.full((M, cols), float("nan"), dtype=dtype, device="cuda")
+
+    def near(got, want, slope=1.0, exact=False):
+        err, scale = (got.double() - want).abs(), want.abs()
+        assert bool((err <= (0 if exact else 2.0 ** -8) * scale + slope * terms + 1e-30).all()), float(err.max())
+
+    y32 = out(torch.float32)
+    _lib.check(lib.bn_gemm_bf16_nt_skinny_f32(x.data_ptr(), w.data_ptr(), M, N, K, y32.data_ptr(), st))
+    near(y32, ref, exact=True)
+    n0, n1 = 1024, 2504
+    parts = [out(cols=n) for n in (n0, n1, N - n0 - n1)]
+    _lib.check(lib.bn_gemm_bf16_nt_skinny(x.data_ptr(), w.data_ptr(), M, N, K, parts[0].data_ptr(), n0, parts[1].data_ptr(), n1, parts[2].data_ptr(), st))
+    near(torch.cat(parts, 1), ref)
+    y = out()
+    _lib.check(lib.bn_gemm_bias_act_bf16_nt_skinny(x.data_ptr(), w.data_ptr(), bias.data_ptr(), y.data_ptr(), M, N, K, 3, st))
+    near(y, (ref + bias.double()).clamp_min(0).square(), slope=2 * float((ref + bias.double()).abs().max()))
+    _lib.check(lib.bn_gemm_act_mul_bf16_nt_skinny(x.data_ptr(), w.data_ptr(), mul.data_ptr(), N + 8, y.data_ptr(), M, N, K, 1, st))
+    silu = torch.nn.functional.silu(ref)
+    near(y, silu * mul[:, :N].double(), slope=1.1 * float(mul.abs().max()) + 2.0 ** -12)
+    _lib.check(lib.bn_gemm_glu_bf16_nt_skinny(x.data_ptr(), w.data_ptr(), u.data_ptr(), y.data_ptr(), M, N, K, 1, st))
+    near(y, silu * up, slope=1.1 * float(up.abs().max()) + 1.1 * float(ref.abs().max()))
+
+
 def test_skinny_swiglu(lib):
     from baranet_bdml_b200 import ops
     rng = np.random.default_rng(77)
