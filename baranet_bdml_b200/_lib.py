@@ -41,6 +41,7 @@ SIGNATURES = {
     "bn_linear_f32": (_i, [_p, _i64, _p, _i64, _p, _i, _p, _i, _i, _i, _p, _sz, _p, _p]),
     "bn_rope_f32": (_i, [_p, _i64, _i64, _p, _i64, _i64, _i, _i, _i, _f, _i, _p]),
     "bn_embedding_gather_f32": (_i, [_p, _i64, _p, _p, _i64, _i, _i, _i, _p, _p]),
+    "bn_embedding_gather_f32_bf16": (_i, [_p, _i64, _p, _p, _i64, _i, _i, _i, _p, _p]),
     "bn_argmax_rows_f32": (_i, [_p, _i64, _i64, _p, _i, _i, _p]),
     "bn_add_rmsnorm_bf16": (_i, [_p, _p, _p, _p, _p, _i, _i, _f, _p]),
     "bn_gemm_bf16_nt": (_i, [_p, _p, _p, _i, _i, _i, _p, _p]),
@@ -82,6 +83,7 @@ SIGNATURES = {
     "bn_gemm_act_mul_bf16_nt_small_m": (_i, [_p, _p, _p, _i64, _p, _i, _i, _i, _i, _p, _sz, _p, _p]),
     "bn_gemm_glu_bf16_nt_skinny": (_i, [_p, _p, _p, _p, _i, _i, _i, _i, _p]),
     "bn_gemm_bf16_nt_skinny_f32": (_i, [_p, _p, _i, _i, _i, _p, _p]),
+    "bn_gemm_bf16_nt_skinny_widened": (_i, [_p, _p, _i, _i, _i, _p, _p]),
     "bn_gemm_act_mul_bf16_nt_skinny": (_i, [_p, _p, _p, _i64, _p, _i, _i, _i, _i, _p]),
     "bn_act_mul_f32": (_i, [_p, _i64, _p, _i64, _p, _i64, _i, _i, _i, _p]),
     "bn_embedding_gather_bf16": (_i, [_p, _i64, _p, _p, _i64, _p, _i64, _i, _i, _i, _p, _p]),

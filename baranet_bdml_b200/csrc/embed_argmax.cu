@@ -4,6 +4,7 @@
 //   bn_embedding_gather_f32  out[i, :] = table[ids[i], :]
 //       reference: LLaMAModel.embed gathers on the HOST, row by row, from a device-to-host copy of the whole table
 //       (262 MB for TinyLLaMA) and uploads the result (mygrad/llama/llama_model.py:58-78)
+//   bn_embedding_gather_f32_bf16  the same, rounded to bf16 on the way (a launch and a pass less than with a cast behind it)
 //   bn_argmax_rows_f32       out[r] = index of the first maximum of row r
 //       reference: op_argmax (src/ops/op_reduction.cuh:196-210) with MaxAccumFunc (:5-19): accum = x[0]; a later
 //       element replaces it only if it is strictly greater, so ties keep the first index and a NaN never wins unless
@@ -47,25 +48,28 @@ embedding_gather_bf16_kernel(const __nv_bfloat16* __restrict__ table, int64_t ta
     }
 }
 
+template <typename TO>
 __global__ void __launch_bounds__(256)
 embedding_gather_kernel(const float* __restrict__ table, int64_t table_rs, const uint32_t* __restrict__ ids,
-                        float* __restrict__ out, int64_t out_rs, int n_ids, int hidden, int vocab,
+                        TO* __restrict__ out, int64_t out_rs, int n_ids, int hidden, int vocab,
                         int* __restrict__ error_word) {
     for (int i = blockIdx.x; i < n_ids; i += gridDim.x) {
         const uint32_t id = ids[i];
         const bool valid = id < (uint32_t)vocab;
         if (!valid && threadIdx.x == 0 && error_word) atomicExch(error_word, BN_ERR_INVALID_ARG);
         const float* src = table + (int64_t)(valid ? id : 0) * table_rs;
-        float* dst = out + (int64_t)i * out_rs;
+        TO* dst = out + (int64_t)i * out_rs;
         const bool vec = (hidden % 4 == 0) && (table_rs % 4 == 0) && (out_rs % 4 == 0) &&
                          ((reinterpret_cast<uintptr_t>(table) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
         if (vec) {
             const float4* s4 = reinterpret_cast<const float4*>(src);
-            float4* d4 = reinterpret_cast<float4*>(dst);
-            for (int c = threadIdx.x; c < hidden / 4; c += blockDim.x)
-                d4[c] = valid ? __ldg(s4 + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int c = threadIdx.x; c < hidden / 4; c += blockDim.x) {
+                const float4 f = valid ? __ldg(s4 + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+                const float v[4] = {f.x, f.y, f.z, f.w};
+                store4(dst + 4 * c, v);
+            }
         } else {
-            for (int c = threadIdx.x; c < hidden; c += blockDim.x) dst[c] = valid ? __ldg(src + c) : 0.f;
+            for (int c = threadIdx.x; c < hidden; c += blockDim.x) dst[c] = from_f<TO>(valid ? __ldg(src + c) : 0.f);
         }
     }
 }
@@ -138,21 +142,31 @@ argmax_rows_kernel(const float* x, int64_t x_rs, int64_t x_cs, uint32_t* out, in
 
 using namespace bn;
 
+template <typename TO>
+static int embedding_gather(const char* what, const float* table, int64_t table_rs, const uint32_t* ids, TO* out, int64_t out_rs,
+                            int n_ids, int hidden, int vocab, int* error_word, bn_stream_t stream) {
+    if (!table || !ids || !out) return fail(BN_ERR_INVALID_ARG, "%s: null pointer", what);
+    if (n_ids < 0 || hidden < 0 || vocab <= 0)
+        return fail(BN_ERR_INVALID_ARG, "%s: bad shape n_ids=%d hidden=%d vocab=%d", what, n_ids, hidden, vocab);
+    if (int rc = require_sm100()) return rc;
+    if (n_ids == 0 || hidden == 0) return BN_OK;
+    const long long cap = (long long)sm_count() * 8;
+    embedding_gather_kernel<<<(unsigned)(n_ids < cap ? n_ids : cap), 256, 0, as_stream(stream)>>>(
+        table, table_rs, ids, out, out_rs, n_ids, hidden, vocab, error_word);
+    return launch_status(what);
+}
+
 extern "C" int bn_embedding_gather_f32(const float* table, int64_t table_rs, const uint32_t* ids, float* out,
                                        int64_t out_rs, int n_ids, int hidden, int vocab, int* error_word,
                                        bn_stream_t stream) {
-    if (!table || !ids || !out) return fail(BN_ERR_INVALID_ARG, "bn_embedding_gather_f32: null pointer");
-    if (n_ids < 0 || hidden < 0 || vocab <= 0)
-        return fail(BN_ERR_INVALID_ARG, "bn_embedding_gather_f32: bad shape n_ids=%d hidden=%d vocab=%d", n_ids, hidden, vocab);
-    if (int rc = require_sm100()) return rc;
-    if (n_ids == 0 || hidden == 0) return BN_OK;
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const long long cap = (long long)sms * 8;
-    embedding_gather_kernel<<<(unsigned)(n_ids < cap ? n_ids : cap), 256, 0, as_stream(stream)>>>(
-        table, table_rs, ids, out, out_rs, n_ids, hidden, vocab, error_word);
-    return launch_status("bn_embedding_gather_f32");
+    return embedding_gather("bn_embedding_gather_f32", table, table_rs, ids, out, out_rs, n_ids, hidden, vocab, error_word, stream);
+}
+
+extern "C" int bn_embedding_gather_f32_bf16(const float* table, int64_t table_rs, const uint32_t* ids, void* out,
+                                            int64_t out_rs, int n_ids, int hidden, int vocab, int* error_word,
+                                            bn_stream_t stream) {
+    return embedding_gather("bn_embedding_gather_f32_bf16", table, table_rs, ids, static_cast<__nv_bfloat16*>(out), out_rs, n_ids, hidden,
+                            vocab, error_word, stream);
 }
 
 extern "C" int bn_embedding_gather_bf16(const void* table, int64_t table_rs, const uint32_t* ids, float* out_f32, int64_t rs_f32,

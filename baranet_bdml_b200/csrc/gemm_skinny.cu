@@ -39,6 +39,7 @@ struct SkinnyParams {
     int ld[3];                          // row stride of out[r] in elements
     int M, N, K, steps;                 // steps = K / (8 * 32), rounded up
     float* out32;                       // when set, the (single) output range in fp32 instead of out[0]
+    bool rounded;                       // ... of the sum rounded to bf16
     const __nv_bfloat16* mul;           // when set, out[0] = act(x W) * mul, mul (M, mul_ld)
     long long mul_ld;
     int act;                            // of the gated pair, of `mul`, or of the result plus bias
@@ -58,7 +59,7 @@ struct SkinnyParams {
 template <bool GLU>
 __device__ __forceinline__ void skinny_store(const SkinnyParams& p, int row, int n, float v) {
     if (p.out32) {
-        p.out32[(size_t)row * p.N + n] = v;
+        p.out32[(size_t)row * p.N + n] = p.rounded ? __bfloat162float(__float2bfloat16(v)) : v;
         return;
     }
     if (p.bias) v += __ldg(p.bias + n);
@@ -406,17 +407,24 @@ extern "C" int bn_gemm_bf16_nt_skinny(const void* a, const void* bt, int M, int 
     return skinny_launch<false, false>(p, as_stream(stream), what);
 }
 
-extern "C" int bn_gemm_bf16_nt_skinny_f32(const void* a, const void* bt, int M, int N, int K, float* out, bn_stream_t stream) {
-    const char* what = "bn_gemm_bf16_nt_skinny_f32";
+static int skinny_f32(const char* what, const void* a, const void* bt, int M, int N, int K, float* out, bool rounded, bn_stream_t stream) {
     if (int rc = skinny_check(what, a, bt, M, N, K)) return rc;
     if (!out) return fail(BN_ERR_INVALID_ARG, "%s: null pointer", what);
     SkinnyParams p{};
     p.a = static_cast<const __nv_bfloat16*>(a);
     p.bt = static_cast<const __nv_bfloat16*>(bt);
-    p.out32 = out;
+    p.out32 = out; p.rounded = rounded;
     p.n_end[0] = p.n_end[1] = p.n_end[2] = N;
     p.M = M; p.N = N; p.K = K; p.steps = (K + SK_WARPS * 32 - 1) / (SK_WARPS * 32);
     return skinny_launch<false, false>(p, as_stream(stream), what);
+}
+
+extern "C" int bn_gemm_bf16_nt_skinny_f32(const void* a, const void* bt, int M, int N, int K, float* out, bn_stream_t stream) {
+    return skinny_f32("bn_gemm_bf16_nt_skinny_f32", a, bt, M, N, K, out, false, stream);
+}
+
+extern "C" int bn_gemm_bf16_nt_skinny_widened(const void* a, const void* bt, int M, int N, int K, float* out, bn_stream_t stream) {
+    return skinny_f32("bn_gemm_bf16_nt_skinny_widened", a, bt, M, N, K, out, true, stream);
 }
 
 extern "C" int bn_gemm_bias_act_bf16_nt_skinny(const void* a, const void* bt, const float* bias, void* out, int M, int N, int K,

@@ -259,19 +259,19 @@ class LLaMAModelBF16(CausalLM):
         the flag, a zeroed int32 `error` of its own, later."""
         ids = input_ids.to(torch.int32).contiguous()
         n, H = ids.numel(), self.config.hidden_size
-        out = torch.empty((n, H), dtype=torch.float32, device="cuda")
-        err = torch.zeros(1, dtype=torch.int32, device="cuda") if error is None else error
-        _lib.check(_lib.load().bn_embedding_gather_f32(self.embed_tokens.data_ptr(), H, ids.data_ptr(), out.data_ptr(), H,
-                                                       n, H, self.config.vocab_size, err.data_ptr(),
-                                                       ops._stream()))
+        out = torch.empty((n, H), dtype=torch.bfloat16, device="cuda")
+        err = torch.zeros(1, dtype=torch.int32, device="cuda") if check and error is None else error
+        _lib.check(_lib.load().bn_embedding_gather_f32_bf16(self.embed_tokens.data_ptr(), H, ids.data_ptr(), out.data_ptr(), H,
+                                                            n, H, self.config.vocab_size, None if err is None else err.data_ptr(),
+                                                            ops._stream()))
         if check and int(err.item()) != 0:
             raise IndexError("token id out of range")
-        return out.to(torch.bfloat16)
+        return out
 
     def _logits(self, residual: torch.Tensor, pending: torch.Tensor) -> torch.Tensor:
         """final norm of (residual + pending), lm_head: (rows, hidden) -> (rows, vocab) fp32"""
         _, normed = ops.add_rmsnorm_bf16(residual, pending, self.norm_weight, self.config.rms_norm_eps, want_sum=False)
-        return ops.linear_bf16(normed, self.lm_head).float()
+        return ops.linear_bf16_widened(normed, self.lm_head)
 
     # ----------------------------------------------------------------- forward
     def __call__(self, input_ids: torch.Tensor, position_offset: int = 0, use_causal_mask: bool = True) -> torch.Tensor:
@@ -299,6 +299,7 @@ class LLaMAModelBF16(CausalLM):
         self.caches = [PagedKVCache(pages, B, pages_per_seq, cfg.num_key_value_heads, cfg.head_dim, cfg.rope_theta,
                                     storage=(pools[i], tables[i], lens)) for i in range(n)]
         self.seq_lens = self.caches[0].seq_lens
+        self._all_seqs = torch.arange(B, dtype=torch.int32, device="cuda")
 
     def prefill(self, input_ids: torch.Tensor, max_len: int) -> torch.Tensor:
         """Prompt pass: (B, S) ids -> logits of the last position (B, vocab); fills the KV caches."""
@@ -335,7 +336,7 @@ class LLaMAModelBF16(CausalLM):
         """One new token per sequence: (B,) ids -> (B, vocab) logits; appends to the caches."""
         B = token_ids.numel()
         h = self.embed(token_ids, check)
-        seq_ids = torch.arange(B, dtype=torch.int32, device="cuda")
+        seq_ids = self._all_seqs if B == self._all_seqs.numel() else torch.arange(B, dtype=torch.int32, device="cuda")
         pending = None
         positions = self.seq_lens.clone()                         # the new token's position = current length
         self.seq_lens.add_(1)

@@ -279,6 +279,18 @@ def linear_bf16(x: torch.Tensor, weight_t: torch.Tensor) -> torch.Tensor:
     return gemm_bf16_nt(x, weight_t)
 
 
+def linear_bf16_widened(x: torch.Tensor, weight_t: torch.Tensor) -> torch.Tensor:
+    """`linear_bf16(x, weight_t).float()`, by one launch for the rows that the weight-streaming kernels take."""
+    rows, k = x.shape
+    if weight_t.shape[1] != k or not skinny_best(rows, weight_t.shape[0], k):
+        return linear_bf16(x, weight_t).float()
+    _need(x, torch.bfloat16, "linear_bf16_widened(x)")
+    _need(weight_t, torch.bfloat16, "linear_bf16_widened(weight_t)")
+    out = torch.empty((rows, weight_t.shape[0]), dtype=torch.float32, device=x.device)
+    _lib.check(_lib.load().bn_gemm_bf16_nt_skinny_widened(x.data_ptr(), weight_t.data_ptr(), rows, weight_t.shape[0], k, out.data_ptr(), _stream()))
+    return out
+
+
 def add_rmsnorm_bf16(a: torch.Tensor, b: Optional[torch.Tensor], weight: torch.Tensor, eps: float = 1e-6, *,
                      want_sum: bool = True) -> Tuple[Optional[torch.Tensor], torch.Tensor]:
     """(a + b rounded to bf16, rmsnorm of that sum) for a bf16 residual stream (tokens, hidden); b None: plain norm."""

@@ -161,6 +161,10 @@ BN_API int bn_rope_f32(const float* x, int64_t x_rs, int64_t x_cs, float* y, int
 BN_API int bn_embedding_gather_f32(const float* table, int64_t table_rs, const uint32_t* ids, float* out,
                                    int64_t out_rs, int n_ids, int hidden, int vocab, int* error_word,
                                    bn_stream_t stream);
+/* The same, each element rounded to bf16. */
+BN_API int bn_embedding_gather_f32_bf16(const float* table, int64_t table_rs, const uint32_t* ids, void* out,
+                                        int64_t out_rs, int n_ids, int hidden, int vocab, int* error_word,
+                                        bn_stream_t stream);
 
 /* out[r] = index of the first maximum of row r of x (rows, cols) fp32 with element strides: element 0 stands unless
  * a later element is strictly greater, so ties keep the first index and a NaN wins only at index 0.
@@ -442,6 +446,8 @@ BN_API int bn_gemm_act_mul_bf16_nt_small_m(const void* a, const void* bt, const 
 BN_API int bn_gemm_glu_bf16_nt_skinny(const void* x, const void* gate_t, const void* up_t, void* h, int M, int inter, int K,
                                       int act, bn_stream_t stream);
 BN_API int bn_gemm_bf16_nt_skinny_f32(const void* a, const void* bt, int M, int N, int K, float* out, bn_stream_t stream);
+/* The bf16 result of bn_gemm_bf16_nt_skinny stored as fp32: logits that are read as fp32. */
+BN_API int bn_gemm_bf16_nt_skinny_widened(const void* a, const void* bt, int M, int N, int K, float* out, bn_stream_t stream);
 BN_API int bn_gemm_act_mul_bf16_nt_skinny(const void* a, const void* bt, const void* mul, int64_t mul_ld, void* out, int M,
                                           int N, int K, int act, bn_stream_t stream);
 BN_API int bn_act_mul_f32(const float* a, int64_t a_ld, const float* b, int64_t b_ld, float* out, int64_t out_ld, int rows,

@@ -60,6 +60,23 @@ def test_embedding_gather_is_the_host_gather(lib, vocab, hidden, n):
     assert np.array_equal(_tensor(table).gather_rows(nxt).to_numpy(), table[np.argmax(logits, axis=1)])
 
 
+@pytest.mark.parametrize("hidden,row", [(64, 64), (2048, 2052), (13, 13), (64, 66)])
+def test_embedding_gather_rounded(lib, hidden, row):
+    """The bf16 form is the fp32 one rounded, in rows that vectors can take and in others; an id that is none gives zeros."""
+    from baranet_bdml_b200 import _lib
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(hidden)
+    table = torch.randn(50, row, generator=g, device="cuda")
+    ids = torch.tensor([0, 49, 7, 7, 50], dtype=torch.int32, device="cuda")
+    out, word = torch.full((5, row), 3.0, dtype=torch.bfloat16, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    args = (table.data_ptr(), row, ids.data_ptr(), out.data_ptr(), row, 5, hidden, 50)
+    _lib.check(lib.bn_embedding_gather_f32_bf16(*args, None, torch.cuda.current_stream().cuda_stream))
+    want = table[ids[:4].long(), :hidden].bfloat16()
+    assert torch.equal(out[:4, :hidden], want) and bool((out[4, :hidden] == 0).all()) and bool((out[:, hidden:] == 3.0).all())
+    _lib.check(lib.bn_embedding_gather_f32_bf16(*args, word.data_ptr(), torch.cuda.current_stream().cuda_stream))
+    assert int(word.item()) != 0
+
+
 def test_embedding_gather_rejects_out_of_range(lib):
     table = np.ones((10, 4), dtype=np.float32)
     with pytest.raises(IndexError):

@@ -440,6 +440,9 @@ def test_wide_products_of_few_rows(lib, M, N, K):
     y32 = out(torch.float32)
     _lib.check(lib.bn_gemm_bf16_nt_skinny_f32(x.data_ptr(), w.data_ptr(), M, N, K, y32.data_ptr(), st))
     near(y32, ref, exact=True)
+    widened = out(torch.float32)
+    _lib.check(lib.bn_gemm_bf16_nt_skinny_widened(x.data_ptr(), w.data_ptr(), M, N, K, widened.data_ptr(), st))
+    assert torch.equal(widened, y32.bfloat16().float())
     n0, n1 = 1024, 2504
     parts = [out(cols=n) for n in (n0, n1, N - n0 - n1)]
     _lib.check(lib.bn_gemm_bf16_nt_skinny(x.data_ptr(), w.data_ptr(), M, N, K, parts[0].data_ptr(), n0, parts[1].data_ptr(), n1, parts[2].data_ptr(), st))
