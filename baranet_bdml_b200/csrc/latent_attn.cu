@@ -280,13 +280,15 @@ rope_heads_kernel(T* q, int64_t q_ld, long long n, int S, int H, int dim, int ro
 // rotation.
 //   q_abs[b][h][0..kv_ld) = sum_i q[b][h][i] W_uk[h * dim + i][:]      q_abs[b][h][kv_ld..) = rotated part
 // ---------------------------------------------------------------------------------------------------------------
-constexpr int LA_N = 128, LA_B = 8;
+// LA_PARTS threads share a column, a range of the weight's rows each; LA_AHEAD: rows whose loads a thread has under way together
+// (one thread a column and a row at a time, fp32, 16 heads of 128 -> 512: 24 us; this 6)
+constexpr int LA_N = 128, LA_B = 8, LA_PARTS = 4, LA_AHEAD = 16;
 
 template <typename T>
-__global__ void __launch_bounds__(LA_N)
+__global__ void __launch_bounds__(LA_N * LA_PARTS)
 latent_absorb_kernel(const T* q, int64_t q_ld, const T* wuk, const double* freq, const int32_t* positions, T* q_abs, int B, int H,
                      int dim, int rot, int kv_ld, int rot_ld) {
-    extern __shared__ __align__(16) float qa_smem[];    // [dim][LA_B]
+    extern __shared__ __align__(16) float qa_smem[];    // [dim][LA_B], then the parts' sums
     float* q_smem = qa_smem;
     ptx::grid_dependency_wait();
     ptx::grid_launch_dependents();
@@ -294,7 +296,7 @@ latent_absorb_kernel(const T* q, int64_t q_ld, const T* wuk, const double* freq,
     const int b0 = blockIdx.x / (H * (n_tiles + 1)) * LA_B, nb = min(LA_B, B - b0);
     const int width = kv_ld + rot_ld;
     if (tile == n_tiles) {
-        for (int i = threadIdx.x; i < nb * (rot_ld / 2); i += LA_N) {
+        for (int i = threadIdx.x; i < nb * (rot_ld / 2); i += LA_N * LA_PARTS) {
             const int b = b0 + i / (rot_ld / 2), j = i % (rot_ld / 2);
             T lo = from_f<T>(0.f), hi = lo;
             if (2 * j < rot) {
@@ -311,41 +313,57 @@ latent_absorb_kernel(const T* q, int64_t q_ld, const T* wuk, const double* freq,
         }
         return;
     }
-    const int n = tile * LA_N + threadIdx.x;
-    for (int i = threadIdx.x; i < LA_B * dim; i += LA_N) {
+    const int n = tile * LA_N + threadIdx.x % LA_N, part = threadIdx.x / LA_N;
+    for (int i = threadIdx.x; i < LA_B * dim; i += LA_N * LA_PARTS) {
         const int b = i / dim, e = i - b * dim;
         q_smem[e * LA_B + b] = b < nb ? to_f(q[(b0 + b) * q_ld + h * (dim + rot) + e]) : 0.f;
     }
     __syncthreads();
-    if (n >= kv_ld) return;
     float acc[LA_B];
 #pragma unroll
     for (int b = 0; b < LA_B; ++b) acc[b] = 0.f;
     const T* w = wuk + (int64_t)h * dim * kv_ld + n;
-#pragma unroll 16
-    for (int e = 0; e < dim; ++e) {
-        const float wv = to_f(w[(int64_t)e * kv_ld]);
-        float q8[LA_B];
-        load4(q_smem + e * LA_B, *reinterpret_cast<float(*)[4]>(q8));
-        load4(q_smem + e * LA_B + 4, *reinterpret_cast<float(*)[4]>(q8 + 4));
+    const int rows = (dim + LA_PARTS - 1) / LA_PARTS, e1 = n < kv_ld ? min(dim, (part + 1) * rows) : 0;
+    for (int e0 = part * rows; e0 < e1; e0 += LA_AHEAD) {
+        float wv[LA_AHEAD];
 #pragma unroll
-        for (int b = 0; b < LA_B; ++b) acc[b] = fmaf(q8[b], wv, acc[b]);
+        for (int i = 0; i < LA_AHEAD; ++i) wv[i] = e0 + i < e1 ? to_f(w[(int64_t)(e0 + i) * kv_ld]) : 0.f;
+#pragma unroll
+        for (int i = 0; i < LA_AHEAD; ++i)
+            if (e0 + i < e1) {
+                float q8[LA_B];
+                load4(q_smem + (e0 + i) * LA_B, *reinterpret_cast<float(*)[4]>(q8));
+                load4(q_smem + (e0 + i) * LA_B + 4, *reinterpret_cast<float(*)[4]>(q8 + 4));
+#pragma unroll
+                for (int b = 0; b < LA_B; ++b) acc[b] = fmaf(q8[b], wv[i], acc[b]);
+            }
     }
+    float* sums = q_smem + dim * LA_B;                  // [LA_PARTS][LA_B][LA_N]
 #pragma unroll
-    for (int b = 0; b < LA_B; ++b)
-        if (b < nb) q_abs[((int64_t)(b0 + b) * H + h) * width + n] = from_f<T>(acc[b]);
+    for (int b = 0; b < LA_B; ++b) sums[(part * LA_B + b) * LA_N + threadIdx.x % LA_N] = acc[b];
+    __syncthreads();
+    if (n < kv_ld)
+        for (int b = part; b < nb; b += LA_PARTS) {
+            float o = 0.f;
+#pragma unroll
+            for (int k = 0; k < LA_PARTS; ++k) o += sums[(k * LA_B + b) * LA_N + threadIdx.x % LA_N];
+            q_abs[((int64_t)(b0 + b) * H + h) * width + n] = from_f<T>(o);
+        }
 }
 
 // ---------------------------------------------------------------------------------------------------------------
 // Scores and weighted latent sum over the ring, any sizes.  Block (row, head, split); warps take 32 keys at a time.
 // The partial result of a split is the normalised sum and its log-sum-exp.
+// VEC: four columns a load, and four lanes share a key's score, a quarter of the columns each; four values are under way at a time.  A
+// lane per key that reads 32 rows a column at a time is one chain of loads: fp32, 16 heads, 512 + 64 columns, 4 sequences of 400 /
+// 1024 tokens 162 / 356 us; this 30 / 42.
 // ---------------------------------------------------------------------------------------------------------------
 constexpr int LD_WARPS = 4, LD_MAXN = 32;              // kv_ld <= 1024
 
-template <typename T>
+template <typename T, bool VEC>
 __global__ void __launch_bounds__(LD_WARPS * 32)
 latent_decode_any_kernel(const LatentDecodeParams p) {
-    extern __shared__ float smem[];
+    extern __shared__ __align__(16) float smem[];
     ptx::grid_dependency_wait();
     ptx::grid_launch_dependents();
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
@@ -353,6 +371,7 @@ latent_decode_any_kernel(const LatentDecodeParams p) {
     float* qs = smem;                                   // [width]
     float* s_acc = smem + width;                        // [LD_WARPS][kv_ld]
     float* s_ml = s_acc + LD_WARPS * p.kv_ld;           // [LD_WARPS][2]
+    float* s_sc = s_ml + LD_WARPS * 2 + warp * 32;      // [LD_WARPS][32]
     const int split = blockIdx.x % p.splits, h = (blockIdx.x / p.splits) % p.H, b = blockIdx.x / (p.splits * p.H);
     const int pos = p.positions[b], slot = p.seq_ids ? p.seq_ids[b] : b;
     const T* q = static_cast<const T*>(p.q_abs) + ((int64_t)b * p.H + h) * width;
@@ -368,7 +387,33 @@ latent_decode_any_kernel(const LatentDecodeParams p) {
     for (int k0 = k_begin + warp * 32; k0 < k_end; k0 += LD_WARPS * 32) {
         const int k = k0 + lane;
         float sc = -INFINITY;
-        if (k < k_end) {
+        if (VEC) {
+#pragma unroll 1
+            for (int s = 0; s < 4; ++s) {
+                const int ks = k0 + s * 8 + lane / 4;
+                float d0 = 0.f, d1 = 0.f;
+                if (ks < k_end) {
+                    const T* row = ring + (int64_t)(ks % p.ring_tokens) * width;
+#pragma unroll 18
+                    for (int e = lane % 4 * 4; e < width; e += 16) {
+                        float kx[4], qx[4];
+                        load4(row + e, kx);
+                        load4(qs + e, qx);
+                        d0 = fmaf(qx[0], kx[0], d0);
+                        d1 = fmaf(qx[1], kx[1], d1);
+                        d0 = fmaf(qx[2], kx[2], d0);
+                        d1 = fmaf(qx[3], kx[3], d1);
+                    }
+                }
+                d0 += d1;
+                d0 += __shfl_xor_sync(0xffffffffu, d0, 1);
+                d0 += __shfl_xor_sync(0xffffffffu, d0, 2);
+                if (lane % 4 == 0) s_sc[s * 8 + lane / 4] = d0;
+            }
+            __syncwarp();
+            if (k < k_end) sc = s_sc[lane] * p.scale;
+            __syncwarp();
+        } else if (k < k_end) {
             const T* row = ring + (int64_t)(k % p.ring_tokens) * width;
             float d = 0.f;
             for (int e = 0; e < width; ++e) d = fmaf(qs[e], to_f(row[e]), d);
@@ -386,15 +431,50 @@ latent_decode_any_kernel(const LatentDecodeParams p) {
 #pragma unroll
         for (int v = 0; v < LD_MAXN; ++v) acc[v] *= shrink;
         const int nk = min(32, k_end - k0);
-        for (int j = 0; j < nk; ++j) {
-            const float wj = __shfl_sync(0xffffffffu, w, j);
-            const T* row = ring + (int64_t)((k0 + j) % p.ring_tokens) * width;
+        if (VEC) {
+            // a lane has columns 128 v + 4 lane ... + 3 in acc[4 v ...]; four keys' loads ahead of their use
+            for (int j0 = 0; j0 < nk; j0 += 4) {
+                const T* rows[4];
+                float wj[4];
 #pragma unroll
-            for (int v = 0; v < LD_MAXN; ++v)
-                if (v * 32 + lane < p.kv_ld) acc[v] = fmaf(wj, to_f(row[v * 32 + lane]), acc[v]);
+                for (int j = 0; j < 4; ++j) {
+                    const int at = min(j0 + j, nk - 1);
+                    rows[j] = ring + (int64_t)((k0 + at) % p.ring_tokens) * width + lane * 4;
+                    wj[j] = __shfl_sync(0xffffffffu, w, at);
+                }
+#pragma unroll
+                for (int v = 0; v < LD_MAXN / 4; ++v)
+                    if (v * 128 + lane * 4 < p.kv_ld) {
+                        float x[4][4];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) load4(rows[j] + v * 128, x[j]);
+#pragma unroll
+                        for (int j = 0; j < 4; ++j)
+                            if (j0 + j < nk) {
+#pragma unroll
+                                for (int e = 0; e < 4; ++e) acc[v * 4 + e] = fmaf(wj[j], x[j][e], acc[v * 4 + e]);
+                            }
+                    }
+            }
+        } else {
+            for (int j = 0; j < nk; ++j) {
+                const float wj = __shfl_sync(0xffffffffu, w, j);
+                const T* row = ring + (int64_t)((k0 + j) % p.ring_tokens) * width;
+#pragma unroll
+                for (int v = 0; v < LD_MAXN; ++v)
+                    if (v * 32 + lane < p.kv_ld) acc[v] = fmaf(wj, to_f(row[v * 32 + lane]), acc[v]);
+            }
         }
     }
-    for (int v = 0; v < LD_MAXN; ++v)
+    if (VEC) {
+#pragma unroll
+        for (int v = 0; v < LD_MAXN / 4; ++v)
+            if (v * 128 + lane * 4 < p.kv_ld)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) s_acc[warp * p.kv_ld + v * 128 + lane * 4 + e] = acc[v * 4 + e];
+    }
+#pragma unroll
+    for (int v = 0; v < LD_MAXN && !VEC; ++v)
         if (v * 32 + lane < p.kv_ld) s_acc[warp * p.kv_ld + v * 32 + lane] = acc[v];
     if (lane == 0) { s_ml[warp * 2] = m; s_ml[warp * 2 + 1] = l; }
     __syncthreads();
@@ -427,48 +507,75 @@ template <typename T>
 __global__ void __launch_bounds__(LO_WARPS * 32)
 latent_expand_out_kernel(const float* partial, const float* lse, int splits, const T* wuv, T* out, int64_t out_ld, int B, int H,
                          int vdim, int kv_ld) {
-    extern __shared__ float o_smem[];                   // [LO_B][kv_ld]
+    extern __shared__ float o_smem[];                   // [LO_B][kv_ld], then the shares
     ptx::grid_dependency_wait();
     ptx::grid_launch_dependents();
     const int v_tiles = (vdim + LO_V - 1) / LO_V;
     const int vt = blockIdx.x % v_tiles, h = (blockIdx.x / v_tiles) % H, b0 = blockIdx.x / (v_tiles * H) * LO_B;
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, nb = min(LO_B, B - b0);
-    for (int b = 0; b < LO_B; ++b) {
-        if (b >= nb) {
-            for (int i = threadIdx.x; i < kv_ld; i += blockDim.x) o_smem[b * kv_ld + i] = 0.f;
-            continue;
+    float* share = o_smem + LO_B * kv_ld;               // [LO_B][splits]: what a split's sum counts
+    if (warp < LO_B) {
+        const int64_t part = ((int64_t)(b0 + min(warp, nb - 1)) * H + h) * splits;
+        float M = -INFINITY, L = 0.f;
+        for (int s = lane; s < splits; s += 32) M = fmaxf(M, lse[part + s]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+        for (int s = lane; s < splits; s += 32) {
+            const float f = expf(lse[part + s] - M);
+            share[warp * splits + s] = f;
+            L += f;
         }
-        const int64_t part = ((int64_t)(b0 + b) * H + h) * splits;
-        float M = -INFINITY;
-        for (int s = 0; s < splits; ++s) M = fmaxf(M, lse[part + s]);
-        float L = 0.f;
-        for (int s = 0; s < splits; ++s) L += expf(lse[part + s] - M);
-        const float inv = 1.f / L;
-        for (int i = threadIdx.x; i < kv_ld; i += blockDim.x) {
-            float o = 0.f;
-            for (int s = 0; s < splits; ++s) o = fmaf(partial[(part + s) * kv_ld + i], expf(lse[part + s] - M), o);
-            o_smem[b * kv_ld + i] = o * inv;
-        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
+        for (int s = lane; s < splits; s += 32) share[warp * splits + s] = warp < nb ? share[warp * splits + s] / L : 0.f;
     }
     __syncthreads();
-    for (int v = vt * LO_V + warp; v < min(vdim, (vt + 1) * LO_V); v += LO_WARPS) {
-        const T* w = wuv + ((int64_t)h * vdim + v) * kv_ld;
-        float acc[LO_B];
+    for (int i = threadIdx.x; i < LO_B * kv_ld; i += blockDim.x) {
+        const int b = i / kv_ld, c = i - b * kv_ld;
+        float o = 0.f;
+        if (b < nb) {
+            const float* from = partial + (((int64_t)(b0 + b) * H + h) * splits) * kv_ld + c;
+            for (int s0 = 0; s0 < splits; s0 += 4) {
+                float x[4];
 #pragma unroll
-        for (int b = 0; b < LO_B; ++b) acc[b] = 0.f;
-#pragma unroll 4
-        for (int i = lane; i < kv_ld; i += 32) {
-            const float wv = to_f(w[i]);
+                for (int k = 0; k < 4; ++k) x[k] = s0 + k < splits ? from[(int64_t)(s0 + k) * kv_ld] : 0.f;
 #pragma unroll
-            for (int b = 0; b < LO_B; ++b) acc[b] = fmaf(wv, o_smem[b * kv_ld + i], acc[b]);
+                for (int k = 0; k < 4; ++k)
+                    if (s0 + k < splits) o = fmaf(x[k], share[b * splits + s0 + k], o);
+            }
         }
+        o_smem[i] = o;
+    }
+    __syncthreads();
+    constexpr int VALS = LO_V / LO_WARPS;               // values of a warp, side by side: their loads are under way together
+    const int first_v = vt * LO_V + warp;
+    float acc[VALS][LO_B];
+#pragma unroll
+    for (int k = 0; k < VALS; ++k)
+#pragma unroll
+        for (int b = 0; b < LO_B; ++b) acc[k][b] = 0.f;
+    const T* w = wuv + ((int64_t)h * vdim + first_v) * kv_ld;
+#pragma unroll 4
+    for (int i = lane; i < kv_ld; i += 32) {
+        float wv[VALS];
+#pragma unroll
+        for (int k = 0; k < VALS; ++k) wv[k] = first_v + k * LO_WARPS < vdim ? to_f(w[(int64_t)k * LO_WARPS * kv_ld + i]) : 0.f;
+#pragma unroll
+        for (int b = 0; b < LO_B; ++b) {
+            const float o = o_smem[b * kv_ld + i];
+#pragma unroll
+            for (int k = 0; k < VALS; ++k) acc[k][b] = fmaf(wv[k], o, acc[k][b]);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < VALS; ++k)
 #pragma unroll
         for (int b = 0; b < LO_B; ++b) {
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) acc[b] += __shfl_xor_sync(0xffffffffu, acc[b], o);
-            if (lane == 0 && b < nb) out[(b0 + b) * out_ld + h * vdim + v] = from_f<T>(acc[b]);
+            for (int o = 16; o > 0; o >>= 1) acc[k][b] += __shfl_xor_sync(0xffffffffu, acc[k][b], o);
+            const int v = first_v + k * LO_WARPS;
+            if (lane == 0 && b < nb && v < vdim) out[(b0 + b) * out_ld + h * vdim + v] = from_f<T>(acc[k][b]);
         }
-    }
     if (h == H - 1 && vt == 0)                          // the padding columns behind the last head
         for (int b = 0; b < nb; ++b)
             for (int i = H * vdim + threadIdx.x; i < out_ld; i += blockDim.x) out[(b0 + b) * out_ld + i] = from_f<T>(0.f);
@@ -559,14 +666,14 @@ extern "C" int bn_latent_absorb_q(const void* q, int64_t q_ld, const void* wuk, 
     if (dtype == 1 && latent_absorb_mma(q, q_ld, wuk, freq, positions, q_abs, B, H, dim, rot, kl, rl, as_stream(stream)))
         return launch_status(what);
     const unsigned grid = (unsigned)(H * ((kl + LA_N - 1) / LA_N + 1) * ((B + LA_B - 1) / LA_B));
-    const size_t smem = (size_t)LA_B * dim * sizeof(float);
+    const size_t smem = (size_t)LA_B * (dim + LA_PARTS * LA_N) * sizeof(float);
     if (dtype == 0) {
         if (int rc = allow_smem(latent_absorb_kernel<float>, smem, what)) return rc;
-        launch_dependent(latent_absorb_kernel<float>, grid, LA_N, smem, as_stream(stream), static_cast<const float*>(q), q_ld,
+        launch_dependent(latent_absorb_kernel<float>, grid, LA_N * LA_PARTS, smem, as_stream(stream), static_cast<const float*>(q), q_ld,
                          static_cast<const float*>(wuk), freq, positions, static_cast<float*>(q_abs), B, H, dim, rot, kl, rl);
     } else {
         if (int rc = allow_smem(latent_absorb_kernel<__nv_bfloat16>, smem, what)) return rc;
-        launch_dependent(latent_absorb_kernel<__nv_bfloat16>, grid, LA_N, smem, as_stream(stream), static_cast<const __nv_bfloat16*>(q),
+        launch_dependent(latent_absorb_kernel<__nv_bfloat16>, grid, LA_N * LA_PARTS, smem, as_stream(stream), static_cast<const __nv_bfloat16*>(q),
                          q_ld, static_cast<const __nv_bfloat16*>(wuk), freq, positions, static_cast<__nv_bfloat16*>(q_abs), B, H, dim,
                          rot, kl, rl);
     }
@@ -576,9 +683,11 @@ extern "C" int bn_latent_absorb_q(const void* q, int64_t q_ld, const void* wuk, 
 extern "C" int bn_latent_decode_splits(int B, int H, int kv_rank, int rot, int window, int dtype) {
     if (B <= 0 || H <= 0 || window <= 0) return 0;
     if (dtype == 1 && latent_decode_mma_ok(H, round8(kv_rank), round8(rot))) return latent_decode_mma_splits(B, H, window, sm_count());
+    // one pass of a CTA's warps each where four CTAs a multiprocessor hold that (4 sequences of 1024 tokens 42 us, with two CTAs 58);
+    // else two (32 sequences of 60 tokens 32 us, with four 52)
     long long want = (2LL * sm_count() + (long long)B * H - 1) / ((long long)B * H);
     const long long most = (window + 127) / 128;
-    if (want > most) want = most;
+    if (want > most || (long long)B * H * most <= 4LL * sm_count()) want = most;
     return (int)(want < 1 ? 1 : want);
 }
 
@@ -594,16 +703,16 @@ extern "C" int bn_latent_decode(const void* q_abs, const void* ring, int num_slo
     LatentDecodeParams p{q_abs, ring, seq_ids, positions, partial, lse, B, H, round8(kv_rank), round8(rot), num_slots, ring_tokens, window, splits, scale};
     if (dtype == 1 && latent_decode_mma_ok(H, p.kv_ld, p.rot_ld)) return latent_decode_mma(p, as_stream(stream));
     if (p.kv_ld > LD_MAXN * 32) return fail(BN_ERR_UNSUPPORTED, "%s: kv_rank=%d (at most %d)", what, kv_rank, LD_MAXN * 32);
-    const size_t smem = (size_t)(p.kv_ld + p.rot_ld + LD_WARPS * p.kv_ld + LD_WARPS * 2) * sizeof(float);
+    const size_t smem = (size_t)(p.kv_ld + p.rot_ld + LD_WARPS * p.kv_ld + LD_WARPS * 34) * sizeof(float);
     const unsigned grid = (unsigned)((long long)B * H * splits);
-    if (dtype == 0) {
-        if (int rc = allow_smem(latent_decode_any_kernel<float>, smem, what)) return rc;
-        launch_dependent(latent_decode_any_kernel<float>, grid, LD_WARPS * 32, smem, as_stream(stream), p);
-    } else {
-        if (int rc = allow_smem(latent_decode_any_kernel<__nv_bfloat16>, smem, what)) return rc;
-        launch_dependent(latent_decode_any_kernel<__nv_bfloat16>, grid, LD_WARPS * 32, smem, as_stream(stream), p);
-    }
-    return launch_status(what);
+    auto run = [&](auto kernel) {
+        if (int rc = allow_smem(kernel, smem, what)) return rc;
+        launch_dependent(kernel, grid, LD_WARPS * 32, smem, as_stream(stream), p);
+        return launch_status(what);
+    };
+    const bool vec = (reinterpret_cast<uintptr_t>(ring) & 15) == 0;        // a row is a multiple of eight elements
+    if (dtype == 0) return vec ? run(latent_decode_any_kernel<float, true>) : run(latent_decode_any_kernel<float, false>);
+    return vec ? run(latent_decode_any_kernel<__nv_bfloat16, true>) : run(latent_decode_any_kernel<__nv_bfloat16, false>);
 }
 
 extern "C" int bn_latent_expand_out(float* partial, const float* lse, int splits, const void* wuv, void* out, int64_t out_ld,
@@ -617,7 +726,7 @@ extern "C" int bn_latent_expand_out(float* partial, const float* lse, int splits
     if (dtype == 1 && latent_expand_mma(partial, lse, splits, wuv, out, out_ld, B, H, vdim, kl, as_stream(stream)))
         return launch_status(what);
     const unsigned grid = (unsigned)(((vdim + LO_V - 1) / LO_V) * H * ((B + LO_B - 1) / LO_B));
-    const size_t smem = (size_t)LO_B * kl * sizeof(float);
+    const size_t smem = (size_t)LO_B * (kl + splits) * sizeof(float);
     if (dtype == 0) {
         if (int rc = allow_smem(latent_expand_out_kernel<float>, smem, what)) return rc;
         launch_dependent(latent_expand_out_kernel<float>, grid, LO_WARPS * 32, smem, as_stream(stream), partial, lse, splits,

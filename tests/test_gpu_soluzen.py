@@ -524,6 +524,31 @@ def test_scan_in_chunks_of_128(lib, S, H, G, pad):
     assert np.array_equal(state[1].double().cpu().numpy(), start[1])
 
 
+@pytest.mark.parametrize("kr,rot,n,splits", [(24, 8, 70, 1), (520, 64, 33, 2), (520, 0, 128, 1), (1024, 72, 300, 3)])
+def test_latent_decode_of_a_ring_that_vectors_cannot_read(lib, kr, rot, n, splits):
+    """An fp32 ring that begins between two 16-byte boundaries takes single loads: the same attention, to the rounding of sums of
+    kr + rot and of n terms"""
+    from baranet_bdml_b200 import _lib
+    g = torch.Generator(device="cuda").manual_seed(kr)
+    B, H, tokens, width = 2, 3, n + 20, kr + rot
+    store = torch.randn(B * tokens * width + 1, generator=g, device="cuda")
+    ring = store[1:].view(B, tokens, width)
+    q = torch.randn(B, H, width, generator=g, device="cuda")
+    pos, scale = torch.tensor([n + 40, n // 2], dtype=torch.int32, device="cuda"), width ** -0.5
+    results = []
+    for r in (ring, ring.clone()):
+        part, lse = torch.empty(B, H, splits, kr, device="cuda"), torch.empty(B, H, splits, device="cuda")
+        _lib.check(lib.bn_latent_decode(q.data_ptr(), r.data_ptr(), B, tokens, None, pos.data_ptr(), part.data_ptr(), lse.data_ptr(), splits, B, H,
+                                        kr, rot, n, scale, 0, torch.cuda.current_stream().cuda_stream))
+        results.append((part * torch.softmax(lse, 2)[..., None]).sum(2).double())
+    for b, p in enumerate(pos.tolist()):
+        at = [k % tokens for k in range(max(0, p - n + 1), p + 1)]
+        keys = ring[b, at].double()
+        want = torch.softmax(q[b].double() @ keys.T * scale, 1) @ keys[:, :kr]
+        for got in results:
+            assert float((got[b] - want).abs().max()) <= 2.0 ** -24 * 8 * (width ** 0.5 * 4 + n)
+
+
 # blocks of 16, 32 and 64 values, values that end inside a block, both sizes of state, groups, portions that end inside a stage of 16
 # tokens and inside four
 @pytest.mark.parametrize("B,H,P,G,N", [(2, 4, 64, 2, 128), (2, 40, 36, 1, 128), (10, 30, 64, 3, 128), (1, 6, 12, 2, 64), (160, 1, 64, 1, 64),
