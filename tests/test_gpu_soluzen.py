@@ -549,6 +549,25 @@ def test_latent_decode_of_a_ring_that_vectors_cannot_read(lib, kr, rot, n, split
             assert float((got[b] - want).abs().max()) <= 2.0 ** -24 * 8 * (width ** 0.5 * 4 + n)
 
 
+# more rows than four a multiprocessor (a block has several, the last blocks one less), narrowest, ragged and widest rows, a row
+# stride beyond the columns; one width and one row count that the other forms take
+@pytest.mark.parametrize("rows,width,pad", [(593, 1032, 8), (700, 4096, 0), (1185, 2056, 16), (1500, 1024, 0), (592, 2048, 0), (650, 4104, 8)])
+def test_gated_norm_of_many_rows(lib, rows, width, pad):
+    """Against fp64, to bf16's rounding of the result (half of its spacing of 2^-7) and the fast exponential's 2^-20; the padding
+    columns are zeros"""
+    from baranet_bdml_b200 import _lib
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    y, proj = (torch.randn(rows, width + 24, generator=g, device="cuda").bfloat16() for _ in range(2))
+    w = torch.randn(width, generator=g, device="cuda")
+    out = torch.full((rows, width + pad), float("nan"), dtype=torch.bfloat16, device="cuda")
+    _lib.check(lib.bn_gated_group_norm(y.data_ptr(), y.stride(0), 1, proj.data_ptr(), proj.stride(0), w.data_ptr(), out.data_ptr(), out.stride(0),
+                                       rows, width, 1, 1e-5, 1, torch.cuda.current_stream().cuda_stream))
+    v = y[:, :width].double() * torch.nn.functional.silu(proj[:, :width].double())
+    want = v * (v.square().mean(1, keepdim=True) + 1e-5).rsqrt() * w.double()
+    assert bool(((out[:, :width].double() - want).abs() <= (2.0 ** -8 + 2.0 ** -18) * want.abs() + 1e-30).all())
+    assert bool((out[:, width:] == 0).all())
+
+
 # blocks of 16, 32 and 64 values, values that end inside a block, both sizes of state, groups, portions that end inside a stage of 16
 # tokens and inside four
 @pytest.mark.parametrize("B,H,P,G,N", [(2, 4, 64, 2, 128), (2, 40, 36, 1, 128), (10, 30, 64, 3, 128), (1, 6, 12, 2, 64), (160, 1, 64, 1, 64),
