@@ -17,6 +17,7 @@
 // launch); the same with the K and V ranges rotated / appended to the paged cache by the epilogue instead (what
 // bn_kv_append would do with them, mygrad/llama/llama_layers.py:161-171 for the new token); and the gated pair (two weights, h = act(x Wg) * (x Wu); SwiGLU: op_silu.cuh:7-15);
 // an fp32 output; the result's activation times a matrix given by the caller; and the activation of the result plus a bias.
+// Most products with a K that is a multiple of 256 take the second kernel of this file, whose CTAs stay (gemm_wide_kernel).
 // K is a multiple of 8 and at most 8192, N a multiple of 8.  When K is a multiple of 256 a warp's eighth is a whole number
 // of 32-wide steps; otherwise (RAGGED) the eighths are rounded up and pieces beyond K read as zero.  Anything else belongs to bn_gemm_bf16_nt_small_m.
 #include "common.cuh"
