@@ -305,7 +305,8 @@ split_parts_kernel(const float* x, int64_t ld, __nv_bfloat16* parts, long long r
 }
 
 // Both operands of a product.  A block has one tile of BN weight rows x 64 k in registers: where one part is all there is, the
-// other two, which nobody will read, are not written.  The blocks behind those of the weight cut the rows of A.
+// other two, which nobody will read, are not written.  The blocks behind those of the weight cut the rows of A.  The weight is
+// read evict-first (cut and product of 64 rows, 7424 -> 2048 94 -> 80 us, 2048 -> 7424 38 -> 34).
 struct CutParams {
     const float *a, *w;
     __nv_bfloat16 *a_parts, *w_parts;
@@ -332,7 +333,12 @@ cut_operands_kernel(const CutParams p) {
         const int n = n0 + i * (BN / 2);
 #pragma unroll
         for (int e = 0; e < 8; ++e) v[i][e] = 0.f;
-        if (n < p.N && k < p.K) load8(p.w + n * p.w_ld + k, v[i]);
+        if (n < p.N && k < p.K) {                              // read once: the parts are what should stay in L2
+            const float4* from = reinterpret_cast<const float4*>(p.w + n * p.w_ld + k);
+            const float4 f0 = __ldcs(from), f1 = __ldcs(from + 1);
+            v[i][0] = f0.x; v[i][1] = f0.y; v[i][2] = f0.z; v[i][3] = f0.w;
+            v[i][4] = f1.x; v[i][5] = f1.y; v[i][6] = f1.z; v[i][7] = f1.w;
+        }
     }
     auto store = [&](int part, int i, const uint4& x) {
         const int n = n0 + i * (BN / 2);
