@@ -41,8 +41,9 @@ constexpr int ST_Q = 128, ST_N = 128, ST_P = 64, ST_WORK = 256, ST_THREADS = ST_
 constexpr int ST_HALF = ST_Q * 128;                                   // 128 rows of 128 bytes
 constexpr int ST_TILES = 5 * ST_HALF;                                 // C (two halves of 64 columns), B (two), x
 constexpr int ST_S = 2 * ST_TILES, ST_WX = ST_S + 2 * ST_HALF, ST_ARRAYS = ST_WX + 2 * ST_HALF;
-// of a chunk: loc_i (running sum within the block, log2), l_j = loc_j - log2 dt_j, the column's factor, the blocks' sums
-struct StArrays { float loc[ST_Q], l[ST_Q], col[ST_Q - 32], total[4]; };
+// of a chunk: loc_i (running sum within the block, log2), dt_j, the column's factor, the blocks' sums.  dt_j stays a factor: in the
+// exponent it would be rounded to the spacing of a sum of 32 decays, and could not be negative.
+struct StArrays { float loc[ST_Q], dt[ST_Q], col[ST_Q - 32], total[4]; };
 struct StTail {
     StArrays arrays[2];
     uint64_t full[2], empty[2], g, ops, u, m, y, out;
@@ -168,17 +169,16 @@ __global__ void __launch_bounds__(ST_THREADS, 1) ssd_scan_tc_kernel(const __grid
             }
             const float total = __shfl_sync(0xffffffffu, before, lane / 8 * 8 + 7);
             before -= s;
-            float own[4], l[4], col[4];
+            float own[4], col[4];
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 own[e] = before + loc[e];
-                l[e] = own[e] - log2f(d[e]);
-                col[e] = exp2f(total - l[e]);
+                col[e] = exp2f(total - own[e]) * d[e];
             }
             if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_empty[k & 1]), ((k >> 1) & 1u) ^ 1u, &s_abort))) break;
             StArrays& w = arrays[k & 1];
             store4(w.loc + lane * 4, own);
-            store4(w.l + lane * 4, l);
+            store4(w.dt + lane * 4, d);
             if (lane < 24) store4(w.col + lane * 4, col);
             if (lane % 8 == 7) w.total[lane / 8] = total;
             __syncwarp();
@@ -273,7 +273,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) ssd_scan_tc_kernel(const __grid
                 after += i > rb ? t : 0.f;
                 sum += t;
             }
-            const float weight = exp2f(w.total[rb] - w.l[row] + after);
+            const float weight = exp2f(w.total[rb] - w.loc[row] + after) * w.dt[row];
             tk.from_start = exp2f(w.loc[row] + before);
             tk.decay = exp2f(sum);
             const uint8_t* xt = base + (k & 1) * ST_TILES + 4 * ST_HALF;
@@ -312,8 +312,8 @@ __global__ void __launch_bounds__(ST_THREADS, 1) ssd_scan_tc_kernel(const __grid
                 uint32_t g[32];
                 tc::ld32(tmem + lanes + ST_G + cb * 32, g);
                 tc::wait_ld(g);
-                const float4* factors = reinterpret_cast<const float4*>(cb < rb ? w.col : w.l) + cb * 8;
                 if (cb < rb) {
+                    const float4* factors = reinterpret_cast<const float4*>(w.col) + cb * 8;
                     float between = 0.f;
 #pragma unroll
                     for (int c = 1; c < 3; ++c) between += c > cb && c < rb ? w.total[c] : 0.f;
@@ -325,12 +325,13 @@ __global__ void __launch_bounds__(ST_THREADS, 1) ssd_scan_tc_kernel(const __grid
                         split2(__uint_as_float(g[4 * e + 2]) * (r * f.z), __uint_as_float(g[4 * e + 3]) * (r * f.w), hi[2 * e + 1], lo[2 * e + 1]);
                     }
                 } else {
-                    auto element = [&](int j, float l) { return j <= lane ? __uint_as_float(g[j]) * ex2(loc - l) : 0.f; };
+                    const float4 *locs = reinterpret_cast<const float4*>(w.loc) + cb * 8, *steps = reinterpret_cast<const float4*>(w.dt) + cb * 8;
+                    auto element = [&](int j, float l, float d) { return j <= lane ? __uint_as_float(g[j]) * (ex2(loc - l) * d) : 0.f; };
 #pragma unroll
                     for (int e = 0; e < 8; ++e) {
-                        const float4 f = factors[e];
-                        split2(element(4 * e, f.x), element(4 * e + 1, f.y), hi[2 * e], lo[2 * e]);
-                        split2(element(4 * e + 2, f.z), element(4 * e + 3, f.w), hi[2 * e + 1], lo[2 * e + 1]);
+                        const float4 l = locs[e], d = steps[e];
+                        split2(element(4 * e, l.x, d.x), element(4 * e + 1, l.y, d.y), hi[2 * e], lo[2 * e]);
+                        split2(element(4 * e + 2, l.z, d.z), element(4 * e + 3, l.w, d.w), hi[2 * e + 1], lo[2 * e + 1]);
                     }
                 }
                 tc::st16(tmem + lanes + ST_MH + cb * 16, hi);

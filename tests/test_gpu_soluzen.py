@@ -524,6 +524,34 @@ def test_scan_in_chunks_of_128(lib, S, H, G, pad):
     assert np.array_equal(state[1].double().cpu().numpy(), start[1])
 
 
+@pytest.mark.parametrize("S", [1, 32, 65, 128, 200])
+@pytest.mark.parametrize("checked", [False, True])
+def test_scan_multiplies_by_the_step_size(lib, S, checked):
+    """Decays that forget everything before a token (e^-300 is 0 in fp32) leave its own term alone, dt x B: the state holds it to the
+    2^-18 that two bf16 parts of dt x leave out, however long the sums of the decays are; and dt is a factor of any sign."""
+    from baranet_bdml_b200 import _lib
+    rng = np.random.default_rng(S)
+    B, H, P, G, N = 2, 5, 64, 1, 128
+    inner = H * P
+    xbc = gpu(rng.standard_normal((B, S, inner + 2 * N)), torch.bfloat16)
+    step = np.exp(rng.uniform(np.log(1e-3), np.log(8.0), (B, S, H)))
+    step[:, :, 1] *= -1.0
+    step[:, :, 2] = 0.0
+    dt, a, D = gpu(step), gpu(np.full((B, S, H), -300.0)), gpu(np.zeros(H))
+    state = gpu(rng.standard_normal((B, H, P, N)))
+    y, word = torch.empty((B, S, inner), dtype=torch.bfloat16, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    head = (xbc.data_ptr(), xbc.stride(1), dt.data_ptr(), a.data_ptr(), D.data_ptr(), state.data_ptr(), None, B, S, H, P, G, N, y.data_ptr(), y.stride(1))
+    st = torch.cuda.current_stream().cuda_stream
+    _lib.check(lib.bn_ssm_scan_checked(*head, word.data_ptr(), 1, st) if checked else lib.bn_ssm_scan(*head, 1, st))
+    x, b, c = (t.double() for t in xbc.split([inner, N, N], 2))
+    x = x.view(B, S, H, P) * dt.double()[..., None]
+    want = x[:, -1, :, :, None] * b[:, -1, None, None, :]
+    assert bool(((state.double() - want).abs() <= 2.0 ** -17 * want.abs()).all())
+    size = (b.abs() * c.abs()).sum(2)[..., None, None] * x.abs()
+    want = (b * c).sum(2)[..., None, None] * x
+    assert bool(((y.view(B, S, H, P).double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -16 * size).all()) and int(word.item()) == 0
+
+
 @pytest.mark.parametrize("kr,rot,n,splits", [(24, 8, 70, 1), (520, 64, 33, 2), (520, 0, 128, 1), (1024, 72, 300, 3)])
 def test_latent_decode_of_a_ring_that_vectors_cannot_read(lib, kr, rot, n, splits):
     """An fp32 ring that begins between two 16-byte boundaries takes single loads: the same attention, to the rounding of sums of
