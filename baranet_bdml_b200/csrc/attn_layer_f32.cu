@@ -24,7 +24,7 @@
 namespace bn {
 
 constexpr int AL_THREADS = 256, AL_KEYS = 64, AL_MAXW = 256, AL_MAXD = 64;
-constexpr size_t AL_SMEM = 200 * 1024;
+constexpr size_t AL_SMEM = SMEM_MOST;
 
 __device__ __forceinline__ float4 add4(const float4& a, const float4& b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
 
@@ -549,19 +549,15 @@ __global__ void __launch_bounds__(WARPS * 32, 1) out_kernel(const OutParams p) {
     }
 }
 
-// Lets `kernel` have so much shared memory; asked of the driver once per thread and device for each kernel (`known`)
-struct SmemKnown {
-    int dev = -1;
-    size_t bytes = 0;
-};
-template <typename K>
-static int allow_smem_once(K kernel, size_t bytes, SmemKnown& known) {
+// allow_smem, asked of the driver once per thread and device for each kernel: what it sets does not depend on the call
+template <auto KERNEL>
+static int allow_smem_once(size_t bytes) {
+    static thread_local int known_dev = -1;
     int dev = 0;
     cudaGetDevice(&dev);
-    if (dev == known.dev && bytes <= known.bytes) return BN_OK;
-    if (int rc = allow_smem(kernel, bytes, "bn_attn_layer_f32")) return rc;
-    known.dev = dev;
-    known.bytes = bytes;
+    if (bytes <= 48 * 1024 || dev == known_dev) return BN_OK;
+    if (int rc = allow_smem(KERNEL, bytes, "bn_attn_layer_f32")) return rc;
+    known_dev = dev;
     return BN_OK;
 }
 
@@ -626,9 +622,8 @@ static bool layer_plan(int S, int hidden, int Hq, int Hkv, int D, int mode, Laye
 
 template <int BM>
 static int project_run(const ProjectParams& p, cudaStream_t st) {
-    static thread_local SmemKnown known;
     constexpr size_t smem = 2 * 3 * (BM * PJ_A_LD + PJ_KC * PJ_B_LD) * sizeof(__nv_bfloat16);
-    if (int rc = allow_smem_once(project_kernel<BM>, smem, known)) return rc;
+    if (int rc = allow_smem_once<project_kernel<BM>>(smem)) return rc;
     launch_dependent(project_kernel<BM>, dim3(p.tile_end[PJ_SETS - 1], ceil_div(p.M, BM), ceil_div(p.K, p.range)), BM * 4, smem, st, p);
     return launch_status("bn_attn_layer_f32");
 }
@@ -644,8 +639,7 @@ static int project(int bm, ProjectParams p, cudaStream_t st) {
 
 template <int BM>
 static int core_run(const LayerPlan& l, const CoreParams& p, cudaStream_t st) {
-    static thread_local SmemKnown known;
-    if (int rc = allow_smem_once(attn_rows_f32_kernel<BM>, l.smem, known)) return rc;
+    if (int rc = allow_smem_once<attn_rows_f32_kernel<BM>>(l.smem)) return rc;
     launch_dependent(attn_rows_f32_kernel<BM>, dim3(ceil_div(p.S, BM), p.problems), AL_THREADS, l.smem, st, p);
     return launch_status("bn_attn_layer_f32");
 }
@@ -671,9 +665,8 @@ static int core(const LayerPlan& l, const CoreParams& p, cudaStream_t st) {
 
 template <int WARPS>
 static int out_run(const OutParams& p, cudaStream_t st) {
-    static thread_local SmemKnown known;
     const size_t smem = (size_t)3 * ceil_div(p.W, 16) * 16 * OUT_LD * sizeof(__nv_bfloat16);
-    if (int rc = allow_smem_once(out_kernel<WARPS>, smem, known)) return rc;
+    if (int rc = allow_smem_once<out_kernel<WARPS>>(smem)) return rc;
     launch_dependent(out_kernel<WARPS>, dim3(ceil_div(p.hidden, OUT_BN), ceil_div(p.S, 16 * WARPS)), WARPS * 32, smem, st, p);
     return launch_status("bn_attn_layer_f32");
 }

@@ -715,8 +715,8 @@ static int attn_step_f32(const AttnPortionParams& p, cudaStream_t st, const char
     int ranks = SA_MAXRANKS;
     while (ranks > 1 && (items * ranks > 2LL * sm_count() || (ranks / 2) * 32LL * SA_WARPS >= keys)) ranks /= 2;
     if (items * ranks > 0x7fffffffLL) return fail(BN_ERR_UNSUPPORTED, "%s: B=%d too large", what, p.B);
-    auto run = [&](auto kernel, size_t smem) {
-        if (int rc = allow_smem(kernel, smem, what)) return rc;
+    auto run = [&](auto kernel, size_t smem) {                                 // always the same for a kernel
+        if (int rc = allow_smem(kernel, smem, what, smem)) return rc;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)(items * ranks));
         cfg.blockDim = dim3(SA_THREADS);

@@ -453,6 +453,24 @@ def test_layer_in_one_call(T, dev_inv_freq, S, hid, Hq, Hkv, D, off, causal, mod
         assert not np.isfinite(bad[S // 2:]).any()
 
 
+def test_layer_in_one_call_from_several_threads(T):
+    """A thread's call of less shared memory (both ask for more than 48 KB, of the same kernel) leaves another thread's limit alone"""
+    import threading
+    import torch
+    from baranet_bdml_b200 import _lib
+
+    def layer(S):
+        g = torch.Generator(device="cuda").manual_seed(S)
+        x, *w = (T.TensorF.from_torch(torch.randn(s, generator=g, device="cuda") * 0.05) for s in ((S, 256), (256, 2048), (256, 256), (256, 256), (2048, 256)))
+        return x.attention_layer(*w, 0.125, False, 0, num_heads=32, num_kv_heads=4, head_dim=64, theta=10000.0, heads_mode=_lib.BN_HEADS_PER_HEAD).to_numpy()
+
+    first, other = layer(512), []
+    thread = threading.Thread(target=lambda: other.append(layer(200)))
+    thread.start()
+    thread.join()
+    assert np.array_equal(layer(512), first) and len(other) == 1 and np.array_equal(layer(200), other[0])
+
+
 def test_layer_in_one_call_refuses_what_it_does_not_take(T):
     import torch
     from baranet_bdml_b200 import _lib
