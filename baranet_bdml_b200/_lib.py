@@ -32,6 +32,7 @@ SIGNATURES = {
     "bn_mm_f32_split": (_i, [_p, _p, _i, _p, _i64, _p, _i64, _p, _i, _p, _i, _i, _i, _p, _p]),
     "bn_mm_f32_each": (_i, [_p, _i64, _i64, _i, _p, _p, _p, _p, _p, _p, _i, _i, _p, _p]),
     "bn_attn_layer_f32_workspace_bytes": (_sz, [_i, _i, _i, _i, _i, _i]),
+    "bn_attn_layer_f32_best_bytes": (_sz, [_i, _i, _i, _i, _i, _i, _i, _i]),
     "bn_attn_layer_f32": (_i, [_p, _i64, _p, _i64, _p, _i64, _p, _i64, _p, _i64, _p, _i64, _i, _i, _i, _i, _i, _f, _f, _i, _i, _i, _p,
                                _sz, _p]),
     "bn_linear_f32_workspace_bytes": (_sz, [_i, _i, _i]),

@@ -562,7 +562,7 @@ static int allow_smem_once(size_t bytes) {
 }
 
 struct LayerPlan {
-    int Wq, Wk, W, problems, reps, ld, in_bm, in_range, out_bm, out_range, BM, p_ld;
+    int Wq, Wk, W, problems, reps, ld, in_bm, in_range, out_bm, out_range, BM, wanted, p_ld;
     bool collapsed, fold, tiled;
     size_t wq_at, wo_at, part_at, rows_at, attn_at, out_at, total, smem;
 };
@@ -600,7 +600,7 @@ static bool layer_plan(int S, int hidden, int Hq, int Hkv, int D, int mode, Laye
     project_plan(S, ceil_div(hidden, PJ_BN), l.Wq, &l.out_bm, &l.out_range);
     // As many rows to a block as leave two blocks for every multiprocessor (rows share the reads of keys and values), and fit.
     const long long rows = (long long)S * l.problems, sms = sm_count();
-    l.BM = rows >= 32 * sms ? 16 : rows >= 16 * sms ? 8 : rows >= 6 * sms ? 4 : rows > sms ? 2 : 1;
+    l.BM = l.wanted = rows >= 32 * sms ? 16 : rows >= 16 * sms ? 8 : rows >= 6 * sms ? 4 : rows > sms ? 2 : 1;
     l.p_ld = ceil_div(S, AL_KEYS) * AL_KEYS + 4;
     for (;; l.BM /= 2) {
         if (l.BM == 0) return false;
@@ -618,6 +618,22 @@ static bool layer_plan(int S, int hidden, int Hq, int Hkv, int D, int mode, Laye
     l.out_at = take(l.fold ? 0 : (size_t)ceil_div(l.Wq, l.out_range) * S * hidden);
     l.total = at;
     return true;
+}
+
+// Whether heads of their own go through tiles of 64 x 64, as a portion from the first position on
+static bool layer_tiled(const LayerPlan& l, int S, int causal, int position_offset) { return !l.collapsed && causal && position_offset == 0 && S >= 64; }
+
+// Whether the layer in one call is faster than its operators one by one.  It is, but for long sequences whose scores leave room for few
+// rows to a block, and so read all keys and values for every one or two: relative times of a row and key here (the columns are read
+// once for the BM rows) and in attn_f32_kernel (16 rows to a block, the scores over all query heads).  us as operators and in
+// one call, collapsed and causal: 16 / 16 heads of 16, 7000 tokens (2 rows a block) 4905, 3911, 7900 tokens (1 row) 6028, 8430; 8 / 4 of
+// 64, 15900 (1) 30500, 31793; 12 / 4 of 64, 15900 (1) 38417, 32037; 32 / 4 of 64, 8192 (1) 24193, 9537; 8 / 8 of 16, 16000 (2) 14091,
+// 11066, 28000 (1) 42194, 62011; 4 / 4 of 16, 6000 (4) 1280, 840, 12000 (2) 3885, 4313; 8 / 2 of 32, 12000 (2) 6234, 4315, 30000 (1)
+// 37041, 50612.  Per head, 4 / 2 of 64, not causal: 10000 (4) 22319, 16976, 13000 (2) 37317, 40138, 21000 (1) 97707, 195304.
+static bool layer_best(const LayerPlan& l, int S, int Hq, int Hkv, int causal, int position_offset) {
+    if (l.BM == l.wanted || layer_tiled(l, S, causal, position_offset)) return true;
+    const float here = (0.8f + 0.0082f * l.W) / l.BM, apart = 0.25f + 0.0062f * l.W + (l.collapsed ? 0.003f * (Hq / Hkv - 1) * l.W : 0.f);
+    return here <= apart;
 }
 
 template <int BM>
@@ -680,6 +696,12 @@ extern "C" size_t bn_attn_layer_f32_workspace_bytes(int S, int hidden, int Hq, i
     return (heads_mode == BN_HEADS_COLLAPSED || heads_mode == BN_HEADS_PER_HEAD) && layer_plan(S, hidden, Hq, Hkv, D, heads_mode, &l) ? l.total : 0;
 }
 
+extern "C" size_t bn_attn_layer_f32_best_bytes(int S, int hidden, int Hq, int Hkv, int D, int position_offset, int causal, int heads_mode) {
+    LayerPlan l;
+    return (heads_mode == BN_HEADS_COLLAPSED || heads_mode == BN_HEADS_PER_HEAD) && layer_plan(S, hidden, Hq, Hkv, D, heads_mode, &l) &&
+           layer_best(l, S, Hq, Hkv, causal, position_offset) ? l.total : 0;
+}
+
 extern "C" int bn_attn_layer_f32(const float* x, int64_t x_rs, const float* wq, int64_t wq_rs, const float* wk, int64_t wk_rs,
                                  const float* wv, int64_t wv_rs, const float* wo, int64_t wo_rs, float* out, int64_t out_rs, int S,
                                  int hidden, int Hq, int Hkv, int D, float scale, float theta, int position_offset, int causal,
@@ -713,7 +735,7 @@ extern "C" int bn_attn_layer_f32(const float* x, int64_t x_rs, const float* wq, 
     launch_dependent(finish_kernel, dim3(S + (l.fold ? 4 * sm_count() : 0)), AL_THREADS, 0, st, fin);
     if (int rc = launch_status(what)) return rc;
     const CoreParams c{at(l.rows_at), at(l.attn_at), S, l.ld, l.Wq, l.Wq + l.Wk, l.W, l.problems, l.reps, l.p_ld, scale, position_offset, causal};
-    l.tiled = !l.collapsed && causal && position_offset == 0 && S >= 64;
+    l.tiled = layer_tiled(l, S, causal, position_offset);
     if (int rc = core(l, c, st)) return rc;
     if (l.collapsed && (l.fold || wo_rs == hidden)) {
         const OutParams o{at(l.attn_at), l.fold ? at(l.wo_at) : wo, out, out_rs, S, l.W, hidden};

@@ -233,7 +233,7 @@ class TensorF:
     def attention_layer(self, wq: "TensorF", wk: "TensorF", wv: "TensorF", wo: "TensorF", scale: float, causal: bool, seq_offset: int, *,
                         num_heads: int, num_kv_heads: int, head_dim: int, theta: float, heads_mode: int) -> Optional["TensorF"]:
         """((self @ wq).attention_fused(self @ wk, self @ wv, ...)) @ wo in one call -> bn_attn_layer_f32; None where the shapes,
-        strides or addresses are none that it takes (then the single operators say what is wrong, or do it)."""
+        strides or addresses are none that it takes, or the single operators are faster (they then do it, or say what is wrong)."""
         hidden, kv = self.w, num_kv_heads * head_dim
         weights = (wq, wk, wv, wo)
         if [(t.h, t.w) for t in weights] != [(hidden, num_heads * head_dim), (hidden, kv), (hidden, kv), (num_heads * head_dim, hidden)]:
@@ -242,7 +242,8 @@ class TensorF:
             if not t.on_device or t.stride_w != 1 or t.stride_h % 4 or t._ptr() % 16:
                 return None
         lib = _lib.load()
-        n = lib.bn_attn_layer_f32_workspace_bytes(self.h, hidden, num_heads, num_kv_heads, head_dim, int(heads_mode)) if seq_offset >= 0 else 0
+        n = lib.bn_attn_layer_f32_best_bytes(self.h, hidden, num_heads, num_kv_heads, head_dim, int(seq_offset), int(bool(causal)),
+                                             int(heads_mode)) if seq_offset >= 0 else 0
         if n == 0:
             return None
         out = TensorF(self.h, hidden, True)

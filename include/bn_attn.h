@@ -111,8 +111,10 @@ BN_API int bn_mm_f32_each(const float* A, int64_t a_rs, int64_t a_cs, int n, con
 /* The whole attention layer: x (S, hidden) -> softmax attention of rotated q = x wq, k = x wk, v = x wv -> @ wo, fp32, rows of
  * contiguous elements: wq (hidden, Hq D), wk and wv (hidden, Hkv D), wo (Hq D, hidden).  Heads, scale, positions and mask as in
  * bn_attn_prefill_f32; sums are shorter and in another order than those of the single operators.  16-byte aligned pointers and
- * strides; `workspace` of bn_attn_layer_f32_workspace_bytes, which is 0 for sizes that this call does not take. */
+ * strides; `workspace` of bn_attn_layer_f32_workspace_bytes, which is 0 for sizes that this call does not take.
+ * bn_attn_layer_f32_best_bytes: the same, and 0 where the single operators are faster (an estimate; long sequences of some shapes). */
 BN_API size_t bn_attn_layer_f32_workspace_bytes(int S, int hidden, int Hq, int Hkv, int D, int heads_mode);
+BN_API size_t bn_attn_layer_f32_best_bytes(int S, int hidden, int Hq, int Hkv, int D, int position_offset, int causal, int heads_mode);
 BN_API int bn_attn_layer_f32(const float* x, int64_t x_rs, const float* wq, int64_t wq_rs, const float* wk, int64_t wk_rs,
                              const float* wv, int64_t wv_rs, const float* wo, int64_t wo_rs, float* out, int64_t out_rs, int S,
                              int hidden, int Hq, int Hkv, int D, float scale, float theta, int position_offset, int causal,

@@ -40,6 +40,25 @@ def test_bad_arguments_return_status_codes(lib):
         _lib.check(lib.bn_rope_f32(None, 0, 0, None, 0, 0, 1, 64, 64, 10000.0, 0, None))
 
 
+# (S, hidden, Hq, Hkv, D, causal, per head): measured faster as single operators, and faster in one call
+@pytest.mark.parametrize("sizes,best", [
+    ((7900, 1024, 16, 16, 16, 1, 0), 0), ((8192, 1024, 16, 16, 16, 0, 0), 0), ((28000, 256, 8, 8, 16, 1, 0), 0), ((28000, 256, 16, 8, 16, 1, 0), 0),
+    ((12000, 256, 4, 4, 16, 1, 0), 0), ((30000, 256, 4, 4, 16, 1, 0), 0), ((13000, 256, 4, 2, 64, 0, 1), 0), ((21000, 256, 4, 2, 64, 0, 1), 0),
+    ((13000, 256, 4, 2, 16, 0, 1), 0), ((40000, 256, 1, 1, 64, 1, 0), 0), ((15900, 512, 8, 4, 64, 1, 0), 0), ((30000, 256, 8, 2, 32, 1, 0), 0),
+    ((128, 2048, 32, 4, 64, 1, 0), 1), ((8192, 2048, 32, 4, 64, 1, 0), 1), ((15000, 2048, 32, 4, 64, 1, 0), 1), ((15900, 768, 12, 4, 64, 1, 0), 1), ((12000, 256, 8, 2, 32, 1, 0), 1),
+    ((7000, 1024, 16, 16, 16, 1, 0), 1), ((16000, 256, 8, 8, 16, 1, 0), 1), ((6000, 256, 4, 4, 16, 1, 0), 1), ((10000, 256, 4, 2, 64, 0, 1), 1),
+    ((10000, 256, 4, 2, 16, 0, 1), 1), ((15000, 2048, 32, 4, 64, 1, 1), 1), ((40000, 256, 4, 2, 64, 1, 1), 1), ((4096, 2048, 32, 1, 64, 0, 1), 1),
+    ((128, 2048, 32, 4, 66, 1, 0), 0)])                                                # (a head that the call does not take)
+def test_layer_in_one_call_where_it_is_the_faster_way(lib, sizes, best):
+    from baranet_bdml_b200 import _lib
+    S, hidden, Hq, Hkv, D, causal, per_head = sizes
+    mode = _lib.BN_HEADS_PER_HEAD if per_head else _lib.BN_HEADS_COLLAPSED
+    bytes_of = lambda *how: lib.bn_attn_layer_f32_best_bytes(S, hidden, Hq, Hkv, D, *how, mode)        # noqa: E731
+    assert bytes_of(0, causal) == best * lib.bn_attn_layer_f32_workspace_bytes(S, hidden, Hq, Hkv, D, mode)
+    if per_head and S >= 13000:                        # positions that do not start at 0 take no tiles
+        assert bytes_of(5, 1) == 0
+
+
 def test_missing_library_fails_loudly(monkeypatch):
     from baranet_bdml_b200 import _lib
     monkeypatch.setattr(_lib, "_lib", None)
