@@ -730,7 +730,7 @@ static int attn_step_f32(const AttnPortionParams& p, cudaStream_t st, const char
         attr[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 2;
-        const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, p, ranks);
+        const cudaError_t e = launch_config(cfg, 1, kernel, p, ranks);
         if (e == cudaSuccess) return launch_status(what);
         (void)cudaGetLastError();
         return fail(BN_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));

@@ -539,7 +539,8 @@ static void splitk_plan(int M, int N, int K, int sms, int* splits, int* k_per_sp
     *splits = (k_steps + per - 1) / per;
 }
 
-// Launches the kernel on `grid` CTAs (PAIR: clusters of two), as a programmatic dependent unless what is ahead has to be complete
+// Launches the kernel on `grid` CTAs (PAIR: clusters of two), as a programmatic dependent unless what is ahead has to be complete or the
+// attribute is refused
 template <int EPI, int BN, bool PAIR = false>
 static int gemm_run(const CUtensorMap& a, const CUtensorMap& b, const GemmParams& p, unsigned grid, cudaStream_t st) {
     constexpr size_t smem = GemmShape<BN, PAIR>::SMEM_BYTES;
@@ -571,7 +572,7 @@ static int gemm_run(const CUtensorMap& a, const CUtensorMap& b, const GemmParams
     }
     cfg.attrs = attr;
     cfg.numAttrs = n;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_bf16_nt_kernel<EPI, BN, PAIR>, a, b, p);
+    cudaError_t e = launch_config(cfg, PAIR ? 1 : 0, gemm_bf16_nt_kernel<EPI, BN, PAIR>, a, b, p);
     if (e != cudaSuccess) {
         (void)cudaGetLastError();
         return fail(BN_ERR_CUDA, "gemm: %s", cudaGetErrorString(e));

@@ -262,7 +262,7 @@ static int rows_launch(const RowsGemm& p, cudaStream_t st, const char* what) {
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_rows_kernel<MT, NW>, mw, ma, p, ranks, (steps + ranks - 1) / ranks);
+    cudaError_t e = launch_config(cfg, 1, gemm_rows_kernel<MT, NW>, mw, ma, p, ranks, (steps + ranks - 1) / ranks);
     if (e != cudaSuccess) {
         (void)cudaGetLastError();
         return fail(BN_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));

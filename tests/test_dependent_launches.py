@@ -5,6 +5,7 @@ an earlier kernel left in L1; only weights, which no kernel of a model writes, m
 import glob
 import os
 import re
+import subprocess
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "baranet_bdml_b200", "csrc")
 WAIT = re.compile(r"grid_dependency_wait\(\)|griddepcontrol\.wait")
@@ -74,3 +75,59 @@ def test_dependents_read_what_others_wrote_by_ordinary_loads():
         if dependents:
             reads = [rest[m.end():closing(rest, m.end() - 1, "()") - 1] for m in re.finditer(r"__ldg\(", rest)]
             assert set(reads) <= WEIGHTS.get(name, set()), (name, set(reads) - WEIGHTS.get(name, set()))
+
+
+FAKE = r"""
+#include <stdio.h>
+#include "launch.cuh"
+// The runtime's two calls, which refuse a programmatic dependence while `refuse` is set, and any launch without the cluster's size
+// while `cluster` is
+static int refuse, cluster, calls, kept;
+static cudaError_t pending;
+extern "C" cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* cfg, const void*, void** args) {
+    bool dependent = false, size = false;
+    for (unsigned i = 0; i < cfg->numAttrs; ++i) {
+        dependent |= cfg->attrs[i].id == cudaLaunchAttributeProgrammaticStreamSerialization;
+        size |= cfg->attrs[i].id == cudaLaunchAttributeClusterDimension;
+    }
+    ++calls;
+    if ((refuse && dependent) || (cluster && !size) || *(int*)args[0] != 7) return pending = cudaErrorNotSupported;
+    kept = cfg->numAttrs;
+    return cudaSuccess;
+}
+extern "C" cudaError_t cudaGetLastError() { cudaError_t e = pending; pending = cudaSuccess; return e; }
+static void kernel(int) {}
+int main() {
+    for (refuse = 0; refuse < 2; ++refuse) {
+        calls = 0;
+        bn::launch_dependent(kernel, dim3(3), 32, 0, (cudaStream_t)0, 7);
+        if (calls != 1 + refuse || kept != 1 - refuse || cudaGetLastError() != cudaSuccess) return 1;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        cudaLaunchConfig_t cfg = {};
+        cfg.attrs = attr;
+        cfg.numAttrs = 2;
+        calls = 0, cluster = 1;
+        if (bn::launch_config(cfg, 1, kernel, 7) != cudaSuccess || calls != 1 + refuse || kept != 2 - refuse) return 2;
+        cluster = 0;
+        // what is refused for another reason stays refused, and says so
+        if (bn::launch_config(cfg, 1, kernel, 8) == cudaSuccess || cudaGetLastError() == cudaSuccess) return 3;
+    }
+    return 0;
+}
+"""
+
+
+def test_a_refused_attribute_costs_the_overlap_alone(tmp_path):
+    """Against a fake runtime; and every launch with attributes goes that way, or has the fallback beside it."""
+    src, exe = tmp_path / "launch.cpp", tmp_path / "launch"
+    src.write_text(FAKE)
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    subprocess.run(["/usr/bin/g++", "-std=c++17", "-w", "-I" + CSRC, "-I" + os.path.join(cuda, "include"), str(src), "-o", str(exe)], check=True)
+    assert subprocess.run([str(exe)]).returncode == 0
+    for name, text, found in sources():
+        waiting = {k for k, _, body, _, _ in found if WAIT.search(body)}
+        assert set(re.findall(r"launch_config\(\w+, [^,]*, (\w+_kernel)", text)) <= waiting, name
+        for m in re.finditer(r"cudaLaunchKernelEx\(&\w+, (\w+)", text):
+            assert m.group(1) + "<<<" in text[m.end():m.end() + 200], name
