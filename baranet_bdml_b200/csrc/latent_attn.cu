@@ -288,7 +288,7 @@ template <typename T>
 __global__ void __launch_bounds__(LA_N * LA_PARTS)
 latent_absorb_kernel(const T* q, int64_t q_ld, const T* wuk, const double* freq, const int32_t* positions, T* q_abs, int B, int H,
                      int dim, int rot, int kv_ld, int rot_ld) {
-    extern __shared__ __align__(16) float qa_smem[];    // [dim][LA_B], then the parts' sums
+    extern __shared__ __align__(16) float qa_smem[];    // [dim][LA_B], in their place the parts' sums
     float* q_smem = qa_smem;
     ptx::grid_dependency_wait();
     ptx::grid_launch_dependents();
@@ -338,7 +338,8 @@ latent_absorb_kernel(const T* q, int64_t q_ld, const T* wuk, const double* freq,
                 for (int b = 0; b < LA_B; ++b) acc[b] = fmaf(q8[b], wv[i], acc[b]);
             }
     }
-    float* sums = q_smem + dim * LA_B;                  // [LA_PARTS][LA_B][LA_N]
+    __syncthreads();                                    // the queries have been read
+    float* sums = q_smem;                               // [LA_PARTS][LA_B][LA_N]
 #pragma unroll
     for (int b = 0; b < LA_B; ++b) sums[(part * LA_B + b) * LA_N + threadIdx.x % LA_N] = acc[b];
     __syncthreads();
@@ -369,9 +370,10 @@ latent_decode_any_kernel(const LatentDecodeParams p) {
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const int width = p.kv_ld + p.rot_ld;
     float* qs = smem;                                   // [width]
-    float* s_acc = smem + width;                        // [LD_WARPS][kv_ld]
-    float* s_ml = s_acc + LD_WARPS * p.kv_ld;           // [LD_WARPS][2]
-    float* s_sc = s_ml + LD_WARPS * 2 + warp * 32;      // [LD_WARPS][32]
+    const int acc_ld = max(p.kv_ld, 32);
+    float* s_acc = smem + width;                        // [LD_WARPS][acc_ld]
+    float* s_ml = s_acc + LD_WARPS * acc_ld;            // [LD_WARPS][2]
+    float* s_sc = s_acc + warp * acc_ld;                // this warp's 32 scores, in the place of its sums
     const int split = blockIdx.x % p.splits, h = (blockIdx.x / p.splits) % p.H, b = blockIdx.x / (p.splits * p.H);
     const int pos = p.positions[b], slot = p.seq_ids ? p.seq_ids[b] : b;
     const T* q = static_cast<const T*>(p.q_abs) + ((int64_t)b * p.H + h) * width;
@@ -471,11 +473,11 @@ latent_decode_any_kernel(const LatentDecodeParams p) {
         for (int v = 0; v < LD_MAXN / 4; ++v)
             if (v * 128 + lane * 4 < p.kv_ld)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) s_acc[warp * p.kv_ld + v * 128 + lane * 4 + e] = acc[v * 4 + e];
+                for (int e = 0; e < 4; ++e) s_acc[warp * acc_ld + v * 128 + lane * 4 + e] = acc[v * 4 + e];
     }
 #pragma unroll
     for (int v = 0; v < LD_MAXN && !VEC; ++v)
-        if (v * 32 + lane < p.kv_ld) s_acc[warp * p.kv_ld + v * 32 + lane] = acc[v];
+        if (v * 32 + lane < p.kv_ld) s_acc[warp * acc_ld + v * 32 + lane] = acc[v];
     if (lane == 0) { s_ml[warp * 2] = m; s_ml[warp * 2 + 1] = l; }
     __syncthreads();
     float M = -INFINITY;
@@ -491,7 +493,7 @@ latent_decode_any_kernel(const LatentDecodeParams p) {
     for (int i = threadIdx.x; i < p.kv_ld; i += blockDim.x) {
         float o = 0.f;
 #pragma unroll
-        for (int w = 0; w < LD_WARPS; ++w) o = fmaf(s_acc[w * p.kv_ld + i], f[w], o);
+        for (int w = 0; w < LD_WARPS; ++w) o = fmaf(s_acc[w * acc_ld + i], f[w], o);
         p.partial[part * p.kv_ld + i] = L > 0.f ? o / L : 0.f;
     }
     if (threadIdx.x == 0) p.lse[part] = L > 0.f ? M + logf(L) : -INFINITY;
@@ -501,52 +503,52 @@ latent_decode_any_kernel(const LatentDecodeParams p) {
 // Merges the splits and expands the latent sum to the head's values: out[b][h][v] = sum_n W_uv[h * vdim + v][n] o[n].
 // Block (value tile of LO_V rows, head, group of LO_B rows); a warp per value row.
 // ---------------------------------------------------------------------------------------------------------------
-constexpr int LO_WARPS = 8, LO_V = 32, LO_B = 4;
+constexpr int LO_WARPS = 8, LO_V = 32, LO_B = 4, LO_SHARES = 256;      // LO_SHARES: splits whose shares are worked out at a time
 
 template <typename T>
 __global__ void __launch_bounds__(LO_WARPS * 32)
 latent_expand_out_kernel(const float* partial, const float* lse, int splits, const T* wuv, T* out, int64_t out_ld, int B, int H,
                          int vdim, int kv_ld) {
-    extern __shared__ float o_smem[];                   // [LO_B][kv_ld], then the shares
+    extern __shared__ float o_smem[];                   // [LO_B][kv_ld]
+    __shared__ float share[LO_B][LO_SHARES];            // what a split's sum counts
     ptx::grid_dependency_wait();
     ptx::grid_launch_dependents();
     const int v_tiles = (vdim + LO_V - 1) / LO_V;
     const int vt = blockIdx.x % v_tiles, h = (blockIdx.x / v_tiles) % H, b0 = blockIdx.x / (v_tiles * H) * LO_B;
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, nb = min(LO_B, B - b0);
-    float* share = o_smem + LO_B * kv_ld;               // [LO_B][splits]: what a split's sum counts
+    const int64_t part = ((int64_t)(b0 + min(warp, nb - 1)) * H + h) * splits;
+    float M = -INFINITY, L = 0.f;                       // of row `warp`
     if (warp < LO_B) {
-        const int64_t part = ((int64_t)(b0 + min(warp, nb - 1)) * H + h) * splits;
-        float M = -INFINITY, L = 0.f;
         for (int s = lane; s < splits; s += 32) M = fmaxf(M, lse[part + s]);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
-        for (int s = lane; s < splits; s += 32) {
-            const float f = expf(lse[part + s] - M);
-            share[warp * splits + s] = f;
-            L += f;
-        }
+        for (int s = lane; s < splits; s += 32) L += expf(lse[part + s] - M);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
-        for (int s = lane; s < splits; s += 32) share[warp * splits + s] = warp < nb ? share[warp * splits + s] / L : 0.f;
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i < LO_B * kv_ld; i += blockDim.x) {
-        const int b = i / kv_ld, c = i - b * kv_ld;
-        float o = 0.f;
-        if (b < nb) {
-            const float* from = partial + (((int64_t)(b0 + b) * H + h) * splits) * kv_ld + c;
-            for (int s0 = 0; s0 < splits; s0 += 4) {
-                float x[4];
+    for (int first = 0; first < splits; first += LO_SHARES) {
+        const int n = min(LO_SHARES, splits - first);
+        if (warp < LO_B)
+            for (int s = lane; s < n; s += 32) share[warp][s] = warp < nb ? expf(lse[part + first + s] - M) / L : 0.f;
+        __syncthreads();
+        for (int i = threadIdx.x; i < LO_B * kv_ld; i += blockDim.x) {
+            const int b = i / kv_ld, c = i - b * kv_ld;
+            float o = first ? o_smem[i] : 0.f;
+            if (b < nb) {
+                const float* from = partial + (((int64_t)(b0 + b) * H + h) * splits + first) * kv_ld + c;
+                for (int s0 = 0; s0 < n; s0 += 4) {
+                    float x[4];
 #pragma unroll
-                for (int k = 0; k < 4; ++k) x[k] = s0 + k < splits ? from[(int64_t)(s0 + k) * kv_ld] : 0.f;
+                    for (int k = 0; k < 4; ++k) x[k] = s0 + k < n ? from[(int64_t)(s0 + k) * kv_ld] : 0.f;
 #pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    if (s0 + k < splits) o = fmaf(x[k], share[b * splits + s0 + k], o);
+                    for (int k = 0; k < 4; ++k)
+                        if (s0 + k < n) o = fmaf(x[k], share[b][s0 + k], o);
+                }
             }
+            o_smem[i] = o;
         }
-        o_smem[i] = o;
+        __syncthreads();
     }
-    __syncthreads();
     constexpr int VALS = LO_V / LO_WARPS;               // values of a warp, side by side: their loads are under way together
     const int first_v = vt * LO_V + warp;
     float acc[VALS][LO_B];
@@ -666,7 +668,7 @@ extern "C" int bn_latent_absorb_q(const void* q, int64_t q_ld, const void* wuk, 
     if (dtype == 1 && latent_absorb_mma(q, q_ld, wuk, freq, positions, q_abs, B, H, dim, rot, kl, rl, as_stream(stream)))
         return launch_status(what);
     const unsigned grid = (unsigned)(H * ((kl + LA_N - 1) / LA_N + 1) * ((B + LA_B - 1) / LA_B));
-    const size_t smem = (size_t)LA_B * (dim + LA_PARTS * LA_N) * sizeof(float);
+    const size_t smem = (size_t)LA_B * (dim > LA_PARTS * LA_N ? dim : LA_PARTS * LA_N) * sizeof(float);
     if (dtype == 0) {
         if (int rc = allow_smem(latent_absorb_kernel<float>, smem, what)) return rc;
         launch_dependent(latent_absorb_kernel<float>, grid, LA_N * LA_PARTS, smem, as_stream(stream), static_cast<const float*>(q), q_ld,
@@ -703,7 +705,7 @@ extern "C" int bn_latent_decode(const void* q_abs, const void* ring, int num_slo
     LatentDecodeParams p{q_abs, ring, seq_ids, positions, partial, lse, B, H, round8(kv_rank), round8(rot), num_slots, ring_tokens, window, splits, scale};
     if (dtype == 1 && latent_decode_mma_ok(H, p.kv_ld, p.rot_ld)) return latent_decode_mma(p, as_stream(stream));
     if (p.kv_ld > LD_MAXN * 32) return fail(BN_ERR_UNSUPPORTED, "%s: kv_rank=%d (at most %d)", what, kv_rank, LD_MAXN * 32);
-    const size_t smem = (size_t)(p.kv_ld + p.rot_ld + LD_WARPS * p.kv_ld + LD_WARPS * 34) * sizeof(float);
+    const size_t smem = (size_t)(p.kv_ld + p.rot_ld + LD_WARPS * (p.kv_ld > 32 ? p.kv_ld : 32) + LD_WARPS * 2) * sizeof(float);
     const unsigned grid = (unsigned)((long long)B * H * splits);
     auto run = [&](auto kernel) {
         if (int rc = allow_smem(kernel, smem, what)) return rc;
@@ -726,7 +728,7 @@ extern "C" int bn_latent_expand_out(float* partial, const float* lse, int splits
     if (dtype == 1 && latent_expand_mma(partial, lse, splits, wuv, out, out_ld, B, H, vdim, kl, as_stream(stream)))
         return launch_status(what);
     const unsigned grid = (unsigned)(((vdim + LO_V - 1) / LO_V) * H * ((B + LO_B - 1) / LO_B));
-    const size_t smem = (size_t)LO_B * (kl + splits) * sizeof(float);
+    const size_t smem = (size_t)LO_B * kl * sizeof(float);
     if (dtype == 0) {
         if (int rc = allow_smem(latent_expand_out_kernel<float>, smem, what)) return rc;
         launch_dependent(latent_expand_out_kernel<float>, grid, LO_WARPS * 32, smem, as_stream(stream), partial, lse, splits,

@@ -577,6 +577,44 @@ def test_latent_decode_of_a_ring_that_vectors_cannot_read(lib, kr, rot, n, split
             assert float((got[b] - want).abs().max()) <= 2.0 ** -24 * 8 * (width ** 0.5 * 4 + n)
 
 
+@pytest.mark.parametrize("splits,kr", [(1, 24), (255, 24), (256, 520), (257, 24), (13000, 24), (2, 12800)])
+def test_latent_values_of_any_number_of_splits(lib, splits, kr):
+    """Sums of any number of splits merged, and expanded: fp32 sums of `splits` and of kr terms of weights that add up to 1"""
+    from baranet_bdml_b200 import _lib
+    g = torch.Generator(device="cuda").manual_seed(splits)
+    B, H, vdim = 5, 2, 40
+    part, wuv = torch.randn(B, H, splits, kr, generator=g, device="cuda"), torch.randn(H, vdim, kr, generator=g, device="cuda")
+    lse, out = 3 * torch.randn(B, H, splits, generator=g, device="cuda"), torch.full((B, H * vdim + 8), 7.0, device="cuda")
+    share = torch.softmax(lse.double(), 2)
+    want = torch.einsum("bhsk,bhs,hvk->bhv", part.double(), share, wuv.double())
+    size = torch.einsum("bhsk,bhs,hvk->bhv", part.double().abs(), share, wuv.double().abs())
+    _lib.check(lib.bn_latent_expand_out(part.data_ptr(), lse.data_ptr(), splits, wuv.data_ptr(), out.data_ptr(), out.stride(0), B, H, vdim, kr, 0,
+                                        torch.cuda.current_stream().cuda_stream))
+    assert bool((out[:, H * vdim:] == 0).all())
+    assert bool(((out[:, :H * vdim].view(B, H, vdim).double() - want).abs() <= 2.0 ** -24 * (splits + kr / 32 + 32) * size).all())
+
+
+def test_latent_attention_of_the_widest_heads(lib):
+    """Queries of 6400 columns and rotated parts of 46072 beside 1024 latent ones: all the shared memory that a block asks for"""
+    from baranet_bdml_b200 import _lib
+    g = torch.Generator(device="cuda").manual_seed(1)
+    st, B, H, dim, kr = torch.cuda.current_stream().cuda_stream, 9, 2, 6400, 136
+    q, wuk = torch.randn(B, H * dim, generator=g, device="cuda"), torch.randn(H * dim, kr, generator=g, device="cuda")
+    freq, pos, q_abs = torch.zeros(8, dtype=torch.float64, device="cuda"), torch.zeros(B, dtype=torch.int32, device="cuda"), torch.empty(B, H, kr, device="cuda")
+    _lib.check(lib.bn_latent_absorb_q(q.data_ptr(), q.stride(0), wuk.data_ptr(), freq.data_ptr(), pos.data_ptr(), q_abs.data_ptr(), B, H, dim, 0, kr, 0, st))
+    a, w = q.double().view(B, H, dim), wuk.double().view(H, dim, kr)
+    err, size = q_abs.double() - torch.einsum("bhe,hek->bhk", a, w), torch.einsum("bhe,hek->bhk", a.abs(), w.abs())
+    assert bool((err.abs() <= 2.0 ** -24 * (dim / 4 + 4) * size).all())
+    kr, rot, n = 1024, 46072, 40
+    ring, query = torch.randn(1, n, kr + rot, generator=g, device="cuda"), torch.randn(1, 1, kr + rot, generator=g, device="cuda")
+    part, lse = torch.empty(1, 1, 1, kr, device="cuda"), torch.empty(1, 1, 1, device="cuda")
+    scale, at = (kr + rot) ** -0.5, torch.full((1,), n - 1, dtype=torch.int32, device="cuda")
+    _lib.check(lib.bn_latent_decode(query.data_ptr(), ring.data_ptr(), 1, n, None, at.data_ptr(), part.data_ptr(), lse.data_ptr(), 1, 1, 1,
+                                    kr, rot, n, scale, 0, st))
+    want = torch.softmax(query[0].double() @ ring[0].double().T * scale, 1) @ ring[0, :, :kr].double()
+    assert float((part[0, 0].double() - want).abs().max()) <= 2.0 ** -24 * 8 * ((kr + rot) ** 0.5 * 4 + n)
+
+
 # more rows than four a multiprocessor (a block has several, the last blocks one less), narrowest, ragged and widest rows, a row
 # stride beyond the columns; one width and one row count that the other forms take
 @pytest.mark.parametrize("rows,width,pad", [(593, 1032, 8), (700, 4096, 0), (1185, 2056, 16), (1500, 1024, 0), (592, 2048, 0), (650, 4104, 8)])
