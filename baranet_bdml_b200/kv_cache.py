@@ -51,6 +51,7 @@ class PagedKVCache:
                        torch.zeros((num_seqs, max_pages_per_seq), dtype=torch.int32, device=device),
                        torch.zeros((num_seqs,), dtype=torch.int32, device=device))
         self.pool, self.page_table, self.seq_lens = storage
+        self.seq_ids: Optional[torch.Tensor] = None            # 0 .. num_seqs - 1, where its maker laid them out with it
         self._ws = {}          # decode scratch per (B, Hq, max_seq_len, chunk_tokens); kept while the cache lives
 
     @property

@@ -299,7 +299,7 @@ class LLaMAModelBF16(CausalLM):
         self.caches = [PagedKVCache(pages, B, pages_per_seq, cfg.num_key_value_heads, cfg.head_dim, cfg.rope_theta,
                                     storage=(pools[i], tables[i], lens)) for i in range(n)]
         self.seq_lens = self.caches[0].seq_lens
-        self._all_seqs = torch.arange(B, dtype=torch.int32, device="cuda")
+        self.caches[0].seq_ids = torch.arange(B, dtype=torch.int32, device="cuda")      # as old as the caches: a captured step reads it
 
     def prefill(self, input_ids: torch.Tensor, max_len: int) -> torch.Tensor:
         """Prompt pass: (B, S) ids -> logits of the last position (B, vocab); fills the KV caches."""
@@ -336,7 +336,9 @@ class LLaMAModelBF16(CausalLM):
         """One new token per sequence: (B,) ids -> (B, vocab) logits; appends to the caches."""
         B = token_ids.numel()
         h = self.embed(token_ids, check)
-        seq_ids = self._all_seqs if B == self._all_seqs.numel() else torch.arange(B, dtype=torch.int32, device="cuda")
+        seq_ids = self.caches[0].seq_ids
+        if seq_ids is None or seq_ids.numel() != B:
+            seq_ids = torch.arange(B, dtype=torch.int32, device="cuda")
         pending = None
         positions = self.seq_lens.clone()                         # the new token's position = current length
         self.seq_lens.add_(1)

@@ -72,6 +72,31 @@ def test_graphed_decode_step_equals_eager(lib):
     assert int(graphed.caches[0].seq_lens[0]) == 34
 
 
+def test_captured_step_lives_as_long_as_its_caches(lib):
+    """A graph captured over one set of caches goes on after another prompt has made its own, as long as the first are kept; and
+    caches that a program made by itself serve a step."""
+    from baranet_bdml_b200.kv_cache import PagedKVCache
+    rng = np.random.default_rng(7)
+    ids = torch.from_numpy(rng.integers(3, 1000, (4, 30)).astype(np.int32)).cuda()
+    tok = torch.from_numpy(rng.integers(3, 1000, (4,)).astype(np.int32)).cuda()
+    model = tiny_model(8)
+    model.prefill(ids, 64)
+    kept, lens = model.caches, model.seq_lens
+    own, cfg = tiny_model(8), model.config
+    own.caches = [PagedKVCache(c.num_pages, 4, c.max_pages, cfg.num_key_value_heads, cfg.head_dim, cfg.rope_theta,
+                               storage=(c.pool.clone(), c.page_table, lens.clone())) for c in kept]
+    own.seq_lens = own.caches[0].seq_lens
+    for c in own.caches:
+        c.seq_lens = own.seq_lens
+    step = model.capture_decode_step()
+    want = own.decode_step(tok)
+    assert torch.equal(step(tok)[0], want)
+    lens.sub_(1)
+    model.prefill(ids[:2].contiguous(), 64)
+    filler = [torch.full((4,), 3, dtype=torch.int32, device="cuda") for _ in range(64)]      # takes what small memory was given back
+    assert torch.equal(step(tok)[0], want) and len(filler) == 64 and len(kept) == len(model.caches)
+
+
 def test_model_rejects_bad_ids(lib):
     model = tiny_model()
     with pytest.raises(IndexError):
