@@ -324,10 +324,12 @@ def test_chunked_attention(lib, dtype, H, G, E, V, S, n_old, chunk):
         assert np.abs(got - want).max() <= (2e-5 if dtype == torch.float32 else 3e-2), bound
 
 
-@pytest.mark.parametrize("H,G,E,V", [(8, 1, 64, 64), (1, 1, 68, 4), (16, 2, 128, 128), (3, 1, 4, 68), (2, 1, 256, 100), (2, 1, 320, 64)])
+@pytest.mark.parametrize("H,G,E,V", [(8, 1, 64, 64), (1, 1, 68, 4), (16, 2, 128, 128), (3, 1, 4, 68), (2, 1, 256, 100), (2, 1, 320, 64), (2, 1, 576, 64),
+                                      (2, 1, 640, 64)])
 @pytest.mark.parametrize("S,n_old,chunk", [(1, 0, 9), (8, 0, 64), (63, 1, 64), (64, 0, 65), (65, 63, 1000), (21, 44, 50)])
 def test_chunked_attention_at_the_edges_of_f32_tiles(lib, H, G, E, V, S, n_old, chunk):
-    """Rows and keys that fill tiles of 64, and one more or less; one to five pieces of columns, the last without the tiled form's room."""
+    """Rows and keys that fill tiles of 64, and one more or less; one to nine pieces of columns, and ten, for which
+    that form has no room."""
     rng = np.random.default_rng(S + chunk + E)
     n = S + n_old
     q, k = 3.0 * rng.standard_normal((S, H, E)), R.unit_rms(rng.standard_normal((n, G, E)), 1e-5)

@@ -409,7 +409,9 @@ def test_layer_config1_matches_oracle(T, cref, dev_inv_freq):
     assert nerr(out, ref64) < 2e-5
 
 
-LAYERS = [  # S, hidden, Hq, Hkv, D, offset, causal: rows to a block 1 .. 16, tiles of 64 keys, groups of 1, 3, 5, 8 and 12 heads
+# S, hidden, Hq, Hkv, D, offset, causal: tiles of 64 keys, groups of 1, 2, 3, 5, 8 and 12 heads; rows to a block, on 148 multiprocessors,
+# 1, 2, 4 and 8 collapsed (4 and 2 where 8 are wanted and have no room) and 1, 2, 4, 8 and 16 per head
+LAYERS = [
     (1, 128, 4, 2, 32, 0, True),
     (16, 2048, 32, 4, 64, 0, True),
     (65, 100, 5, 5, 20, 3, False),
@@ -418,6 +420,11 @@ LAYERS = [  # S, hidden, Hq, Hkv, D, offset, causal: rows to a block 1 .. 16, ti
     (333, 768, 12, 1, 64, 0, True),
     (512, 256, 32, 4, 64, 0, False),
     (600, 128, 8, 2, 4, 0, True),
+    (900, 128, 8, 4, 64, 0, True),
+    (2400, 64, 4, 2, 16, 0, True),
+    (2400, 128, 8, 4, 64, 0, False),
+    (4200, 64, 8, 4, 64, 0, True),
+    (300, 192, 12, 4, 16, 3, True),
 ]
 
 
@@ -433,11 +440,13 @@ def test_layer_in_one_call(T, dev_inv_freq, S, hid, Hq, Hkv, D, off, causal, mod
     ws = [(rng.standard_normal(s) * hid ** -0.5).astype(np.float32) for s in ((hid, Hq * D), (hid, Hkv * D), (hid, Hkv * D), (Hq * D, hid))]
     scale, hm = D ** -0.5, _lib.BN_HEADS_COLLAPSED if mode == "collapsed" else _lib.BN_HEADS_PER_HEAD
     tx, *tw = (T.TensorF.from_torch(torch.from_numpy(a).cuda()) for a in (x, *ws))
-    sizes = dict(num_heads=Hq, num_kv_heads=Hkv, head_dim=D, theta=10000.0, heads_mode=hm)
+    theta = 10000.0 if S <= 1000 else 1.0      # far from the start a frequency's rounding on one side shows; those of theta 1 are exact
+    sizes = dict(num_heads=Hq, num_kv_heads=Hkv, head_dim=D, theta=theta, heads_mode=hm)
     layer = lambda t: t.attention_layer(*tw, scale, causal, off, **sizes)                         # noqa: E731
     got = layer(tx).to_numpy()
     inv = np.array([np.float32(1.0 / float(np.float32(10000.0) ** (np.float32(2 * i) / np.float32(D)))) for i in range(D // 2)], dtype=np.float32)
     inv = dev_inv_freq[D].astype(np.float32) if D in dev_inv_freq else inv
+    inv = inv if theta > 1.0 else np.ones_like(inv)
     q, k, v = (x.astype(np.float64) @ w.astype(np.float64) for w in ws[:3])
     core = R.attention_collapsed if mode == "collapsed" else R.attention_per_head
     want = core(q, k, v, num_heads=Hq, num_kv_heads=Hkv, head_dim=D, position_offset=off, causal=causal, dtype=np.float64,

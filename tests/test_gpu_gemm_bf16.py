@@ -415,8 +415,9 @@ def test_skinny_gemm(lib, M, N, K):
 
 
 # Wide products of few rows: one column group more than three a multiprocessor, a number of groups that the CTAs do not share evenly,
-# K of one, two, seven and eight steps a warp, rows in the low half of a fragment and in both
-@pytest.mark.parametrize("N,K", [(3560, 256), (4608, 512), (3704, 1792), (8520, 2048)])
+# K of one, two, seven and eight steps a warp, rows in the low half of a fragment and in both; K in two parts, of which the last is one
+# step or eight, and in four, the last of five, with groups that follow one another in a CTA (the rows are read again for each)
+@pytest.mark.parametrize("N,K", [(3560, 256), (4608, 512), (3704, 1792), (8520, 2048), (3560, 2304), (4616, 4096), (8520, 7424)])
 @pytest.mark.parametrize("M", [1, 8, 9, 16])
 def test_wide_products_of_few_rows(lib, M, N, K):
     """Every output form against fp64: bf16's rounding (2^-9 of the result) and fp32 sums of K terms"""
@@ -473,7 +474,8 @@ def test_skinny_swiglu(lib):
     assert lib.bn_gemm_bf16_nt_skinny(tx.data_ptr(), tg.data_ptr(), 17, inter, K, tx.data_ptr(), inter, None, 0, None, None) != 0
 
 
-@pytest.mark.parametrize("M,Hq,Hkv,D,hidden", [(16, 32, 4, 64, 2048), (3, 4, 2, 64, 256), (7, 6, 3, 32, 512)])
+@pytest.mark.parametrize("M,Hq,Hkv,D,hidden", [(16, 32, 4, 64, 2048), (3, 4, 2, 64, 256), (7, 6, 3, 32, 512), (16, 32, 4, 64, 2304),
+                                               (5, 32, 4, 64, 4096)])
 def test_skinny_qkv_with_cache_append(lib, M, Hq, Hkv, D, hidden):
     """One launch for the q, k and v projections of a decode step with RoPE(K) and the cache append against the
     two-launch path (three-output skinny GEMM, then bn_kv_append): q equal, and every page of the cache equal bit for
