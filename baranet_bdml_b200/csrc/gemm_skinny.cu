@@ -233,7 +233,8 @@ gemm_skinny_kernel(const SkinnyParams p) {
 // (5.4); gated pair 2048 -> 5632 11.7 / 12.8, 9.0 / 10.0 (7.1); 2048 -> 2560 4.5 / 5.7, 3.5 / 5.0 (1.6).  Three slices of
 // room instead of two: the same for the widest, 10 % slower for 2048 -> 4608; one CTA a multiprocessor with six: 12 - 40 %
 // slower; slices asked for in L2 further ahead: 2 - 10 % slower.
-// MULTI: K above 2048, in parts of which a warp holds one at a time.
+// MULTI: K above 2048, in parts of which a warp holds one at a time, so that the rows are read again for every group, of which a CTA has
+// few (2048 columns: one).
 // ---------------------------------------------------------------------------------------------------------------
 constexpr int WD_STAGES = 2, WD_STEPS = 8, WD_SLICE = 8 * WD_STEPS * 64;
 constexpr int WD_SMEM = SK_WARPS * WD_STAGES * WD_SLICE, WD_CTAS = 2;

@@ -462,16 +462,16 @@ static bool split_fits(int M, int N, int K) {
 
 extern "C" size_t bn_linear_f32_workspace_bytes(int M, int N, int K) { return M <= 0 || N <= 0 || K <= 0 ? 0 : cut_layout(M, N, K).total; }
 
-// How a product is taken, by estimates in us (measured, one part / three): operands cut, where that takes less time than bn_mm_f32;
-// with up to 16 rows it does not, the weight being cut for them alone (2048 -> 32000, 4 / 16 / 32 rows: 169, 115, 114 / 251, 192,
-// 192 us, chains 87, 100, 153).  Where the parts alone would have been faster (4 rows 108 us with the cut elsewhere, 16 rows 59), the
-// weight is wide enough for bn_mm_f32_sums to hide its additions (4 / 12 rows 86.5 / 94.7 us, chains 86.5 / 91.9), and the error is
-// the smaller one again; narrower weights, whose time is a chain's latency, keep the chains (1 x 2048 -> 2048 23.0 us, sums 27.1).
 // The time of bn_linear_f32: starts, the cut of the weight (6 or 10 bytes each) and of A, the product
 static float parts_estimate(int M, int N, int K, int w_nparts, float product) {
     return 6.f + (float)N * (float)K * (w_nparts == 1 ? 0.8e-6f : 1.4e-6f) + (float)M * (float)K * 1.0e-6f + product;
 }
 
+// How a product is taken that bn_linear_f32_streams leaves (it has most of those of up to 16 rows, and many of up to 48), by estimates
+// in us (measured, one part / three): operands cut, where that takes less time than bn_mm_f32; with up to 16 rows it does not, the
+// weight being cut for them alone (2048 -> 32000, 4 / 16 / 32 rows: 169, 115, 114 / 251, 192, 192 us, chains 87, 100, 153).  Where the parts alone would have been faster (4 rows 108 us with the cut elsewhere, 16 rows 59), the
+// weight is wide enough for bn_mm_f32_sums to hide its additions (4 / 12 rows 86.5 / 94.7 us, chains 86.5 / 91.9), and the error is
+// the smaller one again; narrower weights, whose time is a chain's latency, keep the chains (1 x 2048 -> 2048 23.0 us, sums 27.1).
 extern "C" int bn_linear_f32_form(int M, int N, int K, int w_nparts) {
     if (M <= 0 || N <= 0 || K <= 0 || N % 8 || K % 8 || !split_fits(M, N, K)) return BN_LINEAR_F32_CHAINS;
     int bn;

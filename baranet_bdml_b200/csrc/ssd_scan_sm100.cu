@@ -21,7 +21,7 @@
 // MMAs; warp 10: decays.  G, Y2 and U of the next chunk run while this one's outputs are finished and its own M is worked out.  160 KB of
 // tiles, one CTA a multiprocessor.  A chunk takes about 4200 cycles, of which 3750 are shared memory's at 128 bytes a cycle (480 KB:
 // tiles in 80, the five products' operands 288, parts, x and outputs through the threads 112), MMAs 2050.
-// 8 x 2048 tokens, 64 heads: 189 us (ssd_scan_kernel 442); 1 x 2048 41 (285); 3 x 333 22 (65); 1 x 128 7.3 (22).
+// 8 x 2048 tokens, 64 heads: 187 us (ssd_scan_kernel 442); 1 x 2048 43 (285); 3 x 333 23 (65); 1 x 128 6.5 (22).
 // On the way: a and dt loaded and summed by the TMA warp behind its waits 206 us; sixteen warps with a quarter of the columns each 242.
 //
 // A token with an x that is not finite reaches the tokens before it in its 16 at most, as in the warp-level form: the MMAs of 16 columns

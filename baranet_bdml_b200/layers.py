@@ -7,10 +7,12 @@ softmax -> p v (llama_layers.py:161-183: four host round trips, seven launches
 and an (S,S) matrix in memory) become ONE fused call.
 
 Two semantics are offered (see `heads_mode`):
-  "collapsed"  exactly what the reference computes: its `_split_heads` is a
-               no-op (llama_layers.py:87-103), so there is ONE softmax over the
+  "collapsed"  what the reference computes: its `_split_heads` is a no-op
+               (llama_layers.py:87-103), so there is ONE softmax over the
                scores summed over all heads.  Default, because it is what makes
-               the layer a numerical drop-in.
+               the layer a numerical drop-in.  Sums are shorter than the
+               reference's chains and in another order: 6e-7 from 64 bits
+               where those are 4e-6 from it (2-norm, 128 tokens).
   "per_head"   standard grouped-query attention, one softmax per query head.
 """
 from __future__ import annotations

@@ -202,7 +202,10 @@ def skinny_any_k(rows: int, n_out: int, k: int) -> bool:
 def skinny_best(rows: int, n_out: int, k: int) -> bool:
     """Those of them for which it is the fastest.  Where K is no multiple of 256 its CTAs read the rows for every 8 columns of the
     weight, which shows with many rows and a wide or a long weight.  With one, us at 16 rows and in the kernel for up to 128 rows:
-    2048 -> 2048 4.1, 4.8, 4096 -> 2048 5.8, 6.4, 7424 -> 2048 9.0, 9.6, 2048 -> 4608 5.9, 6.6, 2048 -> 7424 7.9, 8.2."""
+    2048 -> 2048 4.1, 4.8, 4096 -> 2048 5.8, 6.4, 7424 -> 2048 9.0, 9.6, 2048 -> 4608 5.9, 6.6, 2048 -> 7424 7.9, 8.2.  Whole steps of
+    9 / 12 / 16 sequences, with the products of K > 2048, whose rows do not stay in registers, here and in the other kernel: Duponex, 4
+    layers, 176.9 / 184.2 / 194.1 and 182.5 / 188.0 / 193.9 (7424 -> 2048), Soluzen 313.4 / 329.2 / 349.2 and 317.2 / 331.5 / 352.3
+    (5632 -> 2048), LLaMA, 4 layers, 183.3 / 186.2 / 193.1 and 182.4 / 184.3 / 193.7 (5632 -> 2048)."""
     return skinny_any_k(rows, n_out, k) and (rows <= 8 or k % 256 == 0 or (n_out < 4096 and k <= 4096) or k < 640)
 
 

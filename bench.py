@@ -1018,7 +1018,7 @@ def measure_layer_f32(torch, args, rank, world, pk):
     ms = e0.elapsed_time(e1) / reps
     out = {"metric": "attention_layer_f32_ms", "value": ms, "unit": "ms", "higher_is_better": False, "dtype": "f32",
            "config": {"workload": "BASELINE config 1: one attention layer forward, fp32, S=128, hidden 2048, 32q/4kv "
-                                  "heads, head_dim 64, device-resident tensors; one call, four launches"}}
+                                  "heads, head_dim 64, device-resident tensors; one call, five launches"}}
     try:
         from oracle import cref
         if os.path.exists(cref._GPU_SO):
