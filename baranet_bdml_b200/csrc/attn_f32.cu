@@ -258,7 +258,7 @@ static int attn_f32_run(AttnF32Params p, int problems, cudaStream_t st) {
     p.stored = fixed + (size_t)BM * all_keys * sizeof(float) <= AF_SMEM;
     p.p_ld = p.stored ? all_keys : AF_KEYS + 4;
     const size_t smem = fixed + (size_t)BM * p.p_ld * sizeof(float);
-    if (int rc = allow_smem(attn_f32_kernel<RPT, GR, PC, D4>, smem, "bn_attn_prefill_f32")) return rc;
+    if (int rc = allow_smem(attn_f32_kernel<RPT, GR, PC, D4>, smem, "bn_attn_prefill_f32", SMEM_MOST, 512)) return rc;      // (its arrays: 144 - 256)
     attn_f32_kernel<RPT, GR, PC, D4><<<dim3(ceil_div(p.S, BM), problems), AF_KEYS * GR, smem, st>>>(p);
     return launch_status("bn_attn_prefill_f32");
 }

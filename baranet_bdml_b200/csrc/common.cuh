@@ -36,11 +36,12 @@ inline int sm_count() {
 
 // Lets `kernel` be launched with this much dynamic shared memory.  The limit belongs to the kernel, in all threads: it is set to the
 // same number for every call, or a call of fewer bytes would take it from under another thread's.  `most`: that number, for kernels
-// whose own arrays leave no room for 200 KB (227 KB are all there is).
+// whose own arrays leave no room for 200 KB (227 KB are all there is); `own`: the bytes of those arrays, which count towards the 48 KB
+// that need no asking.
 constexpr size_t SMEM_MOST = 200 * 1024;
 template <typename K>
-inline int allow_smem(K kernel, size_t bytes, const char* what, size_t most = SMEM_MOST) {
-    if (bytes <= 48 * 1024) return BN_OK;
+inline int allow_smem(K kernel, size_t bytes, const char* what, size_t most = SMEM_MOST, size_t own = 0) {
+    if (bytes + own <= 48 * 1024) return BN_OK;
     if (bytes > most) return fail(BN_ERR_UNSUPPORTED, "%s: %zu bytes of shared memory", what, bytes);
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
     return e == cudaSuccess ? BN_OK : fail(BN_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));

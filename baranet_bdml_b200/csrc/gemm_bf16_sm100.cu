@@ -548,7 +548,7 @@ static int gemm_run(const CUtensorMap& a, const CUtensorMap& b, const GemmParams
     int dev = 0;
     cudaGetDevice(&dev);
     if (configured_dev != dev) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_bf16_nt_kernel<EPI, BN, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = cudaFuncSetAttribute(gemm_bf16_nt_kernel<EPI, BN, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmShape<BN, PAIR>::SMEM_BYTES);
         if (e != cudaSuccess) return fail(BN_ERR_CUDA, "cudaFuncSetAttribute(gemm): %s", cudaGetErrorString(e));
         configured_dev = dev;
     }

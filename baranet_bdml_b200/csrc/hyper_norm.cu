@@ -182,10 +182,7 @@ static int hyper_any(unsigned grid, cudaStream_t st, const HyperParams& p) {
     const char* what = "bn_hyper_norm";
     const size_t smem = (size_t)p.hidden * sizeof(float);
     if (smem > 200 * 1024) return fail(BN_ERR_UNSUPPORTED, "%s: hidden=%d (at most 51200)", what, p.hidden);
-    if (smem > 40 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(hyper_norm_any_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return fail(BN_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
-    }
+    if (int rc = allow_smem(hyper_norm_any_kernel<T>, smem, what, SMEM_MOST, 2048)) return rc;      // (its arrays: 1184)
     launch_dependent(hyper_norm_any_kernel<T>, grid, HY_THREADS, smem, st, p);
     return launch_status(what);
 }

@@ -728,13 +728,13 @@ extern "C" int bn_latent_expand_out(float* partial, const float* lse, int splits
     if (dtype == 1 && latent_expand_mma(partial, lse, splits, wuv, out, out_ld, B, H, vdim, kl, as_stream(stream)))
         return launch_status(what);
     const unsigned grid = (unsigned)(((vdim + LO_V - 1) / LO_V) * H * ((B + LO_B - 1) / LO_B));
-    const size_t smem = (size_t)LO_B * kl * sizeof(float);
+    const size_t smem = (size_t)LO_B * kl * sizeof(float), own = (size_t)LO_B * LO_SHARES * sizeof(float);
     if (dtype == 0) {
-        if (int rc = allow_smem(latent_expand_out_kernel<float>, smem, what)) return rc;
+        if (int rc = allow_smem(latent_expand_out_kernel<float>, smem, what, SMEM_MOST, own)) return rc;
         launch_dependent(latent_expand_out_kernel<float>, grid, LO_WARPS * 32, smem, as_stream(stream), partial, lse, splits,
                          static_cast<const float*>(wuv), static_cast<float*>(out), out_ld, B, H, vdim, kl);
     } else {
-        if (int rc = allow_smem(latent_expand_out_kernel<__nv_bfloat16>, smem, what)) return rc;
+        if (int rc = allow_smem(latent_expand_out_kernel<__nv_bfloat16>, smem, what, SMEM_MOST, own)) return rc;
         launch_dependent(latent_expand_out_kernel<__nv_bfloat16>, grid, LO_WARPS * 32, smem, as_stream(stream), partial, lse, splits,
                          static_cast<const __nv_bfloat16*>(wuv), static_cast<__nv_bfloat16*>(out), out_ld, B, H, vdim, kl);
     }

@@ -712,10 +712,7 @@ static int gated_norm_launch(const GatedNormParams& p, bn_stream_t stream) {
     else {
         const size_t smem = (size_t)n * sizeof(float);
         if (smem > 200 * 1024) return fail(BN_ERR_UNSUPPORTED, "%s: part of %d columns (at most 51200)", what, n);
-        if (smem > 48 * 1024) {
-            cudaError_t e = cudaFuncSetAttribute(gated_norm_kernel<T, TY, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e != cudaSuccess) return fail(BN_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
-        }
+        if (int rc = allow_smem(gated_norm_kernel<T, TY, 0>, smem, what, SMEM_MOST, 64)) return rc;      // (its arrays: 32)
         launch_dependent(gated_norm_kernel<T, TY, 0>, grid, GN_THREADS, smem, st, p);
     }
     return launch_status(what);

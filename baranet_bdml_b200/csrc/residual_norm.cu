@@ -240,11 +240,8 @@ static int residual_norm_launch(const ResidualNormParams& p, bn_stream_t stream)
     else {
         const size_t smem = (size_t)p.hidden * sizeof(float);
         if (smem > 200 * 1024) return fail(BN_ERR_UNSUPPORTED, "%s: hidden=%d (at most 51200)", what, p.hidden);
-        if (smem > 48 * 1024) {
-            cudaError_t e = cudaFuncSetAttribute(residual_norm_any_kernel<T, TD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)smem);
-            if (e != cudaSuccess) return fail(BN_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
-        }
+        const int rc = allow_smem(residual_norm_any_kernel<T, TD>, smem, what, SMEM_MOST, 64);      // (its arrays: 32)
+        if (rc) return rc;
         launch_dependent(residual_norm_any_kernel<T, TD>, grid, RS_THREADS, smem, st, p);
     }
     return launch_status(what);

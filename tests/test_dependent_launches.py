@@ -131,3 +131,16 @@ def test_a_refused_attribute_costs_the_overlap_alone(tmp_path):
         assert set(re.findall(r"launch_config\(\w+, [^,]*, (\w+_kernel)", text)) <= waiting, name
         for m in re.finditer(r"cudaLaunchKernelEx\(&\w+, (\w+)", text):
             assert m.group(1) + "<<<" in text[m.end():m.end() + 200], name
+
+
+def test_a_kernel_has_one_limit_of_shared_memory():
+    """The limit that a kernel may ask for belongs to it in all threads: what sets it, outside allow_smem, is a constant of the kernel."""
+    asked = 0
+    for name, text, _ in sources():
+        for m in re.finditer(r"cudaFuncSetAttribute\(", text):
+            args = text[m.end():closing(text, m.end() - 1, "()") - 1]
+            if "," not in args:                     # (the name in a message)
+                continue
+            assert re.search(r"(SMEM_\w+|\w+_SMEM|96 \* 1024)$", args.rsplit(",", 1)[1].strip()), (name, args)
+            asked += 1
+    assert asked > 5

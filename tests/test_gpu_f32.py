@@ -384,6 +384,20 @@ def test_attention_core_f32(T, cref, dev_inv_freq, S, Hq, Hkv, D, off, causal, m
     assert nerr(got, ref64) < 2e-5
 
 
+@pytest.mark.parametrize("S,Hq,Hkv,D", [(149, 2, 1, 40), (385, 4, 2, 24), (1, 4, 4, 18), (641, 5, 5, 10)])
+def test_attention_core_f32_of_just_under_48_kb(T, S, Hq, Hkv, D):
+    """Scores, keys and queries that together with the kernel's own arrays are a few bytes above what needs no asking"""
+    import torch
+    from baranet_bdml_b200 import _lib
+    rng = np.random.default_rng(S)
+    q, k, v = (rng.standard_normal((S, h * D), dtype=np.float32) for h in (Hq, Hkv, Hkv))
+    tq, tk, tv = (T.TensorF.from_torch(torch.from_numpy(a).cuda()) for a in (q, k, v))
+    sizes = dict(num_heads=Hq, num_kv_heads=Hkv, head_dim=D)
+    got = tq.attention_fused(tk, tv, D ** -0.5, True, 0, theta=1.0, heads_mode=_lib.BN_HEADS_COLLAPSED, **sizes).to_numpy()
+    want = R.attention_collapsed(q, k, v, position_offset=0, causal=True, dtype=np.float64, inv_freq=np.ones(D // 2, np.float32), **sizes)
+    assert nerr(got, want) < 2e-5
+
+
 def test_layer_config1_matches_oracle(T, cref, dev_inv_freq):
     """one TinyLLaMA attention layer, fp32, S=128, through the
     mirrored GroupedQueryAttention API with injected seeded weights."""

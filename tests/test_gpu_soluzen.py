@@ -227,7 +227,7 @@ def test_the_gates_see_planted_mistakes(lib):
 
 # ------------------------------------------------------------------------------------------ mechanisms alone
 @DTYPES
-@pytest.mark.parametrize("hidden", [72, 74, 2048, 5000])
+@pytest.mark.parametrize("hidden", [72, 74, 2048, 5000, 12288])
 def test_residual_norm(lib, dtype, hidden):
     from baranet_bdml_b200 import ops
     rng = np.random.default_rng(0)
@@ -580,7 +580,7 @@ def test_latent_decode_of_a_ring_that_vectors_cannot_read(lib, kr, rot, n, split
             assert float((got[b] - want).abs().max()) <= 2.0 ** -24 * 8 * (width ** 0.5 * 4 + n)
 
 
-@pytest.mark.parametrize("splits,kr", [(1, 24), (255, 24), (256, 520), (257, 24), (13000, 24), (2, 12800)])
+@pytest.mark.parametrize("splits,kr", [(1, 24), (255, 24), (256, 520), (257, 24), (13000, 24), (3, 2904), (2, 12800)])
 def test_latent_values_of_any_number_of_splits(lib, splits, kr):
     """Sums of any number of splits merged, and expanded: fp32 sums of `splits` and of kr terms of weights that add up to 1"""
     from baranet_bdml_b200 import _lib
@@ -620,7 +620,7 @@ def test_latent_attention_of_the_widest_heads(lib):
 
 # more rows than four a multiprocessor (a block has several, the last blocks one less), narrowest, ragged and widest rows, a row
 # stride beyond the columns; one width and one row count that the other forms take
-@pytest.mark.parametrize("rows,width,pad", [(593, 1032, 8), (700, 4096, 0), (1185, 2056, 16), (1500, 1024, 0), (592, 2048, 0), (650, 4104, 8)])
+@pytest.mark.parametrize("rows,width,pad", [(593, 1032, 8), (700, 4096, 0), (1185, 2056, 16), (1500, 1024, 0), (592, 2048, 0), (650, 4104, 8), (40, 12288, 0)])
 def test_gated_norm_of_many_rows(lib, rows, width, pad):
     """Against fp64, to bf16's rounding of the result (half of its spacing of 2^-7) and the fast exponential's 2^-20; the padding
     columns are zeros"""
